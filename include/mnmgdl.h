@@ -78,9 +78,11 @@ typedef enum dl_wcc_stop {
 
 /* How TC removes known tuples from a join output (same results either way). */
 typedef enum dl_dedup {
-    DL_DEDUP_AUTO = 0,  /* the engine's choice: BITMAP for TC when the bit matrix (and the column
-                           offsets of its result rows, 1/16 of its size) fit in
-                           dl_tuning.bitmap_max_gib and half the free device memory, else SORT */
+    DL_DEDUP_AUTO = 0,  /* the engine's choice. TC: a breadth-first search per source, with bit rows
+                           for the sources that reach much of the graph, when those rows fit in
+                           dl_tuning.bitmap_max_gib and half the free device memory (and
+                           bitmap_result is 0); else BITMAP when its matrix (and the column offsets
+                           of its result rows, 1/16 of its size) fits likewise; else SORT */
     DL_DEDUP_SORT = 1,  /* radix sort of the join output + merge-path difference against sorted full */
     DL_DEDUP_HASH = 2,  /* full as a hash set of tuple words; one sort of the result at the end
                            (no per-iteration sort, but random-access bound: 1.7x slower on

@@ -25,6 +25,7 @@
 // The new bits of the unit are its part of the next delta: all of them count
 // in |delta|, and those whose target has out-edges (the only ones that can
 // join next step) become its rows.
+#include "dl_closure.h"
 #include "dl_engine_detail.h"
 #include "dl_join.cuh"
 
@@ -1487,6 +1488,10 @@ u64 bitmat_unit_index(const Run &r, u64 unit) {
 void bitmat_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 u0, u64 u1) {
     using namespace detail;
     if (r.info.output_rows == 0 || u0 >= u1) return;
+    if (r.cl_rows) {
+        closure_extract_rows(ctx, r, out, u0, u1);
+        return;
+    }
     const u64 n = r.bm_n;
     if (!r.bm_cols) {
         if (r.bm_row_first)

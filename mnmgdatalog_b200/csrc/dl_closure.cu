@@ -1,0 +1,1251 @@
+// TC as one breadth-first search per source.
+//
+// The reference's TC is left-linear: an iteration joins the newest paths
+// (x, y) with the edges (y, w) and keeps the pairs not seen before
+// (tc.cu:216-314), so Delta_k holds exactly the pairs (x, w) at distance k + 1
+// and the join output of an iteration is the out-edges of the newest pairs'
+// targets. Both depend on one source x at a time: every source's fixpoint is
+// its own breadth-first search, with no other source's state in it. A whole
+// run is then one launch of independent searches instead of a launch, a full
+// relation in HBM and a host wait per iteration, and the per-iteration sizes
+// are sums of the searches' level sizes.
+//
+// Two kinds of work, by what a source reaches:
+//  * closure_warp_kernel / closure_cta_kernel: a search whose visited set
+//    fits in shared memory (a hash set and the visit queue: up to 512 targets
+//    in a warp's slice, up to 4096 in a CTA's). Result pairs leave as words,
+//    sorted afterwards.
+//  * closure_pull_kernel: the sources that reach more ("heavy"), 32 of them
+//    to a word: bit c of row z of T says whether heavy source c reaches z.
+//    One iteration ORs, for every target z, the newest bits of its
+//    in-neighbours and keeps the bits T does not have: whole 128-byte lines
+//    (1024 sources) for one edge instead of one operation per source. Heavy
+//    sources reach much of the graph, so their rows share most edges.
+//
+// Measured on B200 against the n x n bit matrix stepped by one launch per
+// iteration (dl_bitmap.cu), edges and result rows on the device: Chung-Lu graph
+// of 317K nodes (1.88e9 pairs; 9.3K heavy sources hold 99 % of them)
+// 45.5 -> 12.4 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 5.0 ms;
+// DAG of 5.5K edges from and to host memory 3.6 -> 0.68 ms.
+#include <type_traits>
+
+#include "dl_closure.h"
+#include "dl_scan.cuh"
+
+namespace dl {
+namespace detail {
+namespace {
+
+constexpr u32 EMPTY = 0xFFFFFFFFu;  // ranks are below 2^32 - 1
+
+// ---- searches by a warp -------------------------------------------------
+
+constexpr int CW_THREADS = 128;
+constexpr u32 CW_REACH = 512;
+constexpr u32 CW_HASH = 2 * CW_REACH;
+constexpr int CW_HASH_SHIFT = 22;     // 32 - log2(CW_HASH)
+constexpr u32 CW_LEVELS = 256;
+constexpr u32 CW_EDGES = 8192;        // join words of one search
+constexpr int CW_REGS = 4;            // levels 1 .. 32 * CW_REGS are summed in registers
+
+struct CwSmem {
+    u32 hash[CW_HASH];
+    u32 queue[CW_REACH];
+    unsigned short lcnt[CW_LEVELS];   // targets of level d at [d - 1]
+    unsigned short ldeg[CW_LEVELS];   // join words out of level d at [d - 1]
+    u32 wbeg[32], wpre[32];           // compacted rows of the group being expanded
+};
+
+// Counters of a search launch (device).
+struct SearchCounters {
+    unsigned long long fetch;   // next source (group)
+    unsigned long long words;   // result words reserved
+    unsigned long long left;    // sources left over
+    unsigned long long levels;  // largest level of a finished source
+};
+
+__device__ __forceinline__ u32 hash_slot(u32 w, int shift) { return (w * 2654435769u) >> shift; }
+
+// Adds w to an open-addressing set of MASK + 1 slots that always has empty
+// ones; true when it was not there.
+template <u32 MASK>
+__device__ __forceinline__ bool set_insert(u32 *hash, u32 w, int shift) {
+    u32 s = hash_slot(w, shift);
+    for (;;) {
+        const u32 o = atomicCAS(&hash[s], EMPTY, w);
+        if (o == EMPTY) return true;
+        if (o == w) return false;
+        s = (s + 1) & MASK;
+    }
+}
+
+// Walks the edge targets of up to 32 rows (beg, deg of this lane's row; deg 0:
+// none) in windows of 32: f(w, have) per window, all lanes; f returns false
+// to stop. Returns the rows' edges. A window's rows are the bits of a
+// start mask, a word's row the number of rows started up to its position.
+template <class F>
+__device__ __forceinline__ u32 walk_rows(u32 *wbeg, u32 *wpre, u32 beg, u32 deg, const u32 *__restrict__ val,
+                                         u32 lane, u32 lt, u32 le, u32 limit, F f) {
+    const u32 nz = __ballot_sync(0xffffffffu, deg != 0);
+    if (!nz) return 0;
+    const u32 incl = warp_inclusive_sum(deg);
+    const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total > limit) return total;
+    const u32 rk = __popc(nz & lt);
+    if (deg) {
+        wbeg[rk] = beg;
+        wpre[rk] = incl - deg;
+    }
+    __syncwarp();
+    const u32 nrows = __popc(nz);
+    const u32 cb = lane < nrows ? wbeg[lane] : 0u;
+    const u32 pre = lane < nrows ? wpre[lane] : 0xFFFFFFFFu;
+    __syncwarp();
+    int base = -1;  // last row started before the window
+    auto load = [&](u32 i0) -> u32 {
+        const u32 st = (pre - i0) < 32u ? 1u << (pre - i0) : 0u;
+        const u32 starts = __reduce_or_sync(0xffffffffu, st);
+        const int o = base + __popc(starts & le);
+        base += __popc(starts);
+        const u32 ob = __shfl_sync(0xffffffffu, cb, o);
+        const u32 op = __shfl_sync(0xffffffffu, pre, o);
+        return i0 + lane < total ? __ldg(val + ob + (i0 + lane - op)) : 0u;
+    };
+    u32 w = load(0);
+    for (u32 i0 = 0; i0 < total; i0 += 32) {
+        const u32 wn = i0 + 32 < total ? load(i0 + 32) : 0u;  // the next window's load is in flight
+        if (!f(w, i0 + lane < total)) break;
+        w = wn;
+    }
+    return total;
+}
+
+// One search per warp at a time; persistent warps take `group` consecutive
+// sources of [lo, hi) at a time. A search that outgrows its slice goes to `left`.
+// Level sizes are kept per search and added when it finishes: levels up to
+// 128 in lane registers (lane l holds levels 32 j + l + 1), flushed to the
+// instance's counters when the instance changes, the rest directly.
+__global__ void __launch_bounds__(CW_THREADS)
+closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 lo, u64 hi, u32 group, int bits,
+                    const u64 *__restrict__ inst_lo, u32 n_inst, u32 max_level, unsigned long long *__restrict__ cnt,
+                    unsigned long long *__restrict__ deg, u64 *__restrict__ out, u64 cap,
+                    SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CwSmem &s = reinterpret_cast<CwSmem *>(smem_raw)[threadIdx.x >> 5];
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
+    const u32 le = lane == 31 ? ~0u : (2u << lane) - 1;
+    u32 rc[CW_REGS], rd[CW_REGS];
+#pragma unroll
+    for (int j = 0; j < CW_REGS; ++j) rc[j] = rd[j] = 0;
+    u32 held = 0;           // searches summed in rc / rd
+    u32 top = 0;            // largest level seen
+    u32 inst = 0;
+    u64 inst_end = inst_lo ? 0 : hi;  // first rank after the current instance
+    auto flush = [&]() {
+        const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + lane;
+#pragma unroll
+        for (int j = 0; j < CW_REGS; ++j) {
+            if (rc[j]) atomicAdd(cnt + at + 32 * j, (unsigned long long) rc[j]);
+            if (deg && rd[j]) atomicAdd(deg + at + 32 * j, (unsigned long long) rd[j]);
+            rc[j] = rd[j] = 0;
+        }
+        held = 0;
+    };
+    for (;;) {
+        unsigned long long g = 0;
+        if (lane == 0) g = atomicAdd(&ctr->fetch, (unsigned long long) group);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (lo + g >= hi) break;
+        const u64 xe = min(hi, (u64) (lo + g + group));
+        for (u64 x = lo + g; x < xe; ++x) {
+            const u32 b0 = __ldg(off + x), d0 = __ldg(off + x + 1) - b0;
+            if (d0 == 0) continue;
+            if (x >= inst_end) {  // another instance: its range by binary search
+                flush();
+                u32 a = 0, b = n_inst;
+                while (a < b) {
+                    const u32 m = (a + b) >> 1;
+                    if (inst_lo[m] <= x) a = m + 1;
+                    else b = m;
+                }
+                inst = a - 1;
+                inst_end = a < n_inst ? inst_lo[a] : hi;
+            }
+            // visited set empty
+            uint4 *hv = reinterpret_cast<uint4 *>(s.hash);
+#pragma unroll
+            for (u32 k = 0; k < CW_HASH / 4 / 32; ++k) hv[k * 32 + lane] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
+            __syncwarp();
+            u32 tail = 0, edges = 0;
+            bool over = false;
+            auto visit = [&](u32 w, bool have) -> bool {
+                const bool fresh = have && set_insert<CW_HASH - 1>(s.hash, w, CW_HASH_SHIFT);
+                const u32 fm = __ballot_sync(0xffffffffu, fresh);
+                const u32 n = __popc(fm);
+                if (tail + n > CW_REACH) {
+                    over = true;
+                    return false;
+                }
+                if (fresh) s.queue[tail + __popc(fm & lt)] = w;
+                tail += n;
+                return true;
+            };
+            // level 1: x's own edges
+            if (walk_rows(s.wbeg, s.wpre, b0, lane == 0 ? d0 : 0u, val, lane, lt, le, CW_REACH, visit) > CW_REACH)
+                over = true;
+            u32 head = 0, level = 1;
+            while (!over) {
+                __syncwarp();
+                const u32 end = tail;
+                u32 ld = 0;
+                if (level != max_level) {
+                    for (u32 h = head; h < end && !over; h += 32) {
+                        u32 b = 0, d = 0;
+                        if (h + lane < end) {
+                            const u32 y = s.queue[h + lane];
+                            b = __ldg(off + y);
+                            d = __ldg(off + y + 1) - b;
+                        }
+                        const u32 t = walk_rows(s.wbeg, s.wpre, b, d, val, lane, lt, le, CW_EDGES - edges, visit);
+                        if (t > CW_EDGES - edges) {
+                            over = true;
+                            break;
+                        }
+                        edges += t;
+                        ld += t;
+                    }
+                }
+                if (over) break;
+                if (lane == 0) {
+                    s.lcnt[level - 1] = (unsigned short) (end - head);
+                    s.ldeg[level - 1] = (unsigned short) ld;
+                }
+                if (tail == end) break;  // no level after this one
+                head = end;
+                if (++level > CW_LEVELS) over = true;
+            }
+            __syncwarp();
+            if (over) {
+                if (lane == 0) left[atomicAdd(&ctr->left, 1ull)] = x;
+                continue;
+            }
+            // level sizes
+            top = max(top, level);
+#pragma unroll
+            for (int j = 0; j < CW_REGS; ++j) {
+                const u32 k = 32 * j + lane;
+                if (k < level) {
+                    rc[j] += s.lcnt[k];
+                    rd[j] += s.ldeg[k];
+                }
+            }
+            for (u32 k = 32 * CW_REGS + lane; k < level; k += 32) {
+                const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + k;
+                atomicAdd(cnt + at, (unsigned long long) s.lcnt[k]);
+                if (deg) atomicAdd(deg + at, (unsigned long long) s.ldeg[k]);
+            }
+            if (++held == (1u << 18)) flush();  // 2^18 searches x 8192 words stay below 2^32
+            // result words
+            unsigned long long p = 0;
+            if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) tail);
+            p = __shfl_sync(0xffffffffu, p, 0);
+            if (p + tail <= cap)
+                for (u32 k = lane; k < tail; k += 32) out[p + k] = ((u64) s.queue[k] << bits) | x;
+            __syncwarp();
+        }
+    }
+    flush();
+    if (lane == 0 && top) atomicMax(&ctr->levels, (unsigned long long) top);
+}
+
+// ---- searches by a CTA --------------------------------------------------
+
+constexpr int CC_THREADS = 256;
+constexpr u32 CC_REACH = 4096;
+constexpr u32 CC_HASH = 2 * CC_REACH;
+constexpr int CC_HASH_SHIFT = 19;  // 32 - log2(CC_HASH)
+constexpr u32 CC_EDGES = 1u << 18;
+
+struct CcSmem {
+    u32 hash[CC_HASH];
+    u32 queue[CC_REACH];
+    u32 wbeg[CC_THREADS / 32][32], wpre[CC_THREADS / 32][32];
+    u32 tail, edges;
+    u64 x, pos;
+};
+
+// The same search by a CTA, for the sources a warp's slice could not hold:
+// each level's rows are shared by the CTA's warps, 32 rows at a time. Level
+// sizes go to the CTA's slice of `lev` (2 * CL_LEVELS words) until the search has
+// finished: in shared memory they would cost a quarter of the resident CTAs.
+__global__ void __launch_bounds__(CC_THREADS)
+closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, const u64 *__restrict__ src, u64 n_src,
+                   u32 reach, int bits, const u64 *__restrict__ inst_lo, u32 n_inst, u32 max_level,
+                   unsigned long long *__restrict__ cnt, unsigned long long *__restrict__ deg, u32 *lev,
+                   u64 *__restrict__ out, u64 cap, SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u32 *lcnt = lev + (u64) blockIdx.x * 2 * CL_LEVELS, *ldeg = lcnt + CL_LEVELS;
+    CcSmem &s = *reinterpret_cast<CcSmem *>(smem_raw);
+    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const u32 lt = lanemask_lt();
+    const u32 le = lane == 31 ? ~0u : (2u << lane) - 1;
+    for (;;) {
+        if (tid == 0) {
+            const u64 i = atomicAdd(&ctr->fetch, 1ull);
+            s.x = i < n_src ? src[i] : ~0ull;
+            s.tail = 0;
+            s.edges = 0;
+        }
+        uint4 *hv = reinterpret_cast<uint4 *>(s.hash);
+        for (u32 k = tid; k < CC_HASH / 4; k += CC_THREADS) hv[k] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
+        __syncthreads();
+        const u64 x = s.x;
+        if (x == ~0ull) break;
+        auto visit = [&](u32 w, bool have) -> bool {
+            // the set holds at most `reach` words and the warps' windows in flight
+            if (__any_sync(0xffffffffu, *reinterpret_cast<volatile u32 *>(&s.tail) > reach)) return false;
+            const bool fresh = have && set_insert<CC_HASH - 1>(s.hash, w, CC_HASH_SHIFT);
+            const u32 fm = __ballot_sync(0xffffffffu, fresh);
+            if (fm) {
+                u32 at = 0;
+                if (lane == 0) at = atomicAdd(&s.tail, (u32) __popc(fm));
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(fm & lt);
+                if (fresh && at < CC_REACH) s.queue[at] = w;
+            }
+            return true;
+        };
+        // rows of a group of up to 32 nodes; the level's edges are added to s.edges
+        auto expand = [&](u32 b, u32 d) {
+            const u32 t = walk_rows(s.wbeg[warp], s.wpre[warp], b, d, val, lane, lt, le, CC_EDGES, visit);
+            if (lane == 0 && t) atomicAdd(&s.edges, min(t, CC_EDGES + 1));
+        };
+        if (warp == 0) {
+            const u32 b0 = __ldg(off + x), d0 = __ldg(off + x + 1) - b0;
+            if (d0 <= reach) expand(b0, lane == 0 ? d0 : 0u);
+            else if (lane == 0) s.tail = reach + 1;
+        }
+        u32 head = 0, level = 1;
+        bool over = false;
+        for (;;) {
+            __syncthreads();  // the level's targets are queued
+            const u32 end = s.tail;
+            if (end > reach || s.edges > CC_EDGES) {
+                over = true;
+                break;
+            }
+            __syncthreads();  // every thread has read the level's bounds
+            if (tid == 0) s.edges = 0;
+            __syncthreads();
+            if (level != max_level) {
+                for (u32 h = head + warp * 32; h < end; h += CC_THREADS) {
+                    u32 b = 0, d = 0;
+                    if (h + lane < end) {
+                        const u32 y = s.queue[h + lane];
+                        b = __ldg(off + y);
+                        d = __ldg(off + y + 1) - b;
+                    }
+                    expand(b, d);
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                lcnt[level - 1] = end - head;
+                ldeg[level - 1] = s.edges;
+            }
+            if (s.tail == end) break;
+            head = end;
+            if (++level > CL_LEVELS) {
+                over = true;
+                break;
+            }
+        }
+        __syncthreads();
+        if (over) {
+            if (tid == 0) left[atomicAdd(&ctr->left, 1ull)] = x;
+            __syncthreads();
+            continue;
+        }
+        const u32 tail = s.tail;
+        u32 inst = 0;
+        if (inst_lo) {
+            u32 a = 0, b = n_inst;
+            while (a < b) {
+                const u32 m = (a + b) >> 1;
+                if (inst_lo[m] <= x) a = m + 1;
+                else b = m;
+            }
+            inst = a - 1;
+        }
+        for (u32 k = tid; k < level; k += CC_THREADS) {
+            const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + k;
+            atomicAdd(cnt + at, (unsigned long long) lcnt[k]);
+            if (deg) atomicAdd(deg + at, (unsigned long long) ldeg[k]);
+        }
+        if (tid == 0) {
+            s.pos = atomicAdd(&ctr->words, (unsigned long long) tail);
+            atomicMax(&ctr->levels, (unsigned long long) level);
+        }
+        __syncthreads();
+        const u64 p = s.pos;
+        if (p + tail <= cap)
+            for (u32 k = tid; k < tail; k += CC_THREADS) out[p + k] = ((u64) s.queue[k] << bits) | x;
+        __syncthreads();  // the queue and x are free
+    }
+}
+
+// ---- heavy sources: 32 to a word ----------------------------------------
+
+constexpr int PU_THREADS = 256;
+// A target with more in-edges than lanes ("hub") is gathered in segments of 32
+// in-edges by as many warps: one warp alone would walk them long after the
+// others are done (at 256 in-edges a warp, 46 % of a level's time was that tail).
+constexpr u32 PU_SEG = 32;
+
+// Rows of heavy-source bits: chunks of 1024 columns (a 128-byte line), 2^shift
+// of which share one activity bit, so that a row's activity is one word
+// whatever the number of columns.
+struct PullShape {
+    u64 n;      // targets
+    u32 words;  // words of a row
+    u32 shift;
+};
+
+// One level's view of the state: row y of `cur` is valid when tag[y] is
+// (activity, level - 1); todo[w] = activity of w's in-neighbours (zero: w is not
+// in the list).
+struct PullLevel {
+    u32 level;
+    const u32 *cur;
+    u32 *nxt;
+    const uint2 *tag;
+    uint2 *tag_next;
+    u32 *todo, *todo_next;
+    const u32 *list;
+    u32 *list_next;
+    unsigned long long *count;  // [level]: targets in the level's list
+    unsigned long long *cnt;    // [level]: new pairs
+    unsigned long long *deg;    // [level]: sum of their targets' out-degrees
+};
+
+// Puts the targets of the newly active nodes on the next level's list: a
+// thread per edge (x, y), sorted by x, so a node's out-degree does not matter
+// (a warp per active node spent half a level on the few nodes with thousands
+// of out-edges).
+__global__ void __launch_bounds__(PU_THREADS)
+closure_push_kernel(PullLevel st, const u64 *__restrict__ edges, u64 ne, int bits) {
+    if (st.level && st.count[st.level] == 0) return;  // the fixpoint was reached earlier
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
+    const u64 mask = (1ull << bits) - 1;
+    for (u64 k0 = (u64) blockIdx.x * PU_THREADS + (threadIdx.x & ~31u); k0 < ne; k0 += (u64) gridDim.x * PU_THREADS) {
+        bool fresh = false;
+        u32 y = 0;
+        if (k0 + lane < ne) {
+            const u64 e = __ldg(edges + k0 + lane);
+            const uint2 tg = st.tag_next[e >> bits];
+            if (tg.y == st.level) {
+                y = (u32) (e & mask);
+                fresh = atomicOr(&st.todo_next[y], tg.x) == 0u;
+            }
+        }
+        const u32 fm = __ballot_sync(0xffffffffu, fresh);
+        if (!fm) continue;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(st.count + st.level + 1, (unsigned long long) __popc(fm));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (fresh) st.list_next[at + __popc(fm & lt)] = y;
+    }
+}
+
+__global__ void pull_swap_kernel(const u64 *__restrict__ e, u64 ne, int bits, u64 *__restrict__ out) {
+    const u64 mask = (1ull << bits) - 1;
+    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (u64) gridDim.x * blockDim.x) {
+        const u64 w = e[i];
+        out[i] = ((w & mask) << bits) | (w >> bits);
+    }
+}
+
+// off[k] = first word whose key (word >> bits) is at least k, k in [0, n].
+template <class T>
+__global__ void key_offsets_kernel(const u64 *__restrict__ w, u64 nw, int bits, u64 n, T *__restrict__ off) {
+    for (u64 k = (u64) blockIdx.x * blockDim.x + threadIdx.x; k <= n; k += (u64) gridDim.x * blockDim.x) {
+        const u64 target = k << bits;
+        u64 l = 0, h = nw;
+        while (l < h) {
+            const u64 m = (l + h) >> 1;
+            if (w[m] < target) l = m + 1;
+            else h = m;
+        }
+        off[k] = (T) l;
+    }
+}
+
+__global__ void low_field_kernel(const u64 *__restrict__ w, u64 n, u64 mask, u32 *__restrict__ out) {
+    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x)
+        out[i] = (u32) (w[i] & mask);
+}
+
+// Hubs: hub_at[w] = accumulator row of hub w, seg[...] = (w, first in-edge of a
+// segment); found[0] = hubs, found[1] = segments.
+__global__ void pull_hubs_kernel(const u32 *__restrict__ roff, u64 n, u32 *__restrict__ hub_at,
+                                 uint2 *__restrict__ seg, unsigned long long *__restrict__ found) {
+    for (u64 w = (u64) blockIdx.x * blockDim.x + threadIdx.x; w < n; w += (u64) gridDim.x * blockDim.x) {
+        const u32 b = roff[w], d = roff[w + 1] - b;
+        if (d <= PU_SEG) continue;
+        hub_at[w] = (u32) atomicAdd(found, 1ull);
+        const u32 k = (d + PU_SEG - 1) / PU_SEG;
+        const unsigned long long at = atomicAdd(found + 1, (unsigned long long) k);
+        for (u32 i = 0; i < k; ++i) seg[at + i] = make_uint2((u32) w, b + i * PU_SEG);
+    }
+}
+
+__global__ void add_counts_kernel(u64 *__restrict__ a, const unsigned long long *__restrict__ b, u64 n) {
+    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x) a[i] += b[i];
+}
+
+// Column i = heavy source src[i] (a warp each): its level-0 row is its own bit
+// at node src[i]; pads the column ids up to `words` * 32.
+__global__ void pull_init_kernel(PullShape sh, PullLevel st, const u64 *__restrict__ src, u64 h,
+                                 u32 *__restrict__ cols) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    for (u64 i = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32; i < (u64) sh.words * 32; i += warps) {
+        if (i >= h) {
+            if (lane == 0) cols[i] = EMPTY;
+            continue;
+        }
+        const u64 x = src[i];
+        const u32 gr = (u32) (i >> 10) >> sh.shift;
+        u32 *row = st.nxt + x * sh.words;
+        const u32 w0 = (gr << sh.shift) * 32, w1 = min(sh.words, w0 + (32u << sh.shift));
+        for (u32 k = w0 + lane; k < w1; k += 32) row[k] = k == (u32) (i >> 5) ? 1u << (i & 31) : 0u;
+        if (lane == 0) {
+            cols[i] = (u32) x;
+            st.tag_next[x] = make_uint2(1u << gr, 0u);
+        }
+    }
+}
+
+// A warp works on K * 128 words of a row at a time: lane l holds words
+// base + 128 k + 4 l .. + 3 (k < K), 16 bytes each, eight lanes to a chunk.
+// Activity bit of the lane's k-th piece.
+template <int K>
+__device__ __forceinline__ u32 piece_bit(const PullShape &sh, u32 base, int k, u32 lane) {
+    return 1u << (((base >> 5) + 4 * k + (lane >> 3)) >> sh.shift);
+}
+
+// ORs the newest words of a group of up to 32 in-neighbours (node y, activity
+// a in the neighbour's lane) into acc: two neighbours' pieces in flight. The
+// pieces whose bit of `need` is clear are not loaded.
+template <int K>
+__device__ __forceinline__ void or_neighbours(const PullShape &sh, const u32 *__restrict__ cur, u32 base, u32 y, u32 a,
+                                              u32 need, u32 lane, uint4 (&acc)[K]) {
+    u32 all = __ballot_sync(0xffffffffu, a != 0);
+    const u32 *mine = cur + base + lane * 4;
+    u32 bit[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) bit[k] = (need >> k) & 1u ? piece_bit<K>(sh, base, k, lane) : 0u;
+    while (all) {
+        uint4 v[2][K];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const u32 j = (__ffs(all) - 1) & 31;
+            u32 aj = __shfl_sync(0xffffffffu, a, j);
+            if (all == 0) aj = 0;
+            all &= all - 1;
+            const uint4 *src = reinterpret_cast<const uint4 *>(mine + (u64) __shfl_sync(0xffffffffu, y, j) * sh.words);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                v[q][k] = make_uint4(0, 0, 0, 0);
+                if (aj & bit[k]) v[q][k] = __ldg(src + 32 * k);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            acc[k].x |= v[0][k].x | v[1][k].x;
+            acc[k].y |= v[0][k].y | v[1][k].y;
+            acc[k].z |= v[0][k].z | v[1][k].z;
+            acc[k].w |= v[0][k].w | v[1][k].w;
+        }
+    }
+}
+
+// Hub targets: a warp ORs the newest words of PU_SEG in-neighbours, K * 128
+// words of the row, into the hub's accumulator (zero before the level).
+template <int K>
+__global__ void __launch_bounds__(PU_THREADS)
+closure_pull_hub_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ roff, const u32 *__restrict__ rval,
+                        const uint2 *__restrict__ seg, u64 n_seg, const u32 *__restrict__ hub_at,
+                        u32 *__restrict__ hub_acc) {
+    if (st.count[st.level] == 0) return;  // the fixpoint was reached earlier
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64) gridDim.x * (PU_THREADS / 32);
+    const u32 passes = (sh.words + K * 128 - 1) / (K * 128);
+    for (u64 it = ((u64) blockIdx.x * PU_THREADS + threadIdx.x) / 32; it < n_seg * passes; it += warps) {
+        const u32 base = (u32) (it % passes) * K * 128;
+        const uint2 sg = seg[it / passes];
+        if (st.todo[sg.x] == 0) continue;
+        const u32 i = sg.y + lane;
+        u32 y = 0, a = 0;
+        if (i < roff[sg.x + 1]) {
+            y = rval[i];
+            const uint2 tg = st.tag[y];
+            a = tg.y == st.level - 1 ? tg.x : 0u;
+        }
+        uint4 acc[K];
+        u32 need = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            acc[k] = make_uint4(0, 0, 0, 0);
+            if (base + 128 * k + lane * 4 < sh.words) need |= 1u << k;
+        }
+        or_neighbours<K>(sh, st.cur, base, y, a, need, lane, acc);
+        u32 *dst = hub_acc + (u64) hub_at[sg.x] * sh.words + base + lane * 4;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (acc[k].x) atomicOr(dst + 128 * k, acc[k].x);
+            if (acc[k].y) atomicOr(dst + 128 * k + 1, acc[k].y);
+            if (acc[k].z) atomicOr(dst + 128 * k + 2, acc[k].z);
+            if (acc[k].w) atomicOr(dst + 128 * k + 3, acc[k].w);
+        }
+    }
+}
+
+// One level: for every target in the level's list (a warp each), the new bits
+// of its row = (OR of its in-neighbours' newest bits) & ~T, K * 512 bytes of the
+// row at a time (K by the row's length: the work per in-neighbour that does
+// not depend on the row is paid once for all K pieces). Only words that are
+// tagged as newest are ever read, so nothing is cleared between levels.
+template <int K>
+__global__ void __launch_bounds__(PU_THREADS, K >= 3 ? 3 : 4)
+closure_pull_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ roff,
+                    const u32 *__restrict__ rval, const u32 *__restrict__ hub_at, u32 *__restrict__ hub_acc,
+                    u32 *__restrict__ t) {
+    const u64 n_list = st.count[st.level];
+    if (n_list == 0) return;  // the fixpoint was reached earlier
+    __shared__ unsigned long long part[2][PU_THREADS / 32];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u64 warps = (u64) gridDim.x * (PU_THREADS / 32);
+    u64 fresh = 0, dsum = 0;
+    for (u64 i = ((u64) blockIdx.x * PU_THREADS + threadIdx.x) / 32; i < n_list; i += warps) {
+        const u32 w = st.list[i];
+        const u32 m = st.todo[w];
+        const u32 b = __ldg(roff + w), n = __ldg(roff + w + 1) - b;
+        const bool hub = n > PU_SEG;
+        u32 y0 = 0, a0 = 0;
+        u32 *hrow = nullptr;
+        if (hub) {
+            hrow = hub_acc + (u64) hub_at[w] * sh.words + lane * 4;
+        } else if (lane < n) {
+            y0 = __ldg(rval + b + lane);
+            const uint2 tg = st.tag[y0];
+            a0 = tg.y == st.level - 1 ? tg.x : 0u;
+        }
+        u32 news = 0, bits_new = 0;
+        const u64 row = (u64) w * sh.words + lane * 4;
+        for (u32 base = 0; base < sh.words; base += K * 128) {
+            u32 in = 0, need = 0;
+            uint4 old[K], acc[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const bool on = base + 128 * k + lane * 4 < sh.words && (m & piece_bit<K>(sh, base, k, lane));
+                if (on) in |= 1u << k;
+                old[k] = on ? *reinterpret_cast<const uint4 *>(t + row + base + 128 * k)
+                            : make_uint4(~0u, ~0u, ~0u, ~0u);
+                acc[k] = make_uint4(0, 0, 0, 0);
+            }
+            if (!__any_sync(0xffffffffu, in != 0)) continue;
+            if (hub) {
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if ((in >> k) & 1u) {
+                        uint4 *hp = reinterpret_cast<uint4 *>(hrow + base + 128 * k);
+                        acc[k] = *hp;
+                        *hp = make_uint4(0, 0, 0, 0);
+                    }
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if ((old[k].x & old[k].y & old[k].z & old[k].w) != ~0u) need |= 1u << k;
+                or_neighbours<K>(sh, st.cur, base, y0, a0, need, lane, acc);
+            }
+            u32 mark = 0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint4 nw = make_uint4(acc[k].x & ~old[k].x, acc[k].y & ~old[k].y, acc[k].z & ~old[k].z,
+                                            acc[k].w & ~old[k].w);
+                const bool any = (nw.x | nw.y | nw.z | nw.w) != 0;
+                if (any) {
+                    *reinterpret_cast<uint4 *>(t + row + base + 128 * k) =
+                        make_uint4(old[k].x | nw.x, old[k].y | nw.y, old[k].z | nw.z, old[k].w | nw.w);
+                    bits_new += __popc(nw.x) + __popc(nw.y) + __popc(nw.z) + __popc(nw.w);
+                }
+                const u32 lines = __ballot_sync(0xffffffffu, any);
+                const bool line = ((lines >> (lane & 24)) & 0xFFu) != 0;  // this piece's chunk has new bits
+                if (line) mark |= piece_bit<K>(sh, base, k, lane);
+                if (((in >> k) & 1u) && (line || sh.shift))
+                    *reinterpret_cast<uint4 *>(st.nxt + row + base + 128 * k) = nw;
+            }
+            news |= __reduce_or_sync(0xffffffffu, mark);
+        }
+        if (lane == 0) {
+            st.todo[w] = 0;
+            if (news) st.tag_next[w] = make_uint2(news, st.level);
+        }
+        if (bits_new) {
+            fresh += bits_new;
+            dsum += (u64) bits_new * (__ldg(off + w + 1) - __ldg(off + w));
+        }
+    }
+    fresh = warp_sum(fresh);
+    dsum = warp_sum(dsum);
+    if (lane == 0) {
+        part[0][warp] = fresh;
+        part[1][warp] = dsum;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long v = 0;
+        for (int i = 0; i < PU_THREADS / 32; ++i) v += part[threadIdx.x][i];
+        if (v) atomicAdd((threadIdx.x == 0 ? st.cnt : st.deg) + st.level, v);
+    }
+}
+
+// ---- results ------------------------------------------------------------
+
+// Row z's result rows by chunk: start[z * chunks + c] = (rows of z before
+// chunk c, light pairs of z before it), a light pair belonging to the chunk of
+// the column it comes before (the last chunk when there is none). counts[z] =
+// rows of z. A warp per target.
+__global__ void closure_counts_kernel(const u32 *__restrict__ t, u64 n, u32 words, const u64 *__restrict__ light,
+                                      const u64 *__restrict__ loff, u64 mask, const u32 *__restrict__ place,
+                                      uint2 *__restrict__ start, u64 *__restrict__ counts) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    const u32 chunks = words / 32;
+    for (u64 z = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32; z < n; z += warps) {
+        const u32 *row = t + z * words;
+        const u64 *lz = light + loff[z];
+        const u32 nl = (u32) (loff[z + 1] - loff[z]);
+        u32 rows = 0, li = 0, wb = 0;
+        u32 lc = lane < nl ? __ldg(place + (__ldg(lz + lane) & mask)) : EMPTY;
+        u32 v = row[lane];
+        for (u32 c = 0; c < chunks; ++c) {
+            const u32 vn = c + 1 < chunks ? row[(c + 1) * 32 + lane] : 0u;
+            if (lane == 0) start[z * chunks + c] = make_uint2(rows + li, li);
+            rows += __reduce_add_sync(0xffffffffu, __popc(v));
+            for (;;) {  // light pairs before columns of this chunk
+                const u32 m = __ballot_sync(0xffffffffu, lc < (c + 1) * 1024);
+                li += __popc(m);
+                if (lc < (c + 1) * 1024) lc = EMPTY;
+                if (li < wb + 32 || li >= nl) break;
+                wb += 32;
+                lc = wb + lane < nl ? __ldg(place + (__ldg(lz + wb + lane) & mask)) : EMPTY;
+            }
+            v = vn;
+        }
+        if (lane == 0) counts[z] = (u64) rows + nl;
+    }
+}
+
+struct SumValue {
+    const u64 *v;
+    __device__ __forceinline__ u64 operator()(u64 i) const { return v[i]; }
+};
+
+// place[r] = heavy sources below rank r.
+__global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u32 *__restrict__ place) {
+    for (u64 r = (u64) blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (u64) gridDim.x * blockDim.x) {
+        u64 a = 0, b = h;
+        while (a < b) {
+            const u64 m = (a + b) >> 1;
+            if (cols[m] < r) a = m + 1;
+            else b = m;
+        }
+        place[r] = (u32) a;
+    }
+}
+
+// Result rows (x, z) of targets [z0, z1), by (z, x): the set bits of row z of
+// T (ascending columns = ascending sources) merged with z's light pairs
+// (ascending sources; one comes before the heavy sources at columns
+// place[source] and up). A warp keeps one chunk of 1024 columns (their node ids
+// in 32 registers) and walks targets; where a target's rows of that chunk go
+// is known from closure_counts_kernel, so chunks and targets are independent.
+// In a chunk, a word's first position comes from a prefix sum over the words
+// plus the light pairs before it; then a lane per bit of a word, whose rows
+// leave as consecutive 8-byte stores (ten instructions a word: with the ids
+// loaded per word it was bound by issue, 40 a word). Light pairs are placed
+// lane-parallel; a word that one falls inside is done last, its lanes shifted
+// by the light pairs below them.
+__global__ void __launch_bounds__(256)
+closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict__ cols,
+                    const u32 *__restrict__ place, const uint2 *__restrict__ start, u64 z0, u64 z1,
+                    const u64 *__restrict__ first, const u64 *__restrict__ light, const u64 *__restrict__ loff,
+                    u64 mask, const int32_t *__restrict__ ids, bool affine, int32_t base, u64 *__restrict__ out) {
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
+    const u32 chunks = words / 32;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    const u64 me = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    auto node = [&](u32 r) -> u32 { return (u32) (affine ? (int32_t) (base + (int64_t) r) : __ldg(ids + r)); };
+    // chunk me % chunks for the targets me / chunks, + warps / chunks, ... (more
+    // chunks than warps: the same warp takes further chunks)
+    const u64 step = max(warps / chunks, (u64) 1);
+    for (u64 c0 = me % min((u64) chunks, warps); c0 < chunks; c0 += warps) {
+        if (me / chunks >= step) break;  // warps beyond a whole number of rounds
+        const u32 k0 = (u32) c0 * 32;
+        const u32 *cc = cols + c0 * 1024;
+        u32 id[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const u32 x = __ldg(cc + j * 32 + lane);
+            id[j] = x == EMPTY ? 0u : node(x);
+        }
+        for (u64 z = z0 + me / chunks; z < z1; z += step) {
+            u32 v = t[z * words + k0 + lane];
+            const uint2 st = start[z * chunks + c0];
+            const u32 lend = c0 + 1 < chunks ? start[z * chunks + c0 + 1].y : (u32) (loff[z + 1] - loff[z]);
+            const u32 any = __ballot_sync(0xffffffffu, v != 0);
+            if (!any && st.y == lend) continue;
+            u64 *dst = out + first[z] + st.x;
+            const u64 zid = (u64) node((u32) z) << 32;
+            const u32 n = __popc(v);
+            const u32 incl = warp_inclusive_sum(n);
+            u32 at = incl - n;
+            u32 inside = 0;
+            const u64 *lz = light + loff[z];
+            // light pairs st.y .. lend - 1: one in word j before bit b
+            auto pair = [&](u32 l, u32 &x, u32 &rel) {
+                x = 0;
+                rel = EMPTY;
+                if (l < lend) {
+                    x = (u32) (__ldg(lz + l) & mask);
+                    rel = min(__ldg(place + x) - k0 * 32, 1024u);
+                }
+            };
+            u32 rel = EMPTY;
+            for (u32 l0 = st.y; l0 < lend; l0 += 32) {
+                u32 x;
+                pair(l0 + lane, x, rel);
+                const bool in = l0 + lane < lend;
+                const u32 j = rel >> 5, b = rel & 31;
+                // (rel 1024: after every column)
+                const u32 wj = __shfl_sync(0xffffffffu, v, j & 31), pj = __shfl_sync(0xffffffffu, incl - n, j & 31);
+                const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+                if (in)
+                    dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + (l0 + lane - st.y)] = zid | node(x);
+                const u32 key = in ? (b ? j : j - 1) : EMPTY - 1;  // words above `key` are shifted whole
+                for (u32 k = 0; k < min(32u, lend - l0); ++k)
+                    at += (int) lane > (int) __shfl_sync(0xffffffffu, key, k);
+                inside |= __reduce_or_sync(0xffffffffu, in && b ? 1u << j : 0u);
+            }
+            u32 slow = any & inside;
+            const u32 v0 = v;
+            if ((inside >> lane) & 1u) v = 0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const u32 word = __shfl_sync(0xffffffffu, v, j);
+                const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
+                if ((word >> lane) & 1u) dst[p] = zid | id[j];
+            }
+            while (slow) {
+                const u32 j = __ffs(slow) - 1;
+                slow &= slow - 1;
+                const u32 word = __shfl_sync(0xffffffffu, v0, j);
+                u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
+                for (u32 l0 = st.y; l0 < lend; l0 += 32) {
+                    u32 x, rl = rel;
+                    if (lend - st.y > 32) pair(l0 + lane, x, rl);  // several windows: read again
+                    for (u32 mm = __ballot_sync(0xffffffffu, (rl >> 5) == j && (rl & 31)); mm; mm &= mm - 1)
+                        p += (__shfl_sync(0xffffffffu, rl, __ffs(mm) - 1) & 31) <= lane;
+                }
+                if ((word >> lane) & 1u) dst[p] = zid | node(__ldg(cc + j * 32 + lane));
+            }
+        }
+    }
+}
+
+template <class K>
+u64 resident_blocks(Context &ctx, K kern, int threads, size_t smem) {
+    if (smem > 48 * 1024)
+        DL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    int per_sm = 0;
+    DL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    return (u64) ctx.sm_count * std::max(per_sm, 1);
+}
+
+// Keeps the first `keep` bytes of buf while it grows to `bytes`.
+void grow_keeping(Context &ctx, DevBuf &buf, u64 bytes, u64 keep) {
+    if (buf.p && buf.cap >= bytes) return;
+    DevBuf nb;
+    ctx.reserve(nb, bytes);
+    if (keep) DL_CUDA(cudaMemcpyAsync(nb.p, buf.p, keep, cudaMemcpyDeviceToDevice, ctx.stream));
+    ctx.give_back(buf);
+    buf = nb;
+}
+
+}  // namespace
+
+ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
+                            u64 max_level, u64 *cnt, u64 *deg) {
+    Workspace &ws = ctx.ws;
+    ClosureLight res;
+    const u64 ns = hi - lo;
+    if (ns == 0) return res;
+    const u64 table = n_inst * (CL_LEVELS + 1) * 8;
+    const u32 ml = (u32) std::min<u64>(max_level, 0xFFFFFFFFull);
+    auto *c = reinterpret_cast<unsigned long long *>(cnt), *d = reinterpret_cast<unsigned long long *>(deg);
+    SearchCounters *ctr = reinterpret_cast<SearchCounters *>(&ctx.ctrl->scalar[40]);
+    ctx.reserve(ws.cl_left, ns * 8);
+    DevBuf &out = ws.jbuf[0];
+    // room for 96 targets a source at first; a run that needs more is repeated with the room it asked for
+    ctx.reserve(out, std::max<u64>(96 * ns, 1 << 16) * 8);
+    const size_t smem = sizeof(CwSmem) * (CW_THREADS / 32);
+    const u64 wave = resident_blocks(ctx, closure_warp_kernel, CW_THREADS, smem);
+    const u32 group = (u32) std::max<u64>(1, std::min<u64>(8, ns / (wave * (CW_THREADS / 32) * 4)));
+    const unsigned grid =
+        (unsigned) std::max<u64>(1, std::min<u64>(wave, (ns + group * (CW_THREADS / 32) - 1) / (group * (CW_THREADS / 32))));
+    SearchCounters got{};
+    auto read_back = [&]() {
+        DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctr, sizeof(got), cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        got.words = ctx.host_scalars[1];
+        got.left = ctx.host_scalars[2];
+        got.levels = ctx.host_scalars[3];
+    };
+    for (;;) {
+        DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
+        DL_CUDA(cudaMemsetAsync(cnt, 0, table, ctx.stream));
+        if (deg) DL_CUDA(cudaMemsetAsync(deg, 0, table, ctx.stream));
+        const u64 cap = out.cap / 8;
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * ns,
+                  closure_warp_kernel<<<grid, CW_THREADS, smem, ctx.stream>>>(
+                      csr.off, csr.val, lo, hi, group, bits, inst_lo, (u32) n_inst, ml, c, d, out.as<u64>(), cap, ctr,
+                      ws.cl_left.as<u64>()));
+        read_back();
+        if (got.words <= cap) break;
+        ctx.reserve(out, got.words * 8);
+    }
+    ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
+    res.n_words = got.words;
+    res.levels = (u32) got.levels;
+    if (got.left == 0) return res;
+    // What the warps left over: CTA searches, unless there are so many that
+    // bit rows are the cheaper form. A CTA search that fails has cost up to
+    // `reach` targets' edges; 10^8 of them are about a millisecond.
+    const u64 nl = got.left, levels_w = res.levels;
+    const double mean_deg = std::max(1.0, (double) csr.n_vals / std::max<u64>(csr.n_keys, 1));
+    u32 reach = CC_REACH;
+    if (!inst_lo) {
+        const double fit = 1e8 / (mean_deg * (double) nl);
+        if (fit < CC_REACH) reach = (u32) fit;
+        if (reach < 2 * CW_REACH) reach = 0;
+    }
+    ctx.reserve(ws.cl_heavy, nl * 8);
+    if (reach == 0) {
+        DL_CUDA(cudaMemcpyAsync(ws.cl_heavy.p, ws.cl_left.p, nl * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+        res.n_heavy = nl;
+        return res;
+    }
+    ctx.reserve(ws.cl_levels, 2 * table);  // their level counts apart: a run that outgrows the room is repeated
+    auto *c2 = ws.cl_levels.as<unsigned long long>();
+    auto *d2 = c2 + table / 8;
+    const u64 wave2 = resident_blocks(ctx, closure_cta_kernel, CC_THREADS, sizeof(CcSmem));
+    const unsigned grid2 = (unsigned) std::min<u64>(wave2, nl);
+    ctx.reserve(ws.cl_act, (u64) grid2 * 2 * CL_LEVELS * 4);
+    grow_keeping(ctx, out, (res.n_words + std::min<u64>(nl * 1024, 1ull << 28)) * 8, res.n_words * 8);
+    for (;;) {
+        DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
+        DL_CUDA(cudaMemsetAsync(c2, 0, 2 * table, ctx.stream));
+        const u64 cap = out.cap / 8 - res.n_words;
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * nl,
+                  closure_cta_kernel<<<grid2, CC_THREADS, sizeof(CcSmem), ctx.stream>>>(
+                      csr.off, csr.val, ws.cl_left.as<u64>(), nl, reach, bits, inst_lo, (u32) n_inst, ml, c2,
+                      deg ? d2 : nullptr, ws.cl_act.as<u32>(), out.as<u64>() + res.n_words, cap, ctr,
+                      ws.cl_heavy.as<u64>()));
+        read_back();
+        if (got.words <= cap) break;
+        grow_keeping(ctx, out, (res.n_words + got.words) * 8, res.n_words * 8);
+    }
+    ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
+    const unsigned ag = grid_for(n_inst * (CL_LEVELS + 1), T256, ctx);
+    DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, n_inst * (CL_LEVELS + 1)));
+    if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, n_inst * (CL_LEVELS + 1)));
+    res.n_words += got.words;
+    res.levels = (u32) std::max<u64>(levels_w, got.levels);
+    res.n_heavy = got.left;
+    return res;
+}
+
+static u64 pull_words(u64 h) { return (h + 1023) / 1024 * 32; }
+
+u64 closure_pull_bytes(u64 n, u64 h) { return n * (3 * pull_words(h) * 4 + pull_words(h) / 4); }
+
+ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne, int bits, u64 n, const u64 *src,
+                          u64 h, u64 max_level, DevBuf &t, DevBuf &cols) {
+    Workspace &ws = ctx.ws;
+    ClosureHeavy res;
+    res.h = h;
+    res.words = pull_words(h);
+    PullShape sh{n, (u32) res.words, 0};
+    while ((32u << sh.shift) < res.words / 32) ++sh.shift;
+    // in-neighbours: the edges sorted by target
+    ctx.reserve(ws.full[0], ne * 8);
+    ctx.reserve(ws.full[1], ne * 8);
+    DL_LAUNCH(ctx, K_PREP, 16.0 * ne,
+              pull_swap_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(edges, ne, bits, ws.full[0].as<u64>()));
+    const u64 *rev = radix_sort(ctx, ws.full[0].as<u64>(), ws.full[1].as<u64>(), ne, Codec::Raw, 2 * bits);
+    ctx.reserve(ws.cl_roff, (n + 1) * 4);
+    ctx.reserve(ws.cl_rval, ne * 4);
+    u32 *roff = ws.cl_roff.as<u32>(), *rval = ws.cl_rval.as<u32>();
+    DL_LAUNCH(ctx, K_PREP, 0,
+              key_offsets_kernel<u32><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, bits, n, roff));
+    DL_LAUNCH(ctx, K_PREP, 12.0 * ne,
+              low_field_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, (1ull << bits) - 1, rval));
+    // targets with many in-edges
+    auto *found = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[44]);
+    ctx.reserve(ws.cl_segs, (ne / PU_SEG * 2 + 1) * 8);  // a hub's segments are at most twice its in-edges / 32
+    ctx.reserve(ws.cl_hub_at, n * 4);
+    DL_CUDA(cudaMemsetAsync(found, 0, 16, ctx.stream));
+    DL_LAUNCH(ctx, K_PREP, 4.0 * n,
+              pull_hubs_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(roff, n, ws.cl_hub_at.as<u32>(),
+                                                                               ws.cl_segs.as<uint2>(), found));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, found, 16, cudaMemcpyDeviceToHost, ctx.stream));
+    // rows: T starts empty; a row of newest bits is read only when its tag says so
+    const u64 row_bytes = n * res.words * 4;
+    ctx.reserve(t, row_bytes);
+    ctx.reserve(ws.cl_rows[0], row_bytes);
+    ctx.reserve(ws.cl_rows[1], row_bytes);
+    ctx.reserve(ws.cl_act, 8 * n * 4);
+    ctx.reserve(cols, (res.words * 32 + n) * 4);
+    DL_CUDA(cudaMemsetAsync(t.p, 0, row_bytes, ctx.stream));
+    // levels: at most one per node (a shortest path), counted on the device
+    const u64 top = max_level ? std::min(max_level, n) : n;
+    ctx.reserve(ws.cl_levels, 3 * (top + 2) * 8);
+    DL_CUDA(cudaMemsetAsync(ws.cl_levels.p, 0, 3 * (top + 2) * 8, ctx.stream));
+    u32 *p = ws.cl_act.as<u32>();
+    DL_CUDA(cudaMemsetAsync(p, 0xFF, 4 * n * 4, ctx.stream));          // tags: no level
+    DL_CUDA(cudaMemsetAsync(p + 4 * n, 0, 2 * n * 4, ctx.stream));     // todo
+    auto view = [&](u64 level) {
+        const u64 in = (level + 1) & 1, out = level & 1;  // buffers by parity; at level 0 only the outputs are used
+        PullLevel v;
+        v.level = (u32) level;
+        v.cur = ws.cl_rows[in].as<u32>();
+        v.nxt = ws.cl_rows[out].as<u32>();
+        v.tag = reinterpret_cast<uint2 *>(p + 2 * in * n);
+        v.tag_next = reinterpret_cast<uint2 *>(p + 2 * out * n);
+        v.todo = p + (4 + out) * n;
+        v.todo_next = p + (4 + in) * n;
+        v.list = p + (6 + out) * n;
+        v.list_next = p + (6 + in) * n;
+        v.count = ws.cl_levels.as<unsigned long long>();
+        v.cnt = v.count + top + 2;
+        v.deg = v.cnt + top + 2;
+        return v;
+    };
+    DL_LAUNCH(ctx, K_PREP, 128.0 * h,
+              pull_init_kernel<<<grid_for(res.words * 32 * 32, T256, ctx), T256, 0, ctx.stream>>>(
+                  sh, view(0), src, h, cols.as<u32>()));
+    auto push = [&](u64 level) {
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                  closure_push_kernel<<<grid_for(ne, PU_THREADS, ctx, 8), PU_THREADS, 0, ctx.stream>>>(
+                      view(level), edges, ne, bits));
+    };
+    push(0);
+    ctx.sync();
+    const u64 n_hubs = ctx.host_scalars[0], n_seg = ctx.host_scalars[1];
+    if (n_hubs) {
+        ctx.reserve(ws.cl_hub_acc, n_hubs * res.words * 4);
+        DL_CUDA(cudaMemsetAsync(ws.cl_hub_acc.p, 0, n_hubs * res.words * 4, ctx.stream));
+    }
+    u32 *hub_acc = ws.cl_hub_acc.as<u32>();
+    auto level_step = [&](auto kc, u64 level) {
+        constexpr int K = decltype(kc)::value;
+        const u64 passes = (res.words + K * 128 - 1) / (K * 128);
+        if (n_hubs)
+            DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                      closure_pull_hub_kernel<K><<<grid_for(n_seg * passes * 32, PU_THREADS, ctx, 8), PU_THREADS, 0,
+                                                   ctx.stream>>>(sh, view(level), roff, rval, ws.cl_segs.as<uint2>(),
+                                                                 n_seg, ws.cl_hub_at.as<u32>(), hub_acc));
+        const u64 wave = resident_blocks(ctx, closure_pull_kernel<K>, PU_THREADS, 0);
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                  closure_pull_kernel<K><<<(unsigned) std::min<u64>(wave, (n + PU_THREADS / 32 - 1) / (PU_THREADS / 32)),
+                                           PU_THREADS, 0, ctx.stream>>>(
+                      sh, view(level), csr.off, roff, rval, ws.cl_hub_at.as<u32>(), hub_acc, t.as<u32>()));
+        push(level);
+    };
+    // Levels are launched eight at a time: one after the fixpoint finds its
+    // list empty and returns.
+    res.cnt.assign(1, 0);
+    res.deg.assign(1, 0);
+    bool done = false;
+    for (u64 level = 1; !done && level <= top;) {
+        const u64 batch = std::min<u64>(8, top - level + 1);
+        for (u64 k = 0; k < batch; ++k) {
+            if (res.words <= 128) level_step(std::integral_constant<int, 1>(), level + k);
+            else if (res.words <= 256) level_step(std::integral_constant<int, 2>(), level + k);
+            else level_step(std::integral_constant<int, 3>(), level + k);
+        }
+        u64 *hs = ctx.host_scalars;
+        DL_CUDA(cudaMemcpyAsync(hs, view(0).cnt + level, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs + 8, view(0).deg + level, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        for (u64 k = 0; k < batch; ++k) {
+            if (hs[k] == 0) {
+                done = true;
+                break;
+            }
+            res.cnt.push_back(hs[k]);
+            res.deg.push_back(hs[8 + k]);
+            ctx.prof_add_bytes(K_BITMAP_EXPAND, 4.0 * hs[8 + k]);
+        }
+        level += batch;
+    }
+    return res;
+}
+
+static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
+                           PhaseTimer &pt, u64 &nfull) {
+    Workspace &ws = ctx.ws;
+    const u64 n = g.n_ids;
+    const u64 max_level = opt.max_iterations > 0 ? (u64) opt.max_iterations + 1 : 0;
+    pt.mark(PH_JOIN);
+    ctx.reserve(ws.offsets, 2 * (CL_LEVELS + 1) * 8);
+    u64 *cnt = ws.offsets.as<u64>(), *deg = cnt + CL_LEVELS + 1;
+    ClosureLight light = closure_search(ctx, g.csr, 0, n, g.bits, nullptr, 1, max_level, cnt, deg);
+    if (light.n_heavy) {
+        const u64 need = closure_pull_bytes(n, light.n_heavy);
+        if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
+        u64 held = r.bm_t.cap + ws.cl_rows[0].cap + ws.cl_rows[1].cap;
+        for (const DevBuf &b : ctx.spares) held += b.cap;
+        if (need > held / 2) {
+            size_t free_b = 0, total_b = 0;
+            DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            if (need > ((u64) free_b + held) / 2) return false;
+        }
+    }
+    // host copies of the level counts (index d)
+    std::vector<u64> hc(light.levels + 1, 0), hd(light.levels + 1, 0);
+    if (light.levels) {
+        DL_CUDA(cudaMemcpyAsync(hc.data(), cnt, (light.levels + 1) * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hd.data(), deg, (light.levels + 1) * 8, cudaMemcpyDeviceToHost, ctx.stream));
+    }
+    pt.mark(PH_DEDUP);
+    // light pairs in result order
+    u64 *lw = ws.jbuf[0].as<u64>();
+    if (light.n_words) {
+        ctx.reserve(ws.jbuf[1], light.n_words * 8);
+        lw = radix_sort(ctx, lw, ws.jbuf[1].as<u64>(), light.n_words, Codec::Raw, 2 * g.bits);
+    }
+    DevBuf &lbuf = holder(ws, lw);
+    r.words = lbuf;
+    lbuf = DevBuf();
+    r.n_words = nfull = light.n_words;
+    if (light.n_heavy) {
+        ctx.reserve(ws.cl_left, light.n_heavy * 8);
+        const u64 *src = radix_sort(ctx, ws.cl_heavy.as<u64>(), ws.cl_left.as<u64>(), light.n_heavy, Codec::Raw, g.bits);
+        pt.mark(PH_MERGE);
+        const ClosureHeavy heavy =
+            closure_pull(ctx, g.csr, edges, ne, g.bits, n, src, light.n_heavy, max_level, r.bm_t, r.cl_cols);
+        if (heavy.cnt.size() > hc.size()) {
+            hc.resize(heavy.cnt.size(), 0);
+            hd.resize(heavy.cnt.size(), 0);
+        }
+        for (size_t d = 1; d < heavy.cnt.size(); ++d) {
+            hc[d] += heavy.cnt[d];
+            hd[d] += heavy.deg[d];
+            nfull += heavy.cnt[d];
+        }
+        pt.mark(PH_FINAL);
+        u32 *place = r.cl_cols.as<u32>() + heavy.words * 32;
+        ctx.reserve(r.cl_start, n * (heavy.words / 32) * 8);
+        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n,
+                  heavy_below_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(r.cl_cols.as<u32>(), heavy.h, n,
+                                                                                     place));
+        // first result row of every target
+        ctx.reserve(r.cl_loff, (n + 1) * 8);
+        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 8.0 * n,
+                  key_offsets_kernel<u64><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(
+                      r.words.as<u64>(), light.n_words, g.bits, n, r.cl_loff.as<u64>()));
+        ctx.reserve(ws.w0, (n + 1) * 8);
+        ctx.reserve(r.bm_first, (n + 1) * 8);
+        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n * heavy.words,
+                  closure_counts_kernel<<<grid_for(n * 32, T256, ctx), T256, 0, ctx.stream>>>(
+                      r.bm_t.as<u32>(), n, (u32) heavy.words, r.words.as<u64>(), r.cl_loff.as<u64>(),
+                      (1ull << g.bits) - 1, place, r.cl_start.as<uint2>(), ws.w0.as<u64>()));
+        const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+        u64 *lb = ctx.lookback_words(tiles);
+        u32 *tc = ctx.tile_counter(62);
+        u64 *tot = &ctx.ctrl->scalar[49];
+        DL_CUDA(cudaMemsetAsync(tc, 0, sizeof(u32), ctx.stream));
+        DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 16.0 * n,
+                  scan_kernel<SumValue><<<(unsigned) tiles, SCAN_THREADS, 0, ctx.stream>>>(
+                      SumValue{ws.w0.as<u64>()}, n, r.bm_first.as<u64>(), lb, tc, ctx.next_epoch(), &ctx.ctrl->err, tot));
+        DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, tot, sizeof(u64), cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        if (ctx.host_scalars[0] != nfull)
+            throw Error(DL_ERR_INTERNAL, "closure holds " + std::to_string(ctx.host_scalars[0]) + " tuples, expected " +
+                                             std::to_string(nfull));
+        r.from_bitmat = true;
+        r.cl_rows = true;
+        r.bm_n = n;
+        r.bm_stride = r.bm_words = heavy.words;
+    } else {
+        pt.mark(PH_FINAL);
+        ctx.sync();  // hc, hd are host memory
+    }
+    // iteration k joins level k + 1 and finds level k + 2 (tc.cu:216-314); the
+    // last one finds nothing, unless max_iterations ends the loop before
+    u64 full = hc.size() > 1 ? hc[1] : 0;
+    for (u64 k = 0;; ++k) {
+        const u64 nnew = k + 2 < hc.size() ? hc[k + 2] : 0;
+        const u64 join = k + 1 < hd.size() ? hd[k + 1] : 0;
+        full += nnew;
+        r.deltas.push_back((i64) nnew);
+        r.joins.push_back((i64) join);
+        r.fulls.push_back((i64) full);
+        ctx.run_join_total += join;
+        ctx.run_join_max = std::max(ctx.run_join_max, join);
+        if (nnew == 0 || (opt.max_iterations > 0 && k + 1 >= (u64) opt.max_iterations)) break;
+    }
+    return true;
+}
+
+bool tc_closure(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
+                PhaseTimer &pt, u64 &nfull) {
+    bool done = false;
+    try {
+        done = tc_closure_run(ctx, r, g, edges, ne, opt, pt, nfull);
+    } catch (const Error &err) {
+        if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
+    }
+    if (!done) {
+        r.deltas.clear();
+        r.joins.clear();
+        r.fulls.clear();
+        r.from_bitmat = r.cl_rows = false;
+        for (DevBuf *b : {&r.words, &r.bm_t, &r.bm_first, &r.cl_cols, &r.cl_loff, &r.cl_start}) ctx.give_back(*b);
+        r.n_words = nfull = 0;
+        ctx.run_join_total = ctx.run_join_max = 0;
+    }
+    return done;
+}
+
+}  // namespace detail
+
+void closure_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 z0, u64 z1) {
+    using namespace detail;
+    const u64 wave = resident_blocks(ctx, closure_rows_kernel, 256, 0);
+    const u32 *cols = r.cl_cols.as<u32>();
+    const u64 chunks = r.bm_words / 32;
+    const unsigned grid = (unsigned) std::max<u64>(1, std::min<u64>(wave, ((z1 - z0) * chunks + 7) / 8));
+    DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * (z1 - z0) * r.bm_words,
+              closure_rows_kernel<<<grid, 256, 0, ctx.stream>>>(
+                  r.bm_t.as<u32>(), (u32) r.bm_words, cols, cols + r.bm_words * 32, r.cl_start.as<uint2>(), z0, z1,
+                  r.bm_first.as<u64>(), r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << r.bits) - 1, r.ids.as<int32_t>(), r.ids_affine, r.id_base,
+                  reinterpret_cast<u64 *>(out)));
+}
+
+}  // namespace dl

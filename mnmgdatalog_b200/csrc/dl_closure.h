@@ -1,0 +1,54 @@
+// Transitive closure as one breadth-first search per source (dl_closure.cu).
+#pragma once
+
+#include "dl_engine_detail.h"
+
+namespace dl {
+namespace detail {
+
+// Levels a searched source may have; level d of a source = its targets at
+// distance d (Delta_{d-1}: level 1 is the edge relation).
+constexpr u32 CL_LEVELS = 4096;
+
+// What the searches of one call found.
+struct ClosureLight {
+    u64 n_words = 0;      // (z << bits) | x words of the finished sources, unsorted, in ws.jbuf[0]
+    u32 levels = 0;       // largest level of a finished source
+    u64 n_heavy = 0;      // sources left over: ranks as u64 words, unsorted, in ws.cl_heavy
+};
+
+// Searches from every source in [lo, hi). Level counts go to
+// cnt[instance * (CL_LEVELS + 1) + d] (and the sum of the out-degrees of the
+// level's targets to deg[...] when not null), instance k being the last one
+// whose first rank inst_lo[k] is at most the source (one instance when
+// inst_lo is null). Sources whose reach or work outgrows the searches' shared
+// memory are left over for the caller. max_level: 0 = no limit.
+ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
+                            u64 max_level, u64 *cnt, u64 *deg);
+
+// The closure of `h` heavy sources (ascending ranks `src`, device) over ranks
+// [0, n) as bit rows: bit c of row z of `t` is set when source c reaches z.
+// `cols`: rank of every column (padded to whole words with all ones), followed
+// by room for n more words.
+struct ClosureHeavy {
+    u64 h = 0;
+    u64 words = 0;                // words of a row (a multiple of 32)
+    std::vector<u64> cnt, deg;    // per level (index d, [0] unused)
+};
+// Device bytes closure_pull needs for h sources over n ranks.
+u64 closure_pull_bytes(u64 n, u64 h);
+ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne, int bits, u64 n, const u64 *src,
+                          u64 h, u64 max_level, DevBuf &t, DevBuf &cols);
+
+// TC of one graph by searches and pulls; false when its buffers do not fit
+// (the workspace's join buffers are overwritten then, the CSR is not).
+// `edges`: sorted (x, y) words.
+bool tc_closure(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
+                PhaseTimer &pt, u64 &nfull);
+
+}  // namespace detail
+
+// Result rows of targets [z0, z1) of a closure run into `out` (all rows' base).
+void closure_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 z0, u64 z1);
+
+}  // namespace dl

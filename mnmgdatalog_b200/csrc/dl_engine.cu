@@ -17,6 +17,7 @@
 #include "dl_internal.h"
 #include "dl_join.cuh"
 #include "dl_scan.cuh"
+#include "dl_closure.h"
 #include "dl_engine.h"
 #include "dl_engine_detail.h"
 
@@ -485,25 +486,42 @@ static void run_tc_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
     int cur = 0;
     FullSet F;
     F.three = true;  // plain runs: large, small and tiny runs
+    bool done = false;
     if (n > 0) {
         rank_nodes(ctx, rows, n, g);
-        // On the bit-matrix path, a dense id range is ranked as is: the
-        // result rows then need no rank -> id table lookups.
+        // Searches from every source (dl_closure.cu) unless a dedup form or a
+        // result form of the bit matrix was asked for.
+        const bool search = opt.dedup == DL_DEDUP_AUTO && ctx.tune.bitmap_max_gib > 0 && ctx.tune.bitmap_result == 0;
+        // On these paths, a dense id range is ranked as is: the result rows
+        // then need no rank -> id table lookups.
         const bool dense = densify_ids(ctx, g, [&](u64 range) {
             try {
-                return bitmat_choose(ctx, opt, range, false);
+                return search || bitmat_choose(ctx, opt, range, false);
             } catch (const Error &) {  // a forced bit matrix that fits only without the absent ids
                 return false;
             }
         });
-        ctx.reserve(ws.jbuf[0], n * 8);
-        ctx.reserve(ws.jbuf[1], n * 8);
-        DL_LAUNCH(ctx, K_PREP, 0, pack_rows_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(rows, n, g.ids, g.n_ids, g.bits,
-                                                                         ws.w0.as<u64>(), ws.jbuf[0].as<u64>()));
         u64 ne;
-        u64 *e = sort_unique_into(ctx, ws.w0, ws.w1, n, 2 * g.bits, ne);
-        build_csr(ctx, e, ne, g);
-        if (dense || bitmat_choose(ctx, opt, g.n_ids, false)) {
+        u64 *e = nullptr;
+        auto edge_words = [&](u64 *rev) {  // the edges as sorted words, and reversed (unsorted) into rev
+            ctx.reserve(ws.w0, n * 8);
+            DL_LAUNCH(ctx, K_PREP, 0, pack_rows_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(rows, n, g.ids, g.n_ids, g.bits,
+                                                                             ws.w0.as<u64>(), rev));
+            e = sort_unique_into(ctx, ws.w0, ws.w1, n, 2 * g.bits, ne);
+        };
+        if (search) {
+            edge_words(nullptr);
+            build_csr(ctx, e, ne, g);
+            done = tc_closure(ctx, r, g, e, ne, opt, pt, nfull);
+        }
+        if (!done) {
+            ctx.reserve(ws.jbuf[0], n * 8);
+            ctx.reserve(ws.jbuf[1], n * 8);
+            edge_words(ws.jbuf[0].as<u64>());
+            if (!search) build_csr(ctx, e, ne, g);
+        }
+        if (done) {
+        } else if ((dense && !search) || bitmat_choose(ctx, opt, g.n_ids, false)) {
             nfull = tc_bitmap_fixpoint(ctx, r, g, e, ne, opt, pt);  // result: the transpose, or the matrix and column offsets, in r
             cur = 0;
         } else {
@@ -537,7 +555,7 @@ static void run_tc_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
     DL_CUDA(cudaEventRecord(ev.b, ctx.stream));
     pt.mark(PH_FINAL);
     adopt_ids(ctx, r, g);
-    if (!r.from_bitmat) {
+    if (!r.from_bitmat && !done) {
         r.words = ws.full[cur];
         ws.full[cur] = DevBuf();
         r.n_words = nfull;
@@ -984,6 +1002,9 @@ void run_destroy(Run *r) {
         r->ctx->give_back(r->bm_first);
         r->ctx->give_back(r->bm_off);
         r->ctx->give_back(r->bm_live);
+        r->ctx->give_back(r->cl_cols);
+        r->ctx->give_back(r->cl_loff);
+        r->ctx->give_back(r->cl_start);
     }
     delete r;
 }

@@ -33,6 +33,12 @@ struct Run {
     DevBuf bm_t, bm_first, bm_off;
     DevBuf bm_live;             // TC column form: the matrix rows that were written (one bit per row)
     u64 bm_n = 0, bm_stride = 0, bm_words = 0;
+    // TC by searches (dl_closure.cu) with heavy sources: bm_t holds a row of
+    // heavy-source bits per target, cl_cols the sources' ranks, `words` the
+    // other pairs in result order, cl_loff each target's first one and
+    // cl_start each (target, 1024 columns)'s first row.
+    bool cl_rows = false;
+    DevBuf cl_cols, cl_loff, cl_start;
 };
 
 Run *run_program(Context &ctx, int program, const int32_t *rows, u64 n, bool on_device, const dl_options &opt);

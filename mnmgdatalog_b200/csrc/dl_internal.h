@@ -77,7 +77,8 @@ enum KernelId : int {
     K_SPARSE_DIFF,     // sparse set difference probes (+ run sampling)
     K_HASH_INSERT,     // hash-set dedup: 8 B read + 32 B probe sector per word, 40 B per new word
     K_BITMAP_EXPAND,   // bit-matrix TC step: 4 B per delta row in and out + 16 B per unit in and out +
-                       // 4 B edge target per join word
+                       // 4 B edge target per join word; TC searches and pulls: 8 B per source and per
+                       // pair written, 4 B per join word
     K_BITMAP_COLUMNS,  // TC result set-up from the bit matrix: its transpose with per-target counts
                        // (2 x matrix), or per (row block, target) counts and their offsets
     K_BITMAP_EXTRACT,  // result rows from the bit matrix: matrix (+ TC offsets) read + 8 B per result row (+ count scan)
@@ -113,6 +114,12 @@ struct Workspace {
     DevBuf wcc_label, wcc_flag, wcc_next;
     DevBuf bitmat[2];      // full relation as a bit matrix; TC's column offsets of the result rows
     DevBuf bit_hasout;     // bit-matrix TC: nodes with out-edges (one bit each)
+    // TC by searches (dl_closure.cu)
+    DevBuf cl_left, cl_heavy;   // sources a warp's / a CTA's search could not hold
+    DevBuf cl_levels;           // level counts
+    DevBuf cl_roff, cl_rval;    // in-neighbours of every node
+    DevBuf cl_segs, cl_hub_at, cl_hub_acc;  // targets with many in-neighbours
+    DevBuf cl_rows[2], cl_act;  // newest bits of the heavy sources' rows, and which rows have any
 };
 
 // Engine knobs the autotuner sets per context (mnmgdatalog_b200/autotune.py);

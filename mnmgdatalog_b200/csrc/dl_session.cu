@@ -790,7 +790,9 @@ void session_destroy(SessionImpl *s) {
     DevBuf *wbufs[] = {&w.input,    &w.ids,      &w.w0,       &w.w1,      &w.csr_off,  &w.csr_val,
                        &w.full[0],  &w.full[1],  &w.small[0], &w.small[1], &w.tiny[0], &w.tiny[1],
                        &w.sample,   &w.sample_small, &w.jbuf[0],
-                       &w.jbuf[1],  &w.offsets,  &w.wcc_label, &w.wcc_flag, &w.wcc_next};
+                       &w.jbuf[1],  &w.offsets,  &w.wcc_label, &w.wcc_flag, &w.wcc_next,
+                       &w.cl_left,  &w.cl_heavy, &w.cl_levels, &w.cl_roff,  &w.cl_rval, &w.cl_segs,
+                       &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act};
     for (DevBuf *b : wbufs) p.give_back(*b);
     for (auto &b : c.spares) p.give_back(b);
     c.spares.clear();
