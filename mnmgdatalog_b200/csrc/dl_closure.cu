@@ -127,8 +127,9 @@ __device__ __forceinline__ u32 walk_rows(u32 *wbeg, u32 *wpre, u32 beg, u32 deg,
 // instance's counters when the instance changes, the rest directly.
 __global__ void __launch_bounds__(CW_THREADS)
 closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 lo, u64 hi, u32 group, int bits,
-                    const u64 *__restrict__ inst_lo, u32 n_inst, u32 max_level, unsigned long long *__restrict__ cnt,
-                    unsigned long long *__restrict__ deg, u64 *__restrict__ out, u64 cap,
+                    const u64 *__restrict__ inst_lo, u32 n_inst, u32 stride, u32 max_level,
+                    unsigned long long *__restrict__ cnt, unsigned long long *__restrict__ deg,
+                    u64 *__restrict__ out, u64 cap,
                     SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CwSmem &s = reinterpret_cast<CwSmem *>(smem_raw)[threadIdx.x >> 5];
@@ -143,7 +144,7 @@ closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u6
     u32 inst = 0;
     u64 inst_end = inst_lo ? 0 : hi;  // first rank after the current instance
     auto flush = [&]() {
-        const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + lane;
+        const u64 at = (u64) inst * stride + 1 + lane;
 #pragma unroll
         for (int j = 0; j < CW_REGS; ++j) {
             if (rc[j]) atomicAdd(cnt + at + 32 * j, (unsigned long long) rc[j]);
@@ -241,7 +242,7 @@ closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u6
                 }
             }
             for (u32 k = 32 * CW_REGS + lane; k < level; k += 32) {
-                const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + k;
+                const u64 at = (u64) inst * stride + 1 + k;
                 atomicAdd(cnt + at, (unsigned long long) s.lcnt[k]);
                 if (deg) atomicAdd(deg + at, (unsigned long long) s.ldeg[k]);
             }
@@ -281,7 +282,7 @@ struct CcSmem {
 // finished: in shared memory they would cost a quarter of the resident CTAs.
 __global__ void __launch_bounds__(CC_THREADS)
 closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, const u64 *__restrict__ src, u64 n_src,
-                   u32 reach, int bits, const u64 *__restrict__ inst_lo, u32 n_inst, u32 max_level,
+                   u32 reach, int bits, const u64 *__restrict__ inst_lo, u32 n_inst, u32 stride, u32 max_level,
                    unsigned long long *__restrict__ cnt, unsigned long long *__restrict__ deg, u32 *lev,
                    u64 *__restrict__ out, u64 cap, SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -378,7 +379,7 @@ closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, con
             inst = a - 1;
         }
         for (u32 k = tid; k < level; k += CC_THREADS) {
-            const u64 at = (u64) inst * (CL_LEVELS + 1) + 1 + k;
+            const u64 at = (u64) inst * stride + 1 + k;
             atomicAdd(cnt + at, (unsigned long long) lcnt[k]);
             if (deg) atomicAdd(deg + at, (unsigned long long) ldeg[k]);
         }
@@ -754,6 +755,36 @@ struct SumValue {
     __device__ __forceinline__ u64 operator()(u64 i) const { return v[i]; }
 };
 
+// Edges of ranks [lo, hi) as words over ranks from lo.
+__global__ void local_edges_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 lo, u64 hi, int bits,
+                                   u64 *__restrict__ out) {
+    const u32 b = off[lo];
+    for (u64 r = lo + (u64) blockIdx.x * blockDim.x + threadIdx.x; r < hi; r += (u64) gridDim.x * blockDim.x)
+        for (u32 k = off[r]; k < off[r + 1]; ++k) out[k - b] = ((r - lo) << bits) | (val[k] - lo);
+}
+
+// The set bits of T as words (z << bits) | x over ranks from lo, unordered.
+__global__ void heavy_words_kernel(const u32 *__restrict__ t, u64 n, u32 words, const u32 *__restrict__ cols, u64 lo,
+                                   int bits, u64 *__restrict__ out, u64 cap, unsigned long long *__restrict__ count) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    for (u64 z = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32; z < n; z += warps) {
+        for (u32 k0 = 0; k0 < words; k0 += 32) {
+            u32 v = t[z * words + k0 + lane];
+            const u32 incl = warp_inclusive_sum((u32) __popc(v));
+            const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+            if (!total) continue;
+            unsigned long long p = 0;
+            if (lane == 0) p = atomicAdd(count, (unsigned long long) total);
+            p = __shfl_sync(0xffffffffu, p, 0);
+            if (p + total > cap) continue;
+            p += incl - __popc(v);
+            for (; v; v &= v - 1)
+                out[p++] = ((z + lo) << bits) | (cols[(k0 + lane) * 32 + __ffs(v) - 1] + lo);
+        }
+    }
+}
+
 // place[r] = heavy sources below rank r.
 __global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u32 *__restrict__ place) {
     for (u64 r = (u64) blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (u64) gridDim.x * blockDim.x) {
@@ -889,12 +920,12 @@ void grow_keeping(Context &ctx, DevBuf &buf, u64 bytes, u64 keep) {
 }  // namespace
 
 ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
-                            u64 max_level, u64 *cnt, u64 *deg) {
+                            u64 stride, u64 max_level, u64 *cnt, u64 *deg) {
     Workspace &ws = ctx.ws;
     ClosureLight res;
     const u64 ns = hi - lo;
     if (ns == 0) return res;
-    const u64 table = n_inst * (CL_LEVELS + 1) * 8;
+    const u64 table = n_inst * stride * 8;
     const u32 ml = (u32) std::min<u64>(max_level, 0xFFFFFFFFull);
     auto *c = reinterpret_cast<unsigned long long *>(cnt), *d = reinterpret_cast<unsigned long long *>(deg);
     SearchCounters *ctr = reinterpret_cast<SearchCounters *>(&ctx.ctrl->scalar[40]);
@@ -922,7 +953,7 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
         const u64 cap = out.cap / 8;
         DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * ns,
                   closure_warp_kernel<<<grid, CW_THREADS, smem, ctx.stream>>>(
-                      csr.off, csr.val, lo, hi, group, bits, inst_lo, (u32) n_inst, ml, c, d, out.as<u64>(), cap, ctr,
+                      csr.off, csr.val, lo, hi, group, bits, inst_lo, (u32) n_inst, (u32) stride, ml, c, d, out.as<u64>(), cap, ctr,
                       ws.cl_left.as<u64>()));
         read_back();
         if (got.words <= cap) break;
@@ -962,7 +993,7 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
         const u64 cap = out.cap / 8 - res.n_words;
         DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * nl,
                   closure_cta_kernel<<<grid2, CC_THREADS, sizeof(CcSmem), ctx.stream>>>(
-                      csr.off, csr.val, ws.cl_left.as<u64>(), nl, reach, bits, inst_lo, (u32) n_inst, ml, c2,
+                      csr.off, csr.val, ws.cl_left.as<u64>(), nl, reach, bits, inst_lo, (u32) n_inst, (u32) stride, ml, c2,
                       deg ? d2 : nullptr, ws.cl_act.as<u32>(), out.as<u64>() + res.n_words, cap, ctr,
                       ws.cl_heavy.as<u64>()));
         read_back();
@@ -970,9 +1001,9 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
         grow_keeping(ctx, out, (res.n_words + got.words) * 8, res.n_words * 8);
     }
     ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
-    const unsigned ag = grid_for(n_inst * (CL_LEVELS + 1), T256, ctx);
-    DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, n_inst * (CL_LEVELS + 1)));
-    if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, n_inst * (CL_LEVELS + 1)));
+    const unsigned ag = grid_for(table / 8, T256, ctx);
+    DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, table / 8));
+    if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, table / 8));
     res.n_words += got.words;
     res.levels = (u32) std::max<u64>(levels_w, got.levels);
     res.n_heavy = got.left;
@@ -1106,6 +1137,68 @@ ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne
     return res;
 }
 
+void closure_heavy_words(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const std::vector<u64> &src,
+                         u64 max_level, std::vector<u64> &cnt, u64 &n_words) {
+    Workspace &ws = ctx.ws;
+    const u64 n = hi - lo;
+    const int lb = bits_for(std::max<u64>(n, 2));
+    // the instance's own edges and CSR over ranks from 0
+    u32 ends[2];
+    DL_CUDA(cudaMemcpyAsync(&ends[0], csr.off + lo, 4, cudaMemcpyDeviceToHost, ctx.stream));
+    DL_CUDA(cudaMemcpyAsync(&ends[1], csr.off + hi, 4, cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    const u64 ne = ends[1] - ends[0];
+    ctx.reserve(ws.w0, ne * 8);
+    ctx.reserve(ws.csr_off, (n + 1) * 4);
+    ctx.reserve(ws.csr_val, ne * 4);
+    u64 *e = ws.w0.as<u64>();
+    DL_LAUNCH(ctx, K_PREP, 0,
+              local_edges_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(csr.off, csr.val, lo, hi, lb, e));
+    Csr local;
+    local.off = ws.csr_off.as<u32>();
+    local.val = ws.csr_val.as<u32>();
+    local.n_keys = (u32) n;
+    local.n_vals = ne;
+    DL_LAUNCH(ctx, K_PREP, 0,
+              key_offsets_kernel<u32><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(e, ne, lb, n, local.off));
+    DL_LAUNCH(ctx, K_PREP, 0,
+              low_field_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(e, ne, (1ull << lb) - 1, local.val));
+    // as many sources at a time as 8 GiB of rows hold (sources are independent)
+    const u64 at_once = std::max<u64>(1024, (8ull << 30) / (closure_pull_bytes(n, 1024) / 1024 + 1) / 1024 * 1024);
+    DevBuf t, cols;
+    try {
+        for (u64 s0 = 0; s0 < src.size(); s0 += at_once) {
+            const u64 h = std::min<u64>(at_once, src.size() - s0);
+            std::vector<u64> l(h);
+            for (u64 i = 0; i < h; ++i) l[i] = src[s0 + i] - lo;
+            ctx.reserve(ws.cl_left, h * 8);
+            DL_CUDA(cudaMemcpyAsync(ws.cl_left.p, l.data(), h * 8, cudaMemcpyHostToDevice, ctx.stream));
+            ctx.sync();  // l is a host temporary
+            const ClosureHeavy hv = closure_pull(ctx, local, e, ne, lb, n, ws.cl_left.as<u64>(), h, max_level, t, cols);
+            u64 total = 0;
+            if (hv.cnt.size() > cnt.size()) cnt.resize(hv.cnt.size(), 0);
+            for (size_t d = 1; d < hv.cnt.size(); ++d) {
+                cnt[d] += hv.cnt[d];
+                total += hv.cnt[d];
+            }
+            grow_keeping(ctx, ws.jbuf[0], (n_words + total) * 8, n_words * 8);
+            auto *count = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[46]);
+            DL_CUDA(cudaMemsetAsync(count, 0, 8, ctx.stream));
+            DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * n * hv.words + 8.0 * total,
+                      heavy_words_kernel<<<grid_for(n * 32, T256, ctx), T256, 0, ctx.stream>>>(
+                          t.as<u32>(), n, (u32) hv.words, cols.as<u32>(), lo, bits, ws.jbuf[0].as<u64>() + n_words,
+                          total, count));
+            n_words += total;
+        }
+    } catch (...) {
+        ctx.give_back(t);
+        ctx.give_back(cols);
+        throw;
+    }
+    ctx.give_back(t);
+    ctx.give_back(cols);
+}
+
 static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
                            PhaseTimer &pt, u64 &nfull) {
     Workspace &ws = ctx.ws;
@@ -1114,7 +1207,7 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
     pt.mark(PH_JOIN);
     ctx.reserve(ws.offsets, 2 * (CL_LEVELS + 1) * 8);
     u64 *cnt = ws.offsets.as<u64>(), *deg = cnt + CL_LEVELS + 1;
-    ClosureLight light = closure_search(ctx, g.csr, 0, n, g.bits, nullptr, 1, max_level, cnt, deg);
+    ClosureLight light = closure_search(ctx, g.csr, 0, n, g.bits, nullptr, 1, CL_LEVELS + 1, max_level, cnt, deg);
     if (light.n_heavy) {
         const u64 need = closure_pull_bytes(n, light.n_heavy);
         if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;

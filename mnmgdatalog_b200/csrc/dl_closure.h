@@ -18,13 +18,14 @@ struct ClosureLight {
 };
 
 // Searches from every source in [lo, hi). Level counts go to
-// cnt[instance * (CL_LEVELS + 1) + d] (and the sum of the out-degrees of the
-// level's targets to deg[...] when not null), instance k being the last one
-// whose first rank inst_lo[k] is at most the source (one instance when
-// inst_lo is null). Sources whose reach or work outgrows the searches' shared
-// memory are left over for the caller. max_level: 0 = no limit.
+// cnt[instance * stride + d] (and the sum of the out-degrees of the level's
+// targets to deg[...] when not null), instance k being the last one whose first
+// rank inst_lo[k] is at most the source (one instance when inst_lo is null);
+// stride: above the levels an instance can have, or CL_LEVELS + 1. Sources
+// whose reach or work outgrows the searches' shared memory are left over for
+// the caller. max_level: 0 = no limit.
 ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
-                            u64 max_level, u64 *cnt, u64 *deg);
+                            u64 stride, u64 max_level, u64 *cnt, u64 *deg);
 
 // The closure of `h` heavy sources (ascending ranks `src`, device) over ranks
 // [0, n) as bit rows: bit c of row z of `t` is set when source c reaches z.
@@ -39,6 +40,13 @@ struct ClosureHeavy {
 u64 closure_pull_bytes(u64 n, u64 h);
 ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne, int bits, u64 n, const u64 *src,
                           u64 h, u64 max_level, DevBuf &t, DevBuf &cols);
+
+// The pairs of heavy sources `src` (ascending, host) of one instance with ranks
+// [lo, hi) of the CSR: appended as (z << bits) | x words to ws.jbuf[0] (n_words
+// of it are kept and counted on), their levels added to cnt (index d, grown as
+// needed).
+void closure_heavy_words(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const std::vector<u64> &src,
+                         u64 max_level, std::vector<u64> &cnt, u64 &n_words);
 
 // TC of one graph by searches and pulls; false when its buffers do not fit
 // (the workspace's join buffers are overwritten then, the CSR is not).

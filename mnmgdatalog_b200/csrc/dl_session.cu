@@ -18,6 +18,7 @@
 #include <cstring>
 #include <memory>
 
+#include "dl_closure.h"
 #include "dl_engine_detail.h"
 #include "dl_join.cuh"
 #include "dl_scan.cuh"
@@ -311,6 +312,7 @@ struct SessionImpl {
     std::vector<SessionInstance> inst;
     std::vector<i64> active;    // instance ids in rank order
     std::vector<i64> finished;  // finished since the last poll
+    std::vector<i64> pending;   // TC: admitted since the last step, not searched yet
     bool inst_dirty = true;
 };
 
@@ -680,25 +682,133 @@ u64 wcc_step(SessionImpl &s) {
     return s.active.size();
 }
 
-u64 fixpoint_step(SessionImpl &s) {
+// TC: the whole fixpoint of the instances admitted since the last step
+// (dl_closure.cu: a search per source, whatever the instance, so all of them
+// run in one launch), their rows sorted into one block and every iteration's
+// |delta|. The steps then only report iteration after iteration.
+void search_pending(SessionImpl &s) {
+    if (s.pending.empty()) return;
+    Context &ctx = s.ctx;
+    Workspace &ws = ctx.ws;
+    const std::vector<i64> ids = s.pending;
+    const u64 n = ids.size();
+    // first ranks; ranks between two of them that no instance holds (a failed
+    // admission's) become an entry of their own
+    std::vector<u64> lo, at(n);
+    u64 end = s.inst[ids[0]].rank_lo, widest = 1;
+    for (u64 k = 0; k < n; ++k) {
+        const SessionInstance &in = s.inst[ids[k]];
+        if (in.rank_lo != end) lo.push_back(end);
+        at[k] = lo.size();
+        lo.push_back(in.rank_lo);
+        end = in.rank_hi;
+        widest = std::max<u64>(widest, in.n_ids);
+    }
+    const u64 first = lo[0], ni = lo.size(), stride = std::min<u64>(CL_LEVELS, widest) + 1;
+    ctx.reserve(s.range_lo, ni * 8);
+    DL_CUDA(cudaMemcpyAsync(s.range_lo.p, lo.data(), ni * 8, cudaMemcpyHostToDevice, ctx.stream));
+    ctx.reserve(s.counts, ni * stride * 8);
+    const u64 max_level = s.opt.max_iterations > 0 ? (u64) s.opt.max_iterations + 1 : 0;
+    Csr csr;
+    csr.off = s.off.as<u32>();
+    csr.val = s.val.as<u32>();
+    csr.n_keys = (u32) s.next_rank;
+    csr.n_vals = s.n_vals;
+    const ClosureLight light = closure_search(ctx, csr, first, end, s.bits, s.range_lo.as<u64>(), ni, stride,
+                                              max_level, s.counts.as<u64>(), nullptr);
+    const u64 width = light.levels + 1;
+    std::vector<u64> hc(ni * width, 0);
+    if (light.levels)
+        DL_CUDA(cudaMemcpy2DAsync(hc.data(), width * 8, s.counts.p, stride * 8, width * 8, ni, cudaMemcpyDeviceToHost,
+                                  ctx.stream));
+    std::vector<u64> heavy(light.n_heavy);
+    if (light.n_heavy)
+        DL_CUDA(cudaMemcpyAsync(heavy.data(), ws.cl_heavy.p, light.n_heavy * 8, cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    std::sort(heavy.begin(), heavy.end());
+    u64 words = light.n_words;
+    auto hp = heavy.begin();
+    for (u64 k = 0; k < n; ++k) {
+        SessionInstance &in = s.inst[ids[k]];
+        std::vector<u64> cnt(hc.begin() + at[k] * width, hc.begin() + (at[k] + 1) * width);
+        hp = std::lower_bound(hp, heavy.end(), in.rank_lo);
+        const auto he = std::lower_bound(hp, heavy.end(), in.rank_hi);
+        if (he != hp)
+            closure_heavy_words(ctx, csr, in.rank_lo, in.rank_hi, s.bits, std::vector<u64>(hp, he), max_level, cnt,
+                                words);
+        hp = he;
+        in.ahead.clear();
+        for (u64 d = 2;; ++d) {  // iteration d - 2 finds the targets at distance d (tc.cu:216-314)
+            const i64 c = d < cnt.size() ? (i64) cnt[d] : 0;
+            in.ahead.push_back(c);
+            if (c == 0 || (s.opt.max_iterations > 0 && (int) in.ahead.size() >= s.opt.max_iterations)) break;
+        }
+    }
+    // result order; every instance's words are one range
+    std::vector<u64> hb(6 * n, 0);
+    auto block = std::shared_ptr<DevBuf>();
+    if (words) {
+        ctx.reserve(ws.jbuf[1], words * 8);
+        int w[8];
+        const int nw = plan_windows(s.bits, bits_for(std::max<u64>(s.next_rank, 2)), w);
+        u64 *r = radix_sort_windows(ctx, ws.jbuf[0].as<u64>(), ws.jbuf[1].as<u64>(), words, w, nw);
+        upload_ranges(s, ids);
+        ctx.reserve(s.counts, 6 * n * 8);
+        Runs3 runs{{r, r, r}, {words, 0, 0}};
+        DL_LAUNCH(ctx, K_PREP, 0,
+                  session_bounds_kernel<<<grid_for(6 * n, 256, ctx, 4), 256, 0, ctx.stream>>>(
+                      runs, s.range_lo.as<u64>(), (u32) n, s.bits, s.counts.as<u64>()));
+        DL_CUDA(cudaMemcpyAsync(hb.data(), s.counts.p, 6 * n * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DevBuf &held = holder(ws, r);
+        if (held.cap <= 2 * words * 8 + (1 << 20)) {  // the sorted buffer becomes the result block
+            block = make_block(ctx, 0);
+            std::swap(*block, held);
+        } else {
+            block = make_block(ctx, words * 8);
+            DL_CUDA(cudaMemcpyAsync(block->p, r, words * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+        }
+        ctx.sync();
+    }
+    for (u64 k = 0; k < n; ++k) {
+        SessionInstance &in = s.inst[ids[k]];
+        in.result_block = block;
+        in.result_off = hb[6 * k];
+        in.n_result = hb[6 * k + 1] - hb[6 * k];
+    }
+    s.pending.clear();
+}
+
+u64 tc_step(SessionImpl &s) {
+    search_pending(s);
+    std::vector<i64> still;
+    for (i64 id : s.active) {
+        SessionInstance &in = s.inst[id];
+        in.deltas.push_back(in.ahead[in.deltas.size()]);
+        if (in.deltas.size() == in.ahead.size()) mark_done(s, in);
+        else still.push_back(id);
+    }
+    if (still.size() != s.active.size()) {
+        s.active = still;
+        s.inst_dirty = true;
+    }
+    reset_if_idle(s);
+    return s.active.size();
+}
+
+// One SG iteration of every active instance (sg.cu:244-390).
+u64 sg_step(SessionImpl &s) {
     Context &ctx = s.ctx;
     Workspace &ws = ctx.ws;
     Graph g = union_graph(s);
     PhaseTimer pt(ctx, false);
     u64 nnew = 0;
     u64 *dnew = nullptr;
-    if (s.program == DL_PROGRAM_TC) {  // tc.cu:216-314
-        u64 nj = 0;
-        u64 *j = join_and_sort(ctx, g, s.delta.as<u64>(), s.n_delta, EmitKind::ZV, nj, nullptr, pt);
-        dnew = absorb(ctx, s.F, j, nj, nnew);
-    } else {  // sg.cu:244-390
-        u64 n1 = 0, n2 = 0;
-        u64 *j1 = join_and_sort(ctx, g, s.delta.as<u64>(), s.n_delta, EmitKind::VZ, n1, nullptr, pt);
-        if (n1) n1 = unique_words(ctx, j1, n1, j1);
-        if (n1) {
-            u64 *j2 = join_and_sort(ctx, g, j1, n1, EmitKind::VZ, n2, nullptr, pt);
-            dnew = absorb(ctx, s.F, j2, n2, nnew);
-        }
+    u64 n1 = 0, n2 = 0;
+    u64 *j1 = join_and_sort(ctx, g, s.delta.as<u64>(), s.n_delta, EmitKind::VZ, n1, nullptr, pt);
+    if (n1) n1 = unique_words(ctx, j1, n1, j1);
+    if (n1) {
+        u64 *j2 = join_and_sort(ctx, g, j1, n1, EmitKind::VZ, n2, nullptr, pt);
+        dnew = absorb(ctx, s.F, j2, n2, nnew);
     }
     // the new delta sits in one of the join buffers: trade it for the old delta's buffer
     if (nnew) std::swap(s.delta, holder(ws, dnew));
@@ -810,6 +920,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
     std::vector<u64> off(count + 1, 0);
     for (u64 k = 0; k < count; ++k) off[k + 1] = off[k] + nrows[k];
     const u64 N = off[count];
+    const bool tc = s.program == DL_PROGRAM_TC;
     const u64 first_id = s.inst.size();
     std::vector<i64> ids(count);
     for (u64 k = 0; k < count; ++k) {
@@ -864,10 +975,9 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
         // rows -> rank words; the edge relation keyed by source (tc.cu:171-176,
         // sg.cu:150-153, wcc.cu:140-167: WCC stores both directions)
         const int bits = s.bits;
-        const bool wcc = s.program == DL_PROGRAM_WCC, tc = s.program == DL_PROGRAM_TC;
-        if (tc) ctx.reserve(ws.jbuf[0], N * 8);
+        const bool wcc = s.program == DL_PROGRAM_WCC;
         u64 *fw = wo.as<u64>();
-        u64 *rv = wcc ? fw + N : (tc ? ws.jbuf[0].as<u64>() : nullptr);
+        u64 *rv = wcc ? fw + N : nullptr;
         DL_LAUNCH(ctx, K_PREP, 0,
                   session_pack_many_kernel<<<grid_for(N, 256, ctx, 16), 256, 0, ctx.stream>>>(
                       in_rows, N, d_off, (u32) count, u, nu, B, bits, fw, rv));
@@ -893,10 +1003,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
         }
         std::vector<bool> empty_base(count, false);
         if (tc) {
-            u64 nd;
-            u64 *d = sort_unique_fields(ctx, ws.jbuf[0], ws.jbuf[1], N, bits, used, nd);  // tc.cu:178-189
-            full_insert_new(s, d, nd);
-            delta_append(s, d, nd);
+            // searched as a whole in the next step
         } else if (s.program == DL_PROGRAM_SG) {
             // sg.cu:170-217: the base rule of the admitted instances, probing the union table
             Graph g = union_graph(s);
@@ -937,6 +1044,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
             } else {
                 in.active = true;
                 s.active.push_back(in.id);
+                if (tc) s.pending.push_back(in.id);
             }
         }
         s.inst_dirty = true;
@@ -957,7 +1065,7 @@ i64 session_admit(SessionImpl &s, const int32_t *rows, u64 n, bool on_device) {
 
 u64 session_step(SessionImpl &s) {
     if (s.active.empty()) return 0;
-    return s.program == DL_PROGRAM_WCC ? wcc_step(s) : fixpoint_step(s);
+    return s.program == DL_PROGRAM_WCC ? wcc_step(s) : s.program == DL_PROGRAM_TC ? tc_step(s) : sg_step(s);
 }
 
 u64 session_poll(SessionImpl &s, int64_t *ids, u64 capacity) {
@@ -1069,7 +1177,8 @@ u64 session_device_bytes(const SessionImpl &s) {
                             &w.full[0], &w.full[1],   &w.small[0], &w.small[1],   &w.tiny[0],    &w.tiny[1],
                             &w.sample,  &w.sample_small, &w.jbuf[0],
                             &w.jbuf[1], &w.offsets,   &c.lookback, &c.radix_part, &c.lbs_splits, &c.sort_hist,
-                            &c.merge_splits};
+                            &c.merge_splits, &w.cl_left, &w.cl_heavy, &w.cl_levels, &w.cl_roff, &w.cl_rval, &w.cl_segs,
+                            &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act};
     for (const DevBuf *x : bufs) b += x->cap;  // cached spare buffers are not counted: they are free memory
     std::vector<const DevBuf *> blocks;
     for (const auto &in : s.inst)
