@@ -11,10 +11,11 @@
 // are sums of the searches' level sizes.
 //
 // Two kinds of work, by what a source reaches:
-//  * closure_warp_kernel / closure_cta_kernel: a search whose visited set
-//    fits in shared memory (a hash set and the visit queue: up to 512 targets
-//    in a warp's slice, up to 4096 in a CTA's). Result pairs leave as words,
-//    sorted afterwards.
+//  * closure_group_kernel / closure_warp_kernel / closure_cta_kernel: a search
+//    whose visited set fits in shared memory (a hash set and the visit queue: up
+//    to 255 targets for eight lanes, 1024 for a warp, 4096 for a CTA; a source
+//    that outgrows one goes to the next). Result pairs leave as words, sorted
+//    afterwards.
 //  * closure_pull_kernel: the sources that reach more ("heavy"), 32 of them
 //    to a word: bit c of row z of T says whether heavy source c reaches z.
 //    One iteration ORs, for every target z, the newest bits of its
@@ -25,8 +26,9 @@
 // Measured on B200 against the n x n bit matrix stepped by one launch per
 // iteration (dl_bitmap.cu), edges and result rows on the device: Chung-Lu graph
 // of 317K nodes (1.88e9 pairs; 9.3K heavy sources hold 99 % of them)
-// 45.5 -> 12.4 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 5.0 ms;
-// DAG of 5.5K edges from and to host memory 3.6 -> 0.68 ms.
+// 45.5 -> 12.4 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 4.0 ms
+// (5.0 with a warp for every source); DAG of 5.5K edges from and to host memory
+// 3.5 -> 0.66 ms.
 #include <type_traits>
 
 #include "dl_closure.h"
@@ -37,24 +39,6 @@ namespace detail {
 namespace {
 
 constexpr u32 EMPTY = 0xFFFFFFFFu;  // ranks are below 2^32 - 1
-
-// ---- searches by a warp -------------------------------------------------
-
-constexpr int CW_THREADS = 128;
-constexpr u32 CW_REACH = 512;
-constexpr u32 CW_HASH = 2 * CW_REACH;
-constexpr int CW_HASH_SHIFT = 22;     // 32 - log2(CW_HASH)
-constexpr u32 CW_LEVELS = 256;
-constexpr u32 CW_EDGES = 8192;        // join words of one search
-constexpr int CW_REGS = 4;            // levels 1 .. 32 * CW_REGS are summed in registers
-
-struct CwSmem {
-    u32 hash[CW_HASH];
-    u32 queue[CW_REACH];
-    unsigned short lcnt[CW_LEVELS];   // targets of level d at [d - 1]
-    unsigned short ldeg[CW_LEVELS];   // join words out of level d at [d - 1]
-    u32 wbeg[32], wpre[32];           // compacted rows of the group being expanded
-};
 
 // Counters of a search launch (device).
 struct SearchCounters {
@@ -78,6 +62,344 @@ __device__ __forceinline__ bool set_insert(u32 *hash, u32 w, int shift) {
         s = (s + 1) & MASK;
     }
 }
+
+// Instance of rank x: the last one whose first rank is at most x.
+__device__ __forceinline__ u32 instance_at(const u64 *__restrict__ inst_lo, u32 n_inst, u64 x) {
+    u32 a = 0, b = n_inst;
+    while (a < b) {
+        const u32 m = (a + b) >> 1;
+        if (inst_lo[m] <= x) a = m + 1;
+        else b = m;
+    }
+    return a - 1;
+}
+
+// Level counts of finished searches, summed in a warp's registers (lane l holds
+// levels 32 j + l + 1) and added to the instance's counters when it changes.
+constexpr int LV_REGS = 4;
+struct LevelSums {
+    u32 rc[LV_REGS], rd[LV_REGS];
+    u32 held, inst;
+    u64 lo, end;  // ranks of the instance
+    __device__ void init(bool one, u64 hi) {
+#pragma unroll
+        for (int j = 0; j < LV_REGS; ++j) rc[j] = rd[j] = 0;
+        held = inst = 0;
+        lo = 0;
+        end = one ? ~0ull : 0;
+    }
+    __device__ void flush(unsigned long long *cnt, unsigned long long *deg, u32 stride, u32 lane) {
+        const u64 at = (u64) inst * stride + 1 + lane;
+#pragma unroll
+        for (int j = 0; j < LV_REGS; ++j) {
+            if (rc[j]) atomicAdd(cnt + at + 32 * j, (unsigned long long) rc[j]);
+            if (deg && rd[j]) atomicAdd(deg + at + 32 * j, (unsigned long long) rd[j]);
+            rc[j] = rd[j] = 0;
+        }
+        held = 0;
+    }
+    // The levels of a search from x: sizes lc[0 .. levels), join words ld[...]. All lanes.
+    template <class C>
+    __device__ void add(u64 x, u32 levels, const C *lc, const unsigned short *ld,
+                        const u64 *__restrict__ inst_lo, u32 n_inst, unsigned long long *cnt, unsigned long long *deg,
+                        u32 stride, u32 lane) {
+        if (x < lo || x >= end) {
+            flush(cnt, deg, stride, lane);
+            inst = instance_at(inst_lo, n_inst, x);
+            lo = inst_lo[inst];
+            end = inst + 1 < n_inst ? inst_lo[inst + 1] : ~0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < LV_REGS; ++j) {
+            const u32 k = 32 * j + lane;
+            if (k < levels) {
+                rc[j] += lc[k];
+                rd[j] += ld[k];
+            }
+        }
+        for (u32 k = 32 * LV_REGS + lane; k < levels; k += 32) {
+            const u64 at = (u64) inst * stride + 1 + k;
+            atomicAdd(cnt + at, (unsigned long long) lc[k]);
+            if (deg) atomicAdd(deg + at, (unsigned long long) ld[k]);
+        }
+        if (++held == (1u << 16)) flush(cnt, deg, stride, lane);  // 2^16 searches x 2^16 words fit 32 bits
+    }
+};
+
+// ---- searches by eight lanes --------------------------------------------
+//
+// Most searches are thin -- a DAG's levels hold two or three targets -- so a
+// warp runs four at a time, eight lanes each, in lockstep: every pass of the
+// loop takes up to eight frontier rows or eight of their edges per search. An
+// edge record brings its target's row along, so a level costs one dependent
+// global load. Bound by the latency of a pass times the searches the shared
+// memory holds, so a search is packed into 2.8 KB: the visited set is a table of
+// one-byte places in the queue, and a target with one in-edge is not looked up
+// at all (only the node it comes from could have brought it).
+constexpr int CG_THREADS = 64;
+constexpr u32 CG_REACH = 255;      // places 0 .. 254; 255 marks an empty slot
+constexpr u32 CG_HASH = 512;
+constexpr int CG_HASH_SHIFT = 23;  // 32 - log2(CG_HASH)
+constexpr u32 CG_LEVELS = 96;
+constexpr u32 CG_EDGES = 4096;     // join words of one search
+constexpr u32 CG_WIDE = 48;        // a source's or eight rows' edges above which a warp is the better form
+constexpr u64 CG_MAX_EDGES = 1ull << 25;
+constexpr u64 CL_FEW = 8192;       // sources that go to the warps at once
+
+struct CgSmem {
+    unsigned char hash[CG_HASH];
+    u32 qw[CG_REACH + 1];             // targets in visiting order
+    u32 qr[CG_REACH + 1];             // their rows (record format)
+    unsigned short ld[CG_LEVELS];     // join words out of level d at [d - 1]
+    unsigned char lc[CG_LEVELS];      // targets of level d at [d - 1]
+};
+static_assert(sizeof(CgSmem) % 16 == 0, "the table is cleared 16 bytes a lane");
+
+// Edge records, 8 bytes: the target, and its row: first edge (25 bits, from
+// k0), whether it has several in-edges (bit 6), degree (6 bits; 63: wide).
+constexpr u32 ROW_WIDE = 63;
+
+// flags[w - lo]: 1 when w has an in-edge, 3 when it has several.
+__global__ void in_edges_kernel(const u32 *__restrict__ val, u64 k0, u64 k1, u64 lo, u32 *flags) {
+    for (u64 k = k0 + (u64) blockIdx.x * blockDim.x + threadIdx.x; k < k1; k += (u64) gridDim.x * blockDim.x) {
+        u32 *f = flags + (val[k] - lo);
+        if (*reinterpret_cast<volatile u32 *>(f) == 3u) continue;
+        if (atomicOr(f, 1u)) atomicOr(f, 3u);
+    }
+}
+
+__global__ void edge_records_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 k0, u64 k1, u64 lo,
+                                    const u32 *__restrict__ flags, uint2 *__restrict__ rec) {
+    for (u64 k = k0 + (u64) blockIdx.x * blockDim.x + threadIdx.x; k < k1; k += (u64) gridDim.x * blockDim.x) {
+        const u32 w = val[k];
+        const u32 b = off[w], d = off[w + 1] - b;
+        const u32 first = d ? b - (u32) k0 : 0u;  // (a sink's row may lie past the last edge)
+        rec[k - k0] = make_uint2(w, (first << 7) | (flags[w - lo] == 3u ? 64u : 0u) | min(d, ROW_WIDE));
+    }
+}
+
+// Searches from the sources of [lo, hi), `batch` (at most 32) consecutive ones
+// per warp at a time. `rec` holds the records of edges k0 and up.
+__global__ void __launch_bounds__(CG_THREADS)
+closure_group_kernel(const u32 *__restrict__ off, const uint2 *__restrict__ rec, u32 k0, u64 lo, u64 hi, u32 batch,
+                     int bits, const u64 *__restrict__ inst_lo, u32 n_inst, u32 stride, u32 max_level,
+                     unsigned long long *__restrict__ cnt, unsigned long long *__restrict__ deg,
+                     u64 *__restrict__ out, u64 cap, SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const u32 lane = threadIdx.x & 31, l = lane & 7, g8 = lane & 24;
+    CgSmem *const all = reinterpret_cast<CgSmem *>(smem_raw) + (threadIdx.x >> 5) * 4;
+    CgSmem &s = all[lane >> 3];
+    LevelSums sums;
+    sums.init(inst_lo == nullptr, hi);
+    u32 top = 0;
+    // the warp's current batch of sources: first edge and degree in the lanes
+    u64 xb = 0;
+    u32 bb = 0, bd = 0, bm = 0;
+    bool more = true;
+    // the group's search
+    bool act = false, done = true, over = false;
+    u32 x = 0, head = 0, end = 0, tail = 0, level = 0, rp = 0, tot = 0, ip = 0, edges = 0, led = 0;
+    u32 cb = 0, incl = 0, pre = 0;
+    for (;;) {
+        // ---- finished searches: result, next source (one group at a time, all lanes) ----
+        u32 fin = __ballot_sync(0xffffffffu, l == 0 && (done || over));
+        while (fin) {
+            const u32 q = __ffs(fin) - 1;
+            fin &= fin - 1;
+            CgSmem &sq = all[q >> 3];
+            const bool was = __shfl_sync(0xffffffffu, act, q), ov = __shfl_sync(0xffffffffu, over, q);
+            const u32 xq = __shfl_sync(0xffffffffu, x, q), tq = __shfl_sync(0xffffffffu, tail, q);
+            if (was && ov) {
+                if (lane == 0) left[atomicAdd(&ctr->left, 1ull)] = lo + xq;
+            } else if (was) {
+                const u32 lq = __shfl_sync(0xffffffffu, level, q);
+                top = max(top, lq);
+                sums.add(lo + xq, lq, sq.lc, sq.ld, inst_lo, n_inst, cnt, deg, stride, lane);
+                unsigned long long p = 0;
+                if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) tq);
+                p = __shfl_sync(0xffffffffu, p, 0);
+                if (p + tq <= cap)
+                    for (u32 k = lane; k < tq; k += 32) out[p + k] = ((u64) sq.qw[k] << bits) | (lo + xq);
+            }
+            while (bm == 0 && more) {
+                unsigned long long f = 0;
+                if (lane == 0) f = atomicAdd(&ctr->fetch, (unsigned long long) batch);
+                xb = __shfl_sync(0xffffffffu, f, 0);
+                if (lo + xb >= hi) {
+                    more = false;
+                    break;
+                }
+                bb = bd = 0;
+                if (lane < batch && lo + xb + lane < hi) {
+                    bb = __ldg(off + lo + xb + lane);
+                    bd = __ldg(off + lo + xb + lane + 1) - bb;
+                    bb -= k0;
+                }
+                bm = __ballot_sync(0xffffffffu, bd != 0);
+            }
+            const bool mine = g8 == q;
+            if (bm) {
+                const u32 j = __ffs(bm) - 1;
+                bm &= bm - 1;
+                const u32 b = __shfl_sync(0xffffffffu, bb, j), d = __shfl_sync(0xffffffffu, bd, j);
+                reinterpret_cast<uint4 *>(sq.hash)[lane] = make_uint4(EMPTY, EMPTY, EMPTY, EMPTY);
+                if (mine) {  // level 0: one row, the source's
+                    x = (u32) (xb + j);
+                    act = true;
+                    done = false;
+                    over = d > CG_WIDE;
+                    head = end = tail = level = rp = ip = edges = led = 0;
+                    tot = over ? 0 : d;
+                    cb = b;
+                    pre = l == 0 ? 0u : tot;
+                    incl = tot;
+                }
+                if (d > CG_WIDE) fin |= 1u << q;  // handed over at once
+            } else if (mine) {
+                act = false;
+                done = over = false;
+                tot = ip = 0;
+            }
+            __syncwarp();
+        }
+        if (!__any_sync(0xffffffffu, act)) break;
+        // ---- rows: the next eight of the frontier, or the next level ----
+        const bool need = act && ip >= tot;
+        if (__any_sync(0xffffffffu, need)) {
+            u32 d = 0;
+            if (need) {
+                rp += 8;
+                if (rp >= end) {  // the level is expanded
+                    if (level && l == 0) {
+                        s.lc[level - 1] = (unsigned char) (end - head);
+                        s.ld[level - 1] = (unsigned short) led;
+                    }
+                    if (tail == end) {
+                        done = true;
+                    } else {
+                        head = rp = end;
+                        end = tail;
+                        led = 0;
+                        if (++level > CG_LEVELS) {
+                            over = true;
+                        } else if (level == max_level) {
+                            if (l == 0) {
+                                s.lc[level - 1] = (unsigned char) (end - head);
+                                s.ld[level - 1] = 0;
+                            }
+                            done = true;
+                        }
+                    }
+                }
+                ip = tot = 0;
+                if (!done && !over && rp + l < end) {
+                    const u32 r = s.qr[rp + l];
+                    cb = r >> 7;
+                    d = r & 63u;
+                }
+            }
+            u32 v = d;
+#pragma unroll
+            for (u32 o = 1; o < 8; o <<= 1) {
+                const u32 y = __shfl_up_sync(0xffffffffu, v, o, 8);
+                if (l >= o) v += y;
+            }
+            const u32 t = __shfl_sync(0xffffffffu, v, 7, 8);
+            if (need && !done && !over) {
+                incl = v;
+                pre = v - d;
+                tot = t;
+                if (t > CG_WIDE || edges + t > CG_EDGES) over = true;
+            }
+        }
+        // ---- edges: eight of the rows' ----
+        const u32 p = ip + l;
+        const bool have = act && !done && !over && p < tot;
+        u32 o = 0;
+        if (__shfl_sync(0xffffffffu, incl, 3, 8) <= p) o = 4;
+        if (__shfl_sync(0xffffffffu, incl, o + 1, 8) <= p) o += 2;
+        if (__shfl_sync(0xffffffffu, incl, o, 8) <= p) o += 1;
+        const u32 at = __shfl_sync(0xffffffffu, cb, o, 8) + (p - __shfl_sync(0xffffffffu, pre, o, 8));
+        uint2 r = make_uint2(0, 0);
+        if (have) r = __ldg(rec + at);
+        // New targets take places in the queue: those with one in-edge at
+        // once, the others when the table does not hold them.
+        bool fresh = have && !(r.y & 64u), look = have && (r.y & 64u);
+        // a source that reaches itself would bring its targets a second time
+        const bool bad = have && (r.x == (u32) lo + x || (r.y & 63u) == ROW_WIDE);
+        if (((__ballot_sync(0xffffffffu, bad) >> g8) & 0xFFu) != 0) {
+            over = true;
+            fresh = look = false;
+        }
+        u32 slot = 0;
+        bool put = false;  // this round's new one goes into the table
+        for (u32 h = hash_slot(r.x, CG_HASH_SHIFT);;) {
+            const u32 gm = (__ballot_sync(0xffffffffu, fresh) >> g8) & 0xFFu;
+            const u32 n = __popc(gm);
+            if (tail + n > CG_REACH) {
+                over = true;
+                fresh = look = put = false;
+            }
+            if (fresh) {
+                const u32 k = tail + __popc(gm & ((1u << l) - 1));
+                s.qw[k] = r.x;
+                s.qr[k] = r.y;
+                if (put) s.hash[slot] = (unsigned char) k;
+            }
+            if (!over) tail += n;
+            fresh = put = false;
+            __syncwarp();
+            if (!__any_sync(0xffffffffu, look)) break;
+            // a step of the probe: found, occupied by another, or empty: then the
+            // lanes that want the slot write their number and the one that stays has it
+            const u32 e = look ? s.hash[h] : 0u;
+            const bool empty = look && e == 255u;
+            if (look && !empty) {
+                if (s.qw[e] == r.x) look = false;
+                else h = (h + 1) & (CG_HASH - 1);
+            }
+            __syncwarp();
+            if (empty) s.hash[h] = (unsigned char) l;
+            __syncwarp();
+            const u32 win = empty ? s.hash[h] : l;
+            const u32 ww = __shfl_sync(0xffffffffu, r.x, win, 8);
+            __syncwarp();
+            if (empty) {
+                if (win == l) {
+                    fresh = put = true;
+                    slot = h;
+                    look = false;
+                } else if (ww == r.x) {
+                    look = false;
+                }
+            }
+        }
+        if (act && !done && !over) {
+            edges += min(8u, tot - ip);
+            led += min(8u, tot - ip);
+            ip += 8;
+        }
+    }
+    sums.flush(cnt, deg, stride, lane);
+    if (lane == 0 && top) atomicMax(&ctr->levels, (unsigned long long) top);
+}
+
+// ---- searches by a warp -------------------------------------------------
+
+constexpr int CW_THREADS = 64;
+constexpr u32 CW_REACH = 1024;
+constexpr u32 CW_HASH = 2 * CW_REACH;
+constexpr int CW_HASH_SHIFT = 21;     // 32 - log2(CW_HASH)
+constexpr u32 CW_LEVELS = 512;
+constexpr u32 CW_EDGES = 16384;       // join words of one search
+
+struct CwSmem {
+    u32 hash[CW_HASH];
+    u32 queue[CW_REACH];
+    unsigned short lcnt[CW_LEVELS];   // targets of level d at [d - 1]
+    unsigned short ldeg[CW_LEVELS];   // join words out of level d at [d - 1]
+    u32 wbeg[32], wpre[32];           // compacted rows of the group being expanded
+};
 
 // Walks the edge targets of up to 32 rows (beg, deg of this lane's row; deg 0:
 // none) in windows of 32: f(w, have) per window, all lanes; f returns false
@@ -120,59 +442,31 @@ __device__ __forceinline__ u32 walk_rows(u32 *wbeg, u32 *wpre, u32 beg, u32 deg,
     return total;
 }
 
-// One search per warp at a time; persistent warps take `group` consecutive
-// sources of [lo, hi) at a time. A search that outgrows its slice goes to `left`.
-// Level sizes are kept per search and added when it finishes: levels up to
-// 128 in lane registers (lane l holds levels 32 j + l + 1), flushed to the
-// instance's counters when the instance changes, the rest directly.
+// The same search by a warp, for the sources eight lanes' slice could not
+// hold (src; null: every rank from lo on). A search that outgrows its slice goes to
+// `left`.
 __global__ void __launch_bounds__(CW_THREADS)
-closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 lo, u64 hi, u32 group, int bits,
-                    const u64 *__restrict__ inst_lo, u32 n_inst, u32 stride, u32 max_level,
+closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, const u64 *__restrict__ src, u64 lo,
+                    u64 n_src, int bits, const u64 *__restrict__ inst_lo, u32 n_inst, u32 stride, u32 max_level,
                     unsigned long long *__restrict__ cnt, unsigned long long *__restrict__ deg,
-                    u64 *__restrict__ out, u64 cap,
-                    SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
+                    u64 *__restrict__ out, u64 cap, SearchCounters *__restrict__ ctr, u64 *__restrict__ left) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CwSmem &s = reinterpret_cast<CwSmem *>(smem_raw)[threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31;
     const u32 lt = lanemask_lt();
     const u32 le = lane == 31 ? ~0u : (2u << lane) - 1;
-    u32 rc[CW_REGS], rd[CW_REGS];
-#pragma unroll
-    for (int j = 0; j < CW_REGS; ++j) rc[j] = rd[j] = 0;
-    u32 held = 0;           // searches summed in rc / rd
+    LevelSums sums;
+    sums.init(inst_lo == nullptr, 0);
     u32 top = 0;            // largest level seen
-    u32 inst = 0;
-    u64 inst_end = inst_lo ? 0 : hi;  // first rank after the current instance
-    auto flush = [&]() {
-        const u64 at = (u64) inst * stride + 1 + lane;
-#pragma unroll
-        for (int j = 0; j < CW_REGS; ++j) {
-            if (rc[j]) atomicAdd(cnt + at + 32 * j, (unsigned long long) rc[j]);
-            if (deg && rd[j]) atomicAdd(deg + at + 32 * j, (unsigned long long) rd[j]);
-            rc[j] = rd[j] = 0;
-        }
-        held = 0;
-    };
     for (;;) {
         unsigned long long g = 0;
-        if (lane == 0) g = atomicAdd(&ctr->fetch, (unsigned long long) group);
+        if (lane == 0) g = atomicAdd(&ctr->fetch, 1ull);
         g = __shfl_sync(0xffffffffu, g, 0);
-        if (lo + g >= hi) break;
-        const u64 xe = min(hi, (u64) (lo + g + group));
-        for (u64 x = lo + g; x < xe; ++x) {
+        if (g >= n_src) break;
+        {
+            const u64 x = src ? src[g] : lo + g;
             const u32 b0 = __ldg(off + x), d0 = __ldg(off + x + 1) - b0;
             if (d0 == 0) continue;
-            if (x >= inst_end) {  // another instance: its range by binary search
-                flush();
-                u32 a = 0, b = n_inst;
-                while (a < b) {
-                    const u32 m = (a + b) >> 1;
-                    if (inst_lo[m] <= x) a = m + 1;
-                    else b = m;
-                }
-                inst = a - 1;
-                inst_end = a < n_inst ? inst_lo[a] : hi;
-            }
             // visited set empty
             uint4 *hv = reinterpret_cast<uint4 *>(s.hash);
 #pragma unroll
@@ -233,20 +527,7 @@ closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u6
             }
             // level sizes
             top = max(top, level);
-#pragma unroll
-            for (int j = 0; j < CW_REGS; ++j) {
-                const u32 k = 32 * j + lane;
-                if (k < level) {
-                    rc[j] += s.lcnt[k];
-                    rd[j] += s.ldeg[k];
-                }
-            }
-            for (u32 k = 32 * CW_REGS + lane; k < level; k += 32) {
-                const u64 at = (u64) inst * stride + 1 + k;
-                atomicAdd(cnt + at, (unsigned long long) s.lcnt[k]);
-                if (deg) atomicAdd(deg + at, (unsigned long long) s.ldeg[k]);
-            }
-            if (++held == (1u << 18)) flush();  // 2^18 searches x 8192 words stay below 2^32
+            sums.add(x, level, s.lcnt, s.ldeg, inst_lo, n_inst, cnt, deg, stride, lane);
             // result words
             unsigned long long p = 0;
             if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) tail);
@@ -256,7 +537,7 @@ closure_warp_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u6
             __syncwarp();
         }
     }
-    flush();
+    sums.flush(cnt, deg, stride, lane);
     if (lane == 0 && top) atomicMax(&ctr->levels, (unsigned long long) top);
 }
 
@@ -368,16 +649,7 @@ closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, con
             continue;
         }
         const u32 tail = s.tail;
-        u32 inst = 0;
-        if (inst_lo) {
-            u32 a = 0, b = n_inst;
-            while (a < b) {
-                const u32 m = (a + b) >> 1;
-                if (inst_lo[m] <= x) a = m + 1;
-                else b = m;
-            }
-            inst = a - 1;
-        }
+        const u32 inst = inst_lo ? instance_at(inst_lo, n_inst, x) : 0;
         for (u32 k = tid; k < level; k += CC_THREADS) {
             const u64 at = (u64) inst * stride + 1 + k;
             atomicAdd(cnt + at, (unsigned long long) lcnt[k]);
@@ -920,92 +1192,118 @@ void grow_keeping(Context &ctx, DevBuf &buf, u64 bytes, u64 keep) {
 }  // namespace
 
 ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
-                            u64 stride, u64 max_level, u64 *cnt, u64 *deg) {
+                            u64 k0, u64 k1, u64 stride, u64 max_level, u64 *cnt, u64 *deg) {
     Workspace &ws = ctx.ws;
     ClosureLight res;
     const u64 ns = hi - lo;
     if (ns == 0) return res;
     const u64 table = n_inst * stride * 8;
     const u32 ml = (u32) std::min<u64>(max_level, 0xFFFFFFFFull);
-    auto *c = reinterpret_cast<unsigned long long *>(cnt), *d = reinterpret_cast<unsigned long long *>(deg);
+    DL_CUDA(cudaMemsetAsync(cnt, 0, table, ctx.stream));
+    if (deg) DL_CUDA(cudaMemsetAsync(deg, 0, table, ctx.stream));
+    ctx.reserve(ws.cl_levels, 2 * table);
+    auto *c2 = ws.cl_levels.as<unsigned long long>();
+    auto *d2 = c2 + table / 8;
     SearchCounters *ctr = reinterpret_cast<SearchCounters *>(&ctx.ctrl->scalar[40]);
     ctx.reserve(ws.cl_left, ns * 8);
     DevBuf &out = ws.jbuf[0];
-    // room for 96 targets a source at first; a run that needs more is repeated with the room it asked for
+    // room for 96 targets a source at first; a launch that needs more is repeated with the room it asked for
     ctx.reserve(out, std::max<u64>(96 * ns, 1 << 16) * 8);
-    const size_t smem = sizeof(CwSmem) * (CW_THREADS / 32);
-    const u64 wave = resident_blocks(ctx, closure_warp_kernel, CW_THREADS, smem);
-    const u32 group = (u32) std::max<u64>(1, std::min<u64>(8, ns / (wave * (CW_THREADS / 32) * 4)));
-    const unsigned grid =
-        (unsigned) std::max<u64>(1, std::min<u64>(wave, (ns + group * (CW_THREADS / 32) - 1) / (group * (CW_THREADS / 32))));
     SearchCounters got{};
-    auto read_back = [&]() {
-        DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctr, sizeof(got), cudaMemcpyDeviceToHost, ctx.stream));
-        ctx.sync();
-        got.words = ctx.host_scalars[1];
-        got.left = ctx.host_scalars[2];
-        got.levels = ctx.host_scalars[3];
+    // One stage: `launch(table, table2, room)` with zeroed counters; repeated when its words outgrow the room.
+    // Its level counts are added to cnt / deg when it went through.
+    auto stage = [&](auto launch) {
+        for (;;) {
+            DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
+            DL_CUDA(cudaMemsetAsync(c2, 0, 2 * table, ctx.stream));
+            const u64 room = out.cap / 8 - res.n_words;
+            launch(out.as<u64>() + res.n_words, room);
+            DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctr, sizeof(got), cudaMemcpyDeviceToHost, ctx.stream));
+            ctx.sync();
+            got.words = ctx.host_scalars[1];
+            got.left = ctx.host_scalars[2];
+            got.levels = ctx.host_scalars[3];
+            if (got.words <= room) break;
+            grow_keeping(ctx, out, (res.n_words + got.words) * 8, res.n_words * 8);
+        }
+        ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
+        res.n_words += got.words;
+        res.levels = (u32) std::max<u64>(res.levels, got.levels);
+        if (got.words) {
+            const unsigned ag = grid_for(table / 8, T256, ctx);
+            DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, table / 8));
+            if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, table / 8));
+        }
     };
-    for (;;) {
-        DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
-        DL_CUDA(cudaMemsetAsync(cnt, 0, table, ctx.stream));
-        if (deg) DL_CUDA(cudaMemsetAsync(deg, 0, table, ctx.stream));
-        const u64 cap = out.cap / 8;
-        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * ns,
-                  closure_warp_kernel<<<grid, CW_THREADS, smem, ctx.stream>>>(
-                      csr.off, csr.val, lo, hi, group, bits, inst_lo, (u32) n_inst, (u32) stride, ml, c, d, out.as<u64>(), cap, ctr,
-                      ws.cl_left.as<u64>()));
-        read_back();
-        if (got.words <= cap) break;
-        ctx.reserve(out, got.words * 8);
+    // Few sources go to the warps at once: one launch and one wait instead of two
+    // (3.6K sources of a 5.5K-edge DAG: 0.78 -> 0.67 ms for the whole run).
+    const bool groups = ns > CL_FEW && k1 - k0 < CG_MAX_EDGES;
+    u64 nl = ns;
+    if (groups) {
+        const u64 m = k1 - k0;
+        ctx.reserve(ws.cl_rec, std::max<u64>(m, 1) * 8);
+        ctx.reserve(ws.cl_act, ns * 4);
+        DL_CUDA(cudaMemsetAsync(ws.cl_act.p, 0, ns * 4, ctx.stream));
+        DL_LAUNCH(ctx, K_PREP, 8.0 * m,
+                  in_edges_kernel<<<grid_for(m, T256, ctx), T256, 0, ctx.stream>>>(csr.val, k0, k1, lo,
+                                                                                  ws.cl_act.as<u32>()));
+        DL_LAUNCH(ctx, K_PREP, 24.0 * m,
+                  edge_records_kernel<<<grid_for(m, T256, ctx), T256, 0, ctx.stream>>>(
+                      csr.off, csr.val, k0, k1, lo, ws.cl_act.as<u32>(), ws.cl_rec.as<uint2>()));
+        const size_t smem_g = sizeof(CgSmem) * (CG_THREADS / 8);
+        const u64 wave_g = resident_blocks(ctx, closure_group_kernel, CG_THREADS, smem_g);
+        const u64 warps_g = wave_g * (CG_THREADS / 32);
+        const u32 batch = (u32) std::max<u64>(4, std::min<u64>(32, ns / (warps_g * 4)));
+        const unsigned grid_g = (unsigned) std::max<u64>(
+            1, std::min<u64>(wave_g, (ns + batch * (CG_THREADS / 32) - 1) / (batch * (CG_THREADS / 32))));
+        stage([&](u64 *to, u64 room) {
+            DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * ns,
+                      closure_group_kernel<<<grid_g, CG_THREADS, smem_g, ctx.stream>>>(
+                          csr.off, ws.cl_rec.as<uint2>(), (u32) k0, lo, hi, batch, bits, inst_lo, (u32) n_inst,
+                          (u32) stride, ml, c2, deg ? d2 : nullptr, to, room, ctr, ws.cl_left.as<u64>()));
+        });
+        if (got.left == 0) return res;
+        nl = got.left;
     }
-    ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
-    res.n_words = got.words;
-    res.levels = (u32) got.levels;
+    ctx.reserve(ws.cl_heavy, nl * 8);
+    grow_keeping(ctx, out, (res.n_words + std::min<u64>(nl * 512, 1ull << 27)) * 8, res.n_words * 8);
+    const size_t smem_w = sizeof(CwSmem) * (CW_THREADS / 32);
+    const u64 wave_w = resident_blocks(ctx, closure_warp_kernel, CW_THREADS, smem_w);
+    const unsigned grid_w = (unsigned) std::min<u64>(wave_w, (nl + CW_THREADS / 32 - 1) / (CW_THREADS / 32));
+    stage([&](u64 *to, u64 room) {
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * nl,
+                  closure_warp_kernel<<<grid_w, CW_THREADS, smem_w, ctx.stream>>>(
+                      csr.off, csr.val, groups ? ws.cl_left.as<u64>() : nullptr, lo, nl, bits, inst_lo, (u32) n_inst,
+                      (u32) stride, ml, c2, deg ? d2 : nullptr, to, room, ctr, ws.cl_heavy.as<u64>()));
+    });
     if (got.left == 0) return res;
     // What the warps left over: CTA searches, unless there are so many that
     // bit rows are the cheaper form. A CTA search that fails has cost up to
     // `reach` targets' edges; 10^8 of them are about a millisecond.
-    const u64 nl = got.left, levels_w = res.levels;
+    nl = got.left;
     const double mean_deg = std::max(1.0, (double) csr.n_vals / std::max<u64>(csr.n_keys, 1));
     u32 reach = CC_REACH;
     if (!inst_lo) {
         const double fit = 1e8 / (mean_deg * (double) nl);
         if (fit < CC_REACH) reach = (u32) fit;
-        if (reach < 2 * CW_REACH) reach = 0;
+        if (reach < CW_REACH + CW_REACH / 2) reach = 0;
     }
-    ctx.reserve(ws.cl_heavy, nl * 8);
     if (reach == 0) {
-        DL_CUDA(cudaMemcpyAsync(ws.cl_heavy.p, ws.cl_left.p, nl * 8, cudaMemcpyDeviceToDevice, ctx.stream));
         res.n_heavy = nl;
         return res;
     }
-    ctx.reserve(ws.cl_levels, 2 * table);  // their level counts apart: a run that outgrows the room is repeated
-    auto *c2 = ws.cl_levels.as<unsigned long long>();
-    auto *d2 = c2 + table / 8;
-    const u64 wave2 = resident_blocks(ctx, closure_cta_kernel, CC_THREADS, sizeof(CcSmem));
-    const unsigned grid2 = (unsigned) std::min<u64>(wave2, nl);
-    ctx.reserve(ws.cl_act, (u64) grid2 * 2 * CL_LEVELS * 4);
-    grow_keeping(ctx, out, (res.n_words + std::min<u64>(nl * 1024, 1ull << 28)) * 8, res.n_words * 8);
-    for (;;) {
-        DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
-        DL_CUDA(cudaMemsetAsync(c2, 0, 2 * table, ctx.stream));
-        const u64 cap = out.cap / 8 - res.n_words;
+    std::swap(ws.cl_left, ws.cl_heavy);  // the sources to search are now in cl_left
+    const u64 wave_c = resident_blocks(ctx, closure_cta_kernel, CC_THREADS, sizeof(CcSmem));
+    const unsigned grid_c = (unsigned) std::min<u64>(wave_c, nl);
+    ctx.reserve(ws.cl_heavy, nl * 8);
+    ctx.reserve(ws.cl_act, (u64) grid_c * 2 * CL_LEVELS * 4);
+    grow_keeping(ctx, out, (res.n_words + std::min<u64>(nl * 2048, 1ull << 27)) * 8, res.n_words * 8);
+    stage([&](u64 *to, u64 room) {
         DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * nl,
-                  closure_cta_kernel<<<grid2, CC_THREADS, sizeof(CcSmem), ctx.stream>>>(
-                      csr.off, csr.val, ws.cl_left.as<u64>(), nl, reach, bits, inst_lo, (u32) n_inst, (u32) stride, ml, c2,
-                      deg ? d2 : nullptr, ws.cl_act.as<u32>(), out.as<u64>() + res.n_words, cap, ctr,
-                      ws.cl_heavy.as<u64>()));
-        read_back();
-        if (got.words <= cap) break;
-        grow_keeping(ctx, out, (res.n_words + got.words) * 8, res.n_words * 8);
-    }
-    ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
-    const unsigned ag = grid_for(table / 8, T256, ctx);
-    DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, table / 8));
-    if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, table / 8));
-    res.n_words += got.words;
-    res.levels = (u32) std::max<u64>(levels_w, got.levels);
+                  closure_cta_kernel<<<grid_c, CC_THREADS, sizeof(CcSmem), ctx.stream>>>(
+                      csr.off, csr.val, ws.cl_left.as<u64>(), nl, reach, bits, inst_lo, (u32) n_inst, (u32) stride, ml,
+                      c2, deg ? d2 : nullptr, ws.cl_act.as<u32>(), to, room, ctr, ws.cl_heavy.as<u64>()));
+    });
     res.n_heavy = got.left;
     return res;
 }
@@ -1207,7 +1505,8 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
     pt.mark(PH_JOIN);
     ctx.reserve(ws.offsets, 2 * (CL_LEVELS + 1) * 8);
     u64 *cnt = ws.offsets.as<u64>(), *deg = cnt + CL_LEVELS + 1;
-    ClosureLight light = closure_search(ctx, g.csr, 0, n, g.bits, nullptr, 1, CL_LEVELS + 1, max_level, cnt, deg);
+    ClosureLight light = closure_search(ctx, g.csr, 0, n, g.bits, nullptr, 1, 0, ne, CL_LEVELS + 1,
+                                       max_level, cnt, deg);
     if (light.n_heavy) {
         const u64 need = closure_pull_bytes(n, light.n_heavy);
         if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;

@@ -21,11 +21,12 @@ struct ClosureLight {
 // cnt[instance * stride + d] (and the sum of the out-degrees of the level's
 // targets to deg[...] when not null), instance k being the last one whose first
 // rank inst_lo[k] is at most the source (one instance when inst_lo is null);
+// [k0, k1): the sources' edges and all edges that can be reached from them;
 // stride: above the levels an instance can have, or CL_LEVELS + 1. Sources
 // whose reach or work outgrows the searches' shared memory are left over for
 // the caller. max_level: 0 = no limit.
 ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
-                            u64 stride, u64 max_level, u64 *cnt, u64 *deg);
+                            u64 k0, u64 k1, u64 stride, u64 max_level, u64 *cnt, u64 *deg);
 
 // The closure of `h` heavy sources (ascending ranks `src`, device) over ranks
 // [0, n) as bit rows: bit c of row z of `t` is set when source c reaches z.

@@ -115,7 +115,8 @@ struct Workspace {
     DevBuf bitmat[2];      // full relation as a bit matrix; TC's column offsets of the result rows
     DevBuf bit_hasout;     // bit-matrix TC: nodes with out-edges (one bit each)
     // TC by searches (dl_closure.cu)
-    DevBuf cl_left, cl_heavy;   // sources a warp's / a CTA's search could not hold
+    DevBuf cl_rec;              // edge records (target, its first edge, its degree)
+    DevBuf cl_left, cl_heavy;   // sources a search could not hold
     DevBuf cl_levels;           // level counts
     DevBuf cl_roff, cl_rval;    // in-neighbours of every node
     DevBuf cl_segs, cl_hub_at, cl_hub_acc;  // targets with many in-neighbours

@@ -313,6 +313,7 @@ struct SessionImpl {
     std::vector<i64> active;    // instance ids in rank order
     std::vector<i64> finished;  // finished since the last poll
     std::vector<i64> pending;   // TC: admitted since the last step, not searched yet
+    u64 pending_vals = 0;       // their first edge
     bool inst_dirty = true;
 };
 
@@ -714,8 +715,8 @@ void search_pending(SessionImpl &s) {
     csr.val = s.val.as<u32>();
     csr.n_keys = (u32) s.next_rank;
     csr.n_vals = s.n_vals;
-    const ClosureLight light = closure_search(ctx, csr, first, end, s.bits, s.range_lo.as<u64>(), ni, stride,
-                                              max_level, s.counts.as<u64>(), nullptr);
+    const ClosureLight light = closure_search(ctx, csr, first, end, s.bits, s.range_lo.as<u64>(), ni, s.pending_vals,
+                                              s.n_vals, stride, max_level, s.counts.as<u64>(), nullptr);
     const u64 width = light.levels + 1;
     std::vector<u64> hc(ni * width, 0);
     if (light.levels)
@@ -902,7 +903,7 @@ void session_destroy(SessionImpl *s) {
                        &w.sample,   &w.sample_small, &w.jbuf[0],
                        &w.jbuf[1],  &w.offsets,  &w.wcc_label, &w.wcc_flag, &w.wcc_next,
                        &w.cl_left,  &w.cl_heavy, &w.cl_levels, &w.cl_roff,  &w.cl_rval, &w.cl_segs,
-                       &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act};
+                       &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec};
     for (DevBuf *b : wbufs) p.give_back(*b);
     for (auto &b : c.spares) p.give_back(b);
     c.spares.clear();
@@ -974,6 +975,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
                   session_ids_kernel<<<grid_for(nu, 256, ctx, 16), 256, 0, ctx.stream>>>(u, nu, block->as<int32_t>()));
         // rows -> rank words; the edge relation keyed by source (tc.cu:171-176,
         // sg.cu:150-153, wcc.cu:140-167: WCC stores both directions)
+        if (tc && s.pending.empty()) s.pending_vals = s.n_vals;
         const int bits = s.bits;
         const bool wcc = s.program == DL_PROGRAM_WCC;
         u64 *fw = wo.as<u64>();
@@ -1178,7 +1180,7 @@ u64 session_device_bytes(const SessionImpl &s) {
                             &w.sample,  &w.sample_small, &w.jbuf[0],
                             &w.jbuf[1], &w.offsets,   &c.lookback, &c.radix_part, &c.lbs_splits, &c.sort_hist,
                             &c.merge_splits, &w.cl_left, &w.cl_heavy, &w.cl_levels, &w.cl_roff, &w.cl_rval, &w.cl_segs,
-                            &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act};
+                            &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec};
     for (const DevBuf *x : bufs) b += x->cap;  // cached spare buffers are not counted: they are free memory
     std::vector<const DevBuf *> blocks;
     for (const auto &in : s.inst)
