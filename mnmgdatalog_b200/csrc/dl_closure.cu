@@ -1073,20 +1073,28 @@ __global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u
 // Result rows (x, z) of targets [z0, z1), by (z, x): the set bits of row z of
 // T (ascending columns = ascending sources) merged with z's light pairs
 // (ascending sources; one comes before the heavy sources at columns
-// place[source] and up). A warp keeps one chunk of 1024 columns (their node ids
-// in 32 registers) and walks targets; where a target's rows of that chunk go
-// is known from closure_counts_kernel, so chunks and targets are independent.
-// In a chunk, a word's first position comes from a prefix sum over the words
-// plus the light pairs before it; then a lane per bit of a word, whose rows
-// leave as consecutive 8-byte stores (ten instructions a word: with the ids
-// loaded per word it was bound by issue, 40 a word). Light pairs are placed
-// lane-parallel; a word that one falls inside is done last, its lanes shifted
-// by the light pairs below them.
+// place[source] and up). A warp walks the targets of one chunk of 1024 columns;
+// where a target's rows of that chunk go is known from the counts, so chunks and
+// targets are independent. In a chunk, a word's first position comes from a
+// prefix sum over the words plus the light pairs before it. Then
+//  * DENSE (a third of the bits set or more): a lane per bit of a word, whose rows
+//    leave as consecutive 8-byte stores, the columns' node ids in 32 registers
+//    (ten instructions a word: with the ids loaded per word it was bound by
+//    issue, 40 a word);
+//  * else a lane per word walks its bits into shared memory, and the chunk's rows
+//    leave with consecutive stores.
+// Light pairs are placed lane-parallel; a word that one falls inside is done
+// last, its lanes shifted by the light pairs below them.
+constexpr u32 ROWS_STAGE = 384;  // a sparse chunk's staged rows
+
+template <bool DENSE>
 __global__ void __launch_bounds__(256)
 closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict__ cols,
                     const u32 *__restrict__ place, const uint2 *__restrict__ start, u64 z0, u64 z1,
                     const u64 *__restrict__ first, const u64 *__restrict__ light, const u64 *__restrict__ loff,
                     u64 mask, const int32_t *__restrict__ ids, bool affine, int32_t base, u64 *__restrict__ out) {
+    __shared__ u32 staged[DENSE ? 1 : 8][ROWS_STAGE];
+    u32 *stage = staged[DENSE ? 0 : threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31;
     const u32 lt = lanemask_lt();
     const u32 chunks = words / 32;
@@ -1100,11 +1108,13 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
         if (me / chunks >= step) break;  // warps beyond a whole number of rounds
         const u32 k0 = (u32) c0 * 32;
         const u32 *cc = cols + c0 * 1024;
-        u32 id[32];
+        u32 id[DENSE ? 32 : 1];
+        if constexpr (DENSE) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const u32 x = __ldg(cc + j * 32 + lane);
-            id[j] = x == EMPTY ? 0u : node(x);
+            for (int j = 0; j < 32; ++j) {
+                const u32 x = __ldg(cc + j * 32 + lane);
+                id[j] = x == EMPTY ? 0u : node(x);
+            }
         }
         for (u64 z = z0 + me / chunks; z < z1; z += step) {
             u32 v = t[z * words + k0 + lane];
@@ -1117,6 +1127,16 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             const u32 n = __popc(v);
             const u32 incl = warp_inclusive_sum(n);
             u32 at = incl - n;
+            if constexpr (!DENSE) {
+                const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+                if (st.y == lend && total <= ROWS_STAGE) {
+                    for (; v; v &= v - 1) stage[at++] = node(__ldg(cc + lane * 32 + __ffs(v) - 1));
+                    __syncwarp();
+                    for (u32 i = lane; i < total; i += 32) dst[i] = zid | stage[i];
+                    __syncwarp();
+                    continue;
+                }
+            }
             u32 inside = 0;
             const u64 *lz = light + loff[z];
             // light pairs st.y .. lend - 1: one in word j before bit b
@@ -1151,7 +1171,11 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             for (int j = 0; j < 32; ++j) {
                 const u32 word = __shfl_sync(0xffffffffu, v, j);
                 const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
-                if ((word >> lane) & 1u) dst[p] = zid | id[j];
+                if constexpr (DENSE) {
+                    if ((word >> lane) & 1u) dst[p] = zid | id[j];
+                } else {
+                    if ((word >> lane) & 1u) dst[p] = zid | node(__ldg(cc + j * 32 + lane));
+                }
             }
             while (slow) {
                 const u32 j = __ffs(slow) - 1;
@@ -1435,6 +1459,25 @@ ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne
     return res;
 }
 
+u64 bit_rows_finish(Context &ctx, Run &r, u64 n, u64 words, const u64 *counts) {
+    ctx.reserve(r.bm_first, (n + 1) * 8);
+    const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    u64 *lb = ctx.lookback_words(tiles);
+    u32 *tc = ctx.tile_counter(62);
+    u64 *tot = &ctx.ctrl->scalar[49];
+    DL_CUDA(cudaMemsetAsync(tc, 0, sizeof(u32), ctx.stream));
+    DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 16.0 * n,
+              scan_kernel<SumValue><<<(unsigned) tiles, SCAN_THREADS, 0, ctx.stream>>>(
+                  SumValue{counts}, n, r.bm_first.as<u64>(), lb, tc, ctx.next_epoch(), &ctx.ctrl->err, tot));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, tot, sizeof(u64), cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    r.from_bitmat = true;
+    r.cl_rows = true;
+    r.bm_n = n;
+    r.bm_stride = r.bm_words = words;
+    return ctx.host_scalars[0];
+}
+
 void closure_heavy_words(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const std::vector<u64> &src,
                          u64 max_level, std::vector<u64> &cnt, u64 &n_words) {
     Workspace &ws = ctx.ws;
@@ -1562,28 +1605,14 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
                   key_offsets_kernel<u64><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(
                       r.words.as<u64>(), light.n_words, g.bits, n, r.cl_loff.as<u64>()));
         ctx.reserve(ws.w0, (n + 1) * 8);
-        ctx.reserve(r.bm_first, (n + 1) * 8);
         DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n * heavy.words,
                   closure_counts_kernel<<<grid_for(n * 32, T256, ctx), T256, 0, ctx.stream>>>(
                       r.bm_t.as<u32>(), n, (u32) heavy.words, r.words.as<u64>(), r.cl_loff.as<u64>(),
                       (1ull << g.bits) - 1, place, r.cl_start.as<uint2>(), ws.w0.as<u64>()));
-        const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-        u64 *lb = ctx.lookback_words(tiles);
-        u32 *tc = ctx.tile_counter(62);
-        u64 *tot = &ctx.ctrl->scalar[49];
-        DL_CUDA(cudaMemsetAsync(tc, 0, sizeof(u32), ctx.stream));
-        DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 16.0 * n,
-                  scan_kernel<SumValue><<<(unsigned) tiles, SCAN_THREADS, 0, ctx.stream>>>(
-                      SumValue{ws.w0.as<u64>()}, n, r.bm_first.as<u64>(), lb, tc, ctx.next_epoch(), &ctx.ctrl->err, tot));
-        DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, tot, sizeof(u64), cudaMemcpyDeviceToHost, ctx.stream));
-        ctx.sync();
-        if (ctx.host_scalars[0] != nfull)
-            throw Error(DL_ERR_INTERNAL, "closure holds " + std::to_string(ctx.host_scalars[0]) + " tuples, expected " +
+        const u64 total = bit_rows_finish(ctx, r, n, heavy.words, ws.w0.as<u64>());
+        if (total != nfull)
+            throw Error(DL_ERR_INTERNAL, "closure holds " + std::to_string(total) + " tuples, expected " +
                                              std::to_string(nfull));
-        r.from_bitmat = true;
-        r.cl_rows = true;
-        r.bm_n = n;
-        r.bm_stride = r.bm_words = heavy.words;
     } else {
         pt.mark(PH_FINAL);
         ctx.sync();  // hc, hd are host memory
@@ -1629,15 +1658,17 @@ bool tc_closure(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, 
 
 void closure_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 z0, u64 z1) {
     using namespace detail;
-    const u64 wave = resident_blocks(ctx, closure_rows_kernel, 256, 0);
     const u32 *cols = r.cl_cols.as<u32>();
     const u64 chunks = r.bm_words / 32;
+    const bool dense = (u64) r.info.output_rows >= r.bm_n * r.bm_words * 32 / 3;
+    auto kern = dense ? closure_rows_kernel<true> : closure_rows_kernel<false>;
+    const u64 wave = resident_blocks(ctx, kern, 256, 0);
     const unsigned grid = (unsigned) std::max<u64>(1, std::min<u64>(wave, ((z1 - z0) * chunks + 7) / 8));
     DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * (z1 - z0) * r.bm_words,
-              closure_rows_kernel<<<grid, 256, 0, ctx.stream>>>(
+              kern<<<grid, 256, 0, ctx.stream>>>(
                   r.bm_t.as<u32>(), (u32) r.bm_words, cols, cols + r.bm_words * 32, r.cl_start.as<uint2>(), z0, z1,
-                  r.bm_first.as<u64>(), r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << r.bits) - 1, r.ids.as<int32_t>(), r.ids_affine, r.id_base,
-                  reinterpret_cast<u64 *>(out)));
+                  r.bm_first.as<u64>(), r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << r.bits) - 1,
+                  r.ids.as<int32_t>(), r.ids_affine, r.id_base, reinterpret_cast<u64 *>(out)));
 }
 
 }  // namespace dl

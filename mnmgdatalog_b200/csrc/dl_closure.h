@@ -42,12 +42,25 @@ u64 closure_pull_bytes(u64 n, u64 h);
 ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne, int bits, u64 n, const u64 *src,
                           u64 h, u64 max_level, DevBuf &t, DevBuf &cols);
 
+// The result of a run as bit rows (r.bm_t, r.cl_cols, r.cl_start, the light
+// pairs in r.words / r.cl_loff): first row of every target from the targets'
+// row counts; returns the number of rows.
+u64 bit_rows_finish(Context &ctx, Run &r, u64 n, u64 words, const u64 *counts);
+
 // The pairs of heavy sources `src` (ascending, host) of one instance with ranks
 // [lo, hi) of the CSR: appended as (z << bits) | x words to ws.jbuf[0] (n_words
 // of it are kept and counted on), their levels added to cnt (index d, grown as
 // needed).
 void closure_heavy_words(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const std::vector<u64> &src,
                          u64 max_level, std::vector<u64> &cnt, u64 &n_words);
+
+// single_join (dl_selfjoin.cu): rows (x, z) with x -> b -> z for some b, over the
+// in-neighbour CSR (off[z]: the y with y -> z), as bit rows; `total`: join rows
+// before dedup. False (nothing done) when the bit rows are not worth it or do
+// not fit; the join and the sort of its output are the better form then.
+bool self_join_rows(Context &ctx, Run &r, const Csr &in, u64 total, PhaseTimer &pt, u64 &rows);
+// Sum over the edges y -> z of y's in-degree: the join rows of the self-join.
+u64 self_join_total(Context &ctx, const Csr &in);
 
 // TC of one graph by searches and pulls; false when its buffers do not fit
 // (the workspace's join buffers are overwritten then, the CSR is not).

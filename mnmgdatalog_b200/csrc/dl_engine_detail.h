@@ -47,8 +47,23 @@ struct PhaseTimer {
 };
 enum { PH_INIT = 0, PH_JOIN = 1, PH_DEDUP = 2, PH_MERGE = 3, PH_FINAL = 4 };
 
+// Node id -> rank: by binary search of the sorted ids, by a presence bit per
+// value from the smallest id on (rank = bits before it), or as id - smallest id.
+// `base` is the smallest id with its sign bit flipped.
+struct Ranker {
+    enum Mode { SORTED, PRESENT, AFFINE };
+    int mode;
+    u32 n;
+    const int32_t *ids;
+    const u32 *present;
+    const u64 *pre;  // set bits before each word of `present`
+    u32 base;
+};
+
 struct Graph {
     u32 n_ids = 0;
+    u32 n_distinct = 0;  // distinct node ids (n_ids counts a dense range's absent ids too)
+    Ranker ranker{};
     int bits = 1;
     int32_t *ids = nullptr;
     // ids[r] == id_base + r for every rank (the ranks cover a dense id range)
@@ -80,14 +95,7 @@ struct FullSet {
 
 
 int bits_for(u64 n);
-// Ranks over every id in [min id, max id] when that range is at most 1/8
-// larger than the distinct ids (absent ids become ranks without edges):
-// rank -> id is then id_base + rank, with no table lookup. Returns whether
-// it did; `fits(range)` decides whether the caller can use that many ranks.
-template <class Fits>
-bool densify_ids(Context &ctx, Graph &g, Fits fits);
 const int32_t *stage_input(Context &ctx, const int32_t *rows, u64 n, bool on_device);
-void rank_nodes(Context &ctx, const int32_t *rows, u64 n, Graph &g);
 u64 *sort_unique_into(Context &ctx, DevBuf &buf, DevBuf &alt, u64 n, int key_bits, u64 &n_out);
 DevBuf &holder(Workspace &ws, const u64 *p);
 DevBuf &other(Workspace &ws, const u64 *p);

@@ -102,6 +102,7 @@ struct Workspace {
     DevBuf input;          // device copy of host edge rows
     DevBuf ids;            // sorted distinct node ids (int32)
     DevBuf w0, w1;         // word buffers for the initial sorts
+    DevBuf rank_bits, rank_pre;  // presence bit per id value, set bits before each word
     DevBuf csr_off, csr_val;
     DevBuf full[2];        // full relation (large run), ping-pong
     DevBuf small[2];       // full relation (small run), ping-pong
