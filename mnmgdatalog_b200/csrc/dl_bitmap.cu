@@ -1105,10 +1105,19 @@ u64 bitmat_stride(u64 n) { return ((n + 31) / 32 + 31) / 32 * 32; }
 u64 bitmat_bytes(u64 n) { return n * bitmat_stride(n) * 4; }
 u64 bitmat_column_offset_bytes(u64 n) { return std::max<u64>((n + CX_ROWS - 1) / CX_ROWS * n * 4, 4); }
 
+// a row (TC), or a row and its touched-word list (SG), must fit in shared memory
+static bool bitmat_row_fits(u64 n, bool sg) {
+    return (n + 31) / 32 * 4 * (sg ? 2 : 1) + sizeof(SgSmem<UW>) + 4096 <= 227 * 1024;
+}
+
+bool bitmat_allowed(const Context &ctx, u64 n, bool sg) {
+    return bitmat_row_fits(n, sg) &&
+           bitmat_bytes(n) + (sg ? 0 : bitmat_column_offset_bytes(n)) <= ((u64) ctx.tune.bitmap_max_gib << 30);
+}
+
 bool bitmat_choose(Context &ctx, const dl_options &opt, u64 n, bool sg) {
     if (opt.dedup != DL_DEDUP_AUTO && opt.dedup != DL_DEDUP_BITMAP) return false;
-    // a row (TC), or a row and its touched-word list (SG), must fit in shared memory
-    if ((n + 31) / 32 * 4 * (sg ? 2 : 1) + sizeof(SgSmem<UW>) + 4096 > 227 * 1024) return false;
+    if (!bitmat_row_fits(n, sg)) return false;
     // TC also keeps the per (row block, target) offsets of its result rows
     const u64 need = bitmat_bytes(n) + (sg ? 0 : bitmat_column_offset_bytes(n));
     // a context that already holds the matrix buffer (a repeated run) needs

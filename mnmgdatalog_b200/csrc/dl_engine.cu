@@ -20,6 +20,7 @@
 #include "dl_closure.h"
 #include "dl_engine.h"
 #include "dl_engine_detail.h"
+#include "dl_pairs.h"
 
 namespace dl {
 namespace detail {
@@ -587,7 +588,7 @@ static void run_tc_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
         // then need no rank -> id table lookups.
         rank_nodes(ctx, rows, n, g, [&](u64 range) {
             try {
-                return search || bitmat_choose(ctx, opt, range, false);
+                return search ? bitmat_allowed(ctx, range, false) : bitmat_choose(ctx, opt, range, false);
             } catch (const Error &) {  // a forced bit matrix that fits only without the absent ids
                 return false;
             }
@@ -738,6 +739,46 @@ static u64 *sg_edge_words(Context &ctx, const int32_t *rows, u64 n, const Graph 
     return sort_unique_into(ctx, ws.jbuf[0], ws.jbuf[1], n, 2 * g.bits, ne);
 }
 
+// SG as a search over pairs; false (nothing reported) when the pairs are many
+// and the bit matrix would take them, or when memory runs out.
+static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_options &opt, PhaseTimer &pt,
+                              u64 &nfull) {
+    Workspace &ws = ctx.ws;
+    pt.mark(PH_JOIN);
+    // up to 64 pairs a node the list is the cheaper form whatever the matrix costs
+    const u64 most = bitmat_allowed(ctx, g.n_ids, true) ? std::max<u64>(64 * (u64) g.n_ids, 1 << 19) : 0;
+    try {
+        const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits,
+                                          opt.max_iterations > 0 ? (u64) opt.max_iterations : 0, most);
+        if (!ps.complete) return false;
+        const u64 n = ps.n_words();
+        pt.mark(PH_DEDUP);
+        u64 *w = ws.jbuf[0].as<u64>();
+        if (n) {
+            ctx.reserve(ws.jbuf[1], n * 8);
+            w = radix_sort(ctx, w, ws.jbuf[1].as<u64>(), n, Codec::Raw, 2 * g.bits);
+        }
+        DevBuf &hold = holder(ws, w);
+        r.words = hold;
+        hold = DevBuf();
+        r.n_words = nfull = n;
+        pt.mark(PH_MERGE);
+        // iteration k finds level k; one that finds nothing ends the program, the
+        // first one also after an empty base (sg.cu:244-390)
+        for (u64 k = 1; k == 1 || k + 1 < ps.bound.size(); ++k) {
+            const u64 at = std::min<u64>(k + 1, ps.bound.size() - 1);
+            const u64 before = std::min<u64>(k, ps.bound.size() - 1);
+            r.deltas.push_back((i64) (ps.bound[at] - ps.bound[before]));
+            r.joins.push_back((i64) (k - 1 < ps.rows.size() ? ps.rows[k - 1] : 0));
+            r.fulls.push_back((i64) ps.bound[at]);
+        }
+    } catch (const Error &err) {
+        if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
+        return false;
+    }
+    return true;
+}
+
 static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, bool on_device, const dl_options &opt) {
     Workspace &ws = ctx.ws;
     PhaseTimer pt(ctx, opt.phase_timing != 0);
@@ -750,12 +791,15 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
     int cur = 0;
     FullSet F;
     F.three = true;  // plain runs: large, small and tiny runs
-    bool on_bitmat = false;
+    bool on_bitmat = false, listed = false;
     if (n > 0) {
+        // Sparse graphs as a search over pairs (dl_pairs.cu) unless a dedup
+        // form was asked for.
+        const bool search = opt.dedup == DL_DEDUP_AUTO && ctx.tune.bitmap_max_gib > 0;
         // As for TC: a dense id range is ranked as is when the bit matrix is used.
         rank_nodes(ctx, rows, n, g, [&](u64 range) {
             try {
-                return bitmat_choose(ctx, opt, range, true);
+                return search ? bitmat_allowed(ctx, range, true) : bitmat_choose(ctx, opt, range, true);
             } catch (const Error &) {
                 return false;
             }
@@ -763,7 +807,9 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
         u64 ne;
         u64 *e = sg_edge_words(ctx, rows, n, g, ne);  // sg.cu:150-153
         build_csr(ctx, e, ne, g);                     // sg.cu:162
-        if (g.ids_affine || bitmat_choose(ctx, opt, g.n_ids, true)) {
+        if (search && pair_search_fits(ctx, g.csr, 0, g.n_ids))
+            listed = sg_pairs_fixpoint(ctx, r, g, opt, pt, nfull);
+        if (!listed && ((g.ids_affine && !search) || bitmat_choose(ctx, opt, g.n_ids, true))) {
             try {
                 nfull = sg_bitmap_fixpoint(ctx, r, g, opt, pt);
                 on_bitmat = true;
@@ -782,6 +828,7 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
             }
         }
     }
+    on_bitmat |= listed;
     if (n > 0 && !on_bitmat) {
         u64 ne;
         u64 *e = sg_edge_words(ctx, rows, n, g, ne);  // again: the bit-matrix attempt reused the buffers

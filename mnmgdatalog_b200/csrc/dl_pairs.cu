@@ -1,0 +1,318 @@
+// SG as a breadth-first search over pairs.
+//
+// sg(x, y) :- e(a, x), sg(a, b), e(b, y) (sg.cu:244-390): an iteration's new
+// pairs are the children pairs of the last one's that were not seen before. The
+// pairs of sparse graphs are few, so the search keeps them as a list in the order
+// found (an iteration's delta is a range of it) and an open-addressing set of
+// their words, which stays in L2: one launch per iteration, levels launched
+// eight at a time without a host wait, and one sort of the list at the end.
+// The base rule sg(x, y) :- e(p, x), e(p, y), x != y is the same expansion of the
+// pairs (p, p).
+//
+// Measured on B200 against the bit matrix stepped by one launch per iteration:
+// lattice of 494K edges (1.5M pairs, 32 iterations, a 28 GB matrix) 41 -> 1.5 ms;
+// 5K edges from and to host memory 1.15 -> 0.6 ms. Against the union of 32
+// instances on the sorted runs (1K-100K edges, host rows) 22 -> 11 ms, most of
+// which is the callers' copies.
+#include "dl_pairs.h"
+#include "dl_scan.cuh"
+
+namespace dl {
+namespace detail {
+namespace {
+
+constexpr int PS_THREADS = 256;
+constexpr u64 FREE = ~0ull;         // never a word: ranks are below 2^32 - 1
+constexpr u32 PS_DEGREE = 64;       // largest out-degree: a pair has at most 4096 children
+constexpr u64 PS_LEVELS = 8;        // levels launched between two host waits
+constexpr u64 PS_SLOTS = 1 << 20;   // smallest set; 148 SMs x 64 warps x 32 words in flight fit half of it
+
+struct PairState {
+    u64 *list;                       // words in the order found
+    u64 cap;                         // words it holds
+    u64 *set;                        // open-addressing set, mask + 1 slots
+    u64 mask;
+    unsigned long long *count;       // words found (may pass cap: the surplus was not stored)
+    unsigned long long *bound;       // bound[k]: first word of level k
+    unsigned long long *rows;        // rows[k]: pairs of level k with children
+    u32 *done;                       // blocks of the current launch that are through
+};
+
+__device__ __forceinline__ u64 pair_slot(u64 w, u64 mask) {
+    // splitmix64's finalizer (Steele, Lea, Flood): structured words spread evenly
+    w ^= w >> 30;
+    w *= 0xbf58476d1ce4e5b9ull;
+    w ^= w >> 27;
+    w *= 0x94d049bb133111ebull;
+    w ^= w >> 31;
+    return w & mask;
+}
+
+// Adds w to the set; true when it was not there. The set is never full: the
+// list's capacity is half of its slots, a launch stops adding once the list is
+// full, and the other half (PS_SLOTS / 2 at least) is more than the resident
+// warps' windows in flight.
+__device__ __forceinline__ bool pair_insert(u64 *set, u64 mask, u64 w) {
+    u64 s = pair_slot(w, mask);
+    for (u64 probe = 0; probe <= mask; ++probe, s = (s + 1) & mask) {
+        const u64 seen = *reinterpret_cast<volatile u64 *>(set + s);
+        if (seen == w) return false;
+        if (seen == FREE) {
+            const u64 o = atomicCAS(reinterpret_cast<unsigned long long *>(set + s), FREE, w);
+            if (o == FREE) return true;
+            if (o == w) return false;
+        }
+    }
+    return false;
+}
+
+// Level `level` (0: the base rule over the nodes [lo, hi)): the children of level
+// - 1's pairs. A warp takes 32 pairs, prefix-sums their child counts and walks
+// the children 32 at a time, so a pair's count does not hold up its lane;
+// what is new is appended with one counter atomic per warp and window.
+__global__ void __launch_bounds__(PS_THREADS)
+pair_level_kernel(PairState st, const u32 *__restrict__ off, const u32 *__restrict__ val, u64 lo, u64 hi, int bits,
+                  u32 level) {
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
+    const u64 mask = (1ull << bits) - 1;
+    u64 i0, i1;
+    if (level == 0) {
+        i0 = lo;
+        i1 = hi;
+    } else {
+        i0 = st.bound[level - 1];
+        i1 = st.bound[level];
+    }
+    const u64 warps = (u64) gridDim.x * (PS_THREADS / 32);
+    u32 rows = 0;
+    for (u64 g = i0 + ((u64) blockIdx.x * PS_THREADS + threadIdx.x) / 32 * 32; g < i1; g += warps * 32) {
+        u32 ab = 0, bb = 0, da = 0, db = 0;
+        if (g + lane < i1) {
+            u64 a, b;
+            if (level == 0) {
+                a = b = g + lane;
+            } else {
+                const u64 w = st.list[g + lane];
+                a = w >> bits;
+                b = w & mask;
+            }
+            ab = __ldg(off + a);
+            da = __ldg(off + a + 1) - ab;
+            bb = __ldg(off + b);
+            db = __ldg(off + b + 1) - bb;
+            if (da && db) ++rows;
+        }
+        const u32 n = da * db;
+        const u32 incl = warp_inclusive_sum(n);
+        const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+        const u32 pre = incl - n;
+        for (u32 c0 = 0; c0 < total; c0 += 32) {
+            const u32 c = c0 + lane;
+            // owner of child c: the first lane whose inclusive sum is above c
+            u32 o = 0;
+#pragma unroll
+            for (u32 step = 16; step >= 1; step >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, o + step - 1) <= c) o += step;
+            o = min(o, 31u);
+            const u32 r = c - __shfl_sync(0xffffffffu, pre, o);
+            const u32 od = __shfl_sync(0xffffffffu, db, o);
+            const u32 oa = __shfl_sync(0xffffffffu, ab, o), ob = __shfl_sync(0xffffffffu, bb, o);
+            bool fresh = false;
+            u64 w = 0;
+            if (c < total && *reinterpret_cast<volatile unsigned long long *>(st.count) < st.cap) {
+                const u32 i = r / od;
+                const u64 x = __ldg(val + oa + i), y = __ldg(val + ob + (r - i * od));
+                w = (x << bits) | y;
+                if (level != 0 || x != y) fresh = pair_insert(st.set, st.mask, w);
+            }
+            const u32 fm = __ballot_sync(0xffffffffu, fresh);
+            if (!fm) continue;
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(st.count, (unsigned long long) __popc(fm));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(fm & lt);
+            if (fresh && at < st.cap) st.list[at] = w;
+        }
+    }
+    rows = warp_sum(rows);
+    if (level && lane == 0 && rows) atomicAdd(st.rows + level - 1, (unsigned long long) rows);
+    // the last block through closes the level
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(st.done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            const unsigned long long n = *reinterpret_cast<volatile unsigned long long *>(st.count);
+            st.bound[level + 1] = n < st.cap ? n : st.cap;
+            *st.done = 0;
+        }
+    }
+}
+
+__global__ void pair_refill_kernel(const u64 *__restrict__ list, u64 n, u64 *set, u64 mask) {
+    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x)
+        pair_insert(set, mask, list[i]);
+}
+
+__global__ void max_degree_kernel(const u32 *__restrict__ off, u64 lo, u64 hi, u32 *__restrict__ most) {
+    u32 m = 0;
+    for (u64 r = lo + (u64) blockIdx.x * blockDim.x + threadIdx.x; r < hi; r += (u64) gridDim.x * blockDim.x)
+        m = max(m, off[r + 1] - off[r]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
+}
+
+__global__ void pair_counts_kernel(const u64 *__restrict__ list, u64 n, int bits, const u64 *__restrict__ bound,
+                                   u32 levels, const u64 *__restrict__ inst_lo, u32 n_inst,
+                                   unsigned long long *__restrict__ counts) {
+    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x) {
+        const u64 x = list[i] >> bits;
+        u32 a = 0, b = n_inst;
+        while (a < b) {
+            const u32 m = (a + b) >> 1;
+            if (inst_lo[m] <= x) a = m + 1;
+            else b = m;
+        }
+        const u32 inst = a - 1;
+        a = 0;
+        b = levels;
+        while (a < b) {  // the last level whose first word is at most i
+            const u32 m = (a + b) >> 1;
+            if (bound[m] <= i) a = m + 1;
+            else b = m;
+        }
+        atomicAdd(counts + (u64) inst * levels + (a - 1), 1ull);
+    }
+}
+
+}  // namespace
+
+bool pair_search_fits(Context &ctx, const Csr &csr, u64 lo, u64 hi) {
+    u32 *most = reinterpret_cast<u32 *>(&ctx.ctrl->scalar[26]);
+    DL_CUDA(cudaMemsetAsync(most, 0, 8, ctx.stream));
+    DL_LAUNCH(ctx, K_PREP, 4.0 * (hi - lo),
+              max_degree_kernel<<<grid_for(hi - lo, T256, ctx, 8), T256, 0, ctx.stream>>>(csr.off, lo, hi, most));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, most, 8, cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    return *reinterpret_cast<u32 *>(ctx.host_scalars) <= PS_DEGREE;
+}
+
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most) {
+    Workspace &ws = ctx.ws;
+    PairSearch ps;
+    DevBuf &list = ws.jbuf[0], &set = ws.jbuf[1];
+    // room for four pairs a node at first, slots for twice as many words (a set of
+    // up to 16M slots stays in L2, where an insert costs a fifth); a level
+    // that needs more is repeated on a set four times the size
+    u64 slots = PS_SLOTS;
+    while (slots < 8 * (hi - lo) && !(most && slots / 2 >= 2 * most)) slots <<= 1;
+    u64 levels = 64;  // level counters: bound[levels + 2], rows[levels + 1], after the list's and blocks' counters
+    ctx.reserve(ws.cl_levels, (2 * levels + 16) * 8);
+    u64 *base = ws.cl_levels.as<u64>();
+    DL_CUDA(cudaMemsetAsync(base, 0, (2 * levels + 16) * 8, ctx.stream));
+    PairState st;
+    auto bind = [&]() {
+        st.list = list.as<u64>();
+        st.cap = slots / 2;
+        st.set = set.as<u64>();
+        st.mask = slots - 1;
+        u64 *b = ws.cl_levels.as<u64>();
+        st.count = reinterpret_cast<unsigned long long *>(b);
+        st.done = reinterpret_cast<u32 *>(b + 1);
+        st.bound = reinterpret_cast<unsigned long long *>(b + 8);
+        st.rows = st.bound + levels + 4;
+    };
+    ctx.reserve(list, slots / 2 * 8);
+    ctx.reserve(set, slots * 8);
+    DL_CUDA(cudaMemsetAsync(set.p, 0xFF, slots * 8, ctx.stream));
+    bind();
+    ps.bound.assign(1, 0);
+    auto launch = [&](u64 level, u64 pairs) {
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                  pair_level_kernel<<<grid_for(pairs, PS_THREADS, ctx, 8), PS_THREADS, 0, ctx.stream>>>(
+                      st, csr.off, csr.val, lo, hi, bits, (u32) level));
+    };
+    for (u64 level = 0;;) {
+        // room for the levels of this batch
+        if (level + PS_LEVELS + 2 > levels) {
+            const u64 old = levels;
+            levels *= 4;
+            DevBuf nb;
+            ctx.reserve(nb, (2 * levels + 16) * 8);
+            DL_CUDA(cudaMemsetAsync(nb.p, 0, (2 * levels + 16) * 8, ctx.stream));
+            u64 *f = ws.cl_levels.as<u64>(), *t = nb.as<u64>();
+            DL_CUDA(cudaMemcpyAsync(t, f, (8 + old + 4) * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+            DL_CUDA(cudaMemcpyAsync(t + 8 + levels + 4, f + 8 + old + 4, old * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+            ctx.give_back(ws.cl_levels);
+            ws.cl_levels = nb;
+            bind();
+        }
+        // an unknown number of pairs: the grid for all nodes, or for the last known level
+        const u64 batch = max_levels ? std::min<u64>(PS_LEVELS, max_levels - level + 1) : PS_LEVELS;
+        const u64 known = level ? ps.bound[level] - ps.bound[level - 1] : hi - lo;
+        for (u64 k = 0; k < batch; ++k) launch(level + k, level || k ? std::max<u64>(4 * known, 1 << 15) : known);
+        u64 *hs = ctx.host_scalars;
+        DL_CUDA(cudaMemcpyAsync(hs, st.count, 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs + 1, st.bound + level + 1, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs + 1 + PS_LEVELS, st.rows + (level ? level - 1 : 0), batch * 8,
+                                cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        const u64 found = hs[0];
+        bool full = found >= st.cap, end = false;
+        u64 good = batch;  // levels of the batch that are whole
+        if (full) {
+            good = 0;
+            while (good < batch && hs[1 + good] < st.cap) ++good;
+        }
+        for (u64 k = 0; k < good; ++k) {
+            const u64 lv = level + k;
+            if (lv) ps.rows.push_back(hs[1 + PS_LEVELS + (level ? k : k - 1)]);
+            ps.bound.push_back(hs[1 + k]);
+            if (ps.bound[lv + 1] == ps.bound[lv]) {  // nothing new
+                ps.complete = end = true;
+                break;
+            }
+        }
+        if (end) break;
+        level += good;
+        if (!full && max_levels && level > max_levels) {
+            ps.complete = true;
+            break;
+        }
+        if (most && (full || ps.n_words() > most)) break;
+        if (full) {  // repeat level `level` with more room: the set again from the words listed before it
+            const u64 keep = ps.bound[level];
+            slots *= 4;
+            DevBuf nl;
+            ctx.reserve(nl, slots / 2 * 8);
+            DL_CUDA(cudaMemcpyAsync(nl.p, list.p, keep * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+            ctx.give_back(list);
+            list = nl;
+            ctx.reserve(set, slots * 8);
+            DL_CUDA(cudaMemsetAsync(set.p, 0xFF, slots * 8, ctx.stream));
+            bind();
+            if (keep)
+                DL_LAUNCH(ctx, K_BITMAP_EXPAND, 16.0 * keep,
+                          pair_refill_kernel<<<grid_for(keep, T256, ctx), T256, 0, ctx.stream>>>(st.list, keep, st.set,
+                                                                                                st.mask));
+            DL_CUDA(cudaMemcpyAsync(st.count, ps.bound.data() + level, 8, cudaMemcpyHostToDevice, ctx.stream));
+            // rows counted by the levels that are repeated
+            DL_CUDA(cudaMemsetAsync(st.rows + (level ? level - 1 : 0), 0, (PS_LEVELS + 1) * 8, ctx.stream));
+            ctx.sync();  // ps.bound is host memory
+        }
+    }
+    return ps;
+}
+
+void pair_level_counts(Context &ctx, const PairSearch &ps, int bits, const u64 *inst_lo, u64 n_inst, u64 *counts) {
+    const u64 levels = ps.bound.size() - 1;
+    DL_CUDA(cudaMemsetAsync(counts, 0, n_inst * levels * 8, ctx.stream));
+    if (ps.n_words() == 0) return;
+    DL_LAUNCH(ctx, K_PREP, 8.0 * ps.n_words(),
+              pair_counts_kernel<<<grid_for(ps.n_words(), T256, ctx), T256, 0, ctx.stream>>>(
+                  ctx.ws.jbuf[0].as<u64>(), ps.n_words(), bits, ctx.ws.cl_levels.as<u64>() + 8, (u32) levels, inst_lo,
+                  (u32) n_inst, reinterpret_cast<unsigned long long *>(counts)));
+}
+
+}  // namespace detail
+}  // namespace dl

@@ -1,0 +1,31 @@
+// SG as a breadth-first search over pairs (dl_pairs.cu).
+#pragma once
+
+#include "dl_engine_detail.h"
+
+namespace dl {
+namespace detail {
+
+// Pairs of one search, in the order found: level 0 = the base rule's, level k =
+// iteration k's new ones.
+struct PairSearch {
+    std::vector<u64> bound;  // level k holds words [bound[k], bound[k + 1])
+    std::vector<u64> rows;   // rows[k]: pairs of level k whose two nodes have out-edges
+    bool complete = false;   // the last level found nothing (or max_levels ended the search)
+    u64 n_words() const { return bound.empty() ? 0 : bound.back(); }
+};
+
+// Whether the degrees of ranks [lo, hi) suit the pair search (a pair's
+// expansion is shared by 32 lanes at most).
+bool pair_search_fits(Context &ctx, const Csr &csr, u64 lo, u64 hi);
+// The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
+// in ws.jbuf[0], unsorted. Stops after level max_levels (0: at the fixpoint),
+// or once more than `most` words are found (0: never; the search is then not
+// complete and its last level may lack words).
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most);
+// counts[instance * levels + k] = words of level k of each instance (instance of
+// a word: the last one whose first rank is at most its key rank).
+void pair_level_counts(Context &ctx, const PairSearch &ps, int bits, const u64 *inst_lo, u64 n_inst, u64 *counts);
+
+}  // namespace detail
+}  // namespace dl

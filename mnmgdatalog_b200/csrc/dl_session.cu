@@ -8,7 +8,11 @@
 // Instances are admitted at any iteration boundary (continuous batching):
 // their edges are appended to the union's offset table (their ranks are above
 // every rank in use, so the table stays sorted) and their initial delta joins
-// the next iteration. Each instance keeps its own iteration count and delta
+// the next iteration. TC's and SG's instances do not need the common steps: a
+// source's (TC, dl_closure.cu) or a pair's (SG, dl_pairs.cu) search never meets
+// another instance's, so the instances admitted together are searched to their
+// fixpoints in one go and the steps report their iterations one by one; SG
+// instances whose degrees do not suit the search keep the common steps. Each instance keeps its own iteration count and delta
 // sequence (a per-instance histogram of every iteration's delta) and leaves
 // the union when it reaches its own fixpoint -- for WCC with the reference's
 // stop rule an instance is frozen (its delta entries dropped) at the iteration
@@ -21,6 +25,7 @@
 #include "dl_closure.h"
 #include "dl_engine_detail.h"
 #include "dl_join.cuh"
+#include "dl_pairs.h"
 #include "dl_scan.cuh"
 #include "dl_session.h"
 
@@ -576,8 +581,7 @@ void mark_done(SessionImpl &s, SessionInstance &in) {
 
 void finish(SessionImpl &s, const std::vector<i64> &ids) {
     if (ids.empty()) return;
-    if (s.program == DL_PROGRAM_WCC) extract_components(s, ids);
-    else extract_words(s, ids);
+    extract_components(s, ids);
     for (i64 id : ids) mark_done(s, s.inst[id]);
 }
 
@@ -683,6 +687,80 @@ u64 wcc_step(SessionImpl &s) {
     return s.active.size();
 }
 
+// The words of a search (ws.jbuf[0], unsorted) in result order, into one block;
+// every instance's are one range of it.
+void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words) {
+    Context &ctx = s.ctx;
+    Workspace &ws = ctx.ws;
+    const u64 n = ids.size();
+    std::vector<u64> hb(6 * n, 0);
+    auto block = std::shared_ptr<DevBuf>();
+    if (words) {
+        ctx.reserve(ws.jbuf[1], words * 8);
+        int w[8];
+        const int nw = plan_windows(s.bits, bits_for(std::max<u64>(s.next_rank, 2)), w);
+        u64 *r = radix_sort_windows(ctx, ws.jbuf[0].as<u64>(), ws.jbuf[1].as<u64>(), words, w, nw);
+        upload_ranges(s, ids);
+        ctx.reserve(s.counts, 6 * n * 8);
+        Runs3 runs{{r, r, r}, {words, 0, 0}};
+        DL_LAUNCH(ctx, K_PREP, 0,
+                  session_bounds_kernel<<<grid_for(6 * n, 256, ctx, 4), 256, 0, ctx.stream>>>(
+                      runs, s.range_lo.as<u64>(), (u32) n, s.bits, s.counts.as<u64>()));
+        DL_CUDA(cudaMemcpyAsync(hb.data(), s.counts.p, 6 * n * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DevBuf &held = holder(ws, r);
+        if (held.cap <= 2 * words * 8 + (1 << 20)) {  // the sorted buffer becomes the result block
+            block = make_block(ctx, 0);
+            std::swap(*block, held);
+        } else {
+            block = make_block(ctx, words * 8);
+            DL_CUDA(cudaMemcpyAsync(block->p, r, words * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+        }
+        ctx.sync();
+    }
+    for (u64 k = 0; k < n; ++k) {
+        SessionInstance &in = s.inst[ids[k]];
+        in.result_block = block;
+        in.result_off = hb[6 * k];
+        in.n_result = hb[6 * k + 1] - hb[6 * k];
+    }
+}
+
+// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi))
+// as one search over pairs (dl_pairs.cu). Returns false when a node's degree
+// does not suit it.
+bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
+    Context &ctx = s.ctx;
+    Csr csr;
+    csr.off = s.off.as<u32>();
+    csr.val = s.val.as<u32>();
+    csr.n_keys = (u32) s.next_rank;
+    csr.n_vals = s.n_vals;
+    if (!pair_search_fits(ctx, csr, lo, hi)) return false;
+    const u64 n = ids.size();
+    const int stop = s.opt.max_iterations;
+    const PairSearch ps = pair_search(ctx, csr, lo, hi, s.bits, stop > 0 ? (u64) stop : 0, 0);
+    const u64 levels = ps.bound.size() - 1;
+    std::vector<u64> first(n), cnt(n * levels);
+    for (u64 k = 0; k < n; ++k) first[k] = s.inst[ids[k]].rank_lo;
+    ctx.reserve(s.range_lo, n * 8);
+    DL_CUDA(cudaMemcpyAsync(s.range_lo.p, first.data(), n * 8, cudaMemcpyHostToDevice, ctx.stream));
+    ctx.reserve(s.counts, n * levels * 8);
+    pair_level_counts(ctx, ps, s.bits, s.range_lo.as<u64>(), n, s.counts.as<u64>());
+    DL_CUDA(cudaMemcpyAsync(cnt.data(), s.counts.p, n * levels * 8, cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    for (u64 k = 0; k < n; ++k) {
+        SessionInstance &in = s.inst[ids[k]];
+        in.ahead.clear();
+        for (u64 d = 1;; ++d) {  // iteration d finds level d (sg.cu:244-390)
+            const i64 c = d < levels ? (i64) cnt[k * levels + d] : 0;
+            in.ahead.push_back(c);
+            if (c == 0 || (stop > 0 && (int) in.ahead.size() >= stop)) break;
+        }
+    }
+    place_results(s, ids, ps.n_words());
+    return true;
+}
+
 // TC: the whole fixpoint of the instances admitted since the last step
 // (dl_closure.cu: a search per source, whatever the instance, so all of them
 // run in one launch), their rows sorted into one block and every iteration's
@@ -745,38 +823,15 @@ void search_pending(SessionImpl &s) {
             if (c == 0 || (s.opt.max_iterations > 0 && (int) in.ahead.size() >= s.opt.max_iterations)) break;
         }
     }
-    // result order; every instance's words are one range
-    std::vector<u64> hb(6 * n, 0);
-    auto block = std::shared_ptr<DevBuf>();
-    if (words) {
-        ctx.reserve(ws.jbuf[1], words * 8);
-        int w[8];
-        const int nw = plan_windows(s.bits, bits_for(std::max<u64>(s.next_rank, 2)), w);
-        u64 *r = radix_sort_windows(ctx, ws.jbuf[0].as<u64>(), ws.jbuf[1].as<u64>(), words, w, nw);
-        upload_ranges(s, ids);
-        ctx.reserve(s.counts, 6 * n * 8);
-        Runs3 runs{{r, r, r}, {words, 0, 0}};
-        DL_LAUNCH(ctx, K_PREP, 0,
-                  session_bounds_kernel<<<grid_for(6 * n, 256, ctx, 4), 256, 0, ctx.stream>>>(
-                      runs, s.range_lo.as<u64>(), (u32) n, s.bits, s.counts.as<u64>()));
-        DL_CUDA(cudaMemcpyAsync(hb.data(), s.counts.p, 6 * n * 8, cudaMemcpyDeviceToHost, ctx.stream));
-        DevBuf &held = holder(ws, r);
-        if (held.cap <= 2 * words * 8 + (1 << 20)) {  // the sorted buffer becomes the result block
-            block = make_block(ctx, 0);
-            std::swap(*block, held);
-        } else {
-            block = make_block(ctx, words * 8);
-            DL_CUDA(cudaMemcpyAsync(block->p, r, words * 8, cudaMemcpyDeviceToDevice, ctx.stream));
-        }
-        ctx.sync();
-    }
-    for (u64 k = 0; k < n; ++k) {
-        SessionInstance &in = s.inst[ids[k]];
-        in.result_block = block;
-        in.result_off = hb[6 * k];
-        in.n_result = hb[6 * k + 1] - hb[6 * k];
-    }
+    place_results(s, ids, words);
     s.pending.clear();
+}
+
+// Reports one iteration of an instance whose fixpoint was searched ahead;
+// true when it was the last.
+bool report_ahead(SessionInstance &in) {
+    in.deltas.push_back(in.ahead[in.deltas.size()]);
+    return in.deltas.size() == in.ahead.size();
 }
 
 u64 tc_step(SessionImpl &s) {
@@ -784,8 +839,7 @@ u64 tc_step(SessionImpl &s) {
     std::vector<i64> still;
     for (i64 id : s.active) {
         SessionInstance &in = s.inst[id];
-        in.deltas.push_back(in.ahead[in.deltas.size()]);
-        if (in.deltas.size() == in.ahead.size()) mark_done(s, in);
+        if (report_ahead(in)) mark_done(s, in);
         else still.push_back(id);
     }
     if (still.size() != s.active.size()) {
@@ -796,49 +850,66 @@ u64 tc_step(SessionImpl &s) {
     return s.active.size();
 }
 
-// One SG iteration of every active instance (sg.cu:244-390).
+// One SG iteration (sg.cu:244-390): the instances searched ahead report theirs,
+// the others (a node of more out-edges than the search takes) advance together
+// on the sorted runs.
 u64 sg_step(SessionImpl &s) {
     Context &ctx = s.ctx;
     Workspace &ws = ctx.ws;
-    Graph g = union_graph(s);
-    PhaseTimer pt(ctx, false);
     u64 nnew = 0;
-    u64 *dnew = nullptr;
-    u64 n1 = 0, n2 = 0;
-    u64 *j1 = join_and_sort(ctx, g, s.delta.as<u64>(), s.n_delta, EmitKind::VZ, n1, nullptr, pt);
-    if (n1) n1 = unique_words(ctx, j1, n1, j1);
-    if (n1) {
-        u64 *j2 = join_and_sort(ctx, g, j1, n1, EmitKind::VZ, n2, nullptr, pt);
-        dnew = absorb(ctx, s.F, j2, n2, nnew);
+    std::vector<u64> c(s.active.size(), 0);
+    bool runs = false;
+    for (i64 id : s.active) runs |= s.inst[id].ahead.empty();
+    if (runs) {
+        Graph g = union_graph(s);
+        PhaseTimer pt(ctx, false);
+        u64 *dnew = nullptr;
+        u64 n1 = 0, n2 = 0;
+        u64 *j1 = join_and_sort(ctx, g, s.delta.as<u64>(), s.n_delta, EmitKind::VZ, n1, nullptr, pt);
+        if (n1) n1 = unique_words(ctx, j1, n1, j1);
+        if (n1) {
+            u64 *j2 = join_and_sort(ctx, g, j1, n1, EmitKind::VZ, n2, nullptr, pt);
+            dnew = absorb(ctx, s.F, j2, n2, nnew);
+        }
+        // the new delta sits in one of the join buffers: trade it for the old delta's buffer
+        if (nnew) std::swap(s.delta, holder(ws, dnew));
+        s.n_delta = nnew;
+        c = delta_counts(s, s.delta.as<u64>(), nnew, s.bits);
     }
-    // the new delta sits in one of the join buffers: trade it for the old delta's buffer
-    if (nnew) std::swap(s.delta, holder(ws, dnew));
-    s.n_delta = nnew;
-    const std::vector<u64> c = delta_counts(s, s.delta.as<u64>(), nnew, s.bits);
-    std::vector<i64> still, done;
+    std::vector<i64> still, done, extract;
+    std::vector<uint8_t> live(s.active.size(), 1);
+    bool rows_left = false;  // an instance stopped by max_iterations keeps rows in the delta
     for (u64 k = 0; k < s.active.size(); ++k) {
         SessionInstance &in = s.inst[s.active[k]];
-        in.deltas.push_back((i64) c[k]);
-        bool stop = c[k] == 0;  // |full| unchanged
-        if (!stop && s.opt.max_iterations > 0 && (int) in.deltas.size() >= s.opt.max_iterations) stop = true;
+        bool stop;
+        if (!in.ahead.empty()) {
+            stop = report_ahead(in);
+        } else {
+            in.deltas.push_back((i64) c[k]);
+            stop = c[k] == 0;  // |full| unchanged
+            if (!stop && s.opt.max_iterations > 0 && (int) in.deltas.size() >= s.opt.max_iterations) stop = true;
+            if (stop) {
+                extract.push_back(s.active[k]);
+                live[k] = 0;
+                rows_left |= c[k] != 0;
+            }
+        }
         (stop ? done : still).push_back(s.active[k]);
     }
-    if (!done.empty() && nnew && still.size() < s.active.size()) {
-        // an instance stopped by max_iterations keeps rows in the delta: drop them
-        bool rows_left = false;
-        for (u64 k = 0; k < s.active.size(); ++k)
-            if (c[k] && std::find(done.begin(), done.end(), s.active[k]) != done.end()) rows_left = true;
-        if (rows_left) {
-            std::vector<uint8_t> live(s.active.size(), 1);
-            for (u64 k = 0; k < s.active.size(); ++k)
-                if (std::find(done.begin(), done.end(), s.active[k]) != done.end()) live[k] = 0;
-            ctx.reserve(s.live, live.size());
-            DL_CUDA(cudaMemcpyAsync(s.live.p, live.data(), live.size(), cudaMemcpyHostToDevice, ctx.stream));
-            KeepActive keep{s.inst_lo.as<u64>(), s.live.as<uint8_t>(), (u32) s.active.size(), s.bits};
-            s.n_delta = session_select(ctx, s.delta.as<u64>(), s.n_delta, keep, 61);
-        }
+    if (rows_left && still.size()) {
+        upload_active(s);
+        ctx.reserve(s.live, live.size());
+        DL_CUDA(cudaMemcpyAsync(s.live.p, live.data(), live.size(), cudaMemcpyHostToDevice, ctx.stream));
+        KeepActive keep{s.inst_lo.as<u64>(), s.live.as<uint8_t>(), (u32) s.active.size(), s.bits};
+        s.n_delta = session_select(ctx, s.delta.as<u64>(), s.n_delta, keep, 61);  // syncs: `live` may go
     }
-    retire(s, done, still);
+    if (!extract.empty()) extract_words(s, extract);
+    for (i64 id : done) mark_done(s, s.inst[id]);
+    if (still.size() != s.active.size()) {
+        s.active = still;
+        s.inst_dirty = true;
+    }
+    reset_if_idle(s);
     maybe_compact(s);
     return s.active.size();
 }
@@ -1004,8 +1075,13 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
             in.ids_off = first[k];
         }
         std::vector<bool> empty_base(count, false);
+        std::vector<i64> with_rows;
+        for (u64 k = 0; k < count; ++k)
+            if (nrows[k]) with_rows.push_back(inst(k).id);
         if (tc) {
             // searched as a whole in the next step
+        } else if (s.program == DL_PROGRAM_SG && search_pairs(s, with_rows, B, B + nu)) {
+            for (u64 k = 0; k < count; ++k) empty_base[k] = nrows[k] && inst(k).ahead[0] == 0 && inst(k).n_result == 0;
         } else if (s.program == DL_PROGRAM_SG) {
             // sg.cu:170-217: the base rule of the admitted instances, probing the union table
             Graph g = union_graph(s);

@@ -1,0 +1,79 @@
+"""SG as a search over pairs (dl_pairs.cu, what AUTO runs on sparse graphs and
+sessions run) against the sorted runs, exactly: rows, iterations and
+per-iteration sizes -- with degrees on both sides of the 64 a pair may have,
+bases that are empty, runs that stop early, results past the first set's size
+(a level repeated on a larger set), and instances of both kinds in a session."""
+import numpy as np
+import pytest
+
+from mnmgdatalog_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def _tree(n, k):
+    return [[i, k * i + 1 + j] for i in range(n) for j in range(k)]
+
+
+def _hubs(d):
+    return [[0, i + 1] for i in range(d)] + [[i + 1, 1000 + i] for i in range(d)]
+
+
+CASES = {
+    "one": [[1, 2]], "loop": [[1, 1], [1, 2]], "siblings": [[1, 2], [1, 3]], "cycle": [[i, (i + 1) % 7] for i in range(7)],
+    "tree2": _tree(500, 2), "tree5": _tree(900, 5), "hub_64": _hubs(64), "hub_65": _hubs(65),
+    "lattice": graphs.lattice3d(side=12, seed=1), "dense_lattice": graphs.lattice3d(side=14, p=0.3, seed=5),
+    "random": np.random.default_rng(0).integers(0, 3000, (5000, 2)), "dag": graphs.dag(n=1500, extra=500, seed=2),
+    "wide_ids": graphs.lattice3d(side=10, seed=4) * 1_000_003 - 10**9,
+}
+STOPS = [0, 1, 4]
+
+
+def _rows(name):
+    return np.ascontiguousarray(CASES[name]).astype(np.int32)
+
+
+@pytest.mark.parametrize("stop", STOPS)
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_sg_pairs_equal_sorted_runs(engine, name, stop):
+    e = _rows(name)
+    want = engine.sg(e, dedup="sort", max_iterations=stop)
+    got = engine.sg(e, max_iterations=stop)
+    assert got.iterations == want.iterations
+    assert got.deltas.tolist() == want.deltas.tolist() and got.full_rows.tolist() == want.full_rows.tolist()
+    assert np.array_equal(got.rows, want.rows)
+    # the delta rows joined per iteration are counted as on the bit matrix
+    assert got.join_rows.tolist() == engine.sg(e, dedup="bitmap", max_iterations=stop).join_rows.tolist()
+
+
+@pytest.mark.parametrize("stop", STOPS)
+@pytest.mark.parametrize("names", [["lattice", "cycle", "tree2", "one"], ["hub_64", "hub_65", "loop", "dense_lattice"]])
+def test_sg_batch_equals_sorted_runs(engine, names, stop):
+    sets = [_rows(k) for k in names] + [np.zeros((0, 2), np.int32)]
+    for e, got in zip(sets, engine.run_batch("sg", sets, max_iterations=stop)):
+        want = engine.sg(e, dedup="sort", max_iterations=stop)
+        assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+
+
+def test_sg_session_of_both_kinds(engine):
+    """Searched instances and instances on the sorted runs advance side by side."""
+    order = [["lattice", "hub_65"], ["dag", "tree5"], ["hub_65", "lattice"], ["dense_lattice"]]
+    with engine.session("sg") as s:
+        ids = []
+        for names in order:
+            ids += list(zip(s.admit_many([_rows(k) for k in names]), names))
+            s.step()
+        s.run()
+        for i, k in ids:
+            want = engine.sg(_rows(k), dedup="sort")
+            got = s.result(i)
+            assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows), k
+
+
+def test_sg_set_outgrown(engine):
+    """More pairs than the first set holds (512K), in one instance of a batch."""
+    sets = [graphs.lattice3d(side=14, p=0.3, seed=5), graphs.lattice3d(side=9, p=0.3, seed=1)]
+    for e, got in zip(sets, engine.run_batch("sg", sets)):
+        want = engine.sg(e, dedup="bitmap")
+        assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+    assert len(got.rows) < 2**19 < len(engine.sg(sets[0]).rows)
