@@ -32,13 +32,12 @@
 #include <type_traits>
 
 #include "dl_closure.h"
+#include "dl_pull.cuh"
 #include "dl_scan.cuh"
 
 namespace dl {
 namespace detail {
 namespace {
-
-constexpr u32 EMPTY = 0xFFFFFFFFu;  // ranks are below 2^32 - 1
 
 // Counters of a search launch (device).
 struct SearchCounters {
@@ -401,47 +400,6 @@ struct CwSmem {
     u32 wbeg[32], wpre[32];           // compacted rows of the group being expanded
 };
 
-// Walks the edge targets of up to 32 rows (beg, deg of this lane's row; deg 0:
-// none) in windows of 32: f(w, have) per window, all lanes; f returns false
-// to stop. Returns the rows' edges. A window's rows are the bits of a
-// start mask, a word's row the number of rows started up to its position.
-template <class F>
-__device__ __forceinline__ u32 walk_rows(u32 *wbeg, u32 *wpre, u32 beg, u32 deg, const u32 *__restrict__ val,
-                                         u32 lane, u32 lt, u32 le, u32 limit, F f) {
-    const u32 nz = __ballot_sync(0xffffffffu, deg != 0);
-    if (!nz) return 0;
-    const u32 incl = warp_inclusive_sum(deg);
-    const u32 total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total > limit) return total;
-    const u32 rk = __popc(nz & lt);
-    if (deg) {
-        wbeg[rk] = beg;
-        wpre[rk] = incl - deg;
-    }
-    __syncwarp();
-    const u32 nrows = __popc(nz);
-    const u32 cb = lane < nrows ? wbeg[lane] : 0u;
-    const u32 pre = lane < nrows ? wpre[lane] : 0xFFFFFFFFu;
-    __syncwarp();
-    int base = -1;  // last row started before the window
-    auto load = [&](u32 i0) -> u32 {
-        const u32 st = (pre - i0) < 32u ? 1u << (pre - i0) : 0u;
-        const u32 starts = __reduce_or_sync(0xffffffffu, st);
-        const int o = base + __popc(starts & le);
-        base += __popc(starts);
-        const u32 ob = __shfl_sync(0xffffffffu, cb, o);
-        const u32 op = __shfl_sync(0xffffffffu, pre, o);
-        return i0 + lane < total ? __ldg(val + ob + (i0 + lane - op)) : 0u;
-    };
-    u32 w = load(0);
-    for (u32 i0 = 0; i0 < total; i0 += 32) {
-        const u32 wn = i0 + 32 < total ? load(i0 + 32) : 0u;  // the next window's load is in flight
-        if (!f(w, i0 + lane < total)) break;
-        w = wn;
-    }
-    return total;
-}
-
 // The same search by a warp, for the sources eight lanes' slice could not
 // hold (src; null: every rank from lo on). A search that outgrows its slice goes to
 // `left`.
@@ -669,95 +627,10 @@ closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, con
 
 // ---- heavy sources: 32 to a word ----------------------------------------
 
-constexpr int PU_THREADS = 256;
 // A target with more in-edges than lanes ("hub") is gathered in segments of 32
 // in-edges by as many warps: one warp alone would walk them long after the
 // others are done (at 256 in-edges a warp, 46 % of a level's time was that tail).
 constexpr u32 PU_SEG = 32;
-
-// Rows of heavy-source bits: chunks of 1024 columns (a 128-byte line), 2^shift
-// of which share one activity bit, so that a row's activity is one word
-// whatever the number of columns.
-struct PullShape {
-    u64 n;      // targets
-    u32 words;  // words of a row
-    u32 shift;
-};
-
-// One level's view of the state: row y of `cur` is valid when tag[y] is
-// (activity, level - 1); todo[w] = activity of w's in-neighbours (zero: w is not
-// in the list).
-struct PullLevel {
-    u32 level;
-    const u32 *cur;
-    u32 *nxt;
-    const uint2 *tag;
-    uint2 *tag_next;
-    u32 *todo, *todo_next;
-    const u32 *list;
-    u32 *list_next;
-    unsigned long long *count;  // [level]: targets in the level's list
-    unsigned long long *cnt;    // [level]: new pairs
-    unsigned long long *deg;    // [level]: sum of their targets' out-degrees
-};
-
-// Puts the targets of the newly active nodes on the next level's list: a
-// thread per edge (x, y), sorted by x, so a node's out-degree does not matter
-// (a warp per active node spent half a level on the few nodes with thousands
-// of out-edges).
-__global__ void __launch_bounds__(PU_THREADS)
-closure_push_kernel(PullLevel st, const u64 *__restrict__ edges, u64 ne, int bits) {
-    if (st.level && st.count[st.level] == 0) return;  // the fixpoint was reached earlier
-    const u32 lane = threadIdx.x & 31;
-    const u32 lt = lanemask_lt();
-    const u64 mask = (1ull << bits) - 1;
-    for (u64 k0 = (u64) blockIdx.x * PU_THREADS + (threadIdx.x & ~31u); k0 < ne; k0 += (u64) gridDim.x * PU_THREADS) {
-        bool fresh = false;
-        u32 y = 0;
-        if (k0 + lane < ne) {
-            const u64 e = __ldg(edges + k0 + lane);
-            const uint2 tg = st.tag_next[e >> bits];
-            if (tg.y == st.level) {
-                y = (u32) (e & mask);
-                fresh = atomicOr(&st.todo_next[y], tg.x) == 0u;
-            }
-        }
-        const u32 fm = __ballot_sync(0xffffffffu, fresh);
-        if (!fm) continue;
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(st.count + st.level + 1, (unsigned long long) __popc(fm));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (fresh) st.list_next[at + __popc(fm & lt)] = y;
-    }
-}
-
-__global__ void pull_swap_kernel(const u64 *__restrict__ e, u64 ne, int bits, u64 *__restrict__ out) {
-    const u64 mask = (1ull << bits) - 1;
-    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (u64) gridDim.x * blockDim.x) {
-        const u64 w = e[i];
-        out[i] = ((w & mask) << bits) | (w >> bits);
-    }
-}
-
-// off[k] = first word whose key (word >> bits) is at least k, k in [0, n].
-template <class T>
-__global__ void key_offsets_kernel(const u64 *__restrict__ w, u64 nw, int bits, u64 n, T *__restrict__ off) {
-    for (u64 k = (u64) blockIdx.x * blockDim.x + threadIdx.x; k <= n; k += (u64) gridDim.x * blockDim.x) {
-        const u64 target = k << bits;
-        u64 l = 0, h = nw;
-        while (l < h) {
-            const u64 m = (l + h) >> 1;
-            if (w[m] < target) l = m + 1;
-            else h = m;
-        }
-        off[k] = (T) l;
-    }
-}
-
-__global__ void low_field_kernel(const u64 *__restrict__ w, u64 n, u64 mask, u32 *__restrict__ out) {
-    for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x)
-        out[i] = (u32) (w[i] & mask);
-}
 
 // Hubs: hub_at[w] = accumulator row of hub w, seg[...] = (w, first in-edge of a
 // segment); found[0] = hubs, found[1] = segments.
@@ -1087,7 +960,7 @@ __global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u
 // last, its lanes shifted by the light pairs below them.
 constexpr u32 ROWS_STAGE = 384;  // a sparse chunk's staged rows
 
-template <bool DENSE>
+template <bool DENSE, bool ROW_FIRST>
 __global__ void __launch_bounds__(256)
 closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict__ cols,
                     const u32 *__restrict__ place, const uint2 *__restrict__ start, u64 z0, u64 z1,
@@ -1123,7 +996,9 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             const u32 any = __ballot_sync(0xffffffffu, v != 0);
             if (!any && st.y == lend) continue;
             u64 *dst = out + first[z] + st.x;
-            const u64 zid = (u64) node((u32) z) << 32;
+            const u32 zid = node((u32) z);
+            // a row (x, z), or (z, x) when the targets come first, as one little-endian word
+            auto pack = [&](u32 x) -> u64 { return ROW_FIRST ? ((u64) x << 32) | zid : ((u64) zid << 32) | x; };
             const u32 n = __popc(v);
             const u32 incl = warp_inclusive_sum(n);
             u32 at = incl - n;
@@ -1132,7 +1007,7 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 if (st.y == lend && total <= ROWS_STAGE) {
                     for (; v; v &= v - 1) stage[at++] = node(__ldg(cc + lane * 32 + __ffs(v) - 1));
                     __syncwarp();
-                    for (u32 i = lane; i < total; i += 32) dst[i] = zid | stage[i];
+                    for (u32 i = lane; i < total; i += 32) dst[i] = pack(stage[i]);
                     __syncwarp();
                     continue;
                 }
@@ -1158,7 +1033,7 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 const u32 wj = __shfl_sync(0xffffffffu, v, j & 31), pj = __shfl_sync(0xffffffffu, incl - n, j & 31);
                 const u32 total = __shfl_sync(0xffffffffu, incl, 31);
                 if (in)
-                    dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + (l0 + lane - st.y)] = zid | node(x);
+                    dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + (l0 + lane - st.y)] = pack(node(x));
                 const u32 key = in ? (b ? j : j - 1) : EMPTY - 1;  // words above `key` are shifted whole
                 for (u32 k = 0; k < min(32u, lend - l0); ++k)
                     at += (int) lane > (int) __shfl_sync(0xffffffffu, key, k);
@@ -1172,9 +1047,9 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 const u32 word = __shfl_sync(0xffffffffu, v, j);
                 const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
                 if constexpr (DENSE) {
-                    if ((word >> lane) & 1u) dst[p] = zid | id[j];
+                    if ((word >> lane) & 1u) dst[p] = pack(id[j]);
                 } else {
-                    if ((word >> lane) & 1u) dst[p] = zid | node(__ldg(cc + j * 32 + lane));
+                    if ((word >> lane) & 1u) dst[p] = pack(node(__ldg(cc + j * 32 + lane)));
                 }
             }
             while (slow) {
@@ -1188,7 +1063,7 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                     for (u32 mm = __ballot_sync(0xffffffffu, (rl >> 5) == j && (rl & 31)); mm; mm &= mm - 1)
                         p += (__shfl_sync(0xffffffffu, rl, __ffs(mm) - 1) & 31) <= lane;
                 }
-                if ((word >> lane) & 1u) dst[p] = zid | node(__ldg(cc + j * 32 + lane));
+                if ((word >> lane) & 1u) dst[p] = pack(node(__ldg(cc + j * 32 + lane)));
             }
         }
     }
@@ -1459,6 +1334,21 @@ ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne
     return res;
 }
 
+void bit_rows_count(Context &ctx, Run &r, u64 n, u64 words, u64 n_light, int bits, const u32 *place, u64 *counts) {
+    ctx.reserve(r.cl_loff, (n + 1) * 8);
+    ctx.reserve(r.cl_start, n * (words / 32) * 8);
+    if (n_light)
+        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 8.0 * n,
+                  key_offsets_kernel<u64><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(
+                      r.words.as<u64>(), n_light, bits, n, r.cl_loff.as<u64>()));
+    else
+        DL_CUDA(cudaMemsetAsync(r.cl_loff.p, 0, (n + 1) * 8, ctx.stream));
+    DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n * words,
+              closure_counts_kernel<<<grid_for(n * 32, T256, ctx), T256, 0, ctx.stream>>>(
+                  r.bm_t.as<u32>(), n, (u32) words, r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << bits) - 1, place,
+                  r.cl_start.as<uint2>(), counts));
+}
+
 u64 bit_rows_finish(Context &ctx, Run &r, u64 n, u64 words, const u64 *counts) {
     ctx.reserve(r.bm_first, (n + 1) * 8);
     const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
@@ -1595,20 +1485,11 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
         }
         pt.mark(PH_FINAL);
         u32 *place = r.cl_cols.as<u32>() + heavy.words * 32;
-        ctx.reserve(r.cl_start, n * (heavy.words / 32) * 8);
         DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n,
                   heavy_below_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(r.cl_cols.as<u32>(), heavy.h, n,
                                                                                      place));
-        // first result row of every target
-        ctx.reserve(r.cl_loff, (n + 1) * 8);
-        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 8.0 * n,
-                  key_offsets_kernel<u64><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(
-                      r.words.as<u64>(), light.n_words, g.bits, n, r.cl_loff.as<u64>()));
         ctx.reserve(ws.w0, (n + 1) * 8);
-        DL_LAUNCH(ctx, K_BITMAP_COLUMNS, 4.0 * n * heavy.words,
-                  closure_counts_kernel<<<grid_for(n * 32, T256, ctx), T256, 0, ctx.stream>>>(
-                      r.bm_t.as<u32>(), n, (u32) heavy.words, r.words.as<u64>(), r.cl_loff.as<u64>(),
-                      (1ull << g.bits) - 1, place, r.cl_start.as<uint2>(), ws.w0.as<u64>()));
+        bit_rows_count(ctx, r, n, heavy.words, light.n_words, g.bits, place, ws.w0.as<u64>());
         const u64 total = bit_rows_finish(ctx, r, n, heavy.words, ws.w0.as<u64>());
         if (total != nfull)
             throw Error(DL_ERR_INTERNAL, "closure holds " + std::to_string(total) + " tuples, expected " +
@@ -1661,7 +1542,8 @@ void closure_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 z0, u64 
     const u32 *cols = r.cl_cols.as<u32>();
     const u64 chunks = r.bm_words / 32;
     const bool dense = (u64) r.info.output_rows >= r.bm_n * r.bm_words * 32 / 3;
-    auto kern = dense ? closure_rows_kernel<true> : closure_rows_kernel<false>;
+    auto kern = r.bm_row_first ? (dense ? closure_rows_kernel<true, true> : closure_rows_kernel<false, true>)
+                               : (dense ? closure_rows_kernel<true, false> : closure_rows_kernel<false, false>);
     const u64 wave = resident_blocks(ctx, kern, 256, 0);
     const unsigned grid = (unsigned) std::max<u64>(1, std::min<u64>(wave, ((z1 - z0) * chunks + 7) / 8));
     DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * (z1 - z0) * r.bm_words,

@@ -42,9 +42,11 @@ u64 closure_pull_bytes(u64 n, u64 h);
 ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne, int bits, u64 n, const u64 *src,
                           u64 h, u64 max_level, DevBuf &t, DevBuf &cols);
 
-// The result of a run as bit rows (r.bm_t, r.cl_cols, r.cl_start, the light
-// pairs in r.words / r.cl_loff): first row of every target from the targets'
-// row counts; returns the number of rows.
+// The result of a run as bit rows (r.bm_t, r.cl_cols, the `n_light` light pairs
+// in r.words): rows of every target (counts) and of its chunks (r.cl_start), the
+// light pairs' place (r.cl_loff).
+void bit_rows_count(Context &ctx, Run &r, u64 n, u64 words, u64 n_light, int bits, const u32 *place, u64 *counts);
+// Then the first row of every target from the counts; returns the number of rows.
 u64 bit_rows_finish(Context &ctx, Run &r, u64 n, u64 words, const u64 *counts);
 
 // The pairs of heavy sources `src` (ascending, host) of one instance with ranks
@@ -53,6 +55,11 @@ u64 bit_rows_finish(Context &ctx, Run &r, u64 n, u64 words, const u64 *counts);
 // needed).
 void closure_heavy_words(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const std::vector<u64> &src,
                          u64 max_level, std::vector<u64> &cnt, u64 &n_words);
+
+// SG as bit rows (dl_sgrows.cu) over the CSR and its sorted edge words; false
+// when the rows do not fit.
+bool sg_rows(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt, PhaseTimer &pt,
+             u64 &nfull);
 
 // single_join (dl_selfjoin.cu): rows (x, z) with x -> b -> z for some b, over the
 // in-neighbour CSR (off[z]: the y with y -> z), as bit rows; `total`: join rows

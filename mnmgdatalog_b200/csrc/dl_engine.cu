@@ -739,6 +739,10 @@ static u64 *sg_edge_words(Context &ctx, const int32_t *rows, u64 n, const Graph 
     return sort_unique_into(ctx, ws.jbuf[0], ws.jbuf[1], n, 2 * g.bits, ne);
 }
 
+// Nodes up to which SG's bit rows are tried before the search over pairs when
+// the graph has edges enough (three matrices of 256 MB at this size).
+constexpr u32 SG_ROWS_FIRST = 46'000;
+
 // SG as a search over pairs; false (nothing reported) when the pairs are many
 // and the bit matrix would take them, or when memory runs out.
 static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_options &opt, PhaseTimer &pt,
@@ -807,8 +811,14 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
         u64 ne;
         u64 *e = sg_edge_words(ctx, rows, n, g, ne);  // sg.cu:150-153
         build_csr(ctx, e, ne, g);                     // sg.cu:162
-        if (search && pair_search_fits(ctx, g.csr, 0, g.n_ids))
+        // a small matrix and more than 1.3 edges a node: most likely many pairs
+        const bool rows_first = g.n_ids <= SG_ROWS_FIRST && ne * 10 > 13 * (u64) g.n_distinct;
+        if (search && !rows_first && pair_search_fits(ctx, g.csr, 0, g.n_ids))
             listed = sg_pairs_fixpoint(ctx, r, g, opt, pt, nfull);
+        if (search && !listed && bitmat_allowed(ctx, g.n_ids, true)) {
+            if (!rows_first) e = sg_edge_words(ctx, rows, n, g, ne);  // again: the search used the buffers
+            listed = sg_rows(ctx, r, g, e, ne, opt, pt, nfull);
+        }
         if (!listed && ((g.ids_affine && !search) || bitmat_choose(ctx, opt, g.n_ids, true))) {
             try {
                 nfull = sg_bitmap_fixpoint(ctx, r, g, opt, pt);

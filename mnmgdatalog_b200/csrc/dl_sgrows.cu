@@ -1,0 +1,464 @@
+// SG on bit rows, one owner per row.
+//
+// sg(x, y) :- e(a, x), sg(a, b), e(b, y) (sg.cu:244-390). sg is symmetric from
+// the base rule on, so with the newest pairs as bit rows D (row b, bit a), the new
+// pairs of row y are
+//     N(y) = union of a's children over a in W(y),   W(y) = OR of D(b), b -> y
+// minus the row's known pairs: everything row y needs is its in-neighbours'
+// newest rows, read as whole lines, and its children's scatter goes to a row in
+// shared memory. A row has one owner (a warp, or a CTA for long rows), so nothing
+// is merged between CTAs: the step on the matrix before this one (dl_bitmap.cu)
+// expanded the pairs of a source once and folded the result into every child's
+// row with an atomic per touched word of the matrix.
+// The base rule is the same step on the identity: N(y) = children of y's
+// parents, without y itself.
+//
+// Measured on B200, a mesh of 22K nodes and 38K edges (2.4e8 pairs, 133
+// iterations), edges and result rows on the device: 67 ms on the matrix, 17 ms here.
+#include "dl_closure.h"
+#include "dl_pull.cuh"
+
+namespace dl {
+namespace detail {
+namespace {
+
+// has[k] bit b = node 32 k + b has out-edges (words padded to the rows' length).
+__global__ void has_children_kernel(const u32 *__restrict__ off, u64 n, u64 words, u32 *__restrict__ has) {
+    for (u64 k = (u64) blockIdx.x * blockDim.x + threadIdx.x; k < words; k += (u64) gridDim.x * blockDim.x) {
+        u32 v = 0;
+        for (u32 b = 0; b < 32; ++b) {
+            const u64 x = k * 32 + b;
+            if (x < n && off[x + 1] > off[x]) v |= 1u << b;
+        }
+        has[k] = v;
+    }
+}
+
+// Level 0: row x = {x} for every node with children; tagged, so that the
+// children of x get on the first list. cols[i] = i (all ones past n).
+__global__ void sg_identity_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, u32 *__restrict__ cols) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    for (u64 x = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32; x < (u64) sh.words * 32; x += warps) {
+        if (lane == 0) cols[x] = x < sh.n ? (u32) x : EMPTY;
+        if (x >= sh.n || off[x + 1] == off[x]) continue;
+        const u32 gr = (u32) (x >> 10) >> sh.shift;
+        const u32 w0 = (gr << sh.shift) * 32, w1 = min(sh.words, w0 + (32u << sh.shift));
+        u32 *row = st.nxt + x * sh.words;
+        for (u32 k = w0 + lane; k < w1; k += 32) row[k] = k == (u32) (x >> 5) ? 1u << (x & 31) : 0u;
+        if (lane == 0) st.tag_next[x] = make_uint2(1u << gr, st.level);
+    }
+}
+
+struct SgTeam {
+    u32 item;            // the team's place in the list
+    u32 touched, news;   // activity bits of the row's touched chunks, and of those with new pairs
+};
+
+constexpr u32 SG_QUEUE = 512;  // bits of W a warp holds before it expands them
+
+// Per-warp part of a team's shared memory.
+struct SgWarp {
+    u32 queue[SG_QUEUE];
+    u32 wbeg[32], wpre[32];
+};
+
+// The children of the queued nodes into the row; returns the activity bits of the
+// chunks this lane's fell into. Not inlined: the kernel calls it in three places,
+// and with three copies of the walk it stalled on instruction fetches two issue
+// slots out of three.
+__device__ __noinline__ u32 sg_expand(SgWarp &mw, u32 qn, u32 *row, const u32 *__restrict__ off,
+                                      const u32 *__restrict__ val, u32 shift) {
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt(), le = lane == 31 ? ~0u : (2u << lane) - 1;
+    u32 mine = 0;
+    __syncwarp();
+    for (u32 q0 = 0; q0 < qn; q0 += 32) {
+        u32 beg = 0, deg = 0;
+        if (q0 + lane < qn) {
+            const u32 a = mw.queue[q0 + lane];
+            beg = __ldg(off + a);
+            deg = __ldg(off + a + 1) - beg;
+        }
+        auto put = [&](u32 x) {
+            atomicOr(&row[x >> 5], 1u << (x & 31));
+            mine |= 1u << ((x >> 10) >> shift);
+        };
+        // a few children each: every lane walks its own node's (a mesh's six at most
+        // cost less than sharing them out); else 32 of the batch's children at a time
+        const u32 most = __reduce_max_sync(0xffffffffu, deg);
+        if (most <= 8) {
+            for (u32 k = 0; k < most; k += 4) {
+                u32 x[4];
+#pragma unroll
+                for (u32 j = 0; j < 4; ++j)
+                    if (k + j < deg) x[j] = __ldg(val + beg + k + j);
+#pragma unroll
+                for (u32 j = 0; j < 4; ++j)
+                    if (k + j < deg) put(x[j]);
+            }
+        } else {
+            walk_rows(mw.wbeg, mw.wpre, beg, deg, val, lane, lt, le, 0xFFFFFFFFu, [&](u32 x, bool have) -> bool {
+                if (have) put(x);
+                return true;
+            });
+        }
+    }
+    __syncwarp();
+    return mine;
+}
+
+// One level: the new pairs of every row in the list, a team of NW warps per row
+// (TEAMS teams to a CTA, each with its row in shared memory). The warps take
+// the active chunks four at a time: OR of the in-neighbours' newest words (32
+// words of W a chunk), whose bits go to a queue across chunks, so that the
+// expansion runs on full batches of 32 pairs; their children are ORed into the
+// shared row. Then the touched chunks are compared with the matrix, four in
+// flight. Bound by latency and instructions, not by the lines: chunk by chunk
+// with batches a quarter full the mesh above took 26 ms, with its walk in three
+// copies 24 ms; 40 warps an SM at 48 registers 17.8 ms against 17.1 for 32 at 64;
+// six or eight chunks in flight spill (17.5 and 20 ms).
+template <int NW, int TEAMS>
+__global__ void __launch_bounds__(NW * TEAMS * 32, 1024 / (NW * TEAMS * 32))
+sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ val,
+               const u32 *__restrict__ roff, const u32 *__restrict__ rval, const u32 *__restrict__ has,
+               u32 *__restrict__ m, int base_rule, unsigned long long *__restrict__ fetch) {
+    extern __shared__ __align__(16) u32 smem[];
+    static_assert(NW == 1 || TEAMS == 1, "a team is a warp or the CTA");
+    const u64 n_list = st.count[st.level];
+    if (n_list == 0) return;  // the fixpoint was reached earlier
+    __shared__ SgTeam teams[TEAMS];
+    __shared__ SgWarp warps[NW * TEAMS];
+    const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const u32 part = NW == 1 ? 0 : wid;  // the warp's number in its team
+    u32 *row = smem + (NW == 1 ? wid : 0) * sh.words;
+    SgTeam &team = teams[NW == 1 ? wid : 0];
+    SgWarp &mw = warps[wid];
+    const u32 tl = NW == 1 ? lane : threadIdx.x;  // thread of the team
+    auto team_sync = [] {
+        if constexpr (NW == 1) __syncwarp();
+        else __syncthreads();
+    };
+    for (u32 k = tl; k < sh.words; k += NW * 32) row[k] = 0;
+    if (tl == 0) team.touched = team.news = 0;
+    u64 fresh = 0, rows = 0;
+    // the next four chunks of the activity mask (EMPTY: none); gc: chunks of the lowest
+    // granule already given out
+    auto four = [&](u32 &mm, u32 &gc, u32 (&c)[4]) {
+#pragma unroll
+        for (u32 q = 0; q < 4; ++q) {
+            c[q] = EMPTY;
+            if (mm) {
+                const u32 at = ((__ffs(mm) - 1) << sh.shift) + gc;
+                if (++gc >> sh.shift) {
+                    gc = 0;
+                    mm &= mm - 1;
+                }
+                if (at < sh.words / 32) c[q] = at;
+            }
+        }
+    };
+    for (;;) {
+        if (tl == 0) team.item = (u32) min(atomicAdd(fetch + st.level, 1ull), (unsigned long long) EMPTY);
+        team_sync();  // the row is clear, nothing marked
+        const u32 i = team.item;
+        if (i >= n_list) break;
+        const u32 y = st.list[i];
+        const u32 act = st.todo[y];
+        const u32 b = __ldg(roff + y), n = __ldg(roff + y + 1) - b;
+        auto parents = [&](u32 e0, u32 &p, u32 &a) {  // 32 in-neighbours from the e0-th on and their activity
+            p = a = 0;
+            if (e0 + lane < n) {
+                p = __ldg(rval + b + e0 + lane);
+                const uint2 tg = st.tag[p];
+                a = tg.y == st.level - 1 ? tg.x : 0u;
+            }
+        };
+        u32 y0, a0;
+        parents(0, y0, a0);
+        u32 mine = 0;  // chunks this lane's children fell into
+        u32 qn = 0;    // queued bits of W
+        auto drain = [&]() {
+            mine |= sg_expand(mw, qn, row, off, val, sh.shift);
+            qn = 0;
+        };
+        {
+            u32 mm = act, gc = 0, turn = 0;
+            while (mm) {
+                u32 c[4];
+                four(mm, gc, c);
+                if (NW > 1 && turn++ % NW != part) continue;
+                u32 w[4] = {0, 0, 0, 0};
+                for (u32 e0 = 0; e0 < n; e0 += 32) {
+                    u32 p = y0, a = a0;
+                    if (e0) parents(e0, p, a);
+                    for (u32 all = __ballot_sync(0xffffffffu, a != 0); all; all &= all - 1) {
+                        const u32 j = __ffs(all) - 1;
+                        const u32 *src = st.cur + (u64) __shfl_sync(0xffffffffu, p, j) * sh.words + lane;
+                        const u32 aj = __shfl_sync(0xffffffffu, a, j);
+#pragma unroll
+                        for (u32 q = 0; q < 4; ++q)
+                            if (c[q] != EMPTY && ((aj >> (c[q] >> sh.shift)) & 1u)) w[q] |= __ldg(src + c[q] * 32);
+                    }
+                }
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q) {
+                    if (c[q] == EMPTY) continue;
+                    u32 v = w[q] & __ldg(has + c[q] * 32 + lane);  // the others have no children
+                    const u32 cnt = __popc(v);
+                    const u32 incl = warp_inclusive_sum(cnt);
+                    const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+                    if (!total) continue;
+                    if (qn + total > SG_QUEUE) drain();
+                    if (total <= SG_QUEUE) {
+                        for (u32 at = qn + incl - cnt; v; v &= v - 1) mw.queue[at++] = (c[q] * 32 + lane) * 32 + __ffs(v) - 1;
+                        qn += total;
+                    } else {  // eight lanes' words at a time
+                        for (u32 g = 0; g < 4; ++g) {
+                            const u32 before = g ? __shfl_sync(0xffffffffu, incl, 8 * g - 1) : 0u;
+                            if ((lane >> 3) == g)
+                                for (u32 at = incl - cnt - before; v; v &= v - 1)
+                                    mw.queue[at++] = (c[q] * 32 + lane) * 32 + __ffs(v) - 1;
+                            qn = __shfl_sync(0xffffffffu, incl, 8 * g + 7) - before;
+                            drain();
+                        }
+                    }
+                }
+            }
+            drain();
+        }
+        u32 touched = __reduce_or_sync(0xffffffffu, mine);
+        if constexpr (NW > 1) {
+            if (lane == 0 && touched) atomicOr(&team.touched, touched);
+            __syncthreads();  // the row is complete
+            touched = team.touched;
+            if (tl == 0) team.news = 0;
+            __syncthreads();
+        } else {
+            __syncwarp();
+        }
+        // new pairs of the touched chunks
+        const bool can = __ldg(off + y + 1) > __ldg(off + y);
+        u32 news = 0;
+        {
+            u32 mm = touched, gc = 0, turn = 0;
+            while (mm) {
+                u32 c[4];
+                four(mm, gc, c);
+                if (NW > 1 && turn++ % NW != part) continue;
+                u32 v[4], old[4];
+                u32 *mp = m + (u64) y * sh.words + lane;
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q) {
+                    v[q] = old[q] = 0;
+                    if (c[q] != EMPTY) {
+                        const u32 k = c[q] * 32 + lane;
+                        v[q] = row[k];
+                        row[k] = 0;
+                        if (base_rule && (y >> 5) == k) v[q] &= ~(1u << (y & 31));  // x != y
+                        if (v[q]) old[q] = mp[c[q] * 32];
+                    }
+                }
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q) {
+                    if (c[q] == EMPTY) continue;
+                    const u32 nw = v[q] & ~old[q];
+                    if (nw) mp[c[q] * 32] = old[q] | nw;
+                    const bool line = __any_sync(0xffffffffu, nw != 0);
+                    if (line || sh.shift) st.nxt[(u64) y * sh.words + c[q] * 32 + lane] = nw;
+                    if (line) {
+                        news |= 1u << (c[q] >> sh.shift);
+                        fresh += __popc(nw);
+                        if (can) rows += __popc(nw & __ldg(has + c[q] * 32 + lane));
+                    }
+                }
+            }
+        }
+        if constexpr (NW > 1) {
+            if (lane == 0 && news) atomicOr(&team.news, news);
+            if (tl == 0) team.touched = 0;  // every warp has read it
+            __syncthreads();
+            news = team.news;
+        }
+        if (tl == 0) {
+            st.todo[y] = 0;
+            if (news) st.tag_next[y] = make_uint2(news, st.level);
+        }
+    }
+    fresh = warp_sum(fresh);
+    rows = warp_sum(rows);
+    if (lane == 0) {
+        if (fresh) atomicAdd(st.cnt + st.level, (unsigned long long) fresh);
+        if (rows) atomicAdd(st.deg + st.level, (unsigned long long) rows);
+    }
+}
+
+constexpr u64 SG_LEVELS = 8;  // levels launched between two host waits
+
+template <int NW, int TEAMS>
+void launch_level(Context &ctx, const PullShape &sh, const PullLevel &st, const Csr &csr, const u32 *roff,
+                  const u32 *rval, const u32 *has, u32 *m, bool base) {
+    const size_t smem = (size_t) TEAMS * sh.words * 4;
+    auto kern = sg_rows_kernel<NW, TEAMS>;
+    DL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    int per_sm = 0;
+    DL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * TEAMS * 32, smem));
+    const u64 grid = std::min<u64>((sh.n + TEAMS - 1) / TEAMS, (u64) ctx.sm_count * std::max(per_sm, 1));
+    DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+              kern<<<(unsigned) grid, NW * TEAMS * 32, smem, ctx.stream>>>(
+                  sh, st, csr.off, csr.val, roff, rval, has, m, base ? 1 : 0, st.deg + SG_LEVELS + 1));
+}
+
+bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
+                 PhaseTimer &pt, u64 &nfull) {
+    Workspace &ws = ctx.ws;
+    const u64 n = g.n_ids, words = (n + 1023) / 1024 * 32;
+    const u64 bytes = n * words * 4;
+    if (words * 4 + 24 * 1024 > 227 * 1024) return false;  // a row in shared memory beside the queues
+    if (3 * bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
+    u64 held = ws.cl_rows[0].cap + ws.cl_rows[1].cap;
+    for (const DevBuf &b : ctx.spares) held += b.cap;
+    if (3 * bytes > held / 2) {
+        size_t free_b = 0, total_b = 0;
+        DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (3 * bytes > ((u64) free_b + held) / 2) return false;
+    }
+    pt.mark(PH_INIT);
+    PullShape sh{n, (u32) words, 0};
+    while ((32u << sh.shift) < words / 32) ++sh.shift;
+    // in-neighbours: the edges sorted by target
+    ctx.reserve(ws.full[0], ne * 8);
+    ctx.reserve(ws.full[1], ne * 8);
+    DL_LAUNCH(ctx, K_PREP, 16.0 * ne,
+              pull_swap_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(edges, ne, g.bits,
+                                                                                ws.full[0].as<u64>()));
+    const u64 *rev = radix_sort(ctx, ws.full[0].as<u64>(), ws.full[1].as<u64>(), ne, Codec::Raw, 2 * g.bits);
+    ctx.reserve(ws.cl_roff, (n + 1) * 4);
+    ctx.reserve(ws.cl_rval, ne * 4);
+    u32 *roff = ws.cl_roff.as<u32>(), *rval = ws.cl_rval.as<u32>();
+    DL_LAUNCH(ctx, K_PREP, 0,
+              key_offsets_kernel<u32><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, g.bits, n, roff));
+    DL_LAUNCH(ctx, K_PREP, 12.0 * ne,
+              low_field_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, (1ull << g.bits) - 1, rval));
+    ctx.reserve(ws.bit_hasout, words * 4);
+    u32 *has = ws.bit_hasout.as<u32>();
+    DL_LAUNCH(ctx, K_PREP, 4.0 * n,
+              has_children_kernel<<<grid_for(words, T256, ctx), T256, 0, ctx.stream>>>(g.csr.off, n, words, has));
+    ctx.reserve(r.bm_t, bytes);
+    ctx.reserve(ws.cl_rows[0], bytes);
+    ctx.reserve(ws.cl_rows[1], bytes);
+    ctx.reserve(ws.cl_act, 8 * n * 4);
+    ctx.reserve(r.cl_cols, words * 32 * 4);
+    DL_CUDA(cudaMemsetAsync(r.bm_t.p, 0, bytes, ctx.stream));
+    u32 *p = ws.cl_act.as<u32>();
+    DL_CUDA(cudaMemsetAsync(p, 0xFF, 4 * n * 4, ctx.stream));       // tags: no level
+    DL_CUDA(cudaMemsetAsync(p + 4 * n, 0, 2 * n * 4, ctx.stream));  // todo
+    // counters of a batch of levels: list lengths (one more than levels), new
+    // pairs, joinable ones, next places of the lists; two sets, the next batch's first list length is copied over
+    constexpr u64 SET = 4 * (SG_LEVELS + 1);
+    ctx.reserve(ws.cl_levels, 2 * SET * 8);
+    u64 *sets[2] = {ws.cl_levels.as<u64>(), ws.cl_levels.as<u64>() + SET};
+    DL_CUDA(cudaMemsetAsync(sets[0], 0, SET * 8, ctx.stream));
+    u64 first = 1;  // first level of the batch
+    int set = 0;
+    auto view = [&](u64 level) {
+        const u64 in = (level + 1) & 1, out = level & 1;
+        PullLevel v;
+        v.level = (u32) level;
+        v.cur = ws.cl_rows[in].as<u32>();
+        v.nxt = ws.cl_rows[out].as<u32>();
+        v.tag = reinterpret_cast<uint2 *>(p + 2 * in * n);
+        v.tag_next = reinterpret_cast<uint2 *>(p + 2 * out * n);
+        v.todo = p + (4 + out) * n;
+        v.todo_next = p + (4 + in) * n;
+        v.list = p + (6 + out) * n;
+        v.list_next = p + (6 + in) * n;
+        v.count = reinterpret_cast<unsigned long long *>(sets[set]) - first;
+        v.cnt = v.count + SG_LEVELS + 1;
+        v.deg = v.cnt + SG_LEVELS + 1;
+        return v;
+    };
+    auto push = [&](u64 level) {
+        DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                  closure_push_kernel<<<grid_for(ne, PU_THREADS, ctx, 8), PU_THREADS, 0, ctx.stream>>>(
+                      view(level), edges, ne, g.bits));
+    };
+    DL_LAUNCH(ctx, K_PREP, 128.0 * n,
+              sg_identity_kernel<<<grid_for(words * 32 * 32, T256, ctx), T256, 0, ctx.stream>>>(
+                  sh, view(0), g.csr.off, r.cl_cols.as<u32>()));
+    push(0);
+    pt.mark(PH_JOIN);
+    // level 1 is the base rule, level k + 1 iteration k; level k + 1's joins are
+    // level k's joinable pairs
+    std::vector<u64> cnt(2, 0), joinable(2, 0);
+    nfull = 0;
+    for (bool done = false; !done;) {
+        // (no level past the last iteration that was asked for)
+        const u64 batch = opt.max_iterations > 0 ? std::min<u64>(SG_LEVELS, (u64) opt.max_iterations + 2 - first)
+                                                 : SG_LEVELS;
+        for (u64 level = first; level < first + batch; ++level) {
+            const bool base = level == 1;
+            if (words <= 1024) launch_level<1, 4>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
+            else if (words <= 4096) launch_level<4, 1>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
+            else launch_level<8, 1>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
+            push(level);
+        }
+        DL_CUDA(cudaMemsetAsync(sets[set ^ 1], 0, SET * 8, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(sets[set ^ 1], sets[set] + SG_LEVELS, 8, cudaMemcpyDeviceToDevice, ctx.stream));
+        u64 *hs = ctx.host_scalars;
+        DL_CUDA(cudaMemcpyAsync(hs, sets[set], SET * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        for (u64 k = 0; k < batch && !done; ++k) {
+            const u64 level = first + k, c = hs[SG_LEVELS + 1 + k], j = hs[2 * (SG_LEVELS + 1) + k];
+            nfull += c;
+            if (level == 1) {
+                cnt[1] = c;
+                joinable[1] = j;
+                continue;
+            }
+            r.deltas.push_back((i64) c);
+            r.joins.push_back((i64) joinable[1]);
+            r.fulls.push_back((i64) nfull);
+            joinable[1] = j;
+            done = c == 0 || (opt.max_iterations > 0 && level - 1 >= (u64) opt.max_iterations);
+        }
+        first += SG_LEVELS;
+        set ^= 1;
+    }
+    pt.mark(PH_FINAL);
+    if (nfull) {
+        ctx.reserve(ws.offsets, (n + 1) * 8);
+        bit_rows_count(ctx, r, n, words, 0, g.bits, nullptr, ws.offsets.as<u64>());
+        const u64 total = bit_rows_finish(ctx, r, n, words, ws.offsets.as<u64>());
+        if (total != nfull)
+            throw Error(DL_ERR_INTERNAL, "bit rows hold " + std::to_string(total) + " tuples, expected " +
+                                             std::to_string(nfull));
+        r.bm_row_first = true;
+    }
+    r.from_bitmat = true;
+    return true;
+}
+
+}  // namespace
+
+bool sg_rows(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt, PhaseTimer &pt,
+             u64 &nfull) {
+    bool done = false;
+    try {
+        done = sg_rows_run(ctx, r, g, edges, ne, opt, pt, nfull);
+    } catch (const Error &err) {
+        if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
+    }
+    if (!done) {
+        r.deltas.clear();
+        r.joins.clear();
+        r.fulls.clear();
+        r.from_bitmat = r.cl_rows = r.bm_row_first = false;
+        for (DevBuf *b : {&r.bm_t, &r.bm_first, &r.cl_cols, &r.cl_loff, &r.cl_start}) ctx.give_back(*b);
+        nfull = 0;
+    }
+    return done;
+}
+
+}  // namespace detail
+}  // namespace dl

@@ -30,7 +30,7 @@ CLASSES = [
     (r"join_emit_kernel|join_emit_bucket_kernel", "join_emit"),
     (r"digit0_hist_kernel", "join_count_scan"),
     (r"bucket_starts_kernel", "join_partition"),
-    (r"bitmat_unit_step_kernel|bitmat_set_edges_kernel|closure_(group|warp|cta|pull|pull_hub|push)_kernel|self_join_kernel|pair_level_kernel|pair_refill_kernel", "bitmap_expand"),
+    (r"bitmat_unit_step_kernel|bitmat_set_edges_kernel|closure_(group|warp|cta|pull|pull_hub|push)_kernel|self_join_kernel|pair_level_kernel|pair_refill_kernel|sg_rows_kernel", "bitmap_expand"),
     (r"bitmat_transpose_count|bitmat_column_count|column_offsets|closure_counts|heavy_below", "bitmap_columns"),
     (r"bitmat_extract|bitmat_column_rows|closure_rows|scan_kernel<.*(CountValue|SumValue)", "bitmap_extract"),
     (r"lbs_partition_kernel", "join_partition"),

@@ -1,0 +1,43 @@
+"""SG on bit rows (dl_sgrows.cu, what AUTO runs on well-connected graphs) against
+the stepped bit matrix, exactly: rows, iterations and per-iteration sizes -- with
+a warp, four and eight warps to a row, more than 32 chunks to an activity word,
+more than 32 in-neighbours and more than 8 children of a node, and runs that
+stop inside and at the end of a batch of levels."""
+import numpy as np
+import pytest
+
+from mnmgdatalog_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def _random(n, m, seed=0):
+    return np.random.default_rng(seed).integers(0, n, (m, 2))
+
+
+def _fan(n):
+    a = np.arange(n)
+    return np.concatenate([np.stack([np.zeros(n), a + 1], 1), np.stack([a + 1, np.full(n, 2 * n)], 1),
+                           np.stack([np.full(n, 2 * n), a + 3 * n], 1)])
+
+
+CASES = [("mesh", graphs.lattice3d(side=14, p=0.3, seed=5), 0), ("mesh_stops", graphs.lattice3d(side=14, p=0.3, seed=5), 7),
+         ("mesh_stops_8", graphs.lattice3d(side=20, p=0.3, seed=1), 8), ("one_chunk", _random(1000, 3000), 0),
+         ("degrees", graphs.chung_lu(n=4000, m=12_000, seed=3), 0), ("fan", _fan(1500), 0),
+         ("children_9", np.stack([np.repeat(np.arange(900), 9), (np.arange(8100) * 7) % 1000], 1), 0),
+         ("chunks_33", _random(34_000, 76_000, 1), 3), ("four_warps", _random(60_000, 130_000, 2), 3),
+         ("eight_warps", _random(135_000, 290_000, 3), 2), ("spread_ids", _random(3000, 9000, 4) * 700_001 - 2**31, 0)]
+
+
+@pytest.mark.parametrize("name,edges,stop", CASES, ids=[c[0] for c in CASES])
+def test_sg_rows_equal_matrix(engine, name, edges, stop):
+    import torch
+    e = np.ascontiguousarray(edges).astype(np.int32)
+    want = engine.sg(e, dedup="bitmap", output="device", max_iterations=stop)
+    got = engine.sg(torch.from_numpy(e).cuda(), output="device", max_iterations=stop)
+    assert got.iterations == want.iterations and got.nodes == want.nodes
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    assert torch.equal(got.rows, want.rows)
+    if want.output_tuples < 10**7:
+        assert np.array_equal(engine.sg(e, max_iterations=stop).rows, want.rows.cpu().numpy())
