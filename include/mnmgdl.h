@@ -304,6 +304,12 @@ DL_API dl_status dl_session_copy_output(dl_session *s, int64_t instance, int32_t
 DL_API dl_status dl_session_copy_deltas(const dl_session *s, int64_t instance, int64_t *dst, int64_t capacity);
 DL_API dl_status dl_session_copy_labels(dl_session *s, int64_t instance, int32_t *node_ids, int32_t *labels,
                                         int64_t capacity);
+/* The same for many finished instances, with one wait for all of them. */
+DL_API dl_status dl_session_copy_outputs(dl_session *s, const int64_t *instances, int64_t count, int32_t *const *dst,
+                                         const int64_t *capacity_rows, int32_t dst_on_device);
+DL_API dl_status dl_session_copy_labels_many(dl_session *s, const int64_t *instances, int64_t count,
+                                             int32_t *const *node_ids, int32_t *const *labels,
+                                             const int64_t *capacity);
 /* Frees a finished instance's result memory (its info stays readable). */
 DL_API dl_status dl_session_release(dl_session *s, int64_t instance);
 /* Device bytes the session's live buffers and unreleased results hold (its

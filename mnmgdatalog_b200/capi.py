@@ -37,7 +37,7 @@ EXPORTS = (
     "dl_compat_get_hash_table", "dl_compat_get_join", "dl_compat_get_join_nl",
     "dl_sort_unique_noalloc", "dl_sort_unique_noalloc_max_rows",
     "dl_session_create", "dl_session_admit", "dl_session_admit_many", "dl_session_step", "dl_session_poll", "dl_session_get_info",
-    "dl_session_copy_output", "dl_session_copy_deltas", "dl_session_copy_labels", "dl_session_release",
+    "dl_session_copy_output", "dl_session_copy_outputs", "dl_session_copy_labels_many", "dl_session_copy_deltas", "dl_session_copy_labels", "dl_session_release",
     "dl_session_memory", "dl_session_destroy", "dl_run_batch",
 )
 
@@ -135,6 +135,8 @@ def lib():
         "dl_session_poll": ([vp, vp, i64, pi64], C.c_int),
         "dl_session_get_info": ([vp, i64, C.POINTER(dl_run_info)], C.c_int),
         "dl_session_copy_output": ([vp, i64, vp, i64, i32], C.c_int),
+        "dl_session_copy_outputs": ([vp, vp, i64, vp, vp, i32], C.c_int),
+        "dl_session_copy_labels_many": ([vp, vp, i64, vp, vp, vp], C.c_int),
         "dl_session_copy_deltas": ([vp, i64, vp, i64], C.c_int),
         "dl_session_copy_labels": ([vp, i64, vp, vp, i64], C.c_int),
         "dl_session_release": ([vp, i64], C.c_int),

@@ -12,7 +12,8 @@ struct dl_context {
 };
 struct dl_hash_table {
     dl::HashTable *ht = nullptr;
-    dl_context *ctx = nullptr;
+    int device = 0;
+    std::shared_ptr<dl::ReturnBox> box;  // of the context that built it
 };
 struct dl_run {
     dl::Run *r = nullptr;
@@ -154,6 +155,10 @@ DL_API dl_status dl_context_destroy(dl_context *ctx) {
     if (!ctx) return DL_OK;
     cudaSetDevice(ctx->c.device);
     if (ctx->c.stream) cudaStreamSynchronize(ctx->c.stream);
+    {
+        std::lock_guard<std::mutex> lock(ctx->c.box->m);
+        ctx->c.box->open = false;  // what comes back later is freed
+    }
     ctx->c.release_all();
     if (ctx->c.ctrl) cudaFree(ctx->c.ctrl);
     if (ctx->c.host_scalars) cudaFreeHost(ctx->c.host_scalars);
@@ -185,7 +190,18 @@ DL_API dl_status dl_free(dl_context *ctx, void *p) {
     return guarded([&] {
         set_device(ctx);
         DL_CUDA(cudaStreamSynchronize(ctx->c.stream));
-        DL_CUDA(cudaFree(p));
+        dl::DevBuf b;
+        {
+            std::lock_guard<std::mutex> lock(ctx->c.box->m);
+            auto it = ctx->c.box->outs.find(p);
+            if (it != ctx->c.box->outs.end()) {
+                b.p = p;
+                b.cap = it->second;
+                ctx->c.box->outs.erase(it);
+            }
+        }
+        if (b.p) ctx->c.box->hand_back(b);
+        else DL_CUDA(cudaFree(p));
     });
 }
 
@@ -293,7 +309,8 @@ DL_API dl_status dl_build_hash_table(dl_context *ctx, const dl_entity *rel, int6
     DL_REQUIRE(ctx && out && n >= 0 && (rel || n == 0), "invalid argument");
     *out = nullptr;
     auto h = std::make_unique<dl_hash_table>();
-    h->ctx = ctx;
+    h->device = ctx->c.device;
+    h->box = ctx->c.box;
     dl_status st = guarded([&] {
         set_device(ctx);
         h->ht = dl::hash_table_build(ctx->c, (const u64 *) rel, (u64) n, load_factor);
@@ -313,10 +330,9 @@ DL_API dl_status dl_hash_table_info(const dl_hash_table *ht, int64_t *slots, int
 DL_API dl_status dl_hash_table_destroy(dl_hash_table *ht) {
     if (!ht) return DL_OK;
     if (ht->ht) {
-        cudaSetDevice(ht->ctx->c.device);
-        cudaStreamSynchronize(ht->ctx->c.stream);
-        ht->ht->table.release();
-        ht->ht->vals.release();
+        cudaSetDevice(ht->device);
+        ht->box->hand_back(ht->ht->table);
+        ht->box->hand_back(ht->ht->vals);
         delete ht->ht;
     }
     delete ht;
@@ -338,15 +354,29 @@ dl_status join_common(dl_context *ctx, int64_t n, dl_entity **out, int64_t *n_ou
         ctx->c.reserve(offs, (u64) n * 8);
         const u64 total = count(offs.as<u64>());
         if (total) {
-            void *p = nullptr;
-            cudaError_t e = cudaMalloc(&p, total * 8);
-            if (e != cudaSuccess) {
-                (void) cudaGetLastError();
+            // small outputs come from the context's cache and go back there (dl_free)
+            const bool pooled = total * 8 <= dl::ReturnBox::kLargest / 2;
+            dl::DevBuf o;
+            try {
+                if (pooled) {
+                    ctx->c.reserve_tight(o, total * 8);
+                } else if (cudaMalloc(&o.p, total * 8) != cudaSuccess) {
+                    (void) cudaGetLastError();
+                    o.p = nullptr;
+                    throw dl::Error(DL_ERR_OUT_OF_MEMORY, "join output of " + std::to_string(total) + " rows");
+                }
+                emit(offs.as<u64>(), total, o.as<u64>());
+                ctx->c.sync();
+            } catch (...) {
+                o.release();
                 ctx->c.give_back(offs);
-                throw dl::Error(DL_ERR_OUT_OF_MEMORY, "join output of " + std::to_string(total) + " rows");
+                throw;
             }
-            emit(offs.as<u64>(), total, (u64 *) p);
-            ctx->c.sync();
+            if (pooled) {
+                std::lock_guard<std::mutex> lock(ctx->c.box->m);
+                ctx->c.box->outs[o.p] = o.cap;
+            }
+            void *p = o.p;
             *out = (dl_entity *) p;
         }
         *n_out = (int64_t) total;
@@ -564,6 +594,34 @@ DL_API dl_status dl_session_copy_labels(dl_session *s, int64_t instance, int32_t
         if ((!node_ids || !labels) && dl::session_instance(*s->s, instance).n_ids)
             throw dl::Error(DL_ERR_INVALID_ARGUMENT, "node_ids/labels is NULL");
         dl::session_copy_labels(*s->s, instance, node_ids, labels, (u64) capacity);
+    });
+}
+
+DL_API dl_status dl_session_copy_outputs(dl_session *s, const int64_t *instances, int64_t count,
+                                         int32_t *const *dst, const int64_t *capacity_rows, int32_t dst_on_device) {
+    DL_REQUIRE(s && s->s && count >= 0 && (count == 0 || (instances && dst && capacity_rows)), "invalid argument");
+    return guarded([&] {
+        set_device(s->ctx);
+        for (int64_t i = 0; i < count; ++i) {
+            if (capacity_rows[i] < 0 || (!dst[i] && dl::session_instance(*s->s, instances[i]).n_result))
+                throw dl::Error(DL_ERR_INVALID_ARGUMENT, "dst is NULL or its capacity negative");
+        }
+        dl::session_copy_outputs(*s->s, instances, (u64) count, dst, capacity_rows, dst_on_device != 0);
+    });
+}
+
+DL_API dl_status dl_session_copy_labels_many(dl_session *s, const int64_t *instances, int64_t count,
+                                             int32_t *const *node_ids, int32_t *const *labels,
+                                             const int64_t *capacity) {
+    DL_REQUIRE(s && s->s && count >= 0 && (count == 0 || (instances && node_ids && labels && capacity)),
+               "invalid argument");
+    return guarded([&] {
+        set_device(s->ctx);
+        for (int64_t i = 0; i < count; ++i)
+            if (capacity[i] < 0 ||
+                ((!node_ids[i] || !labels[i]) && dl::session_instance(*s->s, instances[i]).n_ids))
+                throw dl::Error(DL_ERR_INVALID_ARGUMENT, "node_ids/labels is NULL or the capacity negative");
+        dl::session_copy_labels_many(*s->s, instances, (u64) count, node_ids, labels, capacity);
     });
 }
 

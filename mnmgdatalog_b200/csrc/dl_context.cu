@@ -37,6 +37,61 @@ void DevBuf::release() {
     cap = 0;
 }
 
+void ReturnBox::hand_back(DevBuf &b) {
+    if (!b.p || b.fixed) return;
+    cudaDeviceSynchronize();
+    {
+        std::lock_guard<std::mutex> lock(m);
+        if (open && b.cap <= kLargest) {
+            bufs.push_back(b);
+            b = DevBuf();
+            return;
+        }
+    }
+    b.release();
+}
+
+void SessionKit::release() {
+    if (ctrl) cudaFree(ctrl);
+    if (host_scalars) cudaFreeHost(host_scalars);
+    for (DevBuf *b : {&lookback, &sort_hist, &lbs_splits, &radix_part, &merge_splits, &bucket_cursor}) b->release();
+    ctrl = nullptr;
+    host_scalars = nullptr;
+}
+
+void *Context::host_staging(size_t bytes) {
+    if (bytes > (size_t(64) << 20)) return nullptr;
+    if (bytes > host_stage_bytes) {
+        if (host_stage) cudaFreeHost(host_stage);
+        host_stage = nullptr;
+        host_stage_bytes = 0;
+        const size_t want = std::max<size_t>(bytes + bytes / 2, 1 << 20);
+        DL_CUDA(cudaMallocHost((void **) &host_stage, want));
+        host_stage_bytes = want;
+    }
+    return host_stage;
+}
+
+void Context::reserve_tight(DevBuf &buf, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lock(box->m);
+        for (DevBuf &b : box->bufs) spares.push_back(b);
+        box->bufs.clear();
+    }
+    int best = -1;
+    for (int i = 0; i < (int) spares.size(); ++i)
+        if (spares[i].cap >= bytes && spares[i].cap <= 2 * bytes + (1 << 20) &&
+            (best < 0 || spares[i].cap < spares[best].cap))
+            best = i;
+    if (best >= 0) {
+        buf = spares[best];
+        spares.erase(spares.begin() + best);
+    } else {
+        allocate(buf, bytes);
+    }
+    trim_spares();
+}
+
 void Context::reserve(DevBuf &buf, size_t bytes, bool zero) {
     if (buf.fixed) {  // a fixed slice: it fits or the request is an error
         buf.reserve(bytes);
@@ -47,6 +102,11 @@ void Context::reserve(DevBuf &buf, size_t bytes, bool zero) {
     // A buffer that outgrows itself grows by half at least, so a relation that
     // grows every iteration is reallocated O(log) times, not at every step.
     const size_t want = buf.p ? std::max(bytes, buf.cap + buf.cap / 2) : bytes;
+    {
+        std::lock_guard<std::mutex> lock(box->m);
+        for (DevBuf &b : box->bufs) spares.push_back(b);
+        box->bufs.clear();
+    }
     // Best fit among the cached buffers, but never one far larger than the
     // request: a small result must not pin a large buffer that a growing
     // relation will need next.
@@ -136,6 +196,16 @@ void Context::release_all() {
     }
     for (auto &s : spares) s.release();
     spares.clear();
+    {
+        std::lock_guard<std::mutex> lock(box->m);
+        for (DevBuf &b : box->bufs) b.release();
+        box->bufs.clear();
+    }
+    for (SessionKit &k : kits) k.release();
+    kits.clear();
+    if (host_stage) cudaFreeHost(host_stage);
+    host_stage = nullptr;
+    host_stage_bytes = 0;
     DevBuf *all[] = {&ws.input, &ws.ids, &ws.w0, &ws.w1, &ws.csr_off, &ws.csr_val, &ws.full[0], &ws.full[1],
                      &ws.small[0], &ws.small[1], &ws.tiny[0], &ws.tiny[1], &ws.sample, &ws.sample_small,
                      &ws.jbuf[0], &ws.jbuf[1], &ws.offsets, &ws.wcc_label, &ws.wcc_flag, &ws.wcc_next,

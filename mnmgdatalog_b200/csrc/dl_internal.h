@@ -7,8 +7,11 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/mnmgdl.h"
@@ -143,6 +146,30 @@ struct Tuning {
 };
 Tuning default_tuning();
 
+// Buffers of handles that outlive a call (hash tables, join outputs) on their
+// way back to the context's cache. A handle may be destroyed on any thread and
+// after the context; hand_back() waits for the device first, like the cudaFree
+// that it replaces, so that no other stream still reads the buffer when the
+// context reuses it.
+struct ReturnBox {
+    static constexpr size_t kLargest = size_t(256) << 20;  // larger ones are freed: the memory is the caller's again
+    std::mutex m;
+    bool open = true;             // the context is alive
+    std::vector<DevBuf> bufs;     // given back, not yet in the cache
+    std::unordered_map<void *, size_t> outs;  // join outputs in callers' hands
+    void hand_back(DevBuf &b);    // frees b or keeps it for the context
+};
+
+// What a session needs besides buffers; kept by its parent context, so that a
+// batch does not pay for page-locking, allocating and freeing them.
+struct SessionKit {
+    Ctrl *ctrl = nullptr;
+    u64 *host_scalars = nullptr;
+    u32 epoch = 0;
+    DevBuf lookback, sort_hist, lbs_splits, radix_part, merge_splits, bucket_cursor;
+    void release();
+};
+
 struct Context {
     int device = 0;
     Tuning tune = default_tuning();
@@ -164,6 +191,13 @@ struct Context {
     Workspace ws;
     u64 run_join_total = 0, run_join_max = 0;  // join statistics of the current run
     std::vector<DevBuf> spares;     // buffers handed back by destroyed runs and sessions
+    std::shared_ptr<ReturnBox> box = std::make_shared<ReturnBox>();
+    std::vector<SessionKit> kits;   // of destroyed sessions
+    static constexpr size_t kKits = 4;
+    u64 *host_stage = nullptr;      // page-locked staging of result labels
+    size_t host_stage_bytes = 0;
+    // Page-locked memory of at least `bytes`, or null past 64 MiB.
+    void *host_staging(size_t bytes);
     // Freeing a multi-GB buffer costs milliseconds and synchronises the
     // device, so outgrown buffers stay cached; an allocation that fails
     // drops the whole cache and retries (Context::allocate).
@@ -190,6 +224,8 @@ struct Context {
     // Ensure buf holds `bytes`, preferring a spare buffer over cudaMalloc.
     void reserve(DevBuf &buf, size_t bytes, bool zero = false);
     void give_back(DevBuf &buf);
+    // A buffer that goes into a caller's hands: at most twice the size asked for.
+    void reserve_tight(DevBuf &buf, size_t bytes);
     void trim_spares();
     // Fresh allocation of `bytes` into an empty buf; on failure frees every
     // cached buffer and tries once more (with `minimum` bytes if given).

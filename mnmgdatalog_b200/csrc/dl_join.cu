@@ -123,8 +123,8 @@ HashTable *hash_table_build(Context &ctx, const u64 *rel, u64 n, double load_fac
     if (n == 0) return ht;
     DevBuf a, b;
     try {
-        a.reserve(n * sizeof(u64));
-        b.reserve(n * sizeof(u64));
+        ctx.reserve(a, n * sizeof(u64));
+        ctx.reserve(b, n * sizeof(u64));
         DL_CUDA(cudaMemcpyAsync(a.p, rel, n * sizeof(u64), cudaMemcpyDeviceToDevice, ctx.stream));
         u64 *sorted = radix_sort(ctx, a.as<u64>(), b.as<u64>(), n, Codec::Entity, 0);
         u64 *other = sorted == a.as<u64>() ? b.as<u64>() : a.as<u64>();
@@ -133,21 +133,21 @@ HashTable *hash_table_build(Context &ctx, const u64 *rel, u64 n, double load_fac
         u64 slots = 1;
         while ((double) slots * load_factor < (double) distinct) slots <<= 1;
         ht->slots = slots;
-        ht->table.reserve(slots * sizeof(HashSlot), true);
-        ht->vals.reserve(n * sizeof(u32));
+        ctx.reserve_tight(ht->table, slots * sizeof(HashSlot));
+        DL_CUDA(cudaMemsetAsync(ht->table.p, 0, slots * sizeof(HashSlot), ctx.stream));
+        ctx.reserve_tight(ht->vals, n * sizeof(u32));
         const unsigned grid = (unsigned) std::min<u64>((n + 255) / 256, (u64) ctx.sm_count * 16);
         DL_LAUNCH(ctx, K_HASH_BUILD, 8.0 * n, hash_insert_kernel<<<grid, 256, 0, ctx.stream>>>(sorted, n, ht->table.as<HashSlot>(), slots - 1,
                                                          &ctx.ctrl->err));
         DL_LAUNCH(ctx, K_HASH_BUILD, 8.0 * n, extract_values_kernel<<<grid, 256, 0, ctx.stream>>>(sorted, n, ht->vals.as<u32>()));
         ctx.sync();
     } catch (...) {
-        a.release();
-        b.release();
+        for (DevBuf *x : {&a, &b, &ht->table, &ht->vals}) ctx.give_back(*x);
         delete ht;
         throw;
     }
-    a.release();
-    b.release();
+    ctx.give_back(a);
+    ctx.give_back(b);
     return ht;
 }
 

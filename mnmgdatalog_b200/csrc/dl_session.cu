@@ -281,10 +281,9 @@ u64 session_select(Context &ctx, u64 *buf, u64 n, Keep keep, int slot) {
 void grow_keep(Context &ctx, DevBuf &b, size_t bytes, size_t keep) {
     if (b.p && b.cap >= bytes) return;
     DevBuf nb;
-    ctx.allocate(nb, std::max(bytes, b.cap * 3 / 2));
+    ctx.reserve(nb, std::max(bytes, b.cap * 3 / 2));
     if (keep && b.p) DL_CUDA(cudaMemcpyAsync(nb.p, b.p, keep, cudaMemcpyDeviceToDevice, ctx.stream));
-    ctx.sync();
-    b.release();
+    ctx.give_back(b);  // reused on the same stream, after the copy
     b = nb;
 }
 
@@ -940,12 +939,31 @@ SessionImpl *session_create(Context &parent, int program, const dl_options &opt,
     c.sm_count = parent.sm_count;
     c.prof_on = parent.prof_on;
     c.tune = parent.tune;
-    void *p = nullptr;
-    DL_CUDA(cudaMalloc(&p, sizeof(Ctrl)));
-    c.ctrl = (Ctrl *) p;
-    DL_CUDA(cudaMemset(p, 0, sizeof(Ctrl)));
-    DL_CUDA(cudaMallocHost((void **) &c.host_scalars, 64 * sizeof(u64)));
+    SessionKit kit;
+    if (!parent.kits.empty()) {
+        kit = parent.kits.back();
+        parent.kits.pop_back();
+    } else {
+        void *p = nullptr;
+        DL_CUDA(cudaMalloc(&p, sizeof(Ctrl)));
+        kit.ctrl = (Ctrl *) p;
+        const cudaError_t e = cudaMallocHost((void **) &kit.host_scalars, 64 * sizeof(u64));
+        if (e != cudaSuccess) {
+            kit.release();
+            DL_CUDA(e);
+        }
+    }
+    c.ctrl = kit.ctrl;
+    c.host_scalars = kit.host_scalars;
+    c.epoch = kit.epoch;
+    c.lookback = kit.lookback;
+    c.sort_hist = kit.sort_hist;
+    c.lbs_splits = kit.lbs_splits;
+    c.radix_part = kit.radix_part;
+    c.merge_splits = kit.merge_splits;
+    c.bucket_cursor = kit.bucket_cursor;
     std::memset(c.host_scalars, 0, 64 * sizeof(u64));
+    DL_CUDA(cudaMemsetAsync(c.ctrl, 0, sizeof(Ctrl), c.stream));
     c.spares = std::move(parent.spares);  // the parent's cached buffers serve the session
     parent.spares.clear();
     return s.release();
@@ -978,9 +996,13 @@ void session_destroy(SessionImpl *s) {
     for (DevBuf *b : wbufs) p.give_back(*b);
     for (auto &b : c.spares) p.give_back(b);
     c.spares.clear();
-    c.release_all();  // look-back words, histograms, split points, events
-    if (c.ctrl) cudaFree(c.ctrl);
-    if (c.host_scalars) cudaFreeHost(c.host_scalars);
+    // the control block, page-locked scalars and scan scratch serve the next session
+    SessionKit kit{c.ctrl, c.host_scalars, c.epoch, c.lookback, c.sort_hist, c.lbs_splits, c.radix_part, c.merge_splits,
+                   c.bucket_cursor};
+    c.lookback = c.sort_hist = c.lbs_splits = c.radix_part = c.merge_splits = c.bucket_cursor = DevBuf();
+    if (p.kits.size() < Context::kKits) p.kits.push_back(kit);
+    else kit.release();
+    c.release_all();  // events
     delete s;
 }
 
@@ -1191,51 +1213,109 @@ static SessionInstance &finished_instance(SessionImpl &s, i64 id) {
     return in;
 }
 
-void session_copy_output(SessionImpl &s, i64 id, int32_t *dst, u64 capacity, bool on_device) {
-    SessionInstance &in = finished_instance(s, id);
+// Rows of a finished instance into device memory (no wait).
+static void unpack_result(SessionImpl &s, const SessionInstance &in, int32_t *out) {
     Context &ctx = s.ctx;
     const u64 n = in.n_result;
-    if (capacity < n) throw Error(DL_ERR_INVALID_ARGUMENT, "output capacity too small");
-    if (n == 0) return;
-    DevBuf stage;
-    int32_t *tmp = dst;
-    if (!on_device) {
-        ctx.reserve(stage, n * 8);
-        tmp = stage.as<int32_t>();
-    }
     const int32_t *ids = in.ids();
     const unsigned g = grid_for(n, 256, ctx, 16);
     if (s.program == DL_PROGRAM_WCC)
-        DL_LAUNCH(ctx, K_PREP, 0, session_unpack_comp_kernel<<<g, 256, 0, ctx.stream>>>(in.result_u32(), n, ids, tmp));
+        DL_LAUNCH(ctx, K_PREP, 0, session_unpack_comp_kernel<<<g, 256, 0, ctx.stream>>>(in.result_u32(), n, ids, out));
     else if (s.program == DL_PROGRAM_SG)
         DL_LAUNCH(ctx, K_PREP, 0,
                   session_unpack_kernel<true><<<g, 256, 0, ctx.stream>>>(in.result_words(), n, s.bits, in.rank_lo,
-                                                                          ids, tmp));
+                                                                          ids, out));
     else
         DL_LAUNCH(ctx, K_PREP, 0,
                   session_unpack_kernel<false><<<g, 256, 0, ctx.stream>>>(in.result_words(), n, s.bits, in.rank_lo,
-                                                                           ids, tmp));
-    if (!on_device) DL_CUDA(cudaMemcpyAsync(dst, tmp, n * 8, cudaMemcpyDeviceToHost, ctx.stream));
+                                                                           ids, out));
+}
+
+void session_copy_outputs(SessionImpl &s, const i64 *ids, u64 count, int32_t *const *dst, const i64 *capacity,
+                          bool on_device) {
+    Context &ctx = s.ctx;
+    u64 largest = 0, total = 0;
+    for (u64 k = 0; k < count; ++k) {
+        const u64 n = finished_instance(s, ids[k]).n_result;
+        if ((u64) capacity[k] < n) throw Error(DL_ERR_INVALID_ARGUMENT, "output capacity too small");
+        largest = std::max(largest, n);
+        total += n;
+    }
+    if (total == 0) return;
+    if (on_device) {
+        for (u64 k = 0; k < count; ++k)
+            if (s.inst[ids[k]].n_result) unpack_result(s, s.inst[ids[k]], dst[k]);
+        ctx.sync();
+        return;
+    }
+    DevBuf stage;
+    ctx.reserve(stage, largest * 8);
+    for (u64 k = 0; k < count; ++k) {
+        const u64 n = s.inst[ids[k]].n_result;
+        if (!n) continue;
+        unpack_result(s, s.inst[ids[k]], stage.as<int32_t>());
+        DL_CUDA(cudaMemcpyAsync(dst[k], stage.p, n * 8, cudaMemcpyDeviceToHost, ctx.stream));
+    }
     ctx.sync();
     ctx.give_back(stage);
 }
 
-void session_copy_labels(SessionImpl &s, i64 id, int32_t *node_ids, int32_t *labels, u64 capacity) {
-    SessionInstance &in = finished_instance(s, id);
+void session_copy_output(SessionImpl &s, i64 id, int32_t *dst, u64 capacity, bool on_device) {
+    const i64 cap = (i64) capacity;
+    session_copy_outputs(s, &id, 1, &dst, &cap, on_device);
+}
+
+void session_copy_labels_many(SessionImpl &s, const i64 *ids, u64 count, int32_t *const *node_ids,
+                              int32_t *const *labels, const i64 *capacity) {
+    u64 total = 0;
+    for (u64 k = 0; k < count; ++k) {
+        const SessionInstance &in = finished_instance(s, ids[k]);
+        if ((u64) capacity[k] < in.n_ids) throw Error(DL_ERR_INVALID_ARGUMENT, "label capacity too small");
+        total += in.n_ids;
+    }
     if (s.program != DL_PROGRAM_WCC) throw Error(DL_ERR_INVALID_ARGUMENT, "labels exist only for WCC sessions");
+    if (total == 0) return;
+    // [node ids, labels] of every instance on the device, then to the host: in one
+    // page-locked copy while that is small, else straight to the destinations
     Context &ctx = s.ctx;
-    const u64 n = in.n_ids;
-    if (capacity < n) throw Error(DL_ERR_INVALID_ARGUMENT, "label capacity too small");
-    if (n == 0) return;
     DevBuf stage;
-    ctx.reserve(stage, n * 4);
-    DL_LAUNCH(ctx, K_PREP, 0,
-              session_unpack_labels_kernel<<<grid_for(n, 256, ctx, 16), 256, 0, ctx.stream>>>(
-                  in.labels(), in.rank_lo, n, in.ids(), stage.as<int32_t>()));
-    DL_CUDA(cudaMemcpyAsync(labels, stage.p, n * 4, cudaMemcpyDeviceToHost, ctx.stream));
-    DL_CUDA(cudaMemcpyAsync(node_ids, in.ids(), n * 4, cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.sync();
+    ctx.reserve(stage, total * 8);
+    int32_t *at = stage.as<int32_t>();
+    for (u64 k = 0; k < count; ++k) {
+        const SessionInstance &in = s.inst[ids[k]];
+        const u64 n = in.n_ids;
+        if (!n) continue;
+        DL_CUDA(cudaMemcpyAsync(at, in.ids(), n * 4, cudaMemcpyDeviceToDevice, ctx.stream));
+        DL_LAUNCH(ctx, K_PREP, 0,
+                  session_unpack_labels_kernel<<<grid_for(n, 256, ctx, 16), 256, 0, ctx.stream>>>(
+                      in.labels(), in.rank_lo, n, in.ids(), at + n));
+        at += 2 * n;
+    }
+    int32_t *host = (int32_t *) s.parent->host_staging(total * 8);
+    if (host) {
+        DL_CUDA(cudaMemcpyAsync(host, stage.p, total * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+    }
+    at = host ? host : stage.as<int32_t>();
+    for (u64 k = 0; k < count; ++k) {
+        const u64 n = s.inst[ids[k]].n_ids;
+        if (!n) continue;
+        if (host) {
+            std::memcpy(node_ids[k], at, n * 4);
+            std::memcpy(labels[k], at + n, n * 4);
+        } else {
+            DL_CUDA(cudaMemcpyAsync(node_ids[k], at, n * 4, cudaMemcpyDeviceToHost, ctx.stream));
+            DL_CUDA(cudaMemcpyAsync(labels[k], at + n, n * 4, cudaMemcpyDeviceToHost, ctx.stream));
+        }
+        at += 2 * n;
+    }
+    if (!host) ctx.sync();
     ctx.give_back(stage);
+}
+
+void session_copy_labels(SessionImpl &s, i64 id, int32_t *node_ids, int32_t *labels, u64 capacity) {
+    const i64 cap = (i64) capacity;
+    session_copy_labels_many(s, &id, 1, &node_ids, &labels, &cap);
 }
 
 void session_release(SessionImpl &s, i64 id) {

@@ -56,6 +56,11 @@ const SessionInstance &session_instance(const SessionImpl &s, i64 id);
 void session_info(const SessionImpl &s, i64 id, dl_run_info &info);
 void session_copy_output(SessionImpl &s, i64 id, int32_t *dst, u64 capacity, bool on_device);
 void session_copy_labels(SessionImpl &s, i64 id, int32_t *node_ids, int32_t *labels, u64 capacity);
+// The same for many instances, with one wait.
+void session_copy_outputs(SessionImpl &s, const i64 *ids, u64 count, int32_t *const *dst, const i64 *capacity,
+                          bool on_device);
+void session_copy_labels_many(SessionImpl &s, const i64 *ids, u64 count, int32_t *const *node_ids,
+                              int32_t *const *labels, const i64 *capacity);
 void session_release(SessionImpl &s, i64 id);
 u64 session_device_bytes(const SessionImpl &s);
 u64 session_active(const SessionImpl &s);

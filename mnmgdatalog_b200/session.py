@@ -170,6 +170,38 @@ class Session:
             res.node_ids, res.labels = ids, lab
         return res
 
+    def results(self, instances, *, output: str = "host", labels: bool = False) -> list:
+        """RunResults of finished instances, copied with one wait for all of them."""
+        from .engine import _torch
+        ids = list(instances)
+        res = [self.result(i, output="none") for i in ids]
+        if output not in ("host", "device", "none"):
+            raise DatalogError(1, f"output must be host, device or none, not {output!r}")
+        n = len(ids)
+        idv = np.asarray(ids, dtype=np.int64)
+        if output != "none" and n:
+            sizes = np.asarray([r.output_tuples for r in res], dtype=np.int64)
+            if output == "host":
+                for r in res:
+                    r.rows = np.empty((r.output_tuples, 2), dtype=np.int32)
+                ptrs = [r.rows.ctypes.data for r in res]
+            else:
+                torch = _torch()
+                for r in res:
+                    r.rows = torch.empty((r.output_tuples, 2), dtype=torch.int32, device=f"cuda:{self.engine.device}")
+                ptrs = [r.rows.data_ptr() for r in res]
+            pv = (C.c_void_p * n)(*[p if k else None for p, k in zip(ptrs, sizes)])
+            check(lib().dl_session_copy_outputs(self.handle, idv.ctypes.data, n, pv, sizes.ctypes.data,
+                                                1 if output == "device" else 0))
+        if labels and self._prog == capi.PROGRAM_WCC and n:
+            for r in res:
+                r.node_ids, r.labels = np.empty(r.nodes, dtype=np.int32), np.empty(r.nodes, dtype=np.int32)
+            nodes = np.asarray([r.nodes for r in res], dtype=np.int64)
+            iv = (C.c_void_p * n)(*[r.node_ids.ctypes.data if r.nodes else None for r in res])
+            lv = (C.c_void_p * n)(*[r.labels.ctypes.data if r.nodes else None for r in res])
+            check(lib().dl_session_copy_labels_many(self.handle, idv.ctypes.data, n, iv, lv, nodes.ctypes.data))
+        return res
+
     def release(self, instance: int) -> None:
         """Frees a finished instance's result memory."""
         check(lib().dl_session_release(self.handle, instance))
@@ -198,4 +230,4 @@ def run_batch(engine, program: str, edge_sets, *, wcc_stop: str = "reference", m
     check(lib().dl_run_batch(engine.ctx, prog, ptrs, rows, count, on_dev.pop() if on_dev else 0, C.byref(opts),
                              C.byref(h)))
     with Session(engine, program, _handle=h) as s:
-        return [s.result(i, output=output, labels=labels) for i in range(count)]
+        return s.results(range(count), output=output, labels=labels)

@@ -1,0 +1,69 @@
+"""Buffers behind handles: hash tables and join outputs come from the context's
+cache and go back to it, whatever the order in which they are given up."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from mnmgdatalog_b200 import DatalogError, Engine, graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(n, m, seed):
+    import torch
+    return torch.from_numpy(np.random.default_rng(seed).integers(0, n, (m, 2)).astype(np.int32)).cuda()
+
+
+def test_hash_table_outlives_its_context():
+    with Engine(0) as eng:
+        ht = eng.get_hash_table(_pairs(50, 400, 1))
+    ht.close()  # the context is gone: the memory is freed
+
+
+def test_reused_buffers_hold_no_old_rows():
+    from oracle import ops
+    with Engine(0) as eng:
+        for seed, (n, m) in enumerate([(500, 4000), (20, 300), (500, 4000), (3000, 9000), (20, 300)]):
+            rel, probe = _pairs(n, m, seed), _pairs(n, m // 2, 100 + seed)
+            ht = eng.get_hash_table(rel)
+            got = eng.get_join(ht, probe).cpu().numpy()
+            want = ops.join(rel.cpu().numpy(), probe.cpu().numpy())
+            order = lambda a: a[np.lexsort((a[:, 1], a[:, 0]))]  # noqa: E731
+            assert np.array_equal(order(got), order(np.asarray(want)))
+            ht.close()
+
+
+def test_join_outputs_are_separate_and_freed_once():
+    from mnmgdatalog_b200.capi import check, lib
+    with Engine(0) as eng:
+        ht = eng.get_hash_table(_pairs(100, 2000, 1))
+        probe = _pairs(100, 500, 2)
+        ptrs = []
+        for _ in range(3):
+            out, n = C.c_void_p(), C.c_int64()
+            check(lib().dl_join(eng.ctx, ht.handle, C.c_void_p(probe.data_ptr()), len(probe), C.byref(out), C.byref(n)))
+            ptrs.append(out.value)
+        assert len(set(ptrs)) == 3
+        for p in ptrs:
+            check(lib().dl_free(eng.ctx, C.c_void_p(p)))
+        ht.close()
+
+
+@pytest.mark.parametrize("prog", ["tc", "sg", "wcc"])
+def test_results_in_one_call(engine, prog):
+    sets = [graphs.dag(n=300, extra=90, seed=1), np.zeros((0, 2), np.int32), graphs.dag(n=80, extra=10, seed=2)]
+    with engine.session(prog) as s:
+        ids = s.admit_many(sets)
+        s.run()
+        for out in ("host", "device", "none"):
+            for i, r in zip(reversed(ids), s.results(reversed(ids), output=out, labels=True)):
+                w = s.result(i, output=out, labels=True)
+                if out != "none":
+                    assert np.array_equal(np.asarray(r.rows.cpu() if out == "device" else r.rows),
+                                          np.asarray(w.rows.cpu() if out == "device" else w.rows))
+                if prog == "wcc":
+                    assert np.array_equal(r.labels, w.labels) and np.array_equal(r.node_ids, w.node_ids)
+        assert s.results([]) == []
+        with pytest.raises(DatalogError):
+            s.results([99])
