@@ -21,6 +21,7 @@
 #include "dl_engine.h"
 #include "dl_engine_detail.h"
 #include "dl_pairs.h"
+#include "dl_wcc.h"
 
 namespace dl {
 namespace detail {
@@ -152,27 +153,6 @@ __global__ void unpack_rows_kernel(const u64 *__restrict__ w, u64 n, int bits, c
         r.y = KeyFirst ? lo : hi;
         reinterpret_cast<int2 *>(out)[i] = r;
     }
-}
-
-__global__ void wcc_init_kernel(u32 n, u32 *__restrict__ label, u32 *__restrict__ flag, u64 *__restrict__ delta) {
-    GRID_STRIDE(u, (u64) n) {
-        label[u] = (u32) u;
-        flag[u] = 0;
-        delta[u] = (u << 32) | u;
-    }
-}
-
-__global__ void wcc_next_delta_kernel(const u32 *__restrict__ nodes, u64 count, const u32 *__restrict__ label,
-                                      u32 *__restrict__ flag, u64 *__restrict__ delta) {
-    GRID_STRIDE(i, count) {
-        const u32 v = nodes[i];
-        delta[i] = ((u64) v << 32) | label[v];
-        flag[v] = 0;
-    }
-}
-
-__global__ void wcc_count_kernel(const u32 *__restrict__ label, u32 n, u32 *__restrict__ cnt) {
-    GRID_STRIDE(u, (u64) n) atomicAdd(&cnt[label[u]], 1u);
 }
 
 // Scan source: 1 for every label rank that names a component.
@@ -912,51 +892,23 @@ static void run_wcc_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, bo
         build_csr(ctx, e, ne, g);
         const u32 nn = g.n_ids;
         ctx.reserve(ws.wcc_label, (u64) nn * 4);
-        ctx.reserve(ws.wcc_flag, (u64) nn * 4);
-        ctx.reserve(ws.wcc_next, ((u64) nn + 1) * 4);
-        ctx.reserve(ws.w0, (u64) nn * 8);
-        ctx.reserve(ws.w1, (u64) nn * 8);
-        u32 *label = ws.wcc_label.as<u32>(), *flag = ws.wcc_flag.as<u32>(), *next = ws.wcc_next.as<u32>();
-        u64 *dcur = ws.w0.as<u64>(), *dnext = ws.w1.as<u64>();
-        DL_LAUNCH(ctx, K_PREP, 0, wcc_init_kernel<<<grid_for(nn, T256, ctx), T256, 0, ctx.stream>>>(nn, label, flag, dcur));  // wcc.cu:211-231
-        DL_CHECK_LAUNCH();
-        u32 *next_count = reinterpret_cast<u32 *>(&ctx.ctrl->scalar[9]);
-        u64 ndelta = nn;
-        i64 prev = (i64) nn;
-        for (int it = 0;; ++it) {  // wcc.cu:255-387
-            pt.mark(PH_JOIN);
-            ctx.reserve(ws.offsets, std::max<u64>(ndelta, 1) * 8);
-            DL_CUDA(cudaMemsetAsync(next_count, 0, sizeof(u32), ctx.stream));
-            WccSrc src{g.csr.off, g.csr.val, dcur, label, flag, next, next_count};
-            const u64 total = count_matches(ctx, src, ndelta, ws.offsets.as<u64>());
-            ctx.run_join_total += total;
-            ctx.run_join_max = std::max(ctx.run_join_max, total);
-            if (total) emit_matches(ctx, src, ndelta, ws.offsets.as<u64>(), total, nullptr, nullptr, 0, nullptr);
-            pt.mark(PH_MERGE);
-            DL_CUDA(cudaMemcpyAsync(ctx.host_scalars + 2, next_count, sizeof(u32), cudaMemcpyDeviceToHost, ctx.stream));
-            ctx.sync();
-            const u64 nnew = *reinterpret_cast<u32 *>(ctx.host_scalars + 2);
-            if (nnew) {
-                DL_LAUNCH(ctx, K_PREP, 0, wcc_next_delta_kernel<<<grid_for(nnew, T256, ctx), T256, 0, ctx.stream>>>(next, nnew, label, flag, dnext));
-            }
-            std::swap(dcur, dnext);
-            ndelta = nnew;
-            r.deltas.push_back((i64) nnew);
-            r.joins.push_back((i64) total);
-            r.fulls.push_back((i64) nn);
-            if (opt.wcc_stop == DL_WCC_STOP_FIXPOINT) {
-                if (nnew == 0) break;
-            } else if ((i64) nnew == prev) {
-                break;  // wcc.cu:366-383
-            }
-            prev = (i64) nnew;
-            if (opt.max_iterations > 0 && it + 1 >= opt.max_iterations) break;
+        u32 *label = ws.wcc_label.as<u32>();
+        pt.mark(PH_JOIN);
+        WccRun run = wcc_propagate(ctx, g.csr, 0, nn, {0}, {nn}, opt.wcc_stop, opt.max_iterations, label);
+        r.deltas = std::move(run.deltas[0]);
+        r.joins = std::move(run.joins);
+        r.fulls.assign(r.deltas.size(), (i64) nn);
+        for (i64 j : r.joins) {
+            ctx.run_join_total += (u64) j;
+            ctx.run_join_max = std::max(ctx.run_join_max, (u64) j);
         }
         // Finalize (wcc.cu:389-472): component ids and the largest size.
         pt.mark(PH_FINAL);
-        u32 *cnt = reinterpret_cast<u32 *>(ws.w1.p);  // reuse: nn u32 counters
+        ctx.reserve(ws.w0, (u64) nn * 8);
+        ctx.reserve(ws.w1, (u64) nn * 4);
+        u32 *cnt = ws.w1.as<u32>();
         DL_CUDA(cudaMemsetAsync(cnt, 0, (u64) nn * 4, ctx.stream));
-        DL_LAUNCH(ctx, K_PREP, 0, wcc_count_kernel<<<grid_for(nn, T256, ctx), T256, 0, ctx.stream>>>(label, nn, cnt));
+        wcc_label_counts(ctx, label, nn, 0, cnt);
         u64 *pos = ws.w0.as<u64>();
         u64 *largest = &ctx.ctrl->scalar[10];
         DL_CUDA(cudaMemsetAsync(largest, 0, sizeof(u64), ctx.stream));

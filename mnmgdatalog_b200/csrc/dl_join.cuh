@@ -25,8 +25,6 @@ struct CsrSrc {
     const u64 *probe;
     int bits;
     static constexpr bool kSelfFilter = (K == EmitKind::ZV_NOSELF);
-    static constexpr bool kWrite = true;
-    static constexpr int kProfKind = K_JOIN_EMIT;
     static double prof_bytes(u64 n, u64 total) { return 8.0 * n + 16.0 * total; }
     __device__ __forceinline__ u64 degree(u64 i) const {
         const u32 k = (u32) (probe[i] >> bits);
@@ -68,8 +66,6 @@ struct HashSrc {
     u64 mask;
     const u64 *probe;
     static constexpr bool kSelfFilter = false;
-    static constexpr bool kWrite = true;
-    static constexpr int kProfKind = K_JOIN_EMIT;
     static double prof_bytes(u64 n, u64 total) { return 8.0 * n + 16.0 * total; }
     __device__ __forceinline__ void lookup(u32 key, u64 &begin, u64 &count) const {
         u64 h = fmix32(key) & mask;
@@ -106,8 +102,6 @@ struct SortedSrc {
     u64 n_rel;
     const u64 *probe;
     static constexpr bool kSelfFilter = false;
-    static constexpr bool kWrite = true;
-    static constexpr int kProfKind = K_JOIN_EMIT;
     static double prof_bytes(u64 n, u64 total) { return 8.0 * n + 16.0 * total; }
     __device__ __forceinline__ u64 bound(int key, bool upper) const {
         u64 lo = 0, hi = n_rel;
@@ -129,44 +123,6 @@ struct SortedSrc {
         payload = p >> 32;
     }
     __device__ __forceinline__ u64 word(u64 idx, u64 v) const { return (v << 32) | (rel[idx] >> 32); }
-};
-
-// WCC min-label propagation (wcc.cu:255-387 as one kernel per iteration).
-// Probe words are delta entries (node << 32) | label, the label being the
-// node's label at the end of the previous iteration (Jacobi semantics, as
-// in the reference's join of t_delta with the edges). Each match lowers the
-// neighbour's label with atomicMin; the first thread that lowers a node in
-// this iteration appends it to the next delta list.
-struct WccSrc {
-    const u32 *off;
-    const u32 *val;
-    const u64 *delta;
-    u32 *label;
-    u32 *flag;
-    u32 *next_nodes;
-    u32 *next_count;
-    static constexpr bool kSelfFilter = false;
-    static constexpr bool kWrite = false;
-    static constexpr int kProfKind = K_WCC_PROPAGATE;
-    static double prof_bytes(u64 n, u64 total) { return 8.0 * n + 36.0 * total; }
-    __device__ __forceinline__ u64 degree(u64 i) const {
-        const u32 k = (u32) (delta[i] >> 32);
-        return (u64) (off[k + 1] - off[k]);
-    }
-    __device__ __forceinline__ void item(u64 i, u64 &begin, u64 &payload) const {
-        const u64 p = delta[i];
-        begin = off[(u32) (p >> 32)];
-        payload = (u32) p;
-    }
-    __device__ __forceinline__ u64 word(u64 idx, u64 l) const {
-        const u32 nbr = val[idx];
-        const u32 lab = (u32) l;
-        if (lab < label[nbr]) {  // cheap pre-check; atomicMin decides
-            const u32 old = atomicMin(&label[nbr], lab);
-            if (lab < old && atomicExch(&flag[nbr], 1u) == 0u) next_nodes[atomicAdd(next_count, 1u)] = nbr;
-        }
-        return 0;
-    }
 };
 
 template <class Src>
@@ -207,7 +163,6 @@ join_emit_kernel(Src src, u64 n_probe, const u64 *__restrict__ offsets, u64 tota
         }
         j = lo - 1;
         const u64 w = src.word(s.begin[j] + (o - s.obeg[j]), s.payload[j]);
-        if (!Src::kWrite) continue;
         out[o] = w;
         if (Src::kSelfFilter && w == ~0ull) ++selfs;
         if (ndig > 0) {
@@ -400,7 +355,7 @@ void emit_matches(Context &ctx, const Src &src, u64 n, const u64 *offsets, u64 t
                                                                                      splits));
     auto kern = join_emit_kernel<Src>;
     DL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(JoinSmem)));
-    DL_LAUNCH(ctx, Src::kProfKind, Src::prof_bytes(n, total), kern<<<(unsigned) tiles, JN_THREADS, sizeof(JoinSmem), ctx.stream>>>(src, n, offsets, total, splits, out, hist,
+    DL_LAUNCH(ctx, K_JOIN_EMIT, Src::prof_bytes(n, total), kern<<<(unsigned) tiles, JN_THREADS, sizeof(JoinSmem), ctx.stream>>>(src, n, offsets, total, splits, out, hist,
                                                                          ndig, self_pairs));
 }
 

@@ -7,16 +7,14 @@
 // per-iteration launch and synchronisation cost is paid once for all of them.
 // Instances are admitted at any iteration boundary (continuous batching):
 // their edges are appended to the union's offset table (their ranks are above
-// every rank in use, so the table stays sorted) and their initial delta joins
-// the next iteration. TC's and SG's instances do not need the common steps: a
-// source's (TC, dl_closure.cu) or a pair's (SG, dl_pairs.cu) search never meets
-// another instance's, so the instances admitted together are searched to their
-// fixpoints in one go and the steps report their iterations one by one; SG
-// instances whose degrees do not suit the search keep the common steps. Each instance keeps its own iteration count and delta
-// sequence (a per-instance histogram of every iteration's delta) and leaves
-// the union when it reaches its own fixpoint -- for WCC with the reference's
-// stop rule an instance is frozen (its delta entries dropped) at the iteration
-// where that rule fires, exactly where the reference program would stop.
+// every rank in use, so the table stays sorted). No instance needs the common
+// steps: a source's (TC, dl_closure.cu) or a pair's (SG, dl_pairs.cu) search and a
+// component's labels (WCC, dl_wcc.cu) never meet another instance's, so the
+// instances admitted together are computed to their own stops in one go -- for
+// WCC with the reference's rule the iteration where that rule fires for the
+// instance -- and the steps report their iterations one by one. SG instances whose
+// degrees do not suit the search keep the common steps: their initial delta joins
+// the next iteration, and each leaves the union at its own fixpoint.
 // Results are bit-exact with running each query alone.
 #include <algorithm>
 #include <cstring>
@@ -28,6 +26,7 @@
 #include "dl_pairs.h"
 #include "dl_scan.cuh"
 #include "dl_session.h"
+#include "dl_wcc.h"
 
 namespace dl {
 namespace {
@@ -164,39 +163,6 @@ __global__ void session_bounds_kernel(Runs3 runs, const u64 *__restrict__ lohi, 
     }
 }
 
-__global__ void session_label_init_kernel(u32 *__restrict__ label, u32 *__restrict__ flag, u64 lo, u64 hi,
-                                          u64 *__restrict__ delta) {
-    GRID_STRIDE(i, hi - lo) {
-        const u64 r = lo + i;
-        label[r] = (u32) r;
-        flag[r] = 0;
-        delta[i] = (r << 32) | r;
-    }
-}
-
-__global__ void session_next_delta_kernel(const u32 *__restrict__ nodes, u64 count, const u32 *__restrict__ label,
-                                          u32 *__restrict__ flag, u64 *__restrict__ delta) {
-    GRID_STRIDE(i, count) {
-        const u32 v = nodes[i];
-        delta[i] = ((u64) v << 32) | label[v];
-        flag[v] = 0;
-    }
-}
-
-// Slot t of a concatenation of instance rank ranges (instance k from slot
-// off[k], ranks lo[k]...): counts the component label of the node into
-// cnt[off[k] + label - lo[k]] and copies the node's label.
-__global__ void session_wcc_count_kernel(const u32 *__restrict__ label, const u64 *__restrict__ lo,
-                                         const u64 *__restrict__ off, u32 n, u64 total, u32 *__restrict__ cnt,
-                                         u32 *__restrict__ labels_out) {
-    GRID_STRIDE(t, total) {
-        const u32 k = segment_of(off, n, t);
-        const u32 l = label[lo[k] + (t - off[k])];
-        labels_out[t] = l;
-        atomicAdd(&cnt[off[k] + (l - lo[k])], 1u);
-    }
-}
-
 struct NonZero {
     const u32 *c;
     __device__ __forceinline__ u64 degree(u64 i) const { return c[i] != 0u; }
@@ -307,12 +273,11 @@ struct SessionImpl {
     u64 dead = 0;  // words of finished instances still in the full runs
     DevBuf delta;  // union delta (probe of the next iteration)
     u64 n_delta = 0;
-    DevBuf label, flag, nextl;  // WCC
     DevBuf inst_lo, inst_hi;    // device copies of the active instances' rank ranges
     DevBuf counts;              // per instance delta counts
     DevBuf range_lo;            // first ranks of the instances of a range count
     DevBuf admit_off, admit_first;  // row offsets / first tagged ids of an admission
-    DevBuf live;                // per active instance flag (WCC freezing)
+    DevBuf live;                // per active instance flag (frozen by max_iterations)
     std::vector<SessionInstance> inst;
     std::vector<i64> active;    // instance ids in rank order
     std::vector<i64> finished;  // finished since the last poll
@@ -526,62 +491,10 @@ void extract_words(SessionImpl &s, const std::vector<i64> &ids) {
     }
 }
 
-// Components (ascending local ranks), largest component and per-node labels
-// of finished WCC instances, all in one pass over their rank ranges.
-void extract_components(SessionImpl &s, const std::vector<i64> &ids) {
-    Context &ctx = s.ctx;
-    const u64 n = ids.size();
-    std::vector<u64> off(n + 1, 0);
-    for (u64 k = 0; k < n; ++k) off[k + 1] = off[k] + s.inst[ids[k]].n_ids;
-    const u64 total = off[n];
-    upload_ranges(s, ids);
-    // s.counts: slot offsets [n + 1] then largest [n] then component starts [n]
-    ctx.reserve(s.counts, (3 * n + 1) * 8);
-    u64 *d_off = s.counts.as<u64>(), *d_big = d_off + n + 1, *d_start = d_big + n;
-    DL_CUDA(cudaMemcpyAsync(d_off, off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, ctx.stream));
-    DL_CUDA(cudaMemsetAsync(d_big, 0, n * 8, ctx.stream));
-    DevBuf cnt, pos;
-    ctx.reserve(cnt, std::max<u64>(total, 1) * 4);
-    ctx.reserve(pos, std::max<u64>(total, 1) * 8);
-    DL_CUDA(cudaMemsetAsync(cnt.p, 0, total * 4, ctx.stream));
-    auto labels = make_block(ctx, total * 4);
-    const u64 *lo = s.range_lo.as<u64>();
-    DL_LAUNCH(ctx, K_PREP, 0,
-              session_wcc_count_kernel<<<grid_for(total, 256, ctx, 8), 256, 0, ctx.stream>>>(
-                  s.label.as<u32>(), lo, d_off, (u32) n, total, cnt.as<u32>(), labels->as<u32>()));
-    const u64 nc = count_matches(ctx, NonZero{cnt.as<u32>()}, total, pos.as<u64>());
-    auto comps = make_block(ctx, nc * 4);
-    DL_LAUNCH(ctx, K_PREP, 0,
-              session_wcc_comp_kernel<<<grid_for(total, 256, ctx, 8), 256, 0, ctx.stream>>>(
-                  cnt.as<u32>(), pos.as<u64>(), d_off, (u32) n, total, comps->as<u32>(),
-                  (unsigned long long *) d_big, d_start));
-    std::vector<u64> h(2 * n);
-    DL_CUDA(cudaMemcpyAsync(h.data(), d_big, 2 * n * 8, cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.sync();
-    for (u64 k = 0; k < n; ++k) {
-        SessionInstance &in = s.inst[ids[k]];
-        const u64 start = h[n + k], end = k + 1 < n ? h[n + k + 1] : nc;
-        in.result_block = comps;
-        in.result_off = start;
-        in.n_result = end - start;
-        in.largest = (i64) h[k];
-        in.labels_block = labels;
-        in.labels_off = off[k];
-    }
-    ctx.give_back(cnt);
-    ctx.give_back(pos);
-}
-
 void mark_done(SessionImpl &s, SessionInstance &in) {
     in.active = false;
     in.done = true;
     s.finished.push_back(in.id);
-}
-
-void finish(SessionImpl &s, const std::vector<i64> &ids) {
-    if (ids.empty()) return;
-    extract_components(s, ids);
-    for (i64 id : ids) mark_done(s, s.inst[id]);
 }
 
 // Drops the union state once no instance is active: ranks, offsets and the
@@ -612,7 +525,7 @@ struct KeepLive {
 // Removes the words of finished instances from the full runs once they are
 // at least half of the full relation.
 void maybe_compact(SessionImpl &s) {
-    if (s.program == DL_PROGRAM_WCC || s.active.empty()) return;
+    if (s.active.empty()) return;
     const u64 total = s.F.size();
     if (s.dead == 0 || s.dead * 2 < total) return;
     Context &ctx = s.ctx;
@@ -626,64 +539,6 @@ void maybe_compact(SessionImpl &s) {
     s.F.ssample_ok = false;
     if (s.F.nsmall == 0) fold_tiny(ctx, s.F);  // a tiny run needs a small run
     s.dead = 0;
-}
-
-void retire(SessionImpl &s, const std::vector<i64> &done, const std::vector<i64> &still) {
-    finish(s, done);
-    if (still.size() != s.active.size()) {
-        s.active = still;
-        s.inst_dirty = true;
-    }
-    reset_if_idle(s);
-}
-
-u64 wcc_step(SessionImpl &s) {
-    Context &ctx = s.ctx;
-    Workspace &ws = ctx.ws;
-    ctx.reserve(ws.offsets, std::max<u64>(s.n_delta, 1) * 8);
-    u32 *next_count = reinterpret_cast<u32 *>(&ctx.ctrl->scalar[32]);
-    DL_CUDA(cudaMemsetAsync(next_count, 0, 4, ctx.stream));
-    Graph g = union_graph(s);
-    WccSrc src{g.csr.off, g.csr.val, s.delta.as<u64>(), s.label.as<u32>(), s.flag.as<u32>(), s.nextl.as<u32>(),
-               next_count};
-    const u64 total = count_matches(ctx, src, s.n_delta, ws.offsets.as<u64>());  // wcc.cu:255-300
-    if (total) emit_matches(ctx, src, s.n_delta, ws.offsets.as<u64>(), total, nullptr, nullptr, 0, nullptr);
-    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars + 6, next_count, 4, cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.sync();
-    const u64 nn = *reinterpret_cast<u32 *>(ctx.host_scalars + 6);
-    grow_keep(ctx, s.delta, std::max<u64>(nn, 1) * 8, 0);  // the emit has read the old delta
-    if (nn)  // rebuild the delta from the appended nodes
-        DL_LAUNCH(ctx, K_PREP, 0,
-                  session_next_delta_kernel<<<grid_for(nn, 256, ctx, 16), 256, 0, ctx.stream>>>(
-                      s.nextl.as<u32>(), nn, s.label.as<u32>(), s.flag.as<u32>(), s.delta.as<u64>()));
-    s.n_delta = nn;
-    const std::vector<u64> c = delta_counts(s, s.delta.as<u64>(), nn, 32);
-    std::vector<i64> still, done;
-    std::vector<uint8_t> live(s.active.size(), 1);
-    bool frozen_rows = false;
-    for (u64 k = 0; k < s.active.size(); ++k) {
-        SessionInstance &in = s.inst[s.active[k]];
-        const i64 cnt = (i64) c[k];
-        in.deltas.push_back(cnt);
-        bool stop = s.opt.wcc_stop == DL_WCC_STOP_FIXPOINT ? cnt == 0 : cnt == in.prev_delta;  // wcc.cu:366-383
-        in.prev_delta = cnt;
-        if (!stop && s.opt.max_iterations > 0 && (int) in.deltas.size() >= s.opt.max_iterations) stop = true;
-        if (stop) {
-            live[k] = 0;
-            frozen_rows |= cnt != 0;
-            done.push_back(s.active[k]);
-        } else {
-            still.push_back(s.active[k]);
-        }
-    }
-    if (frozen_rows) {  // an instance stopped with a non-empty delta: drop its rows
-        ctx.reserve(s.live, live.size());
-        DL_CUDA(cudaMemcpyAsync(s.live.p, live.data(), live.size(), cudaMemcpyHostToDevice, ctx.stream));
-        KeepActive keep{s.inst_lo.as<u64>(), s.live.as<uint8_t>(), (u32) s.active.size(), 32};
-        s.n_delta = session_select(ctx, s.delta.as<u64>(), s.n_delta, keep, 61);  // syncs: `live` may go
-    }
-    retire(s, done, still);
-    return s.active.size();
 }
 
 // The words of a search (ws.jbuf[0], unsorted) in result order, into one block;
@@ -760,6 +615,62 @@ bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
     return true;
 }
 
+// WCC: the fixpoints of the newly admitted instances `ids` (ranks [lo, hi), in
+// instance order) and their results: components (ascending local ranks), largest
+// component and per-node labels.
+void propagate_labels(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi, u64 edges) {
+    if (ids.empty()) return;
+    Context &ctx = s.ctx;
+    const u64 n = ids.size(), total = hi - lo;
+    Csr csr;
+    csr.off = s.off.as<u32>();
+    csr.val = s.val.as<u32>();
+    csr.n_keys = (u32) hi;
+    csr.n_vals = edges;
+    std::vector<u64> first(n), n_ids(n), off(n + 1);
+    for (u64 k = 0; k < n; ++k) {
+        first[k] = s.inst[ids[k]].rank_lo;
+        n_ids[k] = s.inst[ids[k]].n_ids;
+        off[k] = first[k] - lo;
+    }
+    off[n] = total;
+    auto labels = make_block(ctx, total * 4);
+    u32 *label = labels->as<u32>();
+    WccRun run = wcc_propagate(ctx, csr, lo, hi, first, n_ids, s.opt.wcc_stop, s.opt.max_iterations, label);
+    // s.counts: slot offsets [n + 1] then largest [n] then component starts [n]
+    ctx.reserve(s.counts, (3 * n + 1) * 8);
+    u64 *d_off = s.counts.as<u64>(), *d_big = d_off + n + 1, *d_start = d_big + n;
+    DL_CUDA(cudaMemcpyAsync(d_off, off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, ctx.stream));
+    DL_CUDA(cudaMemsetAsync(d_big, 0, n * 8, ctx.stream));
+    DevBuf cnt, pos;
+    ctx.reserve(cnt, total * 4);
+    ctx.reserve(pos, total * 8);
+    DL_CUDA(cudaMemsetAsync(cnt.p, 0, total * 4, ctx.stream));
+    wcc_label_counts(ctx, label, total, (u32) lo, cnt.as<u32>());
+    const u64 nc = count_matches(ctx, NonZero{cnt.as<u32>()}, total, pos.as<u64>());
+    auto comps = make_block(ctx, nc * 4);
+    DL_LAUNCH(ctx, K_PREP, 0,
+              session_wcc_comp_kernel<<<grid_for(total, 256, ctx, 8), 256, 0, ctx.stream>>>(
+                  cnt.as<u32>(), pos.as<u64>(), d_off, (u32) n, total, comps->as<u32>(),
+                  (unsigned long long *) d_big, d_start));
+    std::vector<u64> h(2 * n);
+    DL_CUDA(cudaMemcpyAsync(h.data(), d_big, 2 * n * 8, cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    for (u64 k = 0; k < n; ++k) {
+        SessionInstance &in = s.inst[ids[k]];
+        const u64 start = h[n + k], end = k + 1 < n ? h[n + k + 1] : nc;
+        in.ahead = std::move(run.deltas[k]);
+        in.result_block = comps;
+        in.result_off = start;
+        in.n_result = end - start;
+        in.largest = (i64) h[k];
+        in.labels_block = labels;
+        in.labels_off = off[k];
+    }
+    ctx.give_back(cnt);
+    ctx.give_back(pos);
+}
+
 // TC: the whole fixpoint of the instances admitted since the last step
 // (dl_closure.cu: a search per source, whatever the instance, so all of them
 // run in one launch), their rows sorted into one block and every iteration's
@@ -833,8 +744,9 @@ bool report_ahead(SessionInstance &in) {
     return in.deltas.size() == in.ahead.size();
 }
 
-u64 tc_step(SessionImpl &s) {
-    search_pending(s);
+// One iteration of instances that were computed ahead.
+u64 ahead_step(SessionImpl &s) {
+    if (s.program == DL_PROGRAM_TC) search_pending(s);
     std::vector<i64> still;
     for (i64 id : s.active) {
         SessionInstance &in = s.inst[id];
@@ -922,7 +834,6 @@ SessionImpl *session_create(Context &parent, int program, const dl_options &opt,
     s->program = program;
     s->opt = opt;
     if (program == DL_PROGRAM_WCC) {
-        // WCC words are (rank << 32 | label rank)
         s->bits = 32;
         s->rank_cap = 0xFFFFFFFFull;
     } else {
@@ -982,8 +893,8 @@ void session_destroy(SessionImpl *s) {
         in.result_block.reset();
         in.labels_block.reset();
     }
-    DevBuf *bufs[] = {&s->off,     &s->val,    &s->delta,    &s->label,     &s->flag,
-                      &s->nextl,   &s->inst_lo, &s->inst_hi, &s->counts,    &s->live,
+    DevBuf *bufs[] = {&s->off,     &s->val,    &s->delta,    &s->inst_lo,   &s->inst_hi,
+                      &s->counts,    &s->live,
                       &s->range_lo, &s->admit_off, &s->admit_first};
     for (DevBuf *b : bufs) p.give_back(*b);
     Workspace &w = c.ws;
@@ -1123,15 +1034,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
             full_insert_new(s, b, nd);
             delta_append(s, b, nd);
         } else {  // wcc.cu:211-231: cc(n, n) for every node, all nodes in the first delta
-            grow_keep(ctx, s.label, (B + nu) * 4, B * 4);
-            grow_keep(ctx, s.flag, (B + nu) * 4, B * 4);
-            grow_keep(ctx, s.nextl, (B + nu + 1) * 4, 0);
-            grow_keep(ctx, s.delta, (s.n_delta + nu) * 8, s.n_delta * 8);
-            DL_LAUNCH(ctx, K_PREP, 0,
-                      session_label_init_kernel<<<grid_for(nu, 256, ctx, 16), 256, 0, ctx.stream>>>(
-                          s.label.as<u32>(), s.flag.as<u32>(), B, B + nu, s.delta.as<u64>() + s.n_delta));
-            s.n_delta += nu;
-            for (u64 k = 0; k < count; ++k) inst(k).prev_delta = (i64) inst(k).n_ids;
+            propagate_labels(s, with_rows, B, B + nu, ne);
         }
         ctx.sync();
         for (u64 k = 0; k < count; ++k) {
@@ -1165,7 +1068,7 @@ i64 session_admit(SessionImpl &s, const int32_t *rows, u64 n, bool on_device) {
 
 u64 session_step(SessionImpl &s) {
     if (s.active.empty()) return 0;
-    return s.program == DL_PROGRAM_WCC ? wcc_step(s) : s.program == DL_PROGRAM_TC ? tc_step(s) : sg_step(s);
+    return s.program == DL_PROGRAM_SG ? sg_step(s) : ahead_step(s);
 }
 
 u64 session_poll(SessionImpl &s, int64_t *ids, u64 capacity) {
@@ -1201,7 +1104,7 @@ void session_info(const SessionImpl &s, i64 id, dl_run_info &info) {
     info.iterations = (int32_t) in.deltas.size();
     info.input_rows = in.input_rows;
     info.output_rows = info.output_tuples = in.done ? (i64) in.n_result : 0;
-    info.largest_component = in.largest;
+    info.largest_component = in.done ? in.largest : 0;
     info.nodes = in.n_ids;
 }
 
@@ -1330,7 +1233,7 @@ u64 session_device_bytes(const SessionImpl &s) {
     const Context &c = s.ctx;
     const Workspace &w = c.ws;
     u64 b = 0;
-    const DevBuf *bufs[] = {&s.off,     &s.val,       &s.delta,    &s.label,      &s.flag,       &s.nextl,
+    const DevBuf *bufs[] = {&s.off,     &s.val,       &s.delta,
                             &w.input,   &w.ids,       &w.w0,       &w.w1,         &w.csr_off,    &w.csr_val,
                             &w.full[0], &w.full[1],   &w.small[0], &w.small[1],   &w.tiny[0],    &w.tiny[1],
                             &w.sample,  &w.sample_small, &w.jbuf[0],

@@ -16,11 +16,10 @@ struct SessionInstance {
     u32 n_ids = 0;
     const int32_t *ids() const { return ids_block ? ids_block->as<int32_t>() + ids_off : nullptr; }
     std::vector<i64> deltas;       // |delta| of this instance after each iteration
-    std::vector<i64> ahead;        // TC: every iteration's |delta|, known before the steps that report them
-    i64 prev_delta = 0;            // WCC reference stop rule
+    std::vector<i64> ahead;        // every iteration's |delta|, known before the steps that report them (SG: empty if it is not)
     bool active = false, done = false, released = false;
-    // TC/SG: sorted union words; WCC: component ranks (local). Instances that
-    // finish in the same step share one block.
+    // TC/SG: sorted union words; WCC: component ranks (local). Instances computed
+    // or extracted together share one block.
     std::shared_ptr<DevBuf> result_block;
     u64 result_off = 0;
     u64 n_result = 0;

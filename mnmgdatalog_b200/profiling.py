@@ -26,7 +26,7 @@ CLASSES = [
     (r"scan_kernel<.*WordValue", "sort_spine_scan"),
     (r"radix_bucket_kernel", "sort_spine_scan"),
     (r"scan_kernel<.*DegreeOp", "join_count_scan"),
-    (r"join_emit_kernel<.*WccSrc", "wcc_propagate"),
+    (r"wcc_(first|level|close|final)_kernel", "wcc_propagate"),
     (r"join_emit_kernel|join_emit_bucket_kernel", "join_emit"),
     (r"digit0_hist_kernel", "join_count_scan"),
     (r"bucket_starts_kernel", "join_partition"),
