@@ -14,9 +14,9 @@
 // Bound by launches and host waits on small graphs: an iteration moves 36 bytes
 // per edge of the changed nodes. Measured on B200 against four launches and two host
 // waits per iteration (count, scan, balanced emit, rebuild): 24K edges over 16K
-// nodes 0.93 -> 0.64 ms for the whole run, 700K edges over 100K nodes 2.22 ->
-// 1.92, one million edges in a long-diameter graph 7.6 -> 0.83; 64 instances
-// in one union 11.3 -> 4.6 (they iterate on the device alone, not step by step).
+// nodes 0.93 -> 0.53 ms for the whole run, 700K edges over 100K nodes 2.22 ->
+// 1.28, 48 instances
+// in one union 11.3 -> 3.7 (they iterate on the device alone, not step by step).
 #include "dl_wcc.h"
 #include "dl_pull.cuh"
 
@@ -25,7 +25,9 @@ namespace detail {
 namespace {
 
 constexpr int WC_THREADS = 256;
-constexpr u32 WC_LONG = 1024;  // longer lists are cut into pieces of this many edges for as many warps
+constexpr int WC_WARPS = WC_THREADS / 32;
+constexpr u32 WC_LONG = 128;   // longer lists are cut into pieces of this many edges for as many warps
+constexpr u32 WC_TAKE = 4;     // nodes a warp takes at least
 constexpr u64 WC_LEVELS = 8;   // iterations launched between two host waits
 
 struct WccState {
@@ -57,24 +59,53 @@ __device__ __forceinline__ u32 wcc_instance(const WccState &st, u64 r) {
     return a - 1;
 }
 
+// A warp's lowered ranks on their way to the iteration's list: 32 at a time, since
+// one atomic per window of edges on the list's length would be the longest queue.
+struct WccOut {
+    u32 *buf;  // 64 words of shared memory
+    u32 held;
+};
+
+__device__ __forceinline__ void wcc_flush(const WccState &st, u32 level, u32 at, WccOut &o, u32 n, u32 lane) {
+    const bool have = lane < n;
+    const u32 r = have ? o.buf[lane] : 0u;
+    unsigned long long p = 0;
+    if (lane == 0) p = atomicAdd(st.cnt + at, (unsigned long long) n);
+    p = __shfl_sync(0xffffffffu, p, 0) + lane;
+    if (have) st.list[level & 1][p] = r;
+    if (st.n_inst > 1) {
+        const u32 inst = have ? wcc_instance(st, r) : EMPTY;
+        const u32 same = __match_any_sync(0xffffffffu, inst);
+        if (have && lane == (u32) __ffs(same) - 1) atomicAdd(st.icnt + (u64) at * st.n_inst + inst, __popc(same));
+    }
+}
+
 // Ranks lowered in iteration `level` by this warp's lanes (all lanes call).
-__device__ __forceinline__ void wcc_append(const WccState &st, u32 level, u32 at, u32 r, bool fresh, u32 lane, u32 lt) {
+__device__ __forceinline__ void wcc_append(const WccState &st, u32 level, u32 at, WccOut &o, u32 r, bool fresh, u32 lane,
+                                           u32 lt) {
     const u32 fm = __ballot_sync(0xffffffffu, fresh);
     if (!fm) return;
-    unsigned long long p = 0;
-    if (lane == 0) p = atomicAdd(st.cnt + at, (unsigned long long) __popc(fm));
-    p = __shfl_sync(0xffffffffu, p, 0) + __popc(fm & lt);
-    if (fresh) st.list[level & 1][p] = r;
-    if (st.n_inst > 1) {
-        const u32 inst = fresh ? wcc_instance(st, r) : EMPTY;
-        const u32 same = __match_any_sync(0xffffffffu, inst);
-        if (fresh && lane == (u32) __ffs(same) - 1) atomicAdd(st.icnt + (u64) at * st.n_inst + inst, __popc(same));
-    }
+    if (fresh) o.buf[o.held + __popc(fm & lt)] = r;
+    o.held += __popc(fm);
+    __syncwarp();
+    if (o.held < 32) return;
+    wcc_flush(st, level, at, o, 32, lane);
+    o.held -= 32;
+    const u32 x = lane < o.held ? o.buf[32 + lane] : 0u;
+    __syncwarp();
+    if (lane < o.held) o.buf[lane] = x;
+    __syncwarp();
+}
+
+__device__ __forceinline__ void wcc_finish(const WccState &st, u32 level, u32 at, WccOut &o, u32 lane) {
+    if (o.held) wcc_flush(st, level, at, o, o.held, lane);
 }
 
 // Iteration 1.
 __global__ void __launch_bounds__(WC_THREADS)
 wcc_first_kernel(WccState st, const u32 *__restrict__ off, const u32 *__restrict__ val, u64 hi) {
+    __shared__ u32 buf[WC_WARPS][64];
+    WccOut o{buf[threadIdx.x >> 5], 0};
     const u32 lane = threadIdx.x & 31;
     const u32 lt = lanemask_lt();
     const u64 step = (u64) gridDim.x * WC_THREADS;
@@ -90,13 +121,14 @@ wcc_first_kernel(WccState st, const u32 *__restrict__ off, const u32 *__restrict
             st.lab[1][r - st.lo] = m;
             st.tag[r - st.lo] = low ? 1u : 0u;
         }
-        wcc_append(st, 1, 0, (u32) r, low, lane, lt);
+        wcc_append(st, 1, 0, o, (u32) r, low, lane, lt);
     }
+    wcc_finish(st, 1, 0, o, lane);
 }
 
 // Edge targets w of changed nodes with label l: lower array level & 1.
-__device__ __forceinline__ void wcc_lower(const WccState &st, u32 level, u32 at, u32 w, u32 l, bool have, u32 lane,
-                                          u32 lt) {
+__device__ __forceinline__ void wcc_lower(const WccState &st, u32 level, u32 at, WccOut &o, u32 w, u32 l, bool have,
+                                          u32 lane, u32 lt) {
     bool fresh = false;
     if (have) {
         const u64 i = w - st.lo;
@@ -108,25 +140,29 @@ __device__ __forceinline__ void wcc_lower(const WccState &st, u32 level, u32 at,
             }
         }
     }
-    wcc_append(st, level, at, w, fresh, lane, lt);
+    wcc_append(st, level, at, o, w, fresh, lane, lt);
 }
 
 // Iteration `level` (2 and up; `at` = its place in the batch's counters; `n_prev`
-// = where the number of nodes changed before it is): a warp takes 32 of them and walks
-// their edges 32 at a time; long lists go to the next launch in pieces.
+// = where the number of nodes changed before it is): a warp takes 4 to 32 of them, so
+// that all warps have some, and walks their edges 32 at a time; long lists go to the
+// next launch in pieces. (Lists of up to 1024 edges in takes of 32 left single warps
+// with thousands of edges: 1.22 ms of 1.92 on 700K edges of skewed degrees.)
 __global__ void __launch_bounds__(WC_THREADS)
 wcc_level_kernel(WccState st, const u32 *__restrict__ off, const u32 *__restrict__ val, u32 level, u32 at,
                  const unsigned long long *__restrict__ n_prev) {
     if (*st.stop) return;
-    __shared__ u32 wbeg[WC_THREADS / 32][32], wpre[WC_THREADS / 32][32], wlab[WC_THREADS / 32][32];
+    __shared__ u32 wbeg[WC_WARPS][32], wpre[WC_WARPS][32], wlab[WC_WARPS][32], buf[WC_WARPS][64];
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u32 lt = lanemask_lt(), le = lane == 31 ? ~0u : (2u << lane) - 1;
     const u64 n = *n_prev;
-    const u64 step = (u64) gridDim.x * WC_THREADS;
+    const u64 warps = (u64) gridDim.x * WC_WARPS;
+    const u32 take = (u32) min((u64) 32, max((u64) WC_TAKE, (n + warps - 1) / warps));
+    WccOut o{buf[warp], 0};
     u64 walked = 0;
-    for (u64 g = (u64) blockIdx.x * WC_THREADS + (threadIdx.x & ~31u); g < n; g += step) {
+    for (u64 g = ((u64) blockIdx.x * WC_WARPS + warp) * take; g < n; g += warps * take) {
         u32 beg = 0, deg = 0, l = 0;
-        if (g + lane < n) {
+        if (lane < take && g + lane < n) {
             const u32 v = st.list[(level + 1) & 1][g + lane];
             if (st.n_inst == 1 || st.istop[wcc_instance(st, v)] == 0) {
                 l = st.lab[(level + 1) & 1][v - st.lo];
@@ -166,20 +202,21 @@ wcc_level_kernel(WccState st, const u32 *__restrict__ off, const u32 *__restrict
         auto load = [&](u32 i0) -> u32 {
             const u32 start = (pre - i0) < 32u ? 1u << (pre - i0) : 0u;
             const u32 starts = __reduce_or_sync(0xffffffffu, start);
-            const int o = base + __popc(starts & le);
+            const int row = base + __popc(starts & le);
             base += __popc(starts);
-            const u32 ob = __shfl_sync(0xffffffffu, cb, o), op = __shfl_sync(0xffffffffu, pre, o);
-            nl = __shfl_sync(0xffffffffu, cl, o);
+            const u32 ob = __shfl_sync(0xffffffffu, cb, row), op = __shfl_sync(0xffffffffu, pre, row);
+            nl = __shfl_sync(0xffffffffu, cl, row);
             return i0 + lane < total ? __ldg(val + ob + (i0 + lane - op)) : 0u;
         };
         u32 w = load(0), wl = nl;
         for (u32 i0 = 0; i0 < total; i0 += 32) {
             const u32 wn = i0 + 32 < total ? load(i0 + 32) : 0u;
-            wcc_lower(st, level, at, w, wl, i0 + lane < total, lane, lt);
+            wcc_lower(st, level, at, o, w, wl, i0 + lane < total, lane, lt);
             w = wn;
             wl = nl;
         }
     }
+    wcc_finish(st, level, at, o, lane);
     walked = warp_sum(walked);
     if (lane == 0 && walked) atomicAdd(st.join + at, (unsigned long long) walked);
 }
@@ -194,17 +231,18 @@ wcc_close_kernel(WccState st, const u32 *__restrict__ val, u32 level, u32 at, in
     const u32 lane = threadIdx.x & 31;
     const u32 lt = lanemask_lt();
     const u64 n = st.pieces[at];
-    const u64 warps = (u64) gridDim.x * (WC_THREADS / 32);
+    const u64 warps = (u64) gridDim.x * WC_WARPS;
+    __shared__ u32 buf[WC_WARPS][64];
+    WccOut o{buf[threadIdx.x >> 5], 0};
     for (u64 i = ((u64) blockIdx.x * WC_THREADS + threadIdx.x) / 32; i < n; i += warps) {
         const uint4 p = st.piece[i];
-        for (u32 k = 0; k < p.y; k += 128) {
-            u32 w[4];
+        u32 w[WC_LONG / 32];
 #pragma unroll
-            for (u32 q = 0; q < 4; ++q) w[q] = k + q * 32 + lane < p.y ? __ldg(val + p.x + k + q * 32 + lane) : 0u;
+        for (u32 q = 0; q < WC_LONG / 32; ++q) w[q] = q * 32 + lane < p.y ? __ldg(val + p.x + q * 32 + lane) : 0u;
 #pragma unroll
-            for (u32 q = 0; q < 4; ++q) wcc_lower(st, level, at, w[q], p.z, k + q * 32 + lane < p.y, lane, lt);
-        }
+        for (u32 q = 0; q < WC_LONG / 32; ++q) wcc_lower(st, level, at, o, w[q], p.z, q * 32 + lane < p.y, lane, lt);
     }
+    wcc_finish(st, level, at, o, lane);
     __shared__ u32 last, running;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -301,7 +339,6 @@ WccRun wcc_propagate(Context &ctx, const Csr &csr, u64 lo, u64 hi, const std::ve
     // the previous batch's last |delta| (the list it left) sits in slot WC_LEVELS
     std::vector<u32> got(WC_LEVELS * ni);
     for (u32 first = 1; live; first += WC_LEVELS) {
-        u64 most = n;  // of any list: for the grids
         for (u32 k = 0; k < WC_LEVELS; ++k) {
             const u32 level = first + k;
             if (level == 1) {
@@ -310,11 +347,11 @@ WccRun wcc_propagate(Context &ctx, const Csr &csr, u64 lo, u64 hi, const std::ve
                               st, csr.off, csr.val, hi));
             } else {
                 DL_LAUNCH(ctx, K_WCC_PROPAGATE, 0,
-                          wcc_level_kernel<<<grid_for(most, WC_THREADS, ctx, 8), WC_THREADS, 0, ctx.stream>>>(
+                          wcc_level_kernel<<<grid_for(n * 32 / WC_TAKE, WC_THREADS, ctx, 8), WC_THREADS, 0, ctx.stream>>>(
                               st, csr.off, csr.val, level, k, k ? st.cnt + k - 1 : st.cnt + WC_LEVELS));
             }
             DL_LAUNCH(ctx, K_WCC_PROPAGATE, 0,
-                      wcc_close_kernel<<<grid_for(std::max<u64>(csr.n_vals / WC_LONG, 1) * 32, WC_THREADS, ctx, 4),
+                      wcc_close_kernel<<<grid_for(std::max<u64>(csr.n_vals / WC_LONG, 1) * 32, WC_THREADS, ctx, 8),
                                          WC_THREADS, 0, ctx.stream>>>(st, csr.val, level, k, fix, cap));
         }
         u64 *hs = ctx.host_scalars;

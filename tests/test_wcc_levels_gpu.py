@@ -1,6 +1,6 @@
 """WCC's iterations launched in batches (dl_wcc.cu) against the iteration written
 out in numpy, exactly: labels, |delta| and joined rows per iteration, both stop
-rules and early stops -- with lists on both sides of the 1024 edges a warp takes
+rules and early stops -- with lists on both sides of the 128 edges a warp takes
 at once, more iterations than one batch, and instances that stop at different
 iterations of a batch."""
 import numpy as np
@@ -18,7 +18,7 @@ def _star(d, base=0):
 CASES = {
     "one": [[1, 2]], "loop": [[5, 5]], "path8": [[i, i + 1] for i in range(8)], "path9": [[i, i + 1] for i in range(9)],
     "path40": [[i, i + 1] for i in range(40)], "back_path": [[40 - i, 39 - i] for i in range(40)],
-    "star_1024": _star(1024), "star_1025": _star(1025),
+    "star_128": _star(128), "star_129": _star(129), "star_1025": _star(1025),
     # hubs whose labels fall late: their long lists are walked in iterations above 1
     "late_hubs": [[0, 1], [1, 2], [2, 3], [3, 100_001]] + [[100_001, 9000 + i] for i in range(5000)]
     + [[14_000 - 1, 200_000]] + [[200_000, 20_000 + i] for i in range(2048)],
