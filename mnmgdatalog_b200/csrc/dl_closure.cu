@@ -954,11 +954,12 @@ __global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u
 //    leave as consecutive 8-byte stores, the columns' node ids in 32 registers
 //    (ten instructions a word: with the ids loaded per word it was bound by
 //    issue, 40 a word);
-//  * else a lane per word walks its bits into shared memory, and the chunk's rows
-//    leave with consecutive stores.
+//  * else a lane per word walks its bits' positions into shared memory, and the
+//    chunk's rows leave with consecutive stores; their columns are looked up there
+//    (not at the walk, which takes as many turns as its fullest word has bits),
+//    or, where the chunk's columns are consecutive ranks, added up.
 // Light pairs are placed lane-parallel; a word that one falls inside is done
 // last, its lanes shifted by the light pairs below them.
-constexpr u32 ROWS_STAGE = 384;  // a sparse chunk's staged rows
 
 template <bool DENSE, bool ROW_FIRST>
 __global__ void __launch_bounds__(256)
@@ -966,8 +967,8 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                     const u32 *__restrict__ place, const uint2 *__restrict__ start, u64 z0, u64 z1,
                     const u64 *__restrict__ first, const u64 *__restrict__ light, const u64 *__restrict__ loff,
                     u64 mask, const int32_t *__restrict__ ids, bool affine, int32_t base, u64 *__restrict__ out) {
-    __shared__ u32 staged[DENSE ? 1 : 8][ROWS_STAGE];
-    u32 *stage = staged[DENSE ? 0 : threadIdx.x >> 5];
+    __shared__ unsigned short staged[DENSE ? 1 : 8][DENSE ? 1 : 1024];
+    unsigned short *stage = staged[DENSE ? 0 : threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31;
     const u32 lt = lanemask_lt();
     const u32 chunks = words / 32;
@@ -989,13 +990,27 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 id[j] = x == EMPTY ? 0u : node(x);
             }
         }
-        for (u64 z = z0 + me / chunks; z < z1; z += step) {
-            u32 v = t[z * words + k0 + lane];
-            const uint2 st = start[z * chunks + c0];
+        const u32 c_first = __ldg(cc);
+        const bool consecutive = __ldg(cc + 1023) - c_first == 1023;  // columns ascend (EMPTY past the last)
+        u64 z = z0 + me / chunks;
+        u32 v_next = 0;
+        uint2 st_next = make_uint2(0, 0);
+        u64 first_next = 0;
+        auto fetch = [&](u64 y) {  // one target ahead
+            if (y >= z1) return;
+            v_next = t[y * words + k0 + lane];
+            st_next = start[y * chunks + c0];
+            first_next = first[y];
+        };
+        fetch(z);
+        for (; z < z1; z += step) {
+            u32 v = v_next;
+            const uint2 st = st_next;
+            u64 *dst = out + first_next + st.x;
+            fetch(z + step);
             const u32 lend = c0 + 1 < chunks ? start[z * chunks + c0 + 1].y : (u32) (loff[z + 1] - loff[z]);
             const u32 any = __ballot_sync(0xffffffffu, v != 0);
             if (!any && st.y == lend) continue;
-            u64 *dst = out + first[z] + st.x;
             const u32 zid = node((u32) z);
             // a row (x, z), or (z, x) when the targets come first, as one little-endian word
             auto pack = [&](u32 x) -> u64 { return ROW_FIRST ? ((u64) x << 32) | zid : ((u64) zid << 32) | x; };
@@ -1004,10 +1019,14 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             u32 at = incl - n;
             if constexpr (!DENSE) {
                 const u32 total = __shfl_sync(0xffffffffu, incl, 31);
-                if (st.y == lend && total <= ROWS_STAGE) {
-                    for (; v; v &= v - 1) stage[at++] = node(__ldg(cc + lane * 32 + __ffs(v) - 1));
+                if (st.y == lend) {
+                    for (; v; v &= v - 1) stage[at++] = (unsigned short) (lane * 32 + __ffs(v) - 1);
                     __syncwarp();
-                    for (u32 i = lane; i < total; i += 32) dst[i] = pack(stage[i]);
+                    if (consecutive) {
+                        for (u32 i = lane; i < total; i += 32) dst[i] = pack(node(c_first + stage[i]));
+                    } else {
+                        for (u32 i = lane; i < total; i += 32) dst[i] = pack(node(__ldg(cc + stage[i])));
+                    }
                     __syncwarp();
                     continue;
                 }
