@@ -28,6 +28,12 @@ struct ClosureLight {
 ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const u64 *inst_lo, u64 n_inst,
                             u64 k0, u64 k1, u64 stride, u64 max_level, u64 *cnt, u64 *deg);
 
+// The words of a search's finished sources (all sources of the call, nothing
+// appended since) sorted; ranks below 2^used_bits. The words of a source are equal
+// below `bits`, so that lining the sources up replaces the passes over that field:
+// a scan and one copy for about half the passes. Result in ws.jbuf[0] or [1].
+u64 *closure_order(Context &ctx, u64 n_sources, u64 n_words, int bits, int used_bits);
+
 // The closure of `h` heavy sources (ascending ranks `src`, device) over ranks
 // [0, n) as bit rows: bit c of row z of `t` is set when source c reaches z.
 // `cols`: rank of every column (padded to whole words with all ones), followed

@@ -210,7 +210,7 @@ void Context::release_all() {
                      &ws.small[0], &ws.small[1], &ws.tiny[0], &ws.tiny[1], &ws.sample, &ws.sample_small,
                      &ws.jbuf[0], &ws.jbuf[1], &ws.offsets, &ws.wcc_label, &ws.wcc_flag, &ws.wcc_next,
                      &ws.bitmat[0], &ws.bitmat[1], &ws.offsets_next, &ws.bit_hasout,
-                     &ws.rank_bits, &ws.rank_pre, &ws.cl_rec, &ws.cl_left, &ws.cl_heavy, &ws.cl_levels, &ws.cl_roff, &ws.cl_rval, &ws.cl_segs, &ws.cl_hub_at,
+                     &ws.rank_bits, &ws.rank_pre, &ws.cl_rec, &ws.cl_left, &ws.cl_heavy, &ws.cl_seg, &ws.cl_seg_at, &ws.cl_levels, &ws.cl_roff, &ws.cl_rval, &ws.cl_segs, &ws.cl_hub_at,
                      &ws.cl_hub_acc, &ws.cl_rows[0], &ws.cl_rows[1], &ws.cl_act,
                      &lookback, &sort_hist, &lbs_splits, &radix_part, &merge_splits, &bucket_cursor,
                      &part_cursor};

@@ -121,6 +121,7 @@ struct Workspace {
     // TC by searches (dl_closure.cu)
     DevBuf cl_rec;              // edge records (target, its first edge, its degree)
     DevBuf cl_left, cl_heavy;   // sources a search could not hold
+    DevBuf cl_seg, cl_seg_at;   // where the searched sources' words are, and go
     DevBuf cl_levels;           // level counts
     DevBuf cl_roff, cl_rval;    // in-neighbours of every node
     DevBuf cl_segs, cl_hub_at, cl_hub_acc;  // targets with many in-neighbours

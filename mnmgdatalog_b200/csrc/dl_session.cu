@@ -542,18 +542,25 @@ void maybe_compact(SessionImpl &s) {
 }
 
 // The words of a search (ws.jbuf[0], unsorted) in result order, into one block;
-// every instance's are one range of it.
-void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words) {
+// every instance's are one range of it. `sources`: ranks searched when the words are
+// those of a TC search alone, else 0.
+void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words, u64 sources) {
     Context &ctx = s.ctx;
     Workspace &ws = ctx.ws;
     const u64 n = ids.size();
     std::vector<u64> hb(6 * n, 0);
     auto block = std::shared_ptr<DevBuf>();
     if (words) {
-        ctx.reserve(ws.jbuf[1], words * 8);
-        int w[8];
-        const int nw = plan_windows(s.bits, bits_for(std::max<u64>(s.next_rank, 2)), w);
-        u64 *r = radix_sort_windows(ctx, ws.jbuf[0].as<u64>(), ws.jbuf[1].as<u64>(), words, w, nw);
+        const int used = bits_for(std::max<u64>(s.next_rank, 2));
+        u64 *r;
+        if (sources) {
+            r = closure_order(ctx, sources, words, s.bits, used);
+        } else {
+            ctx.reserve(ws.jbuf[1], words * 8);
+            int w[8];
+            const int nw = plan_windows(s.bits, used, w);
+            r = radix_sort_windows(ctx, ws.jbuf[0].as<u64>(), ws.jbuf[1].as<u64>(), words, w, nw);
+        }
         upload_ranges(s, ids);
         ctx.reserve(s.counts, 6 * n * 8);
         Runs3 runs{{r, r, r}, {words, 0, 0}};
@@ -611,7 +618,7 @@ bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
             if (c == 0 || (stop > 0 && (int) in.ahead.size() >= stop)) break;
         }
     }
-    place_results(s, ids, ps.n_words());
+    place_results(s, ids, ps.n_words(), 0);
     return true;
 }
 
@@ -733,7 +740,7 @@ void search_pending(SessionImpl &s) {
             if (c == 0 || (s.opt.max_iterations > 0 && (int) in.ahead.size() >= s.opt.max_iterations)) break;
         }
     }
-    place_results(s, ids, words);
+    place_results(s, ids, words, words == light.n_words ? end - first : 0);
     s.pending.clear();
 }
 
@@ -902,7 +909,7 @@ void session_destroy(SessionImpl *s) {
                        &w.full[0],  &w.full[1],  &w.small[0], &w.small[1], &w.tiny[0], &w.tiny[1],
                        &w.sample,   &w.sample_small, &w.jbuf[0],
                        &w.jbuf[1],  &w.offsets,  &w.wcc_label, &w.wcc_flag, &w.wcc_next,
-                       &w.cl_left,  &w.cl_heavy, &w.cl_levels, &w.cl_roff,  &w.cl_rval, &w.cl_segs,
+                       &w.cl_left,  &w.cl_heavy, &w.cl_seg, &w.cl_seg_at, &w.cl_levels, &w.cl_roff,  &w.cl_rval, &w.cl_segs,
                        &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec};
     for (DevBuf *b : wbufs) p.give_back(*b);
     for (auto &b : c.spares) p.give_back(b);
@@ -1238,7 +1245,7 @@ u64 session_device_bytes(const SessionImpl &s) {
                             &w.full[0], &w.full[1],   &w.small[0], &w.small[1],   &w.tiny[0],    &w.tiny[1],
                             &w.sample,  &w.sample_small, &w.jbuf[0],
                             &w.jbuf[1], &w.offsets,   &c.lookback, &c.radix_part, &c.lbs_splits, &c.sort_hist,
-                            &c.merge_splits, &w.cl_left, &w.cl_heavy, &w.cl_levels, &w.cl_roff, &w.cl_rval, &w.cl_segs,
+                            &c.merge_splits, &w.cl_left, &w.cl_heavy, &w.cl_seg, &w.cl_seg_at, &w.cl_levels, &w.cl_roff, &w.cl_rval, &w.cl_segs,
                             &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec};
     for (const DevBuf *x : bufs) b += x->cap;  // cached spare buffers are not counted: they are free memory
     std::vector<const DevBuf *> blocks;
