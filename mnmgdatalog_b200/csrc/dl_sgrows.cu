@@ -1,20 +1,24 @@
 // SG on bit rows, one owner per row.
 //
 // sg(x, y) :- e(a, x), sg(a, b), e(b, y) (sg.cu:244-390). sg is symmetric from
-// the base rule on, so with the newest pairs as bit rows D (row b, bit a), the new
-// pairs of row y are
-//     N(y) = union of a's children over a in W(y),   W(y) = OR of D(b), b -> y
-// minus the row's known pairs: everything row y needs is its in-neighbours'
-// newest rows, read as whole lines, and its children's scatter goes to a row in
-// shared memory. A row has one owner (a warp, or a CTA for long rows), so nothing
-// is merged between CTAs: the step on the matrix before this one (dl_bitmap.cu)
-// expanded the pairs of a source once and folded the result into every child's
-// row with an atomic per touched word of the matrix.
-// The base rule is the same step on the identity: N(y) = children of y's
-// parents, without y itself.
+// the base rule on, so with E(b) = the children of b's newest partners as a bit row,
+// the new pairs of row y are
+//     N(y) = OR of E(b) over y's in-neighbours b
+// minus the row's known pairs, and E(y) = the children of the nodes in N(y): all
+// that row y needs is its in-neighbours' rows, read as whole lines, and its
+// children's scatter goes to a row in shared memory. A row has one owner (a warp,
+// or a CTA for long rows), so nothing is merged between CTAs, and every new
+// pair is expanded once, whatever the out-degree of its row. (The step on the matrix
+// before this one, dl_bitmap.cu, expanded the pairs of a source once and folded the
+// result into every child's row with an atomic per touched word of the matrix.)
+// The base rule is the same step on the identity: E(x) = x's children, and N(y)
+// without y itself.
 //
 // Measured on B200, a mesh of 22K nodes and 38K edges (2.4e8 pairs, 133
-// iterations), edges and result rows on the device: 67 ms on the matrix, 17 ms here.
+// iterations), edges and result rows on the device: 67 ms on the matrix; 17.1 ms with
+// the newest pairs themselves as rows, which expands the union of the in-neighbours'
+// pairs for every row (also those of nodes without children) and reads the known pairs
+// only after that; 14.7 ms here.
 #include "dl_closure.h"
 #include "dl_pull.cuh"
 
@@ -34,28 +38,37 @@ __global__ void has_children_kernel(const u32 *__restrict__ off, u64 n, u64 word
     }
 }
 
-// Level 0: row x = {x} for every node with children; tagged, so that the
-// children of x get on the first list. cols[i] = i (all ones past n).
-__global__ void sg_identity_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, u32 *__restrict__ cols) {
+// Level 0: the newest pair of a node x is (x, x), so its row holds x's children;
+// tagged, so that the children of x get on the first list. cols[i] = i (all
+// ones past n).
+__global__ void sg_identity_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off,
+                                   const u32 *__restrict__ val, u32 *__restrict__ cols) {
     const u32 lane = threadIdx.x & 31;
     const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
     for (u64 x = ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32; x < (u64) sh.words * 32; x += warps) {
         if (lane == 0) cols[x] = x < sh.n ? (u32) x : EMPTY;
         if (x >= sh.n || off[x + 1] == off[x]) continue;
-        const u32 gr = (u32) (x >> 10) >> sh.shift;
-        const u32 w0 = (gr << sh.shift) * 32, w1 = min(sh.words, w0 + (32u << sh.shift));
+        const u32 b = off[x], e = off[x + 1];
+        u32 act = 0;
+        for (u32 k = b + lane; k < e; k += 32) act |= 1u << ((val[k] >> 10) >> sh.shift);
+        act = __reduce_or_sync(0xffffffffu, act);
         u32 *row = st.nxt + x * sh.words;
-        for (u32 k = w0 + lane; k < w1; k += 32) row[k] = k == (u32) (x >> 5) ? 1u << (x & 31) : 0u;
-        if (lane == 0) st.tag_next[x] = make_uint2(1u << gr, st.level);
+        for (u32 mm = act; mm; mm &= mm - 1) {
+            const u32 w0 = ((u32) (__ffs(mm) - 1) << sh.shift) * 32, w1 = min(sh.words, w0 + (32u << sh.shift));
+            for (u32 k = w0 + lane; k < w1; k += 32) row[k] = 0;
+        }
+        __syncwarp();
+        for (u32 k = b + lane; k < e; k += 32) atomicOr(&row[val[k] >> 5], 1u << (val[k] & 31));
+        if (lane == 0) st.tag_next[x] = make_uint2(act, st.level);
     }
 }
 
 struct SgTeam {
     u32 item;            // the team's place in the list
-    u32 touched, news;   // activity bits of the row's touched chunks, and of those with new pairs
+    u32 touched;         // activity bits of the chunks its children fell into
 };
 
-constexpr u32 SG_QUEUE = 512;  // bits of W a warp holds before it expands them
+constexpr u32 SG_QUEUE = 512;  // new pairs a warp holds before it expands them
 
 // Per-warp part of a team's shared memory.
 struct SgWarp {
@@ -73,13 +86,19 @@ __device__ __noinline__ u32 sg_expand(SgWarp &mw, u32 qn, u32 *row, const u32 *_
     const u32 lt = lanemask_lt(), le = lane == 31 ? ~0u : (2u << lane) - 1;
     u32 mine = 0;
     __syncwarp();
-    for (u32 q0 = 0; q0 < qn; q0 += 32) {
-        u32 beg = 0, deg = 0;
+    u32 nbeg = 0, nend = 0;
+    auto fetch = [&](u32 q0) {  // one batch ahead
+        nbeg = nend = 0;
         if (q0 + lane < qn) {
             const u32 a = mw.queue[q0 + lane];
-            beg = __ldg(off + a);
-            deg = __ldg(off + a + 1) - beg;
+            nbeg = __ldg(off + a);
+            nend = __ldg(off + a + 1);
         }
+    };
+    fetch(0);
+    for (u32 q0 = 0; q0 < qn; q0 += 32) {
+        const u32 beg = nbeg, deg = nend - nbeg;
+        fetch(q0 + 32);
         auto put = [&](u32 x) {
             atomicOr(&row[x >> 5], 1u << (x & 31));
             mine |= 1u << ((x >> 10) >> shift);
@@ -110,14 +129,16 @@ __device__ __noinline__ u32 sg_expand(SgWarp &mw, u32 qn, u32 *row, const u32 *_
 
 // One level: the new pairs of every row in the list, a team of NW warps per row
 // (TEAMS teams to a CTA, each with its row in shared memory). The warps take
-// the active chunks four at a time: OR of the in-neighbours' newest words (32
-// words of W a chunk), whose bits go to a queue across chunks, so that the
-// expansion runs on full batches of 32 pairs; their children are ORed into the
-// shared row. Then the touched chunks are compared with the matrix, four in
-// flight. Bound by latency and instructions, not by the lines: chunk by chunk
-// with batches a quarter full the mesh above took 26 ms, with its walk in three
-// copies 24 ms; 40 warps an SM at 48 registers 17.8 ms against 17.1 for 32 at 64;
-// six or eight chunks in flight spill (17.5 and 20 ms).
+// the active chunks four at a time: OR of the in-neighbours' words and the row's known
+// pairs, whose difference goes to a queue across chunks, so that the expansion
+// runs on full batches of 32 pairs; their children are ORed into the shared row,
+// which leaves chunk by chunk. Bound by latency and instructions (at the mesh's
+// fullest level 60 % of the issue slots, 8200 instructions for a row of 960 new
+// pairs in 22 chunks), not by the lines. Measured on the mesh above in the form before
+// this one: chunk by chunk with batches a quarter full 26 ms, the walk in three
+// copies 24 ms, 40 warps an SM at 48 registers 17.8 ms against 17.1 for 32 at 64, six
+// or eight chunks in flight 17.5 and 20 ms (spills), two in-neighbours at a time
+// 16.4; in this one, one prefix sum over four chunks 15.2 against 14.7 ms.
 template <int NW, int TEAMS>
 __global__ void __launch_bounds__(NW * TEAMS * 32, 1024 / (NW * TEAMS * 32))
 sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ val,
@@ -140,7 +161,7 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
         else __syncthreads();
     };
     for (u32 k = tl; k < sh.words; k += NW * 32) row[k] = 0;
-    if (tl == 0) team.touched = team.news = 0;
+    if (tl == 0) team.touched = 0;
     u64 fresh = 0, rows = 0;
     // the next four chunks of the activity mask (EMPTY: none); gc: chunks of the lowest
     // granule already given out
@@ -177,38 +198,63 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
         u32 y0, a0;
         parents(0, y0, a0);
         u32 mine = 0;  // chunks this lane's children fell into
-        u32 qn = 0;    // queued bits of W
+        u32 qn = 0;    // queued new pairs
         auto drain = [&]() {
             mine |= sg_expand(mw, qn, row, off, val, sh.shift);
             qn = 0;
         };
+        const bool can = __ldg(off + y + 1) > __ldg(off + y);
+        u32 *mp = m + (u64) y * sh.words + lane;
         {
             u32 mm = act, gc = 0, turn = 0;
             while (mm) {
                 u32 c[4];
                 four(mm, gc, c);
                 if (NW > 1 && turn++ % NW != part) continue;
-                u32 w[4] = {0, 0, 0, 0};
+                u32 w[4], old[4];
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q) {
+                    w[q] = old[q] = 0;
+                    if (c[q] != EMPTY) old[q] = mp[c[q] * 32];
+                }
                 for (u32 e0 = 0; e0 < n; e0 += 32) {
                     u32 p = y0, a = a0;
                     if (e0) parents(e0, p, a);
+                    // two in-neighbours at a time: eight lines in flight
                     for (u32 all = __ballot_sync(0xffffffffu, a != 0); all; all &= all - 1) {
                         const u32 j = __ffs(all) - 1;
+                        all &= all - 1;
+                        const u32 j2 = all ? __ffs(all) - 1 : j;
                         const u32 *src = st.cur + (u64) __shfl_sync(0xffffffffu, p, j) * sh.words + lane;
+                        const u32 *src2 = st.cur + (u64) __shfl_sync(0xffffffffu, p, j2) * sh.words + lane;
                         const u32 aj = __shfl_sync(0xffffffffu, a, j);
+                        const u32 aj2 = __shfl_sync(0xffffffffu, j2 == j ? 0u : a, j2);
+                        u32 x[4], x2[4];
 #pragma unroll
-                        for (u32 q = 0; q < 4; ++q)
-                            if (c[q] != EMPTY && ((aj >> (c[q] >> sh.shift)) & 1u)) w[q] |= __ldg(src + c[q] * 32);
+                        for (u32 q = 0; q < 4; ++q) {
+                            x[q] = x2[q] = 0;
+                            if (c[q] == EMPTY) continue;
+                            if ((aj >> (c[q] >> sh.shift)) & 1u) x[q] = __ldg(src + c[q] * 32);
+                            if ((aj2 >> (c[q] >> sh.shift)) & 1u) x2[q] = __ldg(src2 + c[q] * 32);
+                        }
+#pragma unroll
+                        for (u32 q = 0; q < 4; ++q) w[q] |= x[q] | x2[q];
                     }
                 }
 #pragma unroll
                 for (u32 q = 0; q < 4; ++q) {
                     if (c[q] == EMPTY) continue;
-                    u32 v = w[q] & __ldg(has + c[q] * 32 + lane);  // the others have no children
+                    u32 v = w[q] & ~old[q];
+                    if (base_rule && (y >> 5) == c[q] * 32 + lane) v &= ~(1u << (y & 31));  // x != y
+                    if (v) mp[c[q] * 32] = old[q] | v;
+                    fresh += __popc(v);
+                    if (!can) continue;
+                    v &= __ldg(has + c[q] * 32 + lane);  // the others have no children
                     const u32 cnt = __popc(v);
                     const u32 incl = warp_inclusive_sum(cnt);
                     const u32 total = __shfl_sync(0xffffffffu, incl, 31);
                     if (!total) continue;
+                    rows += cnt;
                     if (qn + total > SG_QUEUE) drain();
                     if (total <= SG_QUEUE) {
                         for (u32 at = qn + incl - cnt; v; v &= v - 1) mw.queue[at++] = (c[q] * 32 + lane) * 32 + __ffs(v) - 1;
@@ -225,64 +271,31 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
                     }
                 }
             }
-            drain();
+            if (qn) drain();
         }
         u32 touched = __reduce_or_sync(0xffffffffu, mine);
         if constexpr (NW > 1) {
             if (lane == 0 && touched) atomicOr(&team.touched, touched);
             __syncthreads();  // the row is complete
             touched = team.touched;
-            if (tl == 0) team.news = 0;
-            __syncthreads();
+            __syncthreads();  // every warp has read it
+            if (tl == 0) team.touched = 0;
         } else {
             __syncwarp();
         }
-        // new pairs of the touched chunks
-        const bool can = __ldg(off + y + 1) > __ldg(off + y);
-        u32 news = 0;
-        {
-            u32 mm = touched, gc = 0, turn = 0;
-            while (mm) {
-                u32 c[4];
-                four(mm, gc, c);
+        // the new pairs' children leave for the next level
+        for (u32 mm = touched, turn = 0; mm; mm &= mm - 1) {
+            const u32 c0 = (u32) (__ffs(mm) - 1) << sh.shift, c1 = min(sh.words / 32, c0 + (1u << sh.shift));
+            for (u32 cc = c0; cc < c1; ++cc) {
                 if (NW > 1 && turn++ % NW != part) continue;
-                u32 v[4], old[4];
-                u32 *mp = m + (u64) y * sh.words + lane;
-#pragma unroll
-                for (u32 q = 0; q < 4; ++q) {
-                    v[q] = old[q] = 0;
-                    if (c[q] != EMPTY) {
-                        const u32 k = c[q] * 32 + lane;
-                        v[q] = row[k];
-                        row[k] = 0;
-                        if (base_rule && (y >> 5) == k) v[q] &= ~(1u << (y & 31));  // x != y
-                        if (v[q]) old[q] = mp[c[q] * 32];
-                    }
-                }
-#pragma unroll
-                for (u32 q = 0; q < 4; ++q) {
-                    if (c[q] == EMPTY) continue;
-                    const u32 nw = v[q] & ~old[q];
-                    if (nw) mp[c[q] * 32] = old[q] | nw;
-                    const bool line = __any_sync(0xffffffffu, nw != 0);
-                    if (line || sh.shift) st.nxt[(u64) y * sh.words + c[q] * 32 + lane] = nw;
-                    if (line) {
-                        news |= 1u << (c[q] >> sh.shift);
-                        fresh += __popc(nw);
-                        if (can) rows += __popc(nw & __ldg(has + c[q] * 32 + lane));
-                    }
-                }
+                const u32 k = cc * 32 + lane;
+                st.nxt[(u64) y * sh.words + k] = row[k];
+                row[k] = 0;
             }
-        }
-        if constexpr (NW > 1) {
-            if (lane == 0 && news) atomicOr(&team.news, news);
-            if (tl == 0) team.touched = 0;  // every warp has read it
-            __syncthreads();
-            news = team.news;
         }
         if (tl == 0) {
             st.todo[y] = 0;
-            if (news) st.tag_next[y] = make_uint2(news, st.level);
+            if (touched) st.tag_next[y] = make_uint2(touched, st.level);
         }
     }
     fresh = warp_sum(fresh);
@@ -385,7 +398,7 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     };
     DL_LAUNCH(ctx, K_PREP, 128.0 * n,
               sg_identity_kernel<<<grid_for(words * 32 * 32, T256, ctx), T256, 0, ctx.stream>>>(
-                  sh, view(0), g.csr.off, r.cl_cols.as<u32>()));
+                  sh, view(0), g.csr.off, g.csr.val, r.cl_cols.as<u32>()));
     push(0);
     pt.mark(PH_JOIN);
     // level 1 is the base rule, level k + 1 iteration k; level k + 1's joins are
