@@ -26,9 +26,9 @@
 // Measured on B200 against the n x n bit matrix stepped by one launch per
 // iteration (dl_bitmap.cu), edges and result rows on the device: Chung-Lu graph
 // of 317K nodes (1.88e9 pairs; 9.3K heavy sources hold 99 % of them)
-// 45.5 -> 12.4 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 4.0 ms
-// (5.0 with a warp for every source); DAG of 5.5K edges from and to host memory
-// 3.5 -> 0.66 ms.
+// 45.5 -> 12.0 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 3.7 ms
+// (with a warp for every source a millisecond more); DAG of 5.5K edges from and to
+// host memory 3.5 -> 0.53 ms.
 #include <type_traits>
 
 #include "dl_closure.h"

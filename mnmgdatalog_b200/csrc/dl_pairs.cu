@@ -12,8 +12,8 @@
 // Measured on B200 against the bit matrix stepped by one launch per iteration:
 // lattice of 494K edges (1.5M pairs, 32 iterations, a 28 GB matrix) 41 -> 1.5 ms;
 // 5K edges from and to host memory 1.15 -> 0.6 ms. Against the union of 32
-// instances on the sorted runs (1K-100K edges, host rows) 22 -> 11 ms, most of
-// which is the callers' copies.
+// instances on the sorted runs (1K-100K edges, host rows) 22 -> 6.6 ms, a
+// third of it the host's waits and copies.
 #include "dl_pairs.h"
 #include "dl_scan.cuh"
 
@@ -274,6 +274,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
             good = 0;
             while (good < batch && hs[1 + good] < st.cap) ++good;
         }
+        const u64 listed = ps.n_words();
         for (u64 k = 0; k < good; ++k) {
             const u64 lv = level + k;
             if (lv) ps.rows.push_back(hs[1 + PS_LEVELS + (level ? k : k - 1)]);
@@ -283,6 +284,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
                 break;
             }
         }
+        ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * (ps.n_words() - listed));  // a new pair's word
         if (end) break;
         level += good;
         if (!full && max_levels && level > max_levels) {

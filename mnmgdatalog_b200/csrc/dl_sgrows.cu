@@ -424,6 +424,7 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
         for (u64 k = 0; k < batch && !done; ++k) {
             const u64 level = first + k, c = hs[SG_LEVELS + 1 + k], j = hs[2 * (SG_LEVELS + 1) + k];
             nfull += c;
+            ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * c);  // a new pair's word
             if (level == 1) {
                 cnt[1] = c;
                 joinable[1] = j;
