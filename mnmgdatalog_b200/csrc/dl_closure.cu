@@ -1532,9 +1532,11 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
     if (light.n_heavy) {
         const u64 need = closure_pull_bytes(n, light.n_heavy);
         if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-        u64 held = r.bm_t.cap + ws.cl_rows[0].cap + ws.cl_rows[1].cap;
+        // memory the context holds (a repeated run) needs no driver query: one in ten
+        // stalls the host for milliseconds
+        u64 held = r.bm_t.cap + ws.cl_rows[0].cap + ws.cl_rows[1].cap + ws.cl_act.cap;
         for (const DevBuf &b : ctx.spares) held += b.cap;
-        if (need > held / 2) {
+        if (need > held) {
             size_t free_b = 0, total_b = 0;
             DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
             if (need > ((u64) free_b + held) / 2) return false;

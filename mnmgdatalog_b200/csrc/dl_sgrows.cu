@@ -331,7 +331,7 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     if (3 * bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
     u64 held = ws.cl_rows[0].cap + ws.cl_rows[1].cap;
     for (const DevBuf &b : ctx.spares) held += b.cap;
-    if (3 * bytes > held / 2) {
+    if (3 * bytes > held) {  // (no driver query for memory that a repeated run holds)
         size_t free_b = 0, total_b = 0;
         DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
         if (3 * bytes > ((u64) free_b + held) / 2) return false;
