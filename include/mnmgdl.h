@@ -96,7 +96,7 @@ typedef struct dl_options {
     int32_t wcc_stop;        /* dl_wcc_stop */
     int32_t max_iterations;  /* 0 = run to the fixpoint */
     int32_t phase_timing;    /* 1 = record per-phase device times (adds events) */
-    int32_t dedup;           /* dl_dedup (TC runs; SG and sessions always sort) */
+    int32_t dedup;           /* dl_dedup (TC and SG runs; sessions choose by themselves) */
     int32_t reserved[4];
 } dl_options;
 
@@ -128,8 +128,7 @@ DL_API dl_status dl_context_create(int32_t device, void *stream, dl_context **ou
 DL_API dl_status dl_context_destroy(dl_context *ctx);
 DL_API dl_status dl_context_synchronize(dl_context *ctx);
 /* Waits for the context's stream, then frees the device memory the context keeps between
- * calls: its workspace and cached buffers (e.g. the bit matrix of the last TC run, 2 x n*n/8
- * bytes). Results of live runs and sessions are not touched; the next call allocates again.
+ * calls: its workspace and cached buffers (e.g. the bit rows or the bit matrix of the last TC run). Results of live runs and sessions are not touched; the next call allocates again.
  * No counterpart in the reference (its drivers free everything per iteration). */
 DL_API dl_status dl_context_release_memory(dl_context *ctx);
 DL_API dl_status dl_free(dl_context *ctx, void *device_ptr);
@@ -145,7 +144,7 @@ typedef struct dl_tuning {
     int32_t sort_input_tma;       /* three-kernel pass input: 1 = TMA double buffer (default), 0 = direct loads */
     double hash_load_factor;      /* dl_build_hash_table's default load factor (0 < lf < 1, default 0.5) */
     int32_t join_first_pass;      /* TC: 1 = the join emit also does the sort's first radix pass (default), 0 = not */
-    int32_t bitmap_max_gib;       /* TC dedup AUTO: largest bit matrix + column offsets, GiB (0..1024, default 48; 0 = never) */
+    int32_t bitmap_max_gib;       /* dedup AUTO: largest bit rows, or bit matrix + column offsets, GiB (0..1024, default 48; 0 = never) */
     int32_t bitmap_unit_rows;     /* bit-matrix TC: delta rows per work unit (1..16777216, default 65536) */
     int32_t cache_max_gib;        /* outgrown or released device buffers the context keeps for reuse, at most
                                      this many GiB (0..1024, default 96; 0 = free them at once) */

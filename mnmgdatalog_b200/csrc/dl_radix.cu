@@ -245,8 +245,8 @@ constexpr int US_THREADS = 512;
 // Up to this many CTAs the downsweep's CTAs scan the counts themselves (a thread adds up
 // its digit's row) instead of a launch of their own: at 36 CTAs the scatter takes 2 us
 // longer and the launch and the clearing before it, 8 us, go. A row is read serially, so
-// that with hundreds of CTAs the launch is the shorter one. Runs of 5.5K to 40K edges
-// (4-8 passes): 0.55 -> 0.53 ms (TC), 0.53 -> 0.51 ms (WCC).
+// that with hundreds of CTAs the launch is the shorter one. Whole runs: TC of 5.5K
+// edges 0.55 -> 0.53 ms (6 passes), WCC of 20K 0.53 -> 0.51 ms (4 passes).
 constexpr u32 DS_OWN_SCAN = 64;
 
 struct DsSmem {

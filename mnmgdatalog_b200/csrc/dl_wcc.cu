@@ -13,10 +13,10 @@
 //
 // Bound by launches and host waits on small graphs: an iteration moves 36 bytes
 // per edge of the changed nodes. Measured on B200 against four launches and two host
-// waits per iteration (count, scan, balanced emit, rebuild): 24K edges over 16K
-// nodes 0.93 -> 0.53 ms for the whole run, 700K edges over 100K nodes 2.22 ->
-// 1.28, 48 instances
-// in one union 11.3 -> 3.7 (they iterate on the device alone, not step by step).
+// waits per iteration (count, scan, balanced emit, rebuild): 20K edges from and
+// to host memory 0.93 -> 0.53 ms for the whole run, 1.05M edges on the device 2.22 ->
+// 1.28, 48 instances of 1K to 200K edges in one union 11.3 -> 3.7
+// (they iterate on the device alone, not step by step).
 #include "dl_wcc.h"
 #include "dl_pull.cuh"
 
@@ -147,7 +147,7 @@ __device__ __forceinline__ void wcc_lower(const WccState &st, u32 level, u32 at,
 // = where the number of nodes changed before it is): a warp takes 4 to 32 of them, so
 // that all warps have some, and walks their edges 32 at a time; long lists go to the
 // next launch in pieces. (Lists of up to 1024 edges in takes of 32 left single warps
-// with thousands of edges: 1.22 ms of 1.92 on 700K edges of skewed degrees.)
+// with thousands of edges: 1.22 ms of 1.92 on 1.05M edges of skewed degrees.)
 __global__ void __launch_bounds__(WC_THREADS)
 wcc_level_kernel(WccState st, const u32 *__restrict__ off, const u32 *__restrict__ val, u32 level, u32 at,
                  const unsigned long long *__restrict__ n_prev) {
