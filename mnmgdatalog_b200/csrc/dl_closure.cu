@@ -575,10 +575,15 @@ closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, con
             }
             return true;
         };
-        // rows of a group of up to 32 nodes; the level's edges are added to s.edges
+        // rows of a group of up to 32 nodes; the level's edges are added to s.edges. A group
+        // past the limit was not walked at all, so the search must not end here even if
+        // nothing else is new: it counts as one that outgrew its reach.
         auto expand = [&](u32 b, u32 d) {
             const u32 t = walk_rows(s.wbeg[warp], s.wpre[warp], b, d, val, lane, lt, le, CC_EDGES, visit);
-            if (lane == 0 && t) atomicAdd(&s.edges, min(t, CC_EDGES + 1));
+            if (lane == 0 && t) {
+                atomicAdd(&s.edges, min(t, CC_EDGES + 1));
+                if (t > CC_EDGES) atomicMax(&s.tail, reach + 1);
+            }
         };
         if (warp == 0) {
             const u32 b0 = __ldg(off + x), d0 = __ldg(off + x + 1) - b0;

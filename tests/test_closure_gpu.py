@@ -81,3 +81,59 @@ def test_tc_searches_equal_sorted_runs(engine, name):
     if want.output_tuples < 5 * 10**7:
         host = engine.tc(e, max_iterations=stop)
         assert np.array_equal(host.rows, want.rows.cpu().numpy())
+
+
+def _chain(n):
+    """0 -> 1 -> n leaves."""
+    return np.concatenate([[[0, 1]], np.stack([np.full(n, 1), 2 + np.arange(n)], 1)])
+
+
+def _hubs(hubs, each):
+    """A source above `hubs` nodes of `each` out-edges, all to their own leaves."""
+    leaves = hubs + 1 + np.arange(hubs * each)
+    return np.concatenate([np.stack([np.zeros(hubs, int), 1 + np.arange(hubs)], 1),
+                           np.stack([np.repeat(1 + np.arange(hubs), each), leaves], 1)])
+
+
+def _two_groups(hubs, each, small):
+    """The same with `small` further nodes of one out-edge each, which another warp takes."""
+    e = _hubs(hubs, each)
+    top = int(e.max()) + 1
+    mid = top + np.arange(small)
+    return np.concatenate([e, np.stack([np.zeros(small, int), mid], 1), np.stack([mid, mid + small], 1)])
+
+
+# join words of one warp's rows on both sides of a CTA's 2^18 and of a warp's 2^14
+WIDE = {f"chain_{n}": _chain(n) for n in (16383, 16384, 16385, 262143, 262144, 262145, 300_000)}
+WIDE |= {"hubs_8191": _hubs(32, 8191), "hubs_8192": _hubs(32, 8192), "hubs_9000": _hubs(32, 9000),
+         "two_groups": _two_groups(32, 9000, 40), "fan_262145": _fan(262_145, 3)}
+
+
+def _check_wide(got, want, name):
+    assert got.deltas.tolist() == want.deltas.tolist(), name
+    assert got.output_tuples == want.output_tuples and np.array_equal(got.rows, want.rows), name
+
+
+@pytest.mark.parametrize("name", sorted(WIDE))
+def test_tc_rows_past_a_searchs_join_words(engine, name):
+    e = np.ascontiguousarray(WIDE[name]).astype(np.int32)
+    want, got = engine.tc(e, dedup="sort"), engine.tc(e)
+    _check_wide(got, want, name)
+    assert got.join_rows.tolist() == want.join_rows.tolist() and got.full_rows.tolist() == want.full_rows.tolist()
+
+
+def test_tc_wide_rows_in_a_batch_and_a_session(engine):
+    """Wide nodes and heavy sources side by side with small instances."""
+    sets = {k: np.ascontiguousarray(v).astype(np.int32) for k, v in WIDE.items()}
+    sets["both"] = np.concatenate([_chain(300_000), 400_000 + _cycle(4200)]).astype(np.int32)
+    sets["path"] = _path(30).astype(np.int32)
+    want = {k: engine.tc(v, dedup="sort") for k, v in sets.items()}
+    for k, got in zip(sets, engine.run_batch("tc", list(sets.values()))):
+        _check_wide(got, want[k], k)
+    with engine.session("tc") as s:
+        ids = [(i, k) for k, i in zip(sets, s.admit_many(list(sets.values())))]
+        s.step()
+        ids += [(s.admit(sets[k]), k) for k in ("chain_262145", "two_groups", "path")]
+        s.run()
+        for i, k in ids:
+            _check_wide(s.result(i), want[k], k)
