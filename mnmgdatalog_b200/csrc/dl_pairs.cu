@@ -274,7 +274,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
             good = 0;
             while (good < batch && hs[1 + good] < st.cap) ++good;
         }
-        const u64 listed = ps.n_words();
+        const u64 listed = ps.n_words(), begun = level;
         for (u64 k = 0; k < good; ++k) {
             const u64 lv = level + k;
             if (lv) ps.rows.push_back(hs[1 + PS_LEVELS + (level ? k : k - 1)]);
@@ -308,8 +308,9 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
                           pair_refill_kernel<<<grid_for(keep, T256, ctx), T256, 0, ctx.stream>>>(st.list, keep, st.set,
                                                                                                 st.mask));
             DL_CUDA(cudaMemcpyAsync(st.count, ps.bound.data() + level, 8, cudaMemcpyHostToDevice, ctx.stream));
-            // rows counted by the levels that are repeated
-            DL_CUDA(cudaMemsetAsync(st.rows + (level ? level - 1 : 0), 0, (PS_LEVELS + 1) * 8, ctx.stream));
+            // rows counted by the levels that are repeated: the batch's last one counted rows[begun + batch - 2]
+            const u64 row = level ? level - 1 : 0;
+            DL_CUDA(cudaMemsetAsync(st.rows + row, 0, (begun + batch - 1 - row) * 8, ctx.stream));
             ctx.sync();  // ps.bound is host memory
         }
     }

@@ -77,3 +77,33 @@ def test_sg_set_outgrown(engine):
         want = engine.sg(e, dedup="bitmap")
         assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
     assert len(got.rows) < 2**19 < len(engine.sg(sets[0]).rows)
+
+
+def _chains(count, length, leaves, first):
+    """A root above `count` chains of `length` nodes, each with `leaves` leaves at its
+    end: count * (count - 1) * leaves^2 pairs of leaves, all found in level `length`."""
+    head = first + 1 + np.arange(count) * length
+    node = (head[:, None] + np.arange(length)).ravel()
+    out = [np.stack([np.full(count, first), head], 1),
+           np.stack([node, node + 1], 1).reshape(count, length, 2)[:, :-1].reshape(-1, 2)]
+    last, leaf = head + length - 1, first + 1 + count * length + np.arange(count * leaves)
+    out.append(np.stack([np.repeat(last, leaves), leaf], 1))
+    return np.concatenate(out), int(leaf[-1]) + 1
+
+
+@pytest.mark.parametrize("first,second", [(0, 9), (6, 61), (6, 60), (7, 62), (14, 61)])
+def test_sg_levels_repeated_near_the_counters_end(engine, first, second):
+    """The set is outgrown in level `first` (past 512K pairs) and again in level
+    `second` (past 2M): the levels after it are repeated, at (6, 61) with the last of
+    the 64 levels' counters."""
+    a, top = _chains(12, first, 64, 0) if first else _chains(1, 1, 1, 0)
+    if not first:  # one node above 64 nodes of 64 leaves would come later: siblings past 512K in the base
+        a = np.stack([np.repeat(np.arange(200), 60), 1000 + np.arange(12_000)], 1)
+        top = 13_000
+    b, _ = _chains(24, second, 64, top)
+    e = np.concatenate([a, b]).astype(np.int32)
+    want, got = engine.sg(e, dedup="bitmap"), engine.sg(e)
+    assert got.deltas.tolist() == want.deltas.tolist() and got.join_rows.tolist() == want.join_rows.tolist()
+    assert np.array_equal(got.rows, want.rows)
+    res = engine.run_batch("sg", [e])[0]
+    assert res.deltas.tolist() == want.deltas.tolist() and np.array_equal(res.rows, want.rows)
