@@ -54,9 +54,11 @@ void ReturnBox::hand_back(DevBuf &b) {
 void SessionKit::release() {
     if (ctrl) cudaFree(ctrl);
     if (host_scalars) cudaFreeHost(host_scalars);
+    if (host_stage) cudaFreeHost(host_stage);
     for (DevBuf *b : {&lookback, &sort_hist, &lbs_splits, &radix_part, &merge_splits, &bucket_cursor}) b->release();
     ctrl = nullptr;
-    host_scalars = nullptr;
+    host_scalars = host_stage = nullptr;
+    host_stage_bytes = 0;
 }
 
 void *Context::host_staging(size_t bytes) {

@@ -168,6 +168,8 @@ struct SessionKit {
     u64 *host_scalars = nullptr;
     u32 epoch = 0;
     DevBuf lookback, sort_hist, lbs_splits, radix_part, merge_splits, bucket_cursor;
+    u64 *host_stage = nullptr;
+    size_t host_stage_bytes = 0;
     void release();
 };
 
@@ -195,7 +197,7 @@ struct Context {
     std::shared_ptr<ReturnBox> box = std::make_shared<ReturnBox>();
     std::vector<SessionKit> kits;   // of destroyed sessions
     static constexpr size_t kKits = 4;
-    u64 *host_stage = nullptr;      // page-locked staging of result labels
+    u64 *host_stage = nullptr;      // a session's page-locked staging of result labels
     size_t host_stage_bytes = 0;
     // Page-locked memory of at least `bytes`, or null past 64 MiB.
     void *host_staging(size_t bytes);

@@ -880,6 +880,8 @@ SessionImpl *session_create(Context &parent, int program, const dl_options &opt,
     c.radix_part = kit.radix_part;
     c.merge_splits = kit.merge_splits;
     c.bucket_cursor = kit.bucket_cursor;
+    c.host_stage = kit.host_stage;
+    c.host_stage_bytes = kit.host_stage_bytes;
     std::memset(c.host_scalars, 0, 64 * sizeof(u64));
     DL_CUDA(cudaMemsetAsync(c.ctrl, 0, sizeof(Ctrl), c.stream));
     c.spares = std::move(parent.spares);  // the parent's cached buffers serve the session
@@ -916,7 +918,9 @@ void session_destroy(SessionImpl *s) {
     c.spares.clear();
     // the control block, page-locked scalars and scan scratch serve the next session
     SessionKit kit{c.ctrl, c.host_scalars, c.epoch, c.lookback, c.sort_hist, c.lbs_splits, c.radix_part, c.merge_splits,
-                   c.bucket_cursor};
+                   c.bucket_cursor, c.host_stage, c.host_stage_bytes};
+    c.host_stage = nullptr;
+    c.host_stage_bytes = 0;
     c.lookback = c.sort_hist = c.lbs_splits = c.radix_part = c.merge_splits = c.bucket_cursor = DevBuf();
     if (p.kits.size() < Context::kKits) p.kits.push_back(kit);
     else kit.release();
@@ -1201,7 +1205,7 @@ void session_copy_labels_many(SessionImpl &s, const i64 *ids, u64 count, int32_t
                       in.labels(), in.rank_lo, n, in.ids(), at + n));
         at += 2 * n;
     }
-    int32_t *host = (int32_t *) s.parent->host_staging(total * 8);
+    int32_t *host = (int32_t *) ctx.host_staging(total * 8);
     if (host) {
         DL_CUDA(cudaMemcpyAsync(host, stage.p, total * 8, cudaMemcpyDeviceToHost, ctx.stream));
         ctx.sync();

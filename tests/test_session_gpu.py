@@ -197,3 +197,34 @@ def test_admit_many_while_running(engine, prog):
             got[i] = s.result(i, labels=True)
     for k, p in enumerate(plain):
         _same(got[k], p, prog, f"input {k}")
+
+
+def test_label_copies_of_two_sessions_on_two_threads(engine):
+    """Sessions of one context may be read at the same time: each has a stage of its own."""
+    import threading
+    sets = [[graphs.chung_lu(n=400 * (k + 1) * (3 if t else 1), m=1500 * (k + 1), seed=10 * t + k) for k in range(6)]
+            for t in range(2)]
+    want = [[engine.wcc(e, labels=True) for e in group] for group in sets]
+    sessions = [engine.session("wcc") for _ in sets]
+    try:
+        ids = [s.admit_many(group) for s, group in zip(sessions, sets)]
+        for s in sessions:
+            s.run()
+        bad = []
+
+        def read(t):
+            for r in range(60):
+                first = r % len(ids[t])  # sizes vary, so that the stages grow at different times
+                for w, got in zip(want[t][first:], sessions[t].results(ids[t][first:], output="none", labels=True)):
+                    if not (np.array_equal(w.labels, got.labels) and np.array_equal(w.node_ids, got.node_ids)):
+                        bad.append((t, r))
+
+        threads = [threading.Thread(target=read, args=(t,)) for t in range(2)]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+        assert not bad
+    finally:
+        for s in sessions:
+            s.close()
