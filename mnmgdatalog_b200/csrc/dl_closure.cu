@@ -1537,15 +1537,14 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
     if (light.n_heavy) {
         const u64 need = closure_pull_bytes(n, light.n_heavy);
         if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-        // memory the context holds (a repeated run) needs no driver query: one in ten
-        // stalls the host for milliseconds
-        u64 held = r.bm_t.cap + ws.cl_rows[0].cap + ws.cl_rows[1].cap + ws.cl_act.cap;
-        for (const DevBuf &b : ctx.spares) held += b.cap;
-        if (need > held) {
-            size_t free_b = 0, total_b = 0;
-            DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-            if (need > ((u64) free_b + held) / 2) return false;
-        }
+        const u64 rows = n * pull_words(light.n_heavy) * 4;
+        if (!ctx.room_for({{&r.bm_t, rows}, {&ws.cl_rows[0], rows}, {&ws.cl_rows[1], rows}, {&ws.cl_act, 8 * n * 4}}))
+            return false;
+        // (now, before smaller requests take the cached buffers that were counted on)
+        ctx.reserve(r.bm_t, rows);
+        ctx.reserve(ws.cl_rows[0], rows);
+        ctx.reserve(ws.cl_rows[1], rows);
+        ctx.reserve(ws.cl_act, 8 * n * 4);
     }
     // host copies of the level counts (index d)
     std::vector<u64> hc(light.levels + 1, 0), hd(light.levels + 1, 0);

@@ -74,12 +74,14 @@ void *Context::host_staging(size_t bytes) {
     return host_stage;
 }
 
+void Context::take_returned() {
+    std::lock_guard<std::mutex> lock(box->m);
+    for (DevBuf &b : box->bufs) spares.push_back(b);
+    box->bufs.clear();
+}
+
 void Context::reserve_tight(DevBuf &buf, size_t bytes) {
-    {
-        std::lock_guard<std::mutex> lock(box->m);
-        for (DevBuf &b : box->bufs) spares.push_back(b);
-        box->bufs.clear();
-    }
+    take_returned();
     int best = -1;
     for (int i = 0; i < (int) spares.size(); ++i)
         if (spares[i].cap >= bytes && spares[i].cap <= 2 * bytes + (1 << 20) &&
@@ -94,6 +96,32 @@ void Context::reserve_tight(DevBuf &buf, size_t bytes) {
     trim_spares();
 }
 
+// Best fit among the cached buffers, but never one far larger than the request: a
+// small result must not pin a large buffer that a growing relation will need next.
+int Context::best_spare(const std::vector<DevBuf> &from, size_t bytes) {
+    const size_t limit = std::max<size_t>(4 * bytes, bytes + (size_t(64) << 20));
+    int best = -1;
+    for (int i = 0; i < (int) from.size(); ++i)
+        if (from[i].cap >= bytes && from[i].cap <= limit && (best < 0 || from[i].cap < from[best].cap)) best = i;
+    return best;
+}
+
+bool Context::room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants) {
+    take_returned();
+    std::vector<DevBuf> left = spares;
+    size_t fresh = 0;
+    for (const auto &w : wants) {
+        if (w.first->p && w.first->cap >= w.second) continue;
+        const int best = best_spare(left, w.second);
+        if (best >= 0) left.erase(left.begin() + best);
+        else fresh += w.first->p ? std::max(w.second, w.first->cap + w.first->cap / 2) : w.second;
+    }
+    if (!fresh) return true;
+    size_t free_b = 0, total_b = 0;
+    DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return fresh <= free_b / 2;
+}
+
 void Context::reserve(DevBuf &buf, size_t bytes, bool zero) {
     if (buf.fixed) {  // a fixed slice: it fits or the request is an error
         buf.reserve(bytes);
@@ -104,19 +132,8 @@ void Context::reserve(DevBuf &buf, size_t bytes, bool zero) {
     // A buffer that outgrows itself grows by half at least, so a relation that
     // grows every iteration is reallocated O(log) times, not at every step.
     const size_t want = buf.p ? std::max(bytes, buf.cap + buf.cap / 2) : bytes;
-    {
-        std::lock_guard<std::mutex> lock(box->m);
-        for (DevBuf &b : box->bufs) spares.push_back(b);
-        box->bufs.clear();
-    }
-    // Best fit among the cached buffers, but never one far larger than the
-    // request: a small result must not pin a large buffer that a growing
-    // relation will need next.
-    const size_t limit = std::max<size_t>(4 * bytes, bytes + (size_t(64) << 20));
-    int best = -1;
-    for (int i = 0; i < (int) spares.size(); ++i)
-        if (spares[i].cap >= bytes && spares[i].cap <= limit && (best < 0 || spares[i].cap < spares[best].cap))
-            best = i;
+    take_returned();
+    const int best = best_spare(spares, bytes);
     if (best >= 0) {
         if (buf.p) spares.push_back(buf);
         buf = spares[best];

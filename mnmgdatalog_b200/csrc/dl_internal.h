@@ -7,11 +7,13 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../../include/mnmgdl.h"
@@ -227,6 +229,14 @@ struct Context {
     // Ensure buf holds `bytes`, preferring a spare buffer over cudaMalloc.
     void reserve(DevBuf &buf, size_t bytes, bool zero = false);
     void give_back(DevBuf &buf);
+    // Buffers handed back on any thread join the cache.
+    void take_returned();
+    // Index of the cached buffer reserve() takes for `bytes`, or -1.
+    static int best_spare(const std::vector<DevBuf> &from, size_t bytes);
+    // Whether buffers of these sizes may be reserved by a form that another one can stand
+    // in for: what they would newly allocate is at most half of the free device memory (the
+    // rest is left to whoever shares the GPU). No driver query when nothing would be.
+    bool room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants);
     // A buffer that goes into a caller's hands: at most twice the size asked for.
     void reserve_tight(DevBuf &buf, size_t bytes);
     void trim_spares();

@@ -172,13 +172,7 @@ bool self_join_rows(Context &ctx, Run &r, const Csr &in, u64 total, PhaseTimer &
     // dozen times: worth it up to 16 bytes of matrix per join word (a result
     // row per 1K bits or so).
     if (smem + 4096 > 227 * 1024 || bytes > 16 * total || bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-    u64 held = 0;
-    for (const DevBuf &b : ctx.spares) held += b.cap;
-    if (bytes > held) {  // (no driver query for memory that a repeated run holds)
-        size_t free_b = 0, total_b = 0;
-        DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        if (bytes > ((u64) free_b + held) / 2) return false;
-    }
+    if (!ctx.room_for({{&r.bm_t, bytes}})) return false;
     pt.mark(PH_JOIN);
     try {
         ctx.reserve(r.bm_t, bytes);

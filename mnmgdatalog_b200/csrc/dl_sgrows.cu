@@ -329,13 +329,11 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     const u64 bytes = n * words * 4;
     if (words * 4 + 24 * 1024 > 227 * 1024) return false;  // a row in shared memory beside the queues
     if (3 * bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-    u64 held = ws.cl_rows[0].cap + ws.cl_rows[1].cap;
-    for (const DevBuf &b : ctx.spares) held += b.cap;
-    if (3 * bytes > held) {  // (no driver query for memory that a repeated run holds)
-        size_t free_b = 0, total_b = 0;
-        DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        if (3 * bytes > ((u64) free_b + held) / 2) return false;
-    }
+    if (!ctx.room_for({{&r.bm_t, bytes}, {&ws.cl_rows[0], bytes}, {&ws.cl_rows[1], bytes}})) return false;
+    // (now, before smaller requests take the cached buffers that were counted on)
+    ctx.reserve(r.bm_t, bytes);
+    ctx.reserve(ws.cl_rows[0], bytes);
+    ctx.reserve(ws.cl_rows[1], bytes);
     pt.mark(PH_INIT);
     PullShape sh{n, (u32) words, 0};
     while ((32u << sh.shift) < words / 32) ++sh.shift;
@@ -357,9 +355,6 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     u32 *has = ws.bit_hasout.as<u32>();
     DL_LAUNCH(ctx, K_PREP, 4.0 * n,
               has_children_kernel<<<grid_for(words, T256, ctx), T256, 0, ctx.stream>>>(g.csr.off, n, words, has));
-    ctx.reserve(r.bm_t, bytes);
-    ctx.reserve(ws.cl_rows[0], bytes);
-    ctx.reserve(ws.cl_rows[1], bytes);
     ctx.reserve(ws.cl_act, 8 * n * 4);
     ctx.reserve(r.cl_cols, words * 32 * 4);
     DL_CUDA(cudaMemsetAsync(r.bm_t.p, 0, bytes, ctx.stream));

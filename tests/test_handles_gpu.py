@@ -67,3 +67,29 @@ def test_results_in_one_call(engine, prog):
         assert s.results([]) == []
         with pytest.raises(DatalogError):
             s.results([99])
+
+
+def test_bit_rows_take_at_most_half_of_the_free_memory():
+    """SG's three bit-row matrices (0.8 GB) while 1.2 GB are free: cached buffers that
+    none of them fits into are no room for them, so another form runs."""
+    import torch
+    rng = np.random.default_rng(3)
+    e = np.concatenate([rng.integers(0, 46_000, (70_000, 2)), [[0, 45_999]]]).astype(np.int32)
+    with Engine(0) as eng:
+        want = eng.sg(e, max_iterations=1)
+    with Engine(0) as eng:
+        eng.sg(e[:3000], max_iterations=1)  # the workspace's small buffers
+        rel = torch.stack([torch.randperm(4_000_000, device="cuda", dtype=torch.int32)] * 2, 1).contiguous()
+        tables = [eng.get_hash_table(rel) for _ in range(12)]  # 0.14 GB each
+        del rel
+        torch.cuda.empty_cache()
+        for t in tables:
+            t.close()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - 1200 * 2**20, dtype=torch.uint8, device="cuda")
+        before = torch.cuda.mem_get_info()[0]
+        got = eng.sg(e, max_iterations=1)
+        after = torch.cuda.mem_get_info()[0]
+        del fill
+        torch.cuda.empty_cache()
+        assert before < 1300 * 2**20 and after >= before // 2
+        assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
