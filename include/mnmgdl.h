@@ -144,7 +144,8 @@ typedef struct dl_tuning {
     int32_t sort_input_tma;       /* three-kernel pass input: 1 = TMA double buffer (default), 0 = direct loads */
     double hash_load_factor;      /* dl_build_hash_table's default load factor (0 < lf < 1, default 0.5) */
     int32_t join_first_pass;      /* TC: 1 = the join emit also does the sort's first radix pass (default), 0 = not */
-    int32_t bitmap_max_gib;       /* dedup AUTO: largest bit rows, or bit matrix + column offsets, GiB (0..1024, default 48; 0 = never) */
+    int32_t bitmap_max_gib;       /* dedup AUTO: largest bit rows, or bit matrix + column offsets, GiB (0..1024, default 48; 0 = never);
+                                     SG in sessions: the search's pair list and set (0 = sorted runs) */
     int32_t bitmap_unit_rows;     /* bit-matrix TC: delta rows per work unit (1..16777216, default 65536) */
     int32_t cache_max_gib;        /* outgrown or released device buffers the context keeps for reuse, at most
                                      this many GiB (0..1024, default 96; 0 = free them at once) */

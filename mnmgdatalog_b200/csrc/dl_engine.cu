@@ -729,11 +729,11 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_opt
                               u64 &nfull) {
     Workspace &ws = ctx.ws;
     pt.mark(PH_JOIN);
-    // up to 64 pairs a node the list is the cheaper form whatever the matrix costs
+    // (the first set holds four to eight pairs a node, 512K at least)
     const u64 most = bitmat_allowed(ctx, g.n_ids, true) ? std::max<u64>(64 * (u64) g.n_ids, 1 << 19) : 0;
     try {
         const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits,
-                                          opt.max_iterations > 0 ? (u64) opt.max_iterations : 0, most);
+                                          opt.max_iterations > 0 ? (u64) opt.max_iterations : 0, most, ~0ull);
         if (!ps.complete) return false;
         const u64 n = ps.n_words();
         pt.mark(PH_DEDUP);
@@ -793,7 +793,7 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
         build_csr(ctx, e, ne, g);                     // sg.cu:162
         // a small matrix and more than 1.3 edges a node: most likely many pairs
         const bool rows_first = g.n_ids <= SG_ROWS_FIRST && ne * 10 > 13 * (u64) g.n_distinct;
-        if (search && !rows_first && pair_search_fits(ctx, g.csr, 0, g.n_ids))
+        if (search && !rows_first && pair_degrees(ctx, g.csr, 0, g.n_ids).fits())
             listed = sg_pairs_fixpoint(ctx, r, g, opt, pt, nfull);
         if (search && !listed && bitmat_allowed(ctx, g.n_ids, true)) {
             if (!rows_first) e = sg_edge_words(ctx, rows, n, g, ne);  // again: the search used the buffers

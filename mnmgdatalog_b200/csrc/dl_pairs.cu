@@ -154,12 +154,20 @@ __global__ void pair_refill_kernel(const u64 *__restrict__ list, u64 n, u64 *set
         pair_insert(set, mask, list[i]);
 }
 
-__global__ void max_degree_kernel(const u32 *__restrict__ off, u64 lo, u64 hi, u32 *__restrict__ most) {
-    u32 m = 0;
-    for (u64 r = lo + (u64) blockIdx.x * blockDim.x + threadIdx.x; r < hi; r += (u64) gridDim.x * blockDim.x)
-        m = max(m, off[r + 1] - off[r]);
+// found[0] = largest degree, found[1] = ranks with out-edges.
+__global__ void degrees_kernel(const u32 *__restrict__ off, u64 lo, u64 hi, unsigned long long *__restrict__ found) {
+    u32 m = 0, c = 0;
+    for (u64 r = lo + (u64) blockIdx.x * blockDim.x + threadIdx.x; r < hi; r += (u64) gridDim.x * blockDim.x) {
+        const u32 d = off[r + 1] - off[r];
+        m = max(m, d);
+        c += d != 0;
+    }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && m) {
+        atomicMax(found, (unsigned long long) m);
+        atomicAdd(found + 1, (unsigned long long) c);
+    }
 }
 
 // counts[instance * levels + level] += words. A warp's words are of one level mostly and
@@ -197,17 +205,22 @@ __global__ void pair_counts_kernel(const u64 *__restrict__ list, u64 n, int bits
 
 }  // namespace
 
-bool pair_search_fits(Context &ctx, const Csr &csr, u64 lo, u64 hi) {
-    u32 *most = reinterpret_cast<u32 *>(&ctx.ctrl->scalar[26]);
-    DL_CUDA(cudaMemsetAsync(most, 0, 8, ctx.stream));
+bool PairDegrees::fits() const { return most <= PS_DEGREE; }
+
+PairDegrees pair_degrees(Context &ctx, const Csr &csr, u64 lo, u64 hi) {
+    auto *found = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[26]);
+    DL_CUDA(cudaMemsetAsync(found, 0, 16, ctx.stream));
     DL_LAUNCH(ctx, K_PREP, 4.0 * (hi - lo),
-              max_degree_kernel<<<grid_for(hi - lo, T256, ctx, 8), T256, 0, ctx.stream>>>(csr.off, lo, hi, most));
-    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, most, 8, cudaMemcpyDeviceToHost, ctx.stream));
+              degrees_kernel<<<grid_for(hi - lo, T256, ctx, 8), T256, 0, ctx.stream>>>(csr.off, lo, hi, found));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, found, 16, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
-    return *reinterpret_cast<u32 *>(ctx.host_scalars) <= PS_DEGREE;
+    PairDegrees d;
+    d.most = (u32) ctx.host_scalars[0];
+    d.sources = ctx.host_scalars[1];
+    return d;
 }
 
-PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most) {
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most, u64 limit) {
     Workspace &ws = ctx.ws;
     PairSearch ps;
     DevBuf &list = ws.jbuf[0], &set = ws.jbuf[1];
@@ -216,6 +229,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
     // that needs more is repeated on a set four times the size
     u64 slots = PS_SLOTS;
     while (slots < 8 * (hi - lo) && !(most && slots / 2 >= 2 * most)) slots <<= 1;
+    if (slots * 12 > limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
     u64 levels = 64;  // level counters: bound[levels + 2], rows[levels + 1], after the list's and blocks' counters
     ctx.reserve(ws.cl_levels, (2 * levels + 16) * 8);
     u64 *base = ws.cl_levels.as<u64>();
@@ -296,6 +310,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
             const u64 keep = ps.bound[level];
             slots *= 4;
             DevBuf nl;
+            if (slots * 12 > limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
             ctx.reserve(nl, slots / 2 * 8);
             DL_CUDA(cudaMemcpyAsync(nl.p, list.p, keep * 8, cudaMemcpyDeviceToDevice, ctx.stream));
             ctx.give_back(list);

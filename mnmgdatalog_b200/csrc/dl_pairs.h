@@ -15,14 +15,22 @@ struct PairSearch {
     u64 n_words() const { return bound.empty() ? 0 : bound.back(); }
 };
 
-// Whether the degrees of ranks [lo, hi) suit the pair search (a pair's
-// expansion is shared by 32 lanes at most).
-bool pair_search_fits(Context &ctx, const Csr &csr, u64 lo, u64 hi);
+// Out-edges of ranks [lo, hi): the largest degree and the ranks that have any.
+struct PairDegrees {
+    u32 most = 0;
+    u64 sources = 0;
+    // A pair's expansion is shared by 32 lanes at most.
+    bool fits() const;
+};
+PairDegrees pair_degrees(Context &ctx, const Csr &csr, u64 lo, u64 hi);
 // The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
-// in ws.jbuf[0], unsorted. Stops after level max_levels (0: at the fixpoint),
-// or once more than `most` words are found (0: never; the search is then not
-// complete and its last level may lack words).
-PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most);
+// in ws.jbuf[0], unsorted. Stops after level max_levels (0: at the fixpoint). The
+// search is not complete, and its last level may lack words,
+//  * with most != 0 (the caller has another form for many pairs): once more than
+//    `most` words are found or the first set is outgrown;
+//  * once the list and the set would need more than `limit` bytes, or more than half
+//    of the free memory.
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most, u64 limit);
 // counts[instance * levels + k] = words of level k of each instance (instance of
 // a word: the last one whose first rank is at most its key rank).
 void pair_level_counts(Context &ctx, const PairSearch &ps, int bits, const u64 *inst_lo, u64 n_inst, u64 *counts);

@@ -12,9 +12,9 @@
 // component's labels (WCC, dl_wcc.cu) never meet another instance's, so the
 // instances admitted together are computed to their own stops in one go -- for
 // WCC with the reference's rule the iteration where that rule fires for the
-// instance -- and the steps report their iterations one by one. SG instances whose
-// degrees do not suit the search keep the common steps: their initial delta joins
-// the next iteration, and each leaves the union at its own fixpoint.
+// instance -- and the steps report their iterations one by one. SG instances that the
+// search does not suit (degrees, memory) keep the common steps: their initial
+// delta joins the next iteration, and each leaves the union at its own fixpoint.
 // Results are bit-exact with running each query alone.
 #include <algorithm>
 #include <cstring>
@@ -586,20 +586,35 @@ void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words, u64 s
     }
 }
 
-// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi))
-// as one search over pairs (dl_pairs.cu). Returns false when a node's degree
-// does not suit it.
+// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi)) as one
+// search over pairs (dl_pairs.cu). False (nothing done) when the sorted runs take them:
+// their degrees do not suit the search, or its list and set would pass bitmap_max_gib or half of the free memory.
 bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
     Context &ctx = s.ctx;
+    Workspace &ws = ctx.ws;
+    const u64 limit = (u64) ctx.tune.bitmap_max_gib << 30;
+    if (limit == 0) return false;
     Csr csr;
     csr.off = s.off.as<u32>();
     csr.val = s.val.as<u32>();
     csr.n_keys = (u32) s.next_rank;
     csr.n_vals = s.n_vals;
-    if (!pair_search_fits(ctx, csr, lo, hi)) return false;
     const u64 n = ids.size();
     const int stop = s.opt.max_iterations;
-    const PairSearch ps = pair_search(ctx, csr, lo, hi, s.bits, stop > 0 ? (u64) stop : 0, 0);
+    const PairDegrees deg = pair_degrees(ctx, csr, lo, hi);
+    if (!deg.fits()) return false;
+    PairSearch ps;
+    try {
+        ps = pair_search(ctx, csr, lo, hi, s.bits, stop > 0 ? (u64) stop : 0, 0, limit);
+    } catch (const Error &err) {
+        if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
+        ps.complete = false;
+    }
+    if (!ps.complete) {
+        ctx.give_back(ws.jbuf[0]);  // the list and the set, for whatever the runs need
+        ctx.give_back(ws.jbuf[1]);
+        return false;
+    }
     const u64 levels = ps.bound.size() - 1;
     std::vector<u64> first(n), cnt(n * levels);
     for (u64 k = 0; k < n; ++k) first[k] = s.inst[ids[k]].rank_lo;

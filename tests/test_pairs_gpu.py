@@ -107,3 +107,29 @@ def test_sg_levels_repeated_near_the_counters_end(engine, first, second):
     assert np.array_equal(got.rows, want.rows)
     res = engine.run_batch("sg", [e])[0]
     assert res.deltas.tolist() == want.deltas.tolist() and np.array_equal(res.rows, want.rows)
+
+
+def _batch_against_sorted(eng, sets, on_runs):
+    """The batch's results, and whether it ran on the sorted runs."""
+    sets = [np.ascontiguousarray(e).astype(np.int32) for e in sets]
+    want = [eng.sg(e, dedup="sort") for e in sets]
+    eng.profile(False)
+    res = eng.run_batch("sg", sets)
+    assert (eng.profile_read()["join_emit"]["launches"] > 0) == on_runs
+    for w, got in zip(want, res):
+        assert got.deltas.tolist() == w.deltas.tolist() and np.array_equal(got.rows, w.rows)
+
+
+def test_sg_session_search_is_bounded():
+    """A search that would pass bitmap_max_gib hands its instances to the sorted runs, before it
+    starts (0) or when its set is outgrown (33M pairs in 0.8 GB, the next size takes 3)."""
+    from mnmgdatalog_b200 import Engine
+    small, mesh = graphs.lattice3d(side=8, seed=1), graphs.lattice3d(side=22, p=0.29, seed=0)
+    with Engine(0) as eng:
+        _batch_against_sorted(eng, [small, mesh], False)
+        assert len(eng.sg(mesh).rows) > 2**25
+        eng.set_tuning(bitmap_max_gib=1)
+        _batch_against_sorted(eng, [small, mesh], True)
+        _batch_against_sorted(eng, [small], False)
+        eng.set_tuning(bitmap_max_gib=0)
+        _batch_against_sorted(eng, [small], True)
