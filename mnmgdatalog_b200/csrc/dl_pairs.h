@@ -23,6 +23,9 @@ struct PairDegrees {
     bool fits() const;
 };
 PairDegrees pair_degrees(Context &ctx, const Csr &csr, u64 lo, u64 hi);
+// Whether sorted runs are the faster form for a session's instances of `n_ids` nodes
+// each, with `edges` between them (see dl_pairs.cu).
+bool pair_search_outrun(const PairDegrees &d, u64 edges, const std::vector<u64> &n_ids);
 // The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
 // in ws.jbuf[0], unsorted. Stops after level max_levels (0: at the fixpoint). The
 // search is not complete, and its last level may lack words,

@@ -13,7 +13,7 @@
 // instances admitted together are computed to their own stops in one go -- for
 // WCC with the reference's rule the iteration where that rule fires for the
 // instance -- and the steps report their iterations one by one. SG instances that the
-// search does not suit (degrees, memory) keep the common steps: their initial
+// search does not suit (degrees, many pairs, memory) keep the common steps: their initial
 // delta joins the next iteration, and each leaves the union at its own fixpoint.
 // Results are bit-exact with running each query alone.
 #include <algorithm>
@@ -586,10 +586,11 @@ void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words, u64 s
     }
 }
 
-// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi)) as one
-// search over pairs (dl_pairs.cu). False (nothing done) when the sorted runs take them:
-// their degrees do not suit the search, or its list and set would pass bitmap_max_gib or half of the free memory.
-bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
+// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi), `edges`
+// between them) as one search over pairs (dl_pairs.cu). False (nothing done) when the
+// sorted runs take them: their degrees do not suit the search, the runs are faster, or
+// its list and set would pass bitmap_max_gib or half of the free memory.
+bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi, u64 edges) {
     Context &ctx = s.ctx;
     Workspace &ws = ctx.ws;
     const u64 limit = (u64) ctx.tune.bitmap_max_gib << 30;
@@ -603,6 +604,9 @@ bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
     const int stop = s.opt.max_iterations;
     const PairDegrees deg = pair_degrees(ctx, csr, lo, hi);
     if (!deg.fits()) return false;
+    std::vector<u64> n_ids(n);
+    for (u64 k = 0; k < n; ++k) n_ids[k] = s.inst[ids[k]].n_ids;
+    if (pair_search_outrun(deg, edges, n_ids)) return false;
     PairSearch ps;
     try {
         ps = pair_search(ctx, csr, lo, hi, s.bits, stop > 0 ? (u64) stop : 0, 0, limit);
@@ -1039,7 +1043,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
             if (nrows[k]) with_rows.push_back(inst(k).id);
         if (tc) {
             // searched as a whole in the next step
-        } else if (s.program == DL_PROGRAM_SG && search_pairs(s, with_rows, B, B + nu)) {
+        } else if (s.program == DL_PROGRAM_SG && search_pairs(s, with_rows, B, B + nu, ne)) {
             for (u64 k = 0; k < count; ++k) empty_base[k] = nrows[k] && inst(k).ahead[0] == 0 && inst(k).n_result == 0;
         } else if (s.program == DL_PROGRAM_SG) {
             // sg.cu:170-217: the base rule of the admitted instances, probing the union table

@@ -133,3 +133,23 @@ def test_sg_session_search_is_bounded():
         _batch_against_sorted(eng, [small], False)
         eng.set_tuning(bitmap_max_gib=0)
         _batch_against_sorted(eng, [small], True)
+
+
+def test_sg_session_many_pairs_of_wide_sources(engine):
+    """Both sides of the rule by sources' out-edges and pairs (pair_search_outrun)."""
+    def rnd(n, d, seed):
+        return np.random.default_rng(seed).integers(0, n, (int(n * d), 2))
+    _batch_against_sorted(engine, [rnd(3000, 3, 1), rnd(3000, 3, 2)], True)
+    _batch_against_sorted(engine, [rnd(3000, 1.8, 1), rnd(3000, 1.8, 2)], False)
+    _batch_against_sorted(engine, [rnd(300, 3, k) for k in range(6)], False)
+    _batch_against_sorted(engine, [_tree(1000, 3), _tree(1800, 3)], True)
+    _batch_against_sorted(engine, [[[0, i + 1] for i in range(60)]] * 20, False)
+    with engine.session("sg") as s:  # a session with both kinds
+        e = [np.asarray(x, np.int32) for x in (rnd(5000, 3, 3), _tree(40, 3))]
+        ids = s.admit_many(e[:1])
+        s.step()
+        ids += s.admit_many(e[1:])
+        s.run()
+        for i, x in zip(ids, e):
+            want, got = engine.sg(x, dedup="sort"), s.result(i)
+            assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
