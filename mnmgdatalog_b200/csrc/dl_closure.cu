@@ -1175,8 +1175,9 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
     ctx.reserve(ws.cl_seg, ns * 8);
     DL_CUDA(cudaMemsetAsync(ws.cl_seg.p, 0, ns * 8, ctx.stream));
     DevBuf &out = ws.jbuf[0];
-    // room for 96 targets a source at first; a launch that needs more is repeated with the room it asked for
-    ctx.reserve(out, std::max<u64>(96 * ns, 1 << 16) * 8);
+    // room for 96 targets a source at first, up to a GiB (nothing is known of the result
+    // yet); a launch that needs more is repeated with the room it asked for
+    ctx.reserve(out, std::min<u64>(std::max<u64>(96 * ns, 1 << 16), 1ull << 27) * 8);
     SearchCounters got{};
     // One stage: `launch(where to)` with zeroed counters; repeated when its words outgrow the room.
     // Its level counts are added to cnt / deg when it went through.
@@ -1623,6 +1624,12 @@ bool tc_closure(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, 
         r.fulls.clear();
         r.from_bitmat = r.cl_rows = false;
         for (DevBuf *b : {&r.words, &r.bm_t, &r.bm_first, &r.cl_cols, &r.cl_loff, &r.cl_start}) ctx.give_back(*b);
+        // the searches' buffers too: the form that runs instead may need their memory
+        Workspace &ws = ctx.ws;
+        for (DevBuf *b : {&ws.jbuf[0], &ws.jbuf[1], &ws.cl_rec, &ws.cl_left, &ws.cl_heavy, &ws.cl_seg, &ws.cl_seg_at,
+                          &ws.cl_levels, &ws.cl_roff, &ws.cl_rval, &ws.cl_segs, &ws.cl_hub_at, &ws.cl_hub_acc,
+                          &ws.cl_rows[0], &ws.cl_rows[1], &ws.cl_act})
+            ctx.give_back(*b);
         r.n_words = nfull = 0;
         ctx.run_join_total = ctx.run_join_max = 0;
     }

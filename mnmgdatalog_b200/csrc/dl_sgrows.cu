@@ -463,7 +463,9 @@ bool sg_rows(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, con
         r.joins.clear();
         r.fulls.clear();
         r.from_bitmat = r.cl_rows = r.bm_row_first = false;
-        for (DevBuf *b : {&r.bm_t, &r.bm_first, &r.cl_cols, &r.cl_loff, &r.cl_start}) ctx.give_back(*b);
+        Workspace &ws = ctx.ws;
+        for (DevBuf *b : {&r.bm_t, &r.bm_first, &r.cl_cols, &r.cl_loff, &r.cl_start, &ws.cl_rows[0], &ws.cl_rows[1]})
+            ctx.give_back(*b);
         nfull = 0;
     }
     return done;

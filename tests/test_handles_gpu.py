@@ -93,3 +93,42 @@ def test_bit_rows_take_at_most_half_of_the_free_memory():
         torch.cuda.empty_cache()
         assert before < 1300 * 2**20 and after >= before // 2
         assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+
+
+def _held(eng, prog, e, **kw):
+    """Device bytes that a run took from a fresh context, and those that its result keeps
+    when the context's workspace and cache are freed."""
+    import torch
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    seen = []
+
+    def at_output(rows):
+        seen.append(before - torch.cuda.mem_get_info()[0])
+        eng.release_memory()
+        seen.append(before - torch.cuda.mem_get_info()[0])
+        return torch.empty((rows, 2), dtype=torch.int32, device="cuda")
+
+    got = eng.run(prog, e, output="device", out=at_output, **kw)
+    return got, seen
+
+
+def test_searches_take_room_by_the_result_not_by_the_nodes():
+    """8M edges to 8M sinks: 64 MB of rows (12 GB were reserved before anything was found)."""
+    import torch
+    k = torch.arange(8_000_000, dtype=torch.int32, device="cuda")
+    e = torch.stack([k, k + 8_000_000], 1).contiguous()
+    with Engine(0) as eng:
+        got, (taken, _) = _held(eng, "tc", e)
+        assert got.output_tuples == len(e) and taken < 4 * 2**30
+        assert torch.equal(got.rows, e)
+
+
+def test_tc_without_room_for_bit_rows():
+    """Heavy sources whose rows pass bitmap_max_gib (2.1 GB at 1 GiB): the bit matrix (0.3 GB) runs."""
+    e = np.random.default_rng(2).integers(0, 76_000, (220_000, 2)).astype(np.int32)
+    with Engine(0) as eng:
+        want = eng.tc(e, output="none", max_iterations=9)
+        eng.set_tuning(bitmap_max_gib=1)
+        got = eng.tc(e, output="none", max_iterations=9)
+        assert got.deltas.tolist() == want.deltas.tolist() and got.output_tuples == want.output_tuples
