@@ -1559,10 +1559,8 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
     if (light.n_words) {
         lw = closure_order(ctx, n, light.n_words, g.bits, g.bits);
     }
-    DevBuf &lbuf = holder(ws, lw);
-    r.words = lbuf;
-    lbuf = DevBuf();
-    r.n_words = nfull = light.n_words;
+    adopt_words(ctx, r, lw, light.n_words);
+    nfull = light.n_words;
     if (light.n_heavy) {
         ctx.reserve(ws.cl_left, light.n_heavy * 8);
         const u64 *src = radix_sort(ctx, ws.cl_heavy.as<u64>(), ws.cl_left.as<u64>(), light.n_heavy, Codec::Raw, g.bits);

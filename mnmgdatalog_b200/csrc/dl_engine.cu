@@ -415,6 +415,21 @@ void adopt_ids(Context &ctx, Run &r, const Graph &g) {
     r.id_base = g.id_base;
 }
 
+// Moves the n result words at w (one of the join buffers) into the run. A search sizes
+// the buffers before it knows the result, so one far larger than the words stays in the
+// workspace and the words are copied (the limit is the one reserve() has for cached buffers).
+void adopt_words(Context &ctx, Run &r, const u64 *w, u64 n) {
+    r.n_words = n;
+    if (n == 0) return;
+    DevBuf &hold = holder(ctx.ws, w);
+    if (hold.cap <= std::max<u64>(4 * n * 8, n * 8 + (64ull << 20))) {
+        std::swap(r.words, hold);
+    } else {
+        ctx.reserve_tight(r.words, n * 8);
+        DL_CUDA(cudaMemcpyAsync(r.words.p, w, n * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+    }
+}
+
 // The full relation of TC/SG as disjoint sorted duplicate-free runs: a large
 // one (ws.full[cur]), a small one (ws.small[scur]) and, for plain runs, a
 // tiny one (ws.tiny[tcur]). The reference keeps one sorted array and
@@ -742,10 +757,8 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_opt
             ctx.reserve(ws.jbuf[1], n * 8);
             w = radix_sort(ctx, w, ws.jbuf[1].as<u64>(), n, Codec::Raw, 2 * g.bits);
         }
-        DevBuf &hold = holder(ws, w);
-        r.words = hold;
-        hold = DevBuf();
-        r.n_words = nfull = n;
+        adopt_words(ctx, r, w, n);
+        nfull = n;
         pt.mark(PH_MERGE);
         // iteration k finds level k; one that finds nothing ends the program, the
         // first one also after an empty base (sg.cu:244-390)

@@ -98,6 +98,7 @@ int bits_for(u64 n);
 const int32_t *stage_input(Context &ctx, const int32_t *rows, u64 n, bool on_device);
 u64 *sort_unique_into(Context &ctx, DevBuf &buf, DevBuf &alt, u64 n, int key_bits, u64 &n_out);
 DevBuf &holder(Workspace &ws, const u64 *p);
+void adopt_words(Context &ctx, Run &r, const u64 *w, u64 n);
 DevBuf &other(Workspace &ws, const u64 *p);
 u64 *join_and_sort(Context &ctx, const Graph &g, const u64 *probe, u64 n_probe, EmitKind kind, u64 &n_j,
                    u64 *self_pairs, PhaseTimer &pt);

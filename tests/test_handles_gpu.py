@@ -119,9 +119,21 @@ def test_searches_take_room_by_the_result_not_by_the_nodes():
     k = torch.arange(8_000_000, dtype=torch.int32, device="cuda")
     e = torch.stack([k, k + 8_000_000], 1).contiguous()
     with Engine(0) as eng:
-        got, (taken, _) = _held(eng, "tc", e)
-        assert got.output_tuples == len(e) and taken < 4 * 2**30
+        got, (taken, kept) = _held(eng, "tc", e)
+        assert got.output_tuples == len(e) and taken < 4 * 2**30 and kept < 2**29
         assert torch.equal(got.rows, e)
+
+
+@pytest.mark.parametrize("prog,edges", [("tc", 300_000), ("tc", 3_000_000), ("sg", 60_000), ("sg", 1_000_000)])
+def test_results_do_not_hold_the_searchs_room(prog, edges):
+    """A few words a node: the run keeps at most 64 MiB beside four times its words and its ids."""
+    k = np.arange(edges, dtype=np.int32)
+    e = np.stack([k // 2 if prog == "sg" else k, k + edges], 1)
+    with Engine(0) as eng:
+        got, (_, kept) = _held(eng, prog, e)
+        assert kept < 4 * 8 * got.output_tuples + 2 * 4 * 2 * edges + (72 << 20)
+        want = eng.run(prog, e, dedup="sort")
+        assert np.array_equal(got.rows.cpu().numpy(), want.rows) and got.deltas.tolist() == want.deltas.tolist()
 
 
 def test_tc_without_room_for_bit_rows():
