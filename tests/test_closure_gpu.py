@@ -137,3 +137,19 @@ def test_tc_wide_rows_in_a_batch_and_a_session(engine):
         s.run()
         for i, k in ids:
             _check_wide(s.result(i), want[k], k)
+
+
+@pytest.mark.parametrize("algorithm", [0, 1])
+def test_tc_result_order_under_both_sorts(algorithm):
+    """The searched words are lined up by source and sorted by target only; as a plain run and
+    in a batch, whose ranks start above those of earlier instances."""
+    from mnmgdatalog_b200 import Engine
+    sets = [np.ascontiguousarray(CASES[k][0]).astype(np.int32) for k in ("dag", "random_sparse_ids", "chung_lu")]
+    with Engine(0) as eng:
+        eng.set_tuning(sort_algorithm=algorithm)
+        want = [eng.tc(e, dedup="sort") for e in sets]
+        res = eng.run_batch("tc", sets)
+        for w, b, e in zip(want, res, sets):
+            got = eng.tc(e)
+            assert np.array_equal(got.rows, w.rows) and np.array_equal(b.rows, w.rows)
+            assert got.deltas.tolist() == w.deltas.tolist() == b.deltas.tolist()
