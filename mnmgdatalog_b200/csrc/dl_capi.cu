@@ -358,13 +358,8 @@ dl_status join_common(dl_context *ctx, int64_t n, dl_entity **out, int64_t *n_ou
             const bool pooled = total * 8 <= dl::ReturnBox::kLargest / 2;
             dl::DevBuf o;
             try {
-                if (pooled) {
-                    ctx->c.reserve_tight(o, total * 8);
-                } else if (cudaMalloc(&o.p, total * 8) != cudaSuccess) {
-                    (void) cudaGetLastError();
-                    o.p = nullptr;
-                    throw dl::Error(DL_ERR_OUT_OF_MEMORY, "join output of " + std::to_string(total) + " rows");
-                }
+                if (pooled) ctx->c.reserve_tight(o, total * 8);
+                else o.p = ctx->c.allocate_for_caller(total * 8);
                 emit(offs.as<u64>(), total, o.as<u64>());
                 ctx->c.sync();
             } catch (...) {

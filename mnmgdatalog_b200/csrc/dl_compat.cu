@@ -93,8 +93,7 @@ DL_API dl_entity *dl_compat_get_hash_table(int, int, dl_entity *relation, int re
         dl::Context &ctx = compat_context();
         dl::HashTable *ht = dl::hash_table_build(ctx, (const u64 *) relation, (u64) relation_size, 0.5);
         const u64 bytes = kHeaderBytes + ht->slots * sizeof(dl::HashSlot) + ht->rows * sizeof(uint32_t);
-        void *p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) die((int) DL_ERR_OUT_OF_MEMORY, "cudaMalloc of the hash table failed");
+        void *p = ctx.allocate_for_caller(bytes);
         CompatHeader h{kCompatMagic, ht->slots, ht->distinct, ht->rows};
         char *c = (char *) p;
         DL_CUDA(cudaMemcpy(c, &h, sizeof(h), cudaMemcpyHostToDevice));
@@ -139,8 +138,7 @@ DL_API dl_entity *dl_compat_get_join(int, int, dl_entity *hash_table, int hash_t
         const u64 total = dl::hash_join_count(ctx, view, (const u64 *) relation, (u64) relation_size, offs.as<u64>());
         to_int_result(ctx, total, join_result_size);
         if (total) {
-            void *p = nullptr;
-            if (cudaMalloc(&p, total * 8) != cudaSuccess) die((int) DL_ERR_OUT_OF_MEMORY, "cudaMalloc of the join result failed");
+            void *p = ctx.allocate_for_caller(total * 8);
             dl::hash_join_emit(ctx, view, (const u64 *) relation, (u64) relation_size, offs.as<u64>(), total, (u64 *) p);
             ctx.sync();
             result = (dl_entity *) p;
@@ -171,8 +169,7 @@ DL_API dl_entity *dl_compat_get_join_nl(int, int, dl_entity *sorted_relation, in
                                                 (const u64 *) relation, (u64) relation_size, offs.as<u64>());
         to_int_result(ctx, total, join_result_size);
         if (total) {
-            void *p = nullptr;
-            if (cudaMalloc(&p, total * 8) != cudaSuccess) die((int) DL_ERR_OUT_OF_MEMORY, "cudaMalloc of the join result failed");
+            void *p = ctx.allocate_for_caller(total * 8);
             dl::sorted_join_emit(ctx, (const u64 *) sorted_relation, (u64) sorted_relation_size, (const u64 *) relation,
                                  (u64) relation_size, offs.as<u64>(), total, (u64 *) p);
             ctx.sync();

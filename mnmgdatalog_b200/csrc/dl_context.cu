@@ -160,8 +160,7 @@ void Context::allocate(DevBuf &buf, size_t bytes, bool zero, size_t minimum) {
         buf.reserve(bytes, zero);
     } catch (const Error &) {
         // Out of memory: drop every cached buffer and retry once.
-        for (auto &s : spares) s.release();
-        spares.clear();
+        drop_cache();
         buf.reserve(minimum ? minimum : bytes, zero);
     }
     KernelStat &k = kstat[K_HOST_MALLOC];
@@ -169,6 +168,22 @@ void Context::allocate(DevBuf &buf, size_t bytes, bool zero, size_t minimum) {
     k.timed++;
     k.seconds += now_s() - t0;
     k.bytes += (double) buf.cap;
+}
+
+void Context::drop_cache() {
+    take_returned();
+    for (auto &s : spares) s.release();
+    spares.clear();
+}
+
+void *Context::allocate_for_caller(size_t bytes) {
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    (void) cudaGetLastError();
+    drop_cache();
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    (void) cudaGetLastError();
+    throw Error(DL_ERR_OUT_OF_MEMORY, "cudaMalloc of " + std::to_string(bytes) + " bytes failed");
 }
 
 void Context::trim_spares() {
@@ -213,13 +228,7 @@ void Context::release_all() {
         cudaStreamDestroy(copy_stream);
         copy_stream = nullptr;
     }
-    for (auto &s : spares) s.release();
-    spares.clear();
-    {
-        std::lock_guard<std::mutex> lock(box->m);
-        for (DevBuf &b : box->bufs) b.release();
-        box->bufs.clear();
-    }
+    drop_cache();
     for (SessionKit &k : kits) k.release();
     kits.clear();
     if (host_stage) cudaFreeHost(host_stage);

@@ -231,6 +231,11 @@ struct Context {
     void give_back(DevBuf &buf);
     // Buffers handed back on any thread join the cache.
     void take_returned();
+    // Frees the cache.
+    void drop_cache();
+    // Memory of the exact size that the caller frees (cudaFree); the cache goes first if
+    // there is not enough.
+    void *allocate_for_caller(size_t bytes);
     // Index of the cached buffer reserve() takes for `bytes`, or -1.
     static int best_spare(const std::vector<DevBuf> &from, size_t bytes);
     // Whether buffers of these sizes may be reserved by a form that another one can stand

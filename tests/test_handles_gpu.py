@@ -144,3 +144,32 @@ def test_tc_without_room_for_bit_rows():
         eng.set_tuning(bitmap_max_gib=1)
         got = eng.tc(e, output="none", max_iterations=9)
         assert got.deltas.tolist() == want.deltas.tolist() and got.output_tuples == want.output_tuples
+
+
+def _permutation(n):
+    import torch
+    return torch.stack([torch.randperm(n, device="cuda", dtype=torch.int32)] * 2, 1).contiguous()
+
+
+def test_large_join_output_while_the_cache_holds_the_memory():
+    """1.7 GB of closed hash tables are cached, 0.7 GB are free: an output of 1.2 GB takes the cache's."""
+    import torch
+    with Engine(0) as eng:
+        rel = _permutation(4_000_000)
+        tables = [eng.get_hash_table(rel) for _ in range(12)]
+        one = torch.zeros((12_000, 2), dtype=torch.int32, device="cuda")
+        ht = eng.get_hash_table(one)  # 12,000 rows of one key
+        probe = one[:12_500]
+        del rel
+        torch.cuda.empty_cache()
+        for t in tables:
+            t.close()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - 700 * 2**20, dtype=torch.uint8, device="cuda")
+        out, n = C.c_void_p(), C.c_int64()
+        from mnmgdatalog_b200.capi import check, lib
+        check(lib().dl_join(eng.ctx, ht.handle, C.c_void_p(probe.data_ptr()), len(probe), C.byref(out), C.byref(n)))
+        assert n.value == 12_000 * len(probe)
+        check(lib().dl_free(eng.ctx, out))
+        ht.close()
+        del fill
+        torch.cuda.empty_cache()
