@@ -719,9 +719,8 @@ DL_API dl_status dl_context_set_tuning(dl_context *ctx, const dl_tuning *t) {
     o.hash_load = t->hash_load_factor;
     o.bitmap_max_gib = t->bitmap_max_gib;
     o.bitmap_unit_rows = (uint32_t) t->bitmap_unit_rows;
-    o.cache_max_gib = t->cache_max_gib;
     o.bitmap_result = t->bitmap_result;
-    ctx->c.trim_spares();
+    ctx->c.set_cache_limit(t->cache_max_gib);
     return DL_OK;
 }
 

@@ -41,6 +41,7 @@ dl::Context &compat_context() {
     if (!g_ctx[dev]) {
         auto *c = new dl::Context();
         c->device = dev;
+        c->set_cache_limit(1);  // the caller manages the device's memory and has no way to ask for it back
         c->stream = cudaStreamLegacy;  // the reference's blocking default stream
         cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, dev);
         void *p = nullptr;

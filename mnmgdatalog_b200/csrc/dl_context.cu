@@ -42,7 +42,9 @@ void ReturnBox::hand_back(DevBuf &b) {
     cudaDeviceSynchronize();
     {
         std::lock_guard<std::mutex> lock(m);
-        if (open && b.cap <= kLargest) {
+        size_t held = b.cap;
+        for (const DevBuf &x : bufs) held += x.cap;
+        if (open && b.cap <= kLargest && held <= limit) {
             bufs.push_back(b);
             b = DevBuf();
             return;
@@ -75,9 +77,23 @@ void *Context::host_staging(size_t bytes) {
 }
 
 void Context::take_returned() {
-    std::lock_guard<std::mutex> lock(box->m);
-    for (DevBuf &b : box->bufs) spares.push_back(b);
-    box->bufs.clear();
+    {
+        std::lock_guard<std::mutex> lock(box->m);
+        if (box->bufs.empty()) return;
+        for (DevBuf &b : box->bufs) spares.push_back(b);
+        box->bufs.clear();
+    }
+    trim_spares();
+}
+
+void Context::set_cache_limit(int gib) {
+    tune.cache_max_gib = gib;
+    {
+        std::lock_guard<std::mutex> lock(box->m);
+        box->limit = (size_t) gib << 30;
+    }
+    take_returned();
+    trim_spares();
 }
 
 void Context::reserve_tight(DevBuf &buf, size_t bytes) {

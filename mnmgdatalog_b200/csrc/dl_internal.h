@@ -158,6 +158,7 @@ struct ReturnBox {
     static constexpr size_t kLargest = size_t(256) << 20;  // larger ones are freed: the memory is the caller's again
     std::mutex m;
     bool open = true;             // the context is alive
+    size_t limit = 0;             // of the context's cache, in bytes
     std::vector<DevBuf> bufs;     // given back, not yet in the cache
     std::unordered_map<void *, size_t> outs;  // join outputs in callers' hands
     void hand_back(DevBuf &b);    // frees b or keeps it for the context
@@ -197,6 +198,8 @@ struct Context {
     u64 run_join_total = 0, run_join_max = 0;  // join statistics of the current run
     std::vector<DevBuf> spares;     // buffers handed back by destroyed runs and sessions
     std::shared_ptr<ReturnBox> box = std::make_shared<ReturnBox>();
+    Context() { set_cache_limit(tune.cache_max_gib); }
+    void set_cache_limit(int gib);
     std::vector<SessionKit> kits;   // of destroyed sessions
     static constexpr size_t kKits = 4;
     u64 *host_stage = nullptr;      // a session's page-locked staging of result labels

@@ -173,3 +173,22 @@ def test_large_join_output_while_the_cache_holds_the_memory():
         ht.close()
         del fill
         torch.cuda.empty_cache()
+
+
+def test_a_cache_of_zero_keeps_no_handles_buffers():
+    import torch
+    rel = _permutation(1_000_000)
+    with Engine(0) as eng:
+        eng.get_hash_table(rel).close()  # the workspace
+        eng.set_tuning(cache_max_gib=0)
+        free = torch.cuda.mem_get_info()[0]
+        tables = [eng.get_hash_table(rel) for _ in range(4)]
+        for t in tables:
+            t.close()
+        assert torch.cuda.mem_get_info()[0] >= free
+        eng.set_tuning(cache_max_gib=96)
+        for t in [eng.get_hash_table(rel) for _ in range(4)]:
+            t.close()
+        assert torch.cuda.mem_get_info()[0] < free
+        eng.set_tuning(cache_max_gib=0)  # what is cached goes too
+        assert torch.cuda.mem_get_info()[0] >= free
