@@ -191,6 +191,7 @@ DL_API dl_status dl_free(dl_context *ctx, void *p) {
         set_device(ctx);
         DL_CUDA(cudaStreamSynchronize(ctx->c.stream));
         dl::DevBuf b;
+        if (ctx->c.in_cache(p)) throw dl::Error(DL_ERR_INVALID_ARGUMENT, "dl_free: the memory was freed before");
         {
             std::lock_guard<std::mutex> lock(ctx->c.box->m);
             auto it = ctx->c.box->outs.find(p);
@@ -367,9 +368,10 @@ dl_status join_common(dl_context *ctx, int64_t n, dl_entity **out, int64_t *n_ou
                 ctx->c.give_back(offs);
                 throw;
             }
-            if (pooled) {
+            {  // (an entry of the same address is of memory that was freed in another way)
                 std::lock_guard<std::mutex> lock(ctx->c.box->m);
-                ctx->c.box->outs[o.p] = o.cap;
+                if (pooled) ctx->c.box->outs[o.p] = o.cap;
+                else ctx->c.box->outs.erase(o.p);
             }
             void *p = o.p;
             *out = (dl_entity *) p;

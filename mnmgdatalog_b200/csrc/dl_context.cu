@@ -192,6 +192,12 @@ void Context::drop_cache() {
     spares.clear();
 }
 
+bool Context::in_cache(const void *p) {
+    auto is = [p](const DevBuf &b) { return b.p == p; };
+    std::lock_guard<std::mutex> lock(box->m);
+    return std::any_of(spares.begin(), spares.end(), is) || std::any_of(box->bufs.begin(), box->bufs.end(), is);
+}
+
 void *Context::allocate_for_caller(size_t bytes) {
     void *p = nullptr;
     if (cudaMalloc(&p, bytes) == cudaSuccess) return p;

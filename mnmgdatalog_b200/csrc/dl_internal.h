@@ -236,6 +236,8 @@ struct Context {
     void take_returned();
     // Frees the cache.
     void drop_cache();
+    // Whether p is a cached buffer's.
+    bool in_cache(const void *p);
     // Memory of the exact size that the caller frees (cudaFree); the cache goes first if
     // there is not enough.
     void *allocate_for_caller(size_t bytes);

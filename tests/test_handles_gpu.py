@@ -192,3 +192,20 @@ def test_a_cache_of_zero_keeps_no_handles_buffers():
         assert torch.cuda.mem_get_info()[0] < free
         eng.set_tuning(cache_max_gib=0)  # what is cached goes too
         assert torch.cuda.mem_get_info()[0] >= free
+
+
+def test_join_output_freed_twice_is_refused():
+    """A freed output is the cache's: freeing it again must not take it from there."""
+    from mnmgdatalog_b200.capi import check, lib
+    from oracle import ops
+    with Engine(0) as eng:
+        rel, probe = _pairs(200, 3000, 5), _pairs(200, 800, 6)
+        ht = eng.get_hash_table(rel)
+        out, n = C.c_void_p(), C.c_int64()
+        check(lib().dl_join(eng.ctx, ht.handle, C.c_void_p(probe.data_ptr()), len(probe), C.byref(out), C.byref(n)))
+        assert lib().dl_free(eng.ctx, out) == 0
+        assert lib().dl_free(eng.ctx, out) != 0
+        got = np.sort(eng.get_join(ht, probe).cpu().numpy().view(np.int64).ravel())  # reuses the buffer
+        want = np.ascontiguousarray(ops.join(rel.cpu().numpy(), probe.cpu().numpy()), dtype=np.int32)
+        assert np.array_equal(got, np.sort(want.view(np.int64).ravel()))
+        ht.close()
