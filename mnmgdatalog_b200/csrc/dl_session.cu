@@ -1269,7 +1269,8 @@ u64 session_device_bytes(const SessionImpl &s) {
                             &w.sample,  &w.sample_small, &w.jbuf[0],
                             &w.jbuf[1], &w.offsets,   &c.lookback, &c.radix_part, &c.lbs_splits, &c.sort_hist,
                             &c.merge_splits, &w.cl_left, &w.cl_heavy, &w.cl_seg, &w.cl_seg_at, &w.cl_levels, &w.cl_roff, &w.cl_rval, &w.cl_segs,
-                            &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec};
+                            &w.cl_hub_at, &w.cl_hub_acc, &w.cl_rows[0], &w.cl_rows[1], &w.cl_act, &w.cl_rec,
+                            &w.wcc_label, &w.wcc_flag, &w.wcc_next};
     for (const DevBuf *x : bufs) b += x->cap;  // cached spare buffers are not counted: they are free memory
     std::vector<const DevBuf *> blocks;
     for (const auto &in : s.inst)

@@ -228,3 +228,12 @@ def test_label_copies_of_two_sessions_on_two_threads(engine):
     finally:
         for s in sessions:
             s.close()
+
+
+def test_memory_of_a_wcc_session_counts_its_labels():
+    """60 bytes a node and edge of a path for input, ranks, edges and results, 20 for labels, tags and lists."""
+    from mnmgdatalog_b200 import Engine
+    n = 500_000
+    with Engine(0) as eng, eng.session("wcc") as s:
+        s.admit(np.stack([np.arange(n), np.arange(n) // 2 + n // 2], 1).astype(np.int32))
+        assert s.memory()[0] >= 80 * n
