@@ -656,25 +656,6 @@ closure_cta_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, con
 
 // ---- heavy sources: 32 to a word ----------------------------------------
 
-// A target with more in-edges than lanes ("hub") is gathered in segments of 32
-// in-edges by as many warps: one warp alone would walk them long after the
-// others are done (at 256 in-edges a warp, 46 % of a level's time was that tail).
-constexpr u32 PU_SEG = 32;
-
-// Hubs: hub_at[w] = accumulator row of hub w, seg[...] = (w, first in-edge of a
-// segment); found[0] = hubs, found[1] = segments.
-__global__ void pull_hubs_kernel(const u32 *__restrict__ roff, u64 n, u32 *__restrict__ hub_at,
-                                 uint2 *__restrict__ seg, unsigned long long *__restrict__ found) {
-    for (u64 w = (u64) blockIdx.x * blockDim.x + threadIdx.x; w < n; w += (u64) gridDim.x * blockDim.x) {
-        const u32 b = roff[w], d = roff[w + 1] - b;
-        if (d <= PU_SEG) continue;
-        hub_at[w] = (u32) atomicAdd(found, 1ull);
-        const u32 k = (d + PU_SEG - 1) / PU_SEG;
-        const unsigned long long at = atomicAdd(found + 1, (unsigned long long) k);
-        for (u32 i = 0; i < k; ++i) seg[at + i] = make_uint2((u32) w, b + i * PU_SEG);
-    }
-}
-
 __global__ void add_counts_kernel(u64 *__restrict__ a, const unsigned long long *__restrict__ b, u64 n) {
     for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x) a[i] += b[i];
 }
@@ -698,91 +679,6 @@ __global__ void pull_init_kernel(PullShape sh, PullLevel st, const u64 *__restri
         if (lane == 0) {
             cols[i] = (u32) x;
             st.tag_next[x] = make_uint2(1u << gr, 0u);
-        }
-    }
-}
-
-// A warp works on K * 128 words of a row at a time: lane l holds words
-// base + 128 k + 4 l .. + 3 (k < K), 16 bytes each, eight lanes to a chunk.
-// Activity bit of the lane's k-th piece.
-template <int K>
-__device__ __forceinline__ u32 piece_bit(const PullShape &sh, u32 base, int k, u32 lane) {
-    return 1u << (((base >> 5) + 4 * k + (lane >> 3)) >> sh.shift);
-}
-
-// ORs the newest words of a group of up to 32 in-neighbours (node y, activity
-// a in the neighbour's lane) into acc: two neighbours' pieces in flight. The
-// pieces whose bit of `need` is clear are not loaded.
-template <int K>
-__device__ __forceinline__ void or_neighbours(const PullShape &sh, const u32 *__restrict__ cur, u32 base, u32 y, u32 a,
-                                              u32 need, u32 lane, uint4 (&acc)[K]) {
-    u32 all = __ballot_sync(0xffffffffu, a != 0);
-    const u32 *mine = cur + base + lane * 4;
-    u32 bit[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) bit[k] = (need >> k) & 1u ? piece_bit<K>(sh, base, k, lane) : 0u;
-    while (all) {
-        uint4 v[2][K];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const u32 j = (__ffs(all) - 1) & 31;
-            u32 aj = __shfl_sync(0xffffffffu, a, j);
-            if (all == 0) aj = 0;
-            all &= all - 1;
-            const uint4 *src = reinterpret_cast<const uint4 *>(mine + (u64) __shfl_sync(0xffffffffu, y, j) * sh.words);
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                v[q][k] = make_uint4(0, 0, 0, 0);
-                if (aj & bit[k]) v[q][k] = __ldg(src + 32 * k);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            acc[k].x |= v[0][k].x | v[1][k].x;
-            acc[k].y |= v[0][k].y | v[1][k].y;
-            acc[k].z |= v[0][k].z | v[1][k].z;
-            acc[k].w |= v[0][k].w | v[1][k].w;
-        }
-    }
-}
-
-// Hub targets: a warp ORs the newest words of PU_SEG in-neighbours, K * 128
-// words of the row, into the hub's accumulator (zero before the level).
-template <int K>
-__global__ void __launch_bounds__(PU_THREADS)
-closure_pull_hub_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ roff, const u32 *__restrict__ rval,
-                        const uint2 *__restrict__ seg, u64 n_seg, const u32 *__restrict__ hub_at,
-                        u32 *__restrict__ hub_acc) {
-    if (st.count[st.level] == 0) return;  // the fixpoint was reached earlier
-    const u32 lane = threadIdx.x & 31;
-    const u64 warps = (u64) gridDim.x * (PU_THREADS / 32);
-    const u32 passes = (sh.words + K * 128 - 1) / (K * 128);
-    for (u64 it = ((u64) blockIdx.x * PU_THREADS + threadIdx.x) / 32; it < n_seg * passes; it += warps) {
-        const u32 base = (u32) (it % passes) * K * 128;
-        const uint2 sg = seg[it / passes];
-        if (st.todo[sg.x] == 0) continue;
-        const u32 i = sg.y + lane;
-        u32 y = 0, a = 0;
-        if (i < roff[sg.x + 1]) {
-            y = rval[i];
-            const uint2 tg = st.tag[y];
-            a = tg.y == st.level - 1 ? tg.x : 0u;
-        }
-        uint4 acc[K];
-        u32 need = 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            acc[k] = make_uint4(0, 0, 0, 0);
-            if (base + 128 * k + lane * 4 < sh.words) need |= 1u << k;
-        }
-        or_neighbours<K>(sh, st.cur, base, y, a, need, lane, acc);
-        u32 *dst = hub_acc + (u64) hub_at[sg.x] * sh.words + base + lane * 4;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (acc[k].x) atomicOr(dst + 128 * k, acc[k].x);
-            if (acc[k].y) atomicOr(dst + 128 * k + 1, acc[k].y);
-            if (acc[k].z) atomicOr(dst + 128 * k + 2, acc[k].z);
-            if (acc[k].w) atomicOr(dst + 128 * k + 3, acc[k].w);
         }
     }
 }

@@ -139,11 +139,16 @@ __device__ __noinline__ u32 sg_expand(SgWarp &mw, u32 qn, u32 *row, const u32 *_
 // copies 24 ms, 40 warps an SM at 48 registers 17.8 ms against 17.1 for 32 at 64, six
 // or eight chunks in flight 17.5 and 20 ms (spills), two in-neighbours at a time
 // 16.4; in this one, one prefix sum over four chunks 15.2 against 14.7 ms.
-template <int NW, int TEAMS>
+// HUBS: rows with more than PU_SEG in-neighbours have the OR of their words in hub_acc
+// already (closure_pull_hub_kernel), which is cleared here. (A warp alone with thousands
+// of in-neighbours held up every level: 20K nodes, 40K edges, a third of them into four
+// nodes: 56 ms, on the matrix 28; now SG_HUB_MS.)
+template <int NW, int TEAMS, bool HUBS>
 __global__ void __launch_bounds__(NW * TEAMS * 32, 1024 / (NW * TEAMS * 32))
 sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ val,
                const u32 *__restrict__ roff, const u32 *__restrict__ rval, const u32 *__restrict__ has,
-               u32 *__restrict__ m, int base_rule, unsigned long long *__restrict__ fetch) {
+               const u32 *__restrict__ hub_at, u32 *__restrict__ hub_acc, u32 *__restrict__ m, int base_rule,
+               unsigned long long *__restrict__ fetch) {
     extern __shared__ __align__(16) u32 smem[];
     static_assert(NW == 1 || TEAMS == 1, "a team is a warp or the CTA");
     const u64 n_list = st.count[st.level];
@@ -195,8 +200,11 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
                 a = tg.y == st.level - 1 ? tg.x : 0u;
             }
         };
-        u32 y0, a0;
-        parents(0, y0, a0);
+        const bool hub = HUBS && n > PU_SEG;
+        u32 *hrow = nullptr;
+        u32 y0 = 0, a0 = 0;
+        if (hub) hrow = hub_acc + (u64) hub_at[y] * sh.words + lane;
+        else parents(0, y0, a0);
         u32 mine = 0;  // chunks this lane's children fell into
         u32 qn = 0;    // queued new pairs
         auto drain = [&]() {
@@ -217,7 +225,15 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
                     w[q] = old[q] = 0;
                     if (c[q] != EMPTY) old[q] = mp[c[q] * 32];
                 }
-                for (u32 e0 = 0; e0 < n; e0 += 32) {
+                if (hub) {
+#pragma unroll
+                    for (u32 q = 0; q < 4; ++q) {
+                        if (c[q] == EMPTY) continue;
+                        w[q] = hrow[c[q] * 32];
+                        hrow[c[q] * 32] = 0;
+                    }
+                }
+                for (u32 e0 = 0; e0 < n && !hub; e0 += 32) {
                     u32 p = y0, a = a0;
                     if (e0) parents(e0, p, a);
                     // two in-neighbours at a time: eight lines in flight
@@ -308,18 +324,40 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
 
 constexpr u64 SG_LEVELS = 8;  // levels launched between two host waits
 
+// Targets with many in-neighbours (pull_hubs_kernel).
+struct SgHubs {
+    u64 n = 0, n_seg = 0;
+    const uint2 *seg = nullptr;
+    const u32 *at = nullptr;
+    u32 *acc = nullptr;
+};
+
+template <int K>
+void launch_hubs(Context &ctx, const PullShape &sh, const PullLevel &st, const u32 *roff, const u32 *rval,
+                 const SgHubs &hubs) {
+    const u64 passes = (sh.words + K * 128 - 1) / (K * 128);
+    DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+              closure_pull_hub_kernel<K><<<grid_for(hubs.n_seg * passes * 32, PU_THREADS, ctx, 8), PU_THREADS, 0,
+                                           ctx.stream>>>(sh, st, roff, rval, hubs.seg, hubs.n_seg, hubs.at, hubs.acc));
+}
+
 template <int NW, int TEAMS>
 void launch_level(Context &ctx, const PullShape &sh, const PullLevel &st, const Csr &csr, const u32 *roff,
-                  const u32 *rval, const u32 *has, u32 *m, bool base) {
+                  const u32 *rval, const u32 *has, const SgHubs &hubs, u32 *m, bool base) {
     const size_t smem = (size_t) TEAMS * sh.words * 4;
-    auto kern = sg_rows_kernel<NW, TEAMS>;
+    if (hubs.n) {
+        if (sh.words <= 128) launch_hubs<1>(ctx, sh, st, roff, rval, hubs);
+        else if (sh.words <= 256) launch_hubs<2>(ctx, sh, st, roff, rval, hubs);
+        else launch_hubs<3>(ctx, sh, st, roff, rval, hubs);
+    }
+    auto kern = hubs.n ? sg_rows_kernel<NW, TEAMS, true> : sg_rows_kernel<NW, TEAMS, false>;
     DL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     int per_sm = 0;
     DL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * TEAMS * 32, smem));
     const u64 grid = std::min<u64>((sh.n + TEAMS - 1) / TEAMS, (u64) ctx.sm_count * std::max(per_sm, 1));
     DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
               kern<<<(unsigned) grid, NW * TEAMS * 32, smem, ctx.stream>>>(
-                  sh, st, csr.off, csr.val, roff, rval, has, m, base ? 1 : 0, st.deg + SG_LEVELS + 1));
+                  sh, st, csr.off, csr.val, roff, rval, has, hubs.at, hubs.acc, m, base ? 1 : 0, st.deg + SG_LEVELS + 1));
 }
 
 bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
@@ -351,6 +389,14 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
               key_offsets_kernel<u32><<<grid_for(n + 1, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, g.bits, n, roff));
     DL_LAUNCH(ctx, K_PREP, 12.0 * ne,
               low_field_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(rev, ne, (1ull << g.bits) - 1, rval));
+    auto *found = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[44]);
+    ctx.reserve(ws.cl_segs, (ne / PU_SEG * 2 + 1) * 8);  // a hub's segments are at most twice its in-edges / 32
+    ctx.reserve(ws.cl_hub_at, n * 4);
+    DL_CUDA(cudaMemsetAsync(found, 0, 16, ctx.stream));
+    DL_LAUNCH(ctx, K_PREP, 4.0 * n,
+              pull_hubs_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(roff, n, ws.cl_hub_at.as<u32>(),
+                                                                               ws.cl_segs.as<uint2>(), found));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, found, 16, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.reserve(ws.bit_hasout, words * 4);
     u32 *has = ws.bit_hasout.as<u32>();
     DL_LAUNCH(ctx, K_PREP, 4.0 * n,
@@ -395,6 +441,13 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
               sg_identity_kernel<<<grid_for(words * 32 * 32, T256, ctx), T256, 0, ctx.stream>>>(
                   sh, view(0), g.csr.off, g.csr.val, r.cl_cols.as<u32>()));
     push(0);
+    ctx.sync();
+    SgHubs hubs{ctx.host_scalars[0], ctx.host_scalars[1], ws.cl_segs.as<uint2>(), ws.cl_hub_at.as<u32>(), nullptr};
+    if (hubs.n) {
+        ctx.reserve(ws.cl_hub_acc, hubs.n * words * 4);
+        hubs.acc = ws.cl_hub_acc.as<u32>();
+        DL_CUDA(cudaMemsetAsync(hubs.acc, 0, hubs.n * words * 4, ctx.stream));
+    }
     pt.mark(PH_JOIN);
     // level 1 is the base rule, level k + 1 iteration k; level k + 1's joins are
     // level k's joinable pairs
@@ -406,9 +459,10 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
                                                  : SG_LEVELS;
         for (u64 level = first; level < first + batch; ++level) {
             const bool base = level == 1;
-            if (words <= 1024) launch_level<1, 4>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
-            else if (words <= 4096) launch_level<4, 1>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
-            else launch_level<8, 1>(ctx, sh, view(level), g.csr, roff, rval, has, r.bm_t.as<u32>(), base);
+            u32 *m = r.bm_t.as<u32>();
+            if (words <= 1024) launch_level<1, 4>(ctx, sh, view(level), g.csr, roff, rval, has, hubs, m, base);
+            else if (words <= 4096) launch_level<4, 1>(ctx, sh, view(level), g.csr, roff, rval, has, hubs, m, base);
+            else launch_level<8, 1>(ctx, sh, view(level), g.csr, roff, rval, has, hubs, m, base);
             push(level);
         }
         DL_CUDA(cudaMemsetAsync(sets[set ^ 1], 0, SET * 8, ctx.stream));

@@ -41,3 +41,34 @@ def test_sg_rows_equal_matrix(engine, name, edges, stop):
     assert torch.equal(got.rows, want.rows)
     if want.output_tuples < 10**7:
         assert np.array_equal(engine.sg(e, max_iterations=stop).rows, want.rows.cpu().numpy())
+
+
+def _into_hubs(n, m, hubs, seed):
+    """A random graph, a third of whose edges go into `hubs` nodes."""
+    rng = np.random.default_rng(seed)
+    b = rng.integers(0, n, m)
+    b[: m // 3] = rng.integers(0, hubs, m // 3)
+    return np.stack([rng.integers(0, n, m), b], 1)
+
+
+def _in_degrees(*ds):
+    """Nodes of d in-neighbours each, below a root and a second generation that mixes them."""
+    out, o = [], 1
+    for d in ds:
+        hub = o + d
+        out += [np.stack([np.zeros(d, int), o + np.arange(d)], 1), np.stack([o + np.arange(d), np.full(d, hub)], 1),
+                [[hub, hub + 1], [hub, hub + 2], [hub + 1, 1], [hub + 2, 2]]]
+        o = hub + 3
+    return np.concatenate(out)
+
+
+HUBS = [("edges_of_segments", _in_degrees(31, 32, 33, 63, 64, 65, 96, 97, 1000), 0),
+        ("small", _into_hubs(900, 2500, 3, 1), 0), ("deep", _into_hubs(9000, 18_000, 4, 2), 0),
+        ("deep_stops", _into_hubs(9000, 18_000, 4, 2), 8), ("three_pieces", _into_hubs(20_000, 40_000, 4, 3), 0),
+        ("four_warps", _into_hubs(60_000, 130_000, 5, 4), 3), ("granules", _into_hubs(36_000, 80_000, 40, 5), 5)]
+
+
+@pytest.mark.parametrize("name,edges,stop", HUBS, ids=[c[0] for c in HUBS])
+def test_sg_rows_of_many_in_neighbours(engine, name, edges, stop):
+    """Accumulated rows of nodes past 32 in-neighbours."""
+    test_sg_rows_equal_matrix(engine, name, edges, stop)
