@@ -142,7 +142,7 @@ __device__ __noinline__ u32 sg_expand(SgWarp &mw, u32 qn, u32 *row, const u32 *_
 // HUBS: rows with more than PU_SEG in-neighbours have the OR of their words in hub_acc
 // already (closure_pull_hub_kernel), which is cleared here. (A warp alone with thousands
 // of in-neighbours held up every level: 20K nodes, 40K edges, a third of them into four
-// nodes: 56 ms, on the matrix 28; now SG_HUB_MS.)
+// nodes: 56 ms, on the matrix 28; now 5.2.)
 template <int NW, int TEAMS, bool HUBS>
 __global__ void __launch_bounds__(NW * TEAMS * 32, 1024 / (NW * TEAMS * 32))
 sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ val,
