@@ -153,3 +153,48 @@ def test_tc_result_order_under_both_sorts(algorithm):
             got = eng.tc(e)
             assert np.array_equal(got.rows, w.rows) and np.array_equal(b.rows, w.rows)
             assert got.deltas.tolist() == w.deltas.tolist() == b.deltas.tolist()
+
+
+def _tiny(seed, count=12_000):
+    """Components around what one lane searches alone (paths of up to three targets, rows of up to
+    four sinks): paths, stars, paths into stars and cycles, self loops, in shuffled id order."""
+    rng = np.random.default_rng(seed)
+    kinds = [_path(k) for k in (1, 2, 3, 4, 5)] + [_cycle(k) for k in (1, 2, 3, 4)]
+    kinds += [np.stack([np.zeros(k, int), 1 + np.arange(k)], 1) for k in (2, 3, 4, 5)]
+    kinds += [np.concatenate([_path(p), [[p, p + 1 + j] for j in range(k)]]) for p in (1, 2) for k in (2, 4)]
+    kinds += [np.array(x) for x in ([[0, 1], [1, 1]], [[0, 1], [1, 2], [2, 1]], [[0, 1], [1, 2], [2, 2]],
+                                    [[0, 1], [0, 2], [1, 2]], [[0, 0], [0, 1]], [[0, 1], [1, 2], [2, 0], [2, 3]],
+                                    [[0, 1], [0, 2], [2, 3]])]
+    out, top = [], 0
+    for k in rng.integers(0, len(kinds), count):
+        out.append(kinds[k] + top)
+        top += int(kinds[k].max()) + 1
+    ids = rng.permutation(top) if seed % 2 else np.arange(top)
+    return ids[np.concatenate(out)].astype(np.int32)
+
+
+@pytest.mark.parametrize("stop", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("seed", [0, 1])
+def test_tc_tiny_searches(engine, seed, stop):
+    e = _tiny(seed)
+    want, got = engine.tc(e, dedup="sort", max_iterations=stop), engine.tc(e, max_iterations=stop)
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    assert np.array_equal(got.rows, want.rows)
+
+
+def test_tc_tiny_searches_in_a_batch(engine):
+    """Instances that begin and end inside a warp's 32 sources."""
+    sets = [_tiny(k, c) for k, c in enumerate((5, 9000, 1, 1, 3, 2, 400, 1, 2000))] + [_path(1).astype(np.int32)] * 40
+    for e, got in zip(sets, engine.run_batch("tc", sets)):
+        want = engine.tc(e, dedup="sort")
+        assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+
+
+def test_tc_many_tiny_searches(engine):
+    """Millions of them beside searches of 400 targets."""
+    k = np.arange(1_500_000, dtype=np.int32)
+    hub = np.stack([np.repeat(np.arange(3_000_000, 3_000_200, dtype=np.int32), 200), np.arange(40_000, dtype=np.int32)], 1)
+    e = np.concatenate([np.stack([k, k // 3 + 1_500_000], 1), hub])
+    want, got = engine.tc(e, dedup="sort"), engine.tc(e)
+    assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
