@@ -105,8 +105,16 @@ __global__ void id_mark_kernel(const int32_t *__restrict__ v, u64 n, const unsig
     }
 }
 
+// Set bits of the presence words; those past the span are not scanned (none when the ids
+// are ranked by a sort: 2M words are 20 us).
 struct PopcValue {
     const u32 *w;
+    const unsigned long long *range;
+    u64 cap;
+    __device__ __forceinline__ u64 count() const {
+        const u64 span = (u64) ((u32) range[1] - ~(u32) range[0]) + 1;
+        return span > cap ? 0 : (span + 31) / 32;
+    }
     __device__ __forceinline__ u64 operator()(u64 i) const { return __popc(w[i]); }
 };
 
@@ -238,7 +246,7 @@ void rank_nodes(Context &ctx, const int32_t *rows, u64 n, Graph &g, Fits fits) {
     DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(u32), ctx.stream));
     DL_LAUNCH(ctx, K_PREP, 12.0 * cap_words,
               scan_kernel<PopcValue><<<(unsigned) tiles, SCAN_THREADS, 0, ctx.stream>>>(
-                  PopcValue{present}, cap_words, pre, lb, ctr, ctx.next_epoch(), &ctx.ctrl->err,
+                  PopcValue{present, range, cap}, cap_words, pre, lb, ctr, ctx.next_epoch(), &ctx.ctrl->err,
                   &ctx.ctrl->scalar[22]));
     DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, range, 24, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
@@ -969,12 +977,7 @@ static void run_single_join_impl(Context &ctx, Run &r, const int32_t *rows_in, u
         if (self_join_rows(ctx, r, g.csr, total, pt, nout)) {
             ctx.run_join_total = ctx.run_join_max = total;
         } else {
-            ctx.reserve(ws.w0, n * 8);
-            DL_LAUNCH(ctx, K_PREP, 0, pack_rows_kernel<<<grid_for(n, T256, ctx), T256, 0, ctx.stream>>>(rows, n, g.ranker, g.bits,
-                                                                             ws.w0.as<u64>(), nullptr));
-            u64 ne;
-            u64 *e = sort_unique_into(ctx, ws.w0, ws.w1, n, 2 * g.bits, ne);  // single_join.cu:165-168
-            build_csr(ctx, e, ne, g);
+            build_csr(ctx, self_join_by_source(ctx, p, np, g.bits), np, g);  // single_join.cu:165-168
             u64 nj = 0;
             u64 *j = join_and_sort(ctx, g, p, np, EmitKind::ZV, nj, nullptr, pt);  // single_join.cu:223
             nout = nj ? unique_words(ctx, j, nj, j) : 0;                           // single_join.cu:259-264

@@ -79,6 +79,16 @@ select_kernel(const u64 *in, u64 n, u64 *out, Keep keep, u64 *lb, u32 *tile_ctr,
     if (base + nv == n && tid == 0) *count = excl + tot;
 }
 
+// The items of a scan: n, or fewer where the values know on the device (count()).
+template <class Value>
+__device__ __forceinline__ auto scan_count(const Value &v, u64, int) -> decltype(v.count()) {
+    return v.count();
+}
+template <class Value>
+__device__ __forceinline__ u64 scan_count(const Value &, u64 n, long) {
+    return n;
+}
+
 // Exclusive scan of value(i) for i < n (64-bit): out[i] = sum_{j<i} value(j).
 // The last tile stores the grand total to *total.
 template <class Value>
@@ -94,6 +104,8 @@ scan_kernel(Value value, u64 n, u64 *out, u64 *lb, u32 *tile_ctr, u32 epoch, u32
     __syncthreads();
     const u32 tile = s_tile;
     const u64 base = (u64) tile * SCAN_TILE;
+    n = scan_count(value, n, 0);
+    if (base >= n) return;
     const u32 nv = (u32) min((u64) SCAN_TILE, n - base);
 #pragma unroll
     for (int j = 0; j < SCAN_IPT; ++j) {
