@@ -973,6 +973,8 @@ __global__ void heavy_below_kernel(const u32 *__restrict__ cols, u64 h, u64 n, u
 // Light pairs are placed lane-parallel; a word that one falls inside is done
 // last, its lanes shifted by the light pairs below them.
 
+constexpr u32 MERGE_PAIRS = 32;  // light pairs of a chunk that closure_rows_kernel takes: a window
+
 template <bool DENSE, bool ROW_FIRST>
 __global__ void __launch_bounds__(256)
 closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict__ cols,
@@ -1022,7 +1024,7 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             fetch(z + step);
             const u32 lend = c0 + 1 < chunks ? start[z * chunks + c0 + 1].y : (u32) (loff[z + 1] - loff[z]);
             const u32 any = __ballot_sync(0xffffffffu, v != 0);
-            if (!any && st.y == lend) continue;
+            if ((!any && st.y == lend) || lend - st.y > MERGE_PAIRS) continue;  // (closure_merge_kernel's)
             const u32 zid = node((u32) z);
             // a row (x, z), or (z, x) when the targets come first, as one little-endian word
             auto pack = [&](u32 x) -> u64 { return ROW_FIRST ? ((u64) x << 32) | zid : ((u64) zid << 32) | x; };
@@ -1055,20 +1057,18 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 }
             };
             u32 rel = EMPTY;
-            for (u32 l0 = st.y; l0 < lend; l0 += 32) {
+            if (st.y < lend) {
                 u32 x;
-                pair(l0 + lane, x, rel);
-                const bool in = l0 + lane < lend;
+                pair(st.y + lane, x, rel);
+                const bool in = st.y + lane < lend;
                 const u32 j = rel >> 5, b = rel & 31;
                 // (rel 1024: after every column)
                 const u32 wj = __shfl_sync(0xffffffffu, v, j & 31), pj = __shfl_sync(0xffffffffu, incl - n, j & 31);
                 const u32 total = __shfl_sync(0xffffffffu, incl, 31);
-                if (in)
-                    dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + (l0 + lane - st.y)] = pack(node(x));
+                if (in) dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + lane] = pack(node(x));
                 const u32 key = in ? (b ? j : j - 1) : EMPTY - 1;  // words above `key` are shifted whole
-                for (u32 k = 0; k < min(32u, lend - l0); ++k)
-                    at += (int) lane > (int) __shfl_sync(0xffffffffu, key, k);
-                inside |= __reduce_or_sync(0xffffffffu, in && b ? 1u << j : 0u);
+                for (u32 k = 0; k < lend - st.y; ++k) at += (int) lane > (int) __shfl_sync(0xffffffffu, key, k);
+                inside = __reduce_or_sync(0xffffffffu, in && b && j < 32 ? 1u << j : 0u);
             }
             u32 slow = any & inside;
             const u32 v0 = v;
@@ -1088,14 +1088,110 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
                 slow &= slow - 1;
                 const u32 word = __shfl_sync(0xffffffffu, v0, j);
                 u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
-                for (u32 l0 = st.y; l0 < lend; l0 += 32) {
-                    u32 x, rl = rel;
-                    if (lend - st.y > 32) pair(l0 + lane, x, rl);  // several windows: read again
-                    for (u32 mm = __ballot_sync(0xffffffffu, (rl >> 5) == j && (rl & 31)); mm; mm &= mm - 1)
-                        p += (__shfl_sync(0xffffffffu, rl, __ffs(mm) - 1) & 31) <= lane;
-                }
+                for (u32 mm = __ballot_sync(0xffffffffu, (rel >> 5) == j && (rel & 31)); mm; mm &= mm - 1)
+                    p += (__shfl_sync(0xffffffffu, rel, __ffs(mm) - 1) & 31) <= lane;
                 if ((word >> lane) & 1u) dst[p] = pack(node(__ldg(cc + j * 32 + lane)));
             }
+        }
+    }
+}
+
+// The rows of (target, chunk)s with more light pairs than a window. Their places in the
+// chunk ascend, so a window of 32 pairs shifts the words by the number of its pairs below each
+// (six shuffles); the last pair of every place leaves its number there, and a
+// column's shift is the largest number up to it. (Going through all of a chunk's pairs again
+// for each of its words was quadratic: 21K nodes in 20 layers, 44M pairs, half of them
+// light, 4.8 ms of 7.2; 3.0 for the whole run here. Within the kernel above it cost every run a
+// third of its resident warps in registers.) A warp looks at `take`
+// (target, chunk)s at a time, up to 32, so that all warps have some.
+__global__ void __launch_bounds__(256)
+closure_merge_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict__ cols, const u32 *__restrict__ place,
+                     const uint2 *__restrict__ start, u64 z0, u64 z1, const u64 *__restrict__ first,
+                     const u64 *__restrict__ light, const u64 *__restrict__ loff, u64 mask,
+                     const int32_t *__restrict__ ids, bool affine, int32_t base, u32 take, u64 *__restrict__ out) {
+    __shared__ __align__(4) unsigned short staged[8][1024];
+    unsigned short *stage = staged[threadIdx.x >> 5];
+    const u32 lane = threadIdx.x & 31;
+    const u32 lt = lanemask_lt();
+    const u32 chunks = words / 32;
+    const u64 warps = (u64) gridDim.x * (blockDim.x / 32);
+    auto node = [&](u32 r) -> u32 { return (u32) (affine ? (int32_t) (base + (int64_t) r) : __ldg(ids + r)); };
+    for (u64 i0 = z0 * chunks + ((u64) blockIdx.x * blockDim.x + threadIdx.x) / 32 * take; i0 < z1 * chunks;
+         i0 += warps * take) {
+        u64 zl = 0;
+        u32 from = 0, to = 0, rows = 0;
+        if (lane < take && i0 + lane < z1 * chunks) {
+            zl = (i0 + lane) / chunks;
+            const uint2 st = start[i0 + lane];
+            rows = st.x;
+            from = st.y;
+            to = (i0 + lane + 1) % chunks ? start[i0 + lane + 1].y : (u32) (loff[zl + 1] - loff[zl]);
+        }
+        for (u32 todo = __ballot_sync(0xffffffffu, to - from > MERGE_PAIRS); todo; todo &= todo - 1) {
+            const u32 q = __ffs(todo) - 1;
+            const u64 z = __shfl_sync(0xffffffffu, zl, q);
+            const u32 k0 = (u32) ((i0 + q) % chunks) * 32;
+            const u32 lbeg = __shfl_sync(0xffffffffu, from, q), lend = __shfl_sync(0xffffffffu, to, q);
+            u64 *dst = out + first[z] + __shfl_sync(0xffffffffu, rows, q);
+            const u64 *lz = light + loff[z];
+            const u64 zid = (u64) node((u32) z) << 32;
+            const u32 v = t[z * words + k0 + lane];
+            const u32 incl = warp_inclusive_sum((u32) __popc(v));
+            const u32 before = incl - __popc(v), total = __shfl_sync(0xffffffffu, incl, 31);
+            auto place_of = [&](u32 x) { return min(__ldg(place + x) - k0 * 32, 1024u); };  // 1024: after every column
+            const bool counted = lend - lbeg <= 0xFFFFu;  // else a column's shift is searched for
+            if (counted)
+                for (u32 k = lane; k < 512; k += 32) reinterpret_cast<u32 *>(stage)[k] = 0;
+            __syncwarp();
+            u32 shift = 0;  // pairs at or before the first column of this lane's word
+            for (u32 l0 = lbeg; l0 < lend; l0 += 32) {
+                const u32 i = l0 + lane - lbeg;
+                const bool in = l0 + lane < lend;
+                u32 x = 0, rel = EMPTY;
+                if (in) {
+                    x = (u32) (__ldg(lz + l0 + lane) & mask);
+                    rel = place_of(x);
+                }
+                const u32 j = rel >> 5, b = rel & 31;
+                const u32 wj = __shfl_sync(0xffffffffu, v, j & 31), pj = __shfl_sync(0xffffffffu, before, j & 31);
+                if (in) dst[(j < 32 ? pj + __popc(wj & ((1u << b) - 1)) : total) + i] = zid | node(x);
+                u32 c = 0;
+#pragma unroll
+                for (u32 step = 16; step >= 1; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, rel, c + step - 1) <= 32 * lane) c += step;
+                if (__shfl_sync(0xffffffffu, rel, c) <= 32 * lane) ++c;
+                shift += c;
+                const u32 next = __shfl_down_sync(0xffffffffu, rel, 1);
+                if (counted && in && rel < 1024 && (lane == 31 || next != rel)) stage[rel] = (unsigned short) (i + 1);
+                __syncwarp();
+            }
+            for (u32 j = 0; j < 32; ++j) {
+                const u32 word = __shfl_sync(0xffffffffu, v, j);
+                if (!word) continue;
+                const u32 p = __shfl_sync(0xffffffffu, before, j) + __popc(word & lt);
+                u32 s = __shfl_sync(0xffffffffu, shift, j);
+                if (counted) {
+                    u32 m = stage[j * 32 + lane];
+                    if (__any_sync(0xffffffffu, m != 0)) {
+#pragma unroll
+                        for (u32 o = 1; o < 32; o <<= 1) {
+                            const u32 y = __shfl_up_sync(0xffffffffu, m, o);
+                            if (lane >= o) m = max(m, y);
+                        }
+                        s = max(s, m);
+                    }
+                } else {
+                    u32 a = lbeg, e = lend;
+                    while (a < e) {
+                        const u32 mid = (a + e) >> 1;
+                        if (place_of((u32) (__ldg(lz + mid) & mask)) <= j * 32 + lane) a = mid + 1;
+                        else e = mid;
+                    }
+                    s = a - lbeg;
+                }
+                if ((word >> lane) & 1u) dst[p + s] = zid | node(__ldg(cols + k0 * 32 + j * 32 + lane));
+            }
+            __syncwarp();  // the stage is free
         }
     }
 }
@@ -1637,6 +1733,15 @@ void closure_extract_rows(Context &ctx, const Run &r, int32_t *out, u64 z0, u64 
                   r.bm_t.as<u32>(), (u32) r.bm_words, cols, cols + r.bm_words * 32, r.cl_start.as<uint2>(), z0, z1,
                   r.bm_first.as<u64>(), r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << r.bits) - 1,
                   r.ids.as<int32_t>(), r.ids_affine, r.id_base, reinterpret_cast<u64 *>(out)));
+    if (r.n_words <= MERGE_PAIRS) return;
+    const u64 parts = (z1 - z0) * chunks;
+    const unsigned mg = grid_for(parts * 32, 256, ctx, 8);
+    const u32 take = (u32) std::max<u64>(1, std::min<u64>(32, parts / (mg * 8)));
+    DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 0,
+              closure_merge_kernel<<<mg, 256, 0, ctx.stream>>>(
+                  r.bm_t.as<u32>(), (u32) r.bm_words, cols, cols + r.bm_words * 32, r.cl_start.as<uint2>(), z0, z1,
+                  r.bm_first.as<u64>(), r.words.as<u64>(), r.cl_loff.as<u64>(), (1ull << r.bits) - 1,
+                  r.ids.as<int32_t>(), r.ids_affine, r.id_base, take, reinterpret_cast<u64 *>(out)));
 }
 
 }  // namespace dl

@@ -198,3 +198,37 @@ def test_tc_many_tiny_searches(engine):
     e = np.concatenate([np.stack([k, k // 3 + 1_500_000], 1), hub])
     want, got = engine.tc(e, dedup="sort"), engine.tc(e)
     assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+
+
+def _layers(width, layers, degree, seed=1):
+    """Each node of a layer has `degree` edges into the next one on average."""
+    rng = np.random.default_rng(seed)
+    return np.concatenate([np.stack([i * width + rng.integers(0, width, degree * width),
+                                     (i + 1) * width + rng.integers(0, width, degree * width)], 1)
+                           for i in range(layers)])
+
+
+def _light_and_heavy(light, heavy, seed):
+    """`light` sources above a hub of 20 targets, and `heavy` ones above it and 5000 leaves of their
+    own, with ids in any order: a target's row has all of them."""
+    hub, out = light + heavy, []
+    out.append(np.stack([np.arange(light + heavy), np.full(light + heavy, hub)], 1))
+    out.append(np.stack([np.full(20, hub), hub + 1 + np.arange(20)], 1))
+    leaf = hub + 21 + np.arange(heavy * 5000)
+    out.append(np.stack([light + np.repeat(np.arange(heavy), 5000), leaf], 1))
+    e = np.concatenate(out)
+    return np.random.default_rng(seed).permutation(int(e.max()) + 1)[e]
+
+
+MERGED = {"layers": _layers(1000, 20, 2), "layers_thin": _layers(3000, 10, 1), "layers_wide": _layers(6000, 5, 5),
+          "one_window": _light_and_heavy(31, 3, 1), "window_edge": _light_and_heavy(33, 5, 2),
+          "one_heavy": _light_and_heavy(3000, 1, 3), "chunks": _light_and_heavy(4000, 40, 4),
+          "past_16_bits": _light_and_heavy(70_000, 6, 5), "at_16_bits": _light_and_heavy(65_535, 2, 6)}
+
+
+@pytest.mark.parametrize("name", sorted(MERGED))
+def test_tc_rows_of_many_light_sources(engine, name):
+    e = np.ascontiguousarray(MERGED[name]).astype(np.int32)
+    want, got = engine.tc(e, dedup="sort"), engine.tc(e)
+    assert got.deltas.tolist() == want.deltas.tolist()
+    assert np.array_equal(got.rows, want.rows)
