@@ -135,7 +135,21 @@ bool Context::room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> 
     if (!fresh) return true;
     size_t free_b = 0, total_b = 0;
     DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    return fresh <= free_b / 2;
+    size_t cached = 0;
+    for (const DevBuf &b : left) cached += b.cap;
+    if (fresh > (free_b + cached) / 2) return false;
+    // the context's own cache makes the room, the largest buffers first
+    std::sort(left.begin(), left.end(), [](const DevBuf &a, const DevBuf &b) { return a.cap > b.cap; });
+    for (size_t i = 0; i < left.size() && fresh > free_b / 2; ++i) {
+        for (size_t k = 0; k < spares.size(); ++k)
+            if (spares[k].p == left[i].p) {
+                free_b += spares[k].cap;
+                spares[k].release();
+                spares.erase(spares.begin() + k);
+                break;
+            }
+    }
+    return true;
 }
 
 void Context::reserve(DevBuf &buf, size_t bytes, bool zero) {

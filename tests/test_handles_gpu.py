@@ -70,8 +70,8 @@ def test_results_in_one_call(engine, prog):
 
 
 def test_bit_rows_take_at_most_half_of_the_free_memory():
-    """SG's three bit-row matrices (0.8 GB) while 1.2 GB are free: cached buffers that
-    none of them fits into are no room for them, so another form runs."""
+    """SG's three bit-row matrices (0.8 GB) while 1.2 GB are free and 1.9 cached in buffers that
+    none of them fits into: those are freed first, or another form runs."""
     import torch
     rng = np.random.default_rng(3)
     e = np.concatenate([rng.integers(0, 46_000, (70_000, 2)), [[0, 45_999]]]).astype(np.int32)
@@ -209,3 +209,31 @@ def test_join_output_freed_twice_is_refused():
         want = np.ascontiguousarray(ops.join(rel.cpu().numpy(), probe.cpu().numpy()), dtype=np.int32)
         assert np.array_equal(got, np.sort(want.view(np.int64).ravel()))
         ht.close()
+
+
+def test_the_cache_makes_room_for_bit_rows():
+    """0.5 GB free, 4.3 GB cached in buffers too small for SG's matrices (0.8 GB): the run takes the
+    form that it takes when the memory is free."""
+    import torch
+    rng = np.random.default_rng(3)
+    e = np.concatenate([rng.integers(0, 46_000, (70_000, 2)), [[0, 45_999]]]).astype(np.int32)
+
+    def launches(eng):
+        eng.profile(False)
+        got = eng.sg(e, max_iterations=3)
+        return got, eng.profile_read()["bitmap_expand"]["launches"]
+
+    with Engine(0) as eng:
+        want, of_rows = launches(eng)
+    with Engine(0) as eng:
+        rel = _permutation(4_000_000)
+        tables = [eng.get_hash_table(rel) for _ in range(30)]
+        del rel
+        torch.cuda.empty_cache()
+        for t in tables:
+            t.close()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - 500 * 2**20, dtype=torch.uint8, device="cuda")
+        got, n = launches(eng)
+        del fill
+        torch.cuda.empty_cache()
+    assert n == of_rows and np.array_equal(got.rows, want.rows)
