@@ -746,17 +746,27 @@ static u64 *sg_edge_words(Context &ctx, const int32_t *rows, u64 n, const Graph 
 // the graph has edges enough (three matrices of 256 MB at this size).
 constexpr u32 SG_ROWS_FIRST = 46'000;
 
-// SG as a search over pairs; false (nothing reported) when the pairs are many
-// and the bit matrix would take them, or when memory runs out.
-static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_options &opt, PhaseTimer &pt,
-                              u64 &nfull) {
+// Nodes from which SG that the search over pairs hands over goes to the bit matrix when an edge's
+// source has few out-edges: bit rows read and write three matrices and walk whole rows, which
+// pays where these fill up. Measured, matrix against bit rows: random graphs of 260K nodes
+// and 300K / 309K / 318K edges 56 / 153 / 334 against 105 / 240 / 314 ms, 170K nodes and 200K / 206K
+// / 212K / 220K edges 33 / 61 / 128 / 344 against 44 / 85 / 120 / 188, 87K nodes and 103K / 110K edges 36 / 68 against
+// 36 / 36; meshes of 190K nodes (2.1 out-edges) 53 against 63, 110K (2.2) 495 against 221.
+constexpr u32 SG_MATRIX_NODES = 120'000;
+constexpr double SG_MATRIX_DEGREE = 2.15;
+
+// SG as a search over pairs; false (nothing reported) when another form is the faster one or
+// when memory runs out.
+static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const PairDegrees &deg, const dl_options &opt,
+                              PhaseTimer &pt, u64 &nfull) {
     Workspace &ws = ctx.ws;
     pt.mark(PH_JOIN);
-    // (the first set holds four to eight pairs a node, 512K at least)
-    const u64 most = bitmat_allowed(ctx, g.n_ids, true) ? std::max<u64>(64 * (u64) g.n_ids, 1 << 19) : 0;
+    PairOptions po;
+    po.max_levels = opt.max_iterations > 0 ? (u64) opt.max_iterations : 0;
+    po.handover = bitmat_allowed(ctx, g.n_ids, true);
+    if (!po.handover && pair_search_outrun(deg, {g.n_ids})) return false;  // the sorted runs are the other form
     try {
-        const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits,
-                                          opt.max_iterations > 0 ? (u64) opt.max_iterations : 0, most, ~0ull);
+        const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits, po);
         if (!ps.complete) return false;
         const u64 n = ps.n_words();
         pt.mark(PH_DEDUP);
@@ -774,7 +784,8 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_opt
             const u64 at = std::min<u64>(k + 1, ps.bound.size() - 1);
             const u64 before = std::min<u64>(k, ps.bound.size() - 1);
             r.deltas.push_back((i64) (ps.bound[at] - ps.bound[before]));
-            r.joins.push_back((i64) (k - 1 < ps.rows.size() ? ps.rows[k - 1] : 0));
+            const bool known = k - 1 < ps.rows.size();
+            r.joins.push_back((i64) (known ? ps.rows[k - 1] : 0));
             r.fulls.push_back((i64) ps.bound[at]);
         }
     } catch (const Error &err) {
@@ -814,9 +825,13 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
         build_csr(ctx, e, ne, g);                     // sg.cu:162
         // a small matrix and more than 1.3 edges a node: most likely many pairs
         const bool rows_first = g.n_ids <= SG_ROWS_FIRST && ne * 10 > 13 * (u64) g.n_distinct;
-        if (search && !rows_first && pair_degrees(ctx, g.csr, 0, g.n_ids).fits())
-            listed = sg_pairs_fixpoint(ctx, r, g, opt, pt, nfull);
-        if (search && !listed && bitmat_allowed(ctx, g.n_ids, true)) {
+        bool matrix_first = false;
+        if (search && !rows_first) {
+            const PairDegrees deg = pair_degrees(ctx, g.csr, 0, g.n_ids);
+            if (deg.fits()) listed = sg_pairs_fixpoint(ctx, r, g, deg, opt, pt, nfull);
+            matrix_first = g.n_ids >= SG_MATRIX_NODES && deg.of_sources() < SG_MATRIX_DEGREE;
+        }
+        if (search && !listed && !matrix_first && bitmat_allowed(ctx, g.n_ids, true)) {
             if (!rows_first) e = sg_edge_words(ctx, rows, n, g, ne);  // again: the search used the buffers
             listed = sg_rows(ctx, r, g, e, ne, opt, pt, nfull);
         }

@@ -154,19 +154,23 @@ __global__ void pair_refill_kernel(const u64 *__restrict__ list, u64 n, u64 *set
         pair_insert(set, mask, list[i]);
 }
 
-// found[0] = largest degree, found[1] = ranks with out-edges.
+// found[0] = largest degree, found[1] = edges, found[2] = sum of the degrees' squares.
 __global__ void degrees_kernel(const u32 *__restrict__ off, u64 lo, u64 hi, unsigned long long *__restrict__ found) {
-    u32 m = 0, c = 0;
+    u32 m = 0;
+    u64 c = 0, s = 0;
     for (u64 r = lo + (u64) blockIdx.x * blockDim.x + threadIdx.x; r < hi; r += (u64) gridDim.x * blockDim.x) {
         const u32 d = off[r + 1] - off[r];
         m = max(m, d);
-        c += d != 0;
+        c += d;
+        s += (u64) d * d;
     }
     m = __reduce_max_sync(0xffffffffu, m);
-    c = __reduce_add_sync(0xffffffffu, c);
+    c = warp_sum(c);
+    s = warp_sum(s);
     if ((threadIdx.x & 31) == 0 && m) {
         atomicMax(found, (unsigned long long) m);
         atomicAdd(found + 1, (unsigned long long) c);
+        atomicAdd(found + 2, (unsigned long long) s);
     }
 }
 
@@ -208,44 +212,46 @@ __global__ void pair_counts_kernel(const u64 *__restrict__ list, u64 n, int bits
 bool PairDegrees::fits() const { return most <= PS_DEGREE; }
 
 PairDegrees pair_degrees(Context &ctx, const Csr &csr, u64 lo, u64 hi) {
-    auto *found = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[26]);
-    DL_CUDA(cudaMemsetAsync(found, 0, 16, ctx.stream));
+    auto *found = reinterpret_cast<unsigned long long *>(&ctx.ctrl->scalar[24]);
+    DL_CUDA(cudaMemsetAsync(found, 0, 24, ctx.stream));
     DL_LAUNCH(ctx, K_PREP, 4.0 * (hi - lo),
               degrees_kernel<<<grid_for(hi - lo, T256, ctx, 8), T256, 0, ctx.stream>>>(csr.off, lo, hi, found));
-    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, found, 16, cudaMemcpyDeviceToHost, ctx.stream));
+    DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, found, 24, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
     PairDegrees d;
-    d.most = (u32) ctx.host_scalars[0];
-    d.sources = ctx.host_scalars[1];
+    d.most = ctx.host_scalars[0];
+    d.edges = ctx.host_scalars[1];
+    d.squares = ctx.host_scalars[2];
     return d;
 }
 
-// The search inserts every child of every pair, d^2 of them for d out-edges a source, at
+// The search inserts every child of every pair, the product of two sources' out-edges, at
 // random places: 0.06 ns each while the set is in L2, 0.25 ns for a new one past it. The
-// sorted runs join twice with d, drop duplicates in between and sort, 0.07 ns a word, but
-// an iteration costs half a millisecond however little it finds. So the search loses
-// where sources have more than about two out-edges and the pairs, or the children to
-// look up, are many. Measured, batches on both forms, sorted runs against the search:
-//   random graphs of 2.5 / 3 / 4 / 6 edges a node, 8 of 3000 nodes: 32 / 42 / 46 / 63 ms
-//   against 46 / 61 / 91 / 147; 8 of 1000 nodes, 4 edges: 10.0 against 9.1, 6 edges: 9.7
-//   against 13.0; 8 trees of three children a node, 1000 inner nodes: 6.8 against 10.9;
-//   below the line: 1.5 edges a node, 8 of 3000: 22 against 10; 2 edges, 8 of 1000: 72
-//   against 4.3; meshes of 1.8 edges a node, 4 of 4096 nodes: 143 against 20, one of 22K:
+// sorted runs join twice, drop duplicates in between and sort, 0.07 ns a word, but an
+// iteration costs half a millisecond however little it finds. So the search loses where
+// an edge's source has three out-edges or more and the pairs, or the children to look up, are
+// many. Measured, batches on both forms, sorted runs against the search:
+//   random graphs (1 + d out-edges of an edge's source) of d = 2.5 / 3 / 4 / 6 edges a node, 8 of
+//   3000 nodes: 32 / 42 / 46 / 63 ms against 46 / 61 / 91 / 147; of 2, one of 10,000 nodes: 31
+//   against 37; 8 of 1000 nodes, 4 edges: 10.0 against 9.1, 6 edges: 9.7 against 13.0;
+//   trees of three children a node (3.0), 8 of 1000 inner nodes: 6.8 against 10.9, 3 of 20K nodes
+//   with both directions: 169 against 323;
+//   below the line: 1.5 edges a node (2.5), 8 of 3000: 22 against 10; 2 edges, 8 of 1000: 72
+//   against 4.3; meshes of 1.8 edges a node (2.5), 4 of 4096 nodes: 143 against 20, one of 22K:
 //   163 against 133.
-bool pair_search_outrun(const PairDegrees &d, u64 edges, const std::vector<u64> &n_ids) {
-    const double degree = (double) edges / (double) std::max<u64>(d.sources, 1);
-    if (degree <= 2.2) return false;
+bool pair_search_outrun(const PairDegrees &d, const std::vector<u64> &n_ids) {
+    if (d.of_sources() <= 2.9) return false;
     double nodes = 0, squares = 0;
     for (u64 n : n_ids) {
         nodes += (double) n;
         squares += (double) n * (double) n;
     }
-    const double share = (double) d.sources / std::max(nodes, 1.0);  // nodes with out-edges
-    const double children = degree * degree * share * share * squares;
+    const double mean = (double) d.edges / std::max(nodes, 1.0);
+    const double children = mean * mean * squares;  // pairs of edges
     return std::min(squares, children) > 1.6e7 || children > 2e8;
 }
 
-PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most, u64 limit) {
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const PairOptions &opt) {
     Workspace &ws = ctx.ws;
     PairSearch ps;
     DevBuf &list = ws.jbuf[0], &set = ws.jbuf[1];
@@ -253,22 +259,30 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
     // up to 16M slots stays in L2, where an insert costs a fifth); a level
     // that needs more is repeated on a set four times the size
     u64 slots = PS_SLOTS;
-    while (slots < 8 * (hi - lo) && !(most && slots / 2 >= 2 * most)) slots <<= 1;
-    if (slots * 12 > limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
-    u64 levels = 64;  // level counters: bound[levels + 2], rows[levels + 1], after the list's and blocks' counters
-    ctx.reserve(ws.cl_levels, (2 * levels + 16) * 8);
-    u64 *base = ws.cl_levels.as<u64>();
-    DL_CUDA(cudaMemsetAsync(base, 0, (2 * levels + 16) * 8, ctx.stream));
+    while (slots < 8 * (hi - lo)) slots <<= 1;
+    // A matrix costs its size whatever it holds and 50 to 200 us an iteration, the list 0.3 ns a
+    // pair: past 16 pairs a node (and the first set), levels of more than one a node are the
+    // matrix's, and so are results past 512. Measured: a binary tree of 100K nodes, two
+    // iterations, 7 pairs a node, 1.9 ms on the matrix, 0.65 on the list; a mesh of 264K nodes, 17 a
+    // node in 67 levels, 20 against 3.1; random graphs past the line lose 1 to 5 % to it.
+    const u64 n = hi - lo, many = std::max<u64>(16 * n, PS_SLOTS / 2);
+    if (slots * 12 > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
+    // after the counters of the list and the blocks, two arrays by level: bound and rows, each levels + 4 words
+    u64 levels = 64;
+    constexpr u64 HEAD = 8, ARRAYS = 2;
+    auto words = [](u64 lv) { return HEAD + ARRAYS * (lv + 4); };
+    ctx.reserve(ws.cl_levels, words(levels) * 8);
+    DL_CUDA(cudaMemsetAsync(ws.cl_levels.p, 0, words(levels) * 8, ctx.stream));
     PairState st;
     auto bind = [&]() {
         st.list = list.as<u64>();
         st.cap = slots / 2;
         st.set = set.as<u64>();
         st.mask = slots - 1;
-        u64 *b = ws.cl_levels.as<u64>();
-        st.count = reinterpret_cast<unsigned long long *>(b);
+        auto *b = ws.cl_levels.as<unsigned long long>();
+        st.count = b;
         st.done = reinterpret_cast<u32 *>(b + 1);
-        st.bound = reinterpret_cast<unsigned long long *>(b + 8);
+        st.bound = b + HEAD;
         st.rows = st.bound + levels + 4;
     };
     ctx.reserve(list, slots / 2 * 8);
@@ -287,37 +301,43 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
             const u64 old = levels;
             levels *= 4;
             DevBuf nb;
-            ctx.reserve(nb, (2 * levels + 16) * 8);
-            DL_CUDA(cudaMemsetAsync(nb.p, 0, (2 * levels + 16) * 8, ctx.stream));
+            ctx.reserve(nb, words(levels) * 8);
+            DL_CUDA(cudaMemsetAsync(nb.p, 0, words(levels) * 8, ctx.stream));
             u64 *f = ws.cl_levels.as<u64>(), *t = nb.as<u64>();
-            DL_CUDA(cudaMemcpyAsync(t, f, (8 + old + 4) * 8, cudaMemcpyDeviceToDevice, ctx.stream));
-            DL_CUDA(cudaMemcpyAsync(t + 8 + levels + 4, f + 8 + old + 4, old * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+            DL_CUDA(cudaMemcpyAsync(t, f, HEAD * 8, cudaMemcpyDeviceToDevice, ctx.stream));
+            for (u64 a = 0; a < ARRAYS; ++a)
+                DL_CUDA(cudaMemcpyAsync(t + HEAD + a * (levels + 4), f + HEAD + a * (old + 4), (old + 4) * 8,
+                                        cudaMemcpyDeviceToDevice, ctx.stream));
             ctx.give_back(ws.cl_levels);
             ws.cl_levels = nb;
             bind();
         }
         // an unknown number of pairs: the grid for all nodes, or for the last known level
-        const u64 batch = max_levels ? std::min<u64>(PS_LEVELS, max_levels - level + 1) : PS_LEVELS;
-        const u64 known = level ? ps.bound[level] - ps.bound[level - 1] : hi - lo;
+        const u64 batch = opt.max_levels ? std::min<u64>(PS_LEVELS, opt.max_levels - level + 1) : PS_LEVELS;
+        const u64 known = level ? ps.bound[level] - ps.bound[level - 1] : n;
         for (u64 k = 0; k < batch; ++k) launch(level + k, level || k ? std::max<u64>(4 * known, 1 << 15) : known);
         u64 *hs = ctx.host_scalars;
+        const u64 row0 = level ? level - 1 : 0;
         DL_CUDA(cudaMemcpyAsync(hs, st.count, 8, cudaMemcpyDeviceToHost, ctx.stream));
-        DL_CUDA(cudaMemcpyAsync(hs + 1, st.bound + level + 1, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
-        DL_CUDA(cudaMemcpyAsync(hs + 1 + PS_LEVELS, st.rows + (level ? level - 1 : 0), batch * 8,
-                                cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs + 4, st.bound + level + 1, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs + 4 + PS_LEVELS, st.rows + row0, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        static_assert(4 + ARRAYS * PS_LEVELS < 2 * 31, "fits the host scalars");
         ctx.sync();
-        const u64 found = hs[0];
+        const u64 found = hs[0], *bounds = hs + 4;
         bool full = found >= st.cap, end = false;
         u64 good = batch;  // levels of the batch that are whole
         if (full) {
             good = 0;
-            while (good < batch && hs[1 + good] < st.cap) ++good;
+            while (good < batch && bounds[good] < st.cap) ++good;
         }
         const u64 listed = ps.n_words(), begun = level;
         for (u64 k = 0; k < good; ++k) {
             const u64 lv = level + k;
-            if (lv) ps.rows.push_back(hs[1 + PS_LEVELS + (level ? k : k - 1)]);
-            ps.bound.push_back(hs[1 + k]);
+            if (lv) {
+                const u64 at = level ? k : k - 1;
+                ps.rows.push_back(hs[4 + PS_LEVELS + at]);
+            }
+            ps.bound.push_back(bounds[k]);
             if (ps.bound[lv + 1] == ps.bound[lv]) {  // nothing new
                 ps.complete = end = true;
                 break;
@@ -326,16 +346,19 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u
         ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * (ps.n_words() - listed));  // a new pair's word
         if (end) break;
         level += good;
-        if (!full && max_levels && level > max_levels) {
+        if (!full && opt.max_levels && level > opt.max_levels) {
             ps.complete = true;
             break;
         }
-        if (most && (full || ps.n_words() > most)) break;
+        if (opt.handover) {
+            const u64 all = full ? found : ps.n_words(), last = all - (level ? ps.bound[full ? level : level - 1] : 0);
+            if (all > 512 * n + many || (all >= many && last > n)) break;
+        }
         if (full) {  // repeat level `level` with more room: the set again from the words listed before it
             const u64 keep = ps.bound[level];
             slots *= 4;
             DevBuf nl;
-            if (slots * 12 > limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
+            if (slots * 12 > opt.limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
             ctx.reserve(nl, slots / 2 * 8);
             DL_CUDA(cudaMemcpyAsync(nl.p, list.p, keep * 8, cudaMemcpyDeviceToDevice, ctx.stream));
             ctx.give_back(list);

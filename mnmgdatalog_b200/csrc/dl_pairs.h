@@ -15,25 +15,29 @@ struct PairSearch {
     u64 n_words() const { return bound.empty() ? 0 : bound.back(); }
 };
 
-// Out-edges of ranks [lo, hi): the largest degree and the ranks that have any.
+// Out-edges of ranks [lo, hi).
 struct PairDegrees {
-    u32 most = 0;
-    u64 sources = 0;
+    u64 most = 0;     // the largest
+    u64 edges = 0;    // all
+    u64 squares = 0;  // sum of their squares
     // A pair's expansion is shared by 32 lanes at most.
     bool fits() const;
+    // Mean out-edges of an edge's source (1 more than a node's mean where degrees are random).
+    double of_sources() const { return edges ? (double) squares / (double) edges : 0.0; }
 };
 PairDegrees pair_degrees(Context &ctx, const Csr &csr, u64 lo, u64 hi);
-// Whether sorted runs are the faster form for a session's instances of `n_ids` nodes
-// each, with `edges` between them (see dl_pairs.cu).
-bool pair_search_outrun(const PairDegrees &d, u64 edges, const std::vector<u64> &n_ids);
+// Whether sorted runs are the faster form for graphs of `n_ids` nodes each (see dl_pairs.cu).
+bool pair_search_outrun(const PairDegrees &d, const std::vector<u64> &n_ids);
+
+struct PairOptions {
+    u64 max_levels = 0;    // the level to stop after (0: at the fixpoint)
+    bool handover = false; // stop where a matrix is the faster form (see dl_pairs.cu)
+    u64 limit = ~0ull;     // bytes of the list and the set
+};
 // The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
-// in ws.jbuf[0], unsorted. Stops after level max_levels (0: at the fixpoint). The
-// search is not complete, and its last level may lack words,
-//  * with most != 0 (the caller has another form for many pairs): once more than
-//    `most` words are found or the first set is outgrown;
-//  * once the list and the set would need more than `limit` bytes, or more than half
-//    of the free memory.
-PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, u64 max_levels, u64 most, u64 limit);
+// in ws.jbuf[0], unsorted. It is not complete, and its last level may lack words, where
+// it stopped for `handover` or for `limit` or half of the free memory.
+PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const PairOptions &opt);
 // counts[instance * levels + k] = words of level k of each instance (instance of
 // a word: the last one whose first rank is at most its key rank).
 void pair_level_counts(Context &ctx, const PairSearch &ps, int bits, const u64 *inst_lo, u64 n_inst, u64 *counts);

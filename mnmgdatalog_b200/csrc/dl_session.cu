@@ -586,11 +586,11 @@ void place_results(SessionImpl &s, const std::vector<i64> &ids, u64 words, u64 s
     }
 }
 
-// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi), `edges`
-// between them) as one search over pairs (dl_pairs.cu). False (nothing done) when the
-// sorted runs take them: their degrees do not suit the search, the runs are faster, or
-// its list and set would pass bitmap_max_gib or half of the free memory.
-bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi, u64 edges) {
+// SG: the whole fixpoint of the newly admitted instances `ids` (ranks [lo, hi)) as one
+// search over pairs (dl_pairs.cu). False (nothing done) when the sorted runs take them:
+// their degrees do not suit the search, the runs are faster, or its list and set would pass
+// bitmap_max_gib or half of the free memory.
+bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi) {
     Context &ctx = s.ctx;
     Workspace &ws = ctx.ws;
     const u64 limit = (u64) ctx.tune.bitmap_max_gib << 30;
@@ -606,10 +606,13 @@ bool search_pairs(SessionImpl &s, const std::vector<i64> &ids, u64 lo, u64 hi, u
     if (!deg.fits()) return false;
     std::vector<u64> n_ids(n);
     for (u64 k = 0; k < n; ++k) n_ids[k] = s.inst[ids[k]].n_ids;
-    if (pair_search_outrun(deg, edges, n_ids)) return false;
+    if (pair_search_outrun(deg, n_ids)) return false;
+    PairOptions po;
+    po.max_levels = stop > 0 ? (u64) stop : 0;
+    po.limit = limit;
     PairSearch ps;
     try {
-        ps = pair_search(ctx, csr, lo, hi, s.bits, stop > 0 ? (u64) stop : 0, 0, limit);
+        ps = pair_search(ctx, csr, lo, hi, s.bits, po);
     } catch (const Error &err) {
         if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
         ps.complete = false;
@@ -1043,7 +1046,7 @@ std::vector<i64> session_admit_many(SessionImpl &s, const int32_t *const *rows, 
             if (nrows[k]) with_rows.push_back(inst(k).id);
         if (tc) {
             // searched as a whole in the next step
-        } else if (s.program == DL_PROGRAM_SG && search_pairs(s, with_rows, B, B + nu, ne)) {
+        } else if (s.program == DL_PROGRAM_SG && search_pairs(s, with_rows, B, B + nu)) {
             for (u64 k = 0; k < count; ++k) empty_base[k] = nrows[k] && inst(k).ahead[0] == 0 && inst(k).n_result == 0;
         } else if (s.program == DL_PROGRAM_SG) {
             // sg.cu:170-217: the base rule of the admitted instances, probing the union table

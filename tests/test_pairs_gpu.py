@@ -153,3 +153,20 @@ def test_sg_session_many_pairs_of_wide_sources(engine):
         for i, x in zip(ids, e):
             want, got = engine.sg(x, dedup="sort"), s.result(i)
             assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
+
+
+def _random_above(n, m, seed):
+    return np.concatenate([np.random.default_rng(seed).integers(0, n, (m, 2)), [[0, n - 1]]]).astype(np.int32)
+
+
+@pytest.mark.parametrize("n,m,stop", [(60_000, 60_000, 0), (140_000, 140_000, 0), (140_000, 152_000, 30),
+                                      (140_000, 175_000, 12), (100_000, 106_000, 25), (125_000, 119_000, 0)])
+def test_sg_handed_over_to_other_forms(engine, n, m, stop):
+    """Lists past 16 pairs a node with small levels, and large ones that go to the matrix or to bit rows."""
+    import torch
+    e = _random_above(n, m, 7)
+    want = engine.sg(e, dedup="bitmap", output="device", max_iterations=stop)
+    got = engine.sg(e, output="device", max_iterations=stop)
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    assert torch.equal(got.rows, want.rows)
