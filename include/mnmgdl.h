@@ -107,8 +107,9 @@ typedef struct dl_run_info {
     int64_t output_rows;         /* rows of the program's output file */
     int64_t output_tuples;       /* TC/SG/single_join: |result|; WCC: # components */
     int64_t largest_component;   /* WCC only */
-    int64_t nodes;               /* node ranks of the run: the distinct node ids of the input (TC on the
-                                    bit-matrix path over a dense id range: every id of that range) */
+    int64_t nodes;               /* node ranks of the run: the distinct node ids of the input (TC and SG
+                                    over a dense id range, but for the sorted runs: every id of that
+                                    range) */
     double seconds_total;        /* device time, H2D of the input through the last iteration */
     double seconds_init;         /* phase times (phase_timing = 1), reference CSV columns */
     double seconds_join;
@@ -255,7 +256,10 @@ DL_API dl_status dl_run_copy_output(const dl_run *run, int32_t *dst, int64_t cap
 /* |delta| after each iteration (length = iterations). */
 DL_API dl_status dl_run_copy_deltas(const dl_run *run, int64_t *dst, int64_t capacity);
 /* Per iteration: join output rows (before dedup) and the size of the full
- * relation after the iteration (TC/SG; WCC: number of labelled nodes). */
+ * relation after the iteration (TC/SG; WCC: number of labelled nodes). SG's join has two
+ * steps: the sorted runs, and every form of a graph too large for the bit matrix, count the
+ * distinct rows of the first and the rows of the second; the others the delta rows that
+ * can be joined (and no join total). */
 DL_API dl_status dl_run_copy_iteration_stats(const dl_run *run, int64_t *join_rows, int64_t *full_rows,
                                              int64_t capacity);
 /* WCC: every node id (ascending) and its final component label. */

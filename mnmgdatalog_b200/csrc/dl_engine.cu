@@ -651,6 +651,7 @@ static void run_tc_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
     pt.mark(PH_FINAL);
     adopt_ids(ctx, r, g);
     if (!r.from_bitmat && !done) {
+        r.info.nodes = g.n_distinct;
         r.words = ws.full[cur];
         ws.full[cur] = DevBuf();
         r.n_words = nfull;
@@ -763,8 +764,11 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const PairDe
     pt.mark(PH_JOIN);
     PairOptions po;
     po.max_levels = opt.max_iterations > 0 ? (u64) opt.max_iterations : 0;
+    // without a matrix to hand over to, the sorted runs are the other form, and their
+    // join sizes the ones to report
     po.handover = bitmat_allowed(ctx, g.n_ids, true);
-    if (!po.handover && pair_search_outrun(deg, {g.n_ids})) return false;  // the sorted runs are the other form
+    po.joins = !po.handover;
+    if (po.joins && pair_search_outrun(deg, {g.n_ids})) return false;
     try {
         const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits, po);
         if (!ps.complete) return false;
@@ -785,8 +789,19 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const PairDe
             const u64 before = std::min<u64>(k, ps.bound.size() - 1);
             r.deltas.push_back((i64) (ps.bound[at] - ps.bound[before]));
             const bool known = k - 1 < ps.rows.size();
-            r.joins.push_back((i64) (known ? ps.rows[k - 1] : 0));
+            if (po.joins) {
+                const u64 one = known ? ps.first[k - 1] : 0, two = known ? ps.second[k - 1] : 0;
+                r.joins.push_back((i64) (known ? ps.middle[k - 1] + two : 0));
+                ctx.run_join_total += one + two;
+                ctx.run_join_max = std::max(ctx.run_join_max, std::max(one, two));
+            } else {
+                r.joins.push_back((i64) (known ? ps.rows[k - 1] : 0));
+            }
             r.fulls.push_back((i64) ps.bound[at]);
+        }
+        if (po.joins) {  // the base rule's join
+            ctx.run_join_total += deg.squares;
+            ctx.run_join_max = std::max(ctx.run_join_max, deg.squares);
         }
     } catch (const Error &err) {
         if (err.status != DL_ERR_OUT_OF_MEMORY) throw;
@@ -899,6 +914,7 @@ static void run_sg_impl(Context &ctx, Run &r, const int32_t *rows_in, u64 n, boo
     pt.mark(PH_FINAL);
     adopt_ids(ctx, r, g);
     if (!on_bitmat) {
+        r.info.nodes = g.n_distinct;
         r.words = ws.full[cur];
         ws.full[cur] = DevBuf();
         r.n_words = nfull;

@@ -36,6 +36,11 @@ struct PairState {
     unsigned long long *bound;       // bound[k]: first word of level k
     unsigned long long *rows;        // rows[k]: pairs of level k with children
     u32 *done;                       // blocks of the current launch that are through
+    // The joins in two steps (PairOptions::joins)
+    u64 *mid;                        // set of a level's (x, b), as many slots as `set`
+    unsigned long long *mids;        // words in it
+    unsigned long long *over;        // they passed half of the slots in some level
+    unsigned long long *first, *middle, *second;  // as in PairSearch
 };
 
 __device__ __forceinline__ u64 pair_slot(u64 w, u64 mask) {
@@ -149,6 +154,48 @@ pair_level_kernel(PairState st, const u32 *__restrict__ off, const u32 *__restri
     }
 }
 
+// The first join of level - 1's pairs (a, b): the distinct (x, b), x a child of a, and the second
+// one's rows, b's children for each. For graphs past the bit matrix, whose join sizes are
+// those of the sorted runs; `mid` is empty before the launch.
+__global__ void __launch_bounds__(PS_THREADS)
+pair_joins_kernel(PairState st, const u32 *__restrict__ off, const u32 *__restrict__ val, int bits, u32 level) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 mask = (1ull << bits) - 1;
+    const u64 i0 = st.bound[level - 1], i1 = st.bound[level];
+    const u64 warps = (u64) gridDim.x * (PS_THREADS / 32);
+    u64 first = 0, middle = 0, second = 0;
+    for (u64 g = i0 + ((u64) blockIdx.x * PS_THREADS + threadIdx.x) / 32 * 32; g < i1; g += warps * 32) {
+        u32 ab = 0, da = 0, b = 0, db = 0;
+        if (g + lane < i1) {
+            const u64 w = st.list[g + lane], a = w >> bits;
+            b = (u32) (w & mask);
+            ab = __ldg(off + a);
+            da = __ldg(off + a + 1) - ab;
+            db = __ldg(off + b + 1) - __ldg(off + b);
+        }
+        first += da;
+        const u32 most = __reduce_max_sync(0xffffffffu, da);  // (64 at most)
+        for (u32 k = 0; k < most; ++k) {
+            const bool room = *reinterpret_cast<volatile unsigned long long *>(st.mids) < st.cap;
+            const bool fresh = k < da && room && pair_insert(st.mid, st.mask, ((u64) __ldg(val + ab + k) << bits) | b);
+            const u32 fm = __ballot_sync(0xffffffffu, fresh);
+            if (!room && lane == 0) *st.over = 1;
+            if (!fm) continue;
+            if (lane == 0) atomicAdd(st.mids, (unsigned long long) __popc(fm));
+            middle += fresh;
+            second += fresh ? db : 0u;
+        }
+    }
+    first = warp_sum(first);
+    middle = warp_sum(middle);
+    second = warp_sum(second);
+    if (lane == 0) {
+        if (first) atomicAdd(st.first + level - 1, (unsigned long long) first);
+        if (middle) atomicAdd(st.middle + level - 1, (unsigned long long) middle);
+        if (second) atomicAdd(st.second + level - 1, (unsigned long long) second);
+    }
+}
+
 __global__ void pair_refill_kernel(const u64 *__restrict__ list, u64 n, u64 *set, u64 mask) {
     for (u64 i = (u64) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64) gridDim.x * blockDim.x)
         pair_insert(set, mask, list[i]);
@@ -254,7 +301,7 @@ bool pair_search_outrun(const PairDegrees &d, const std::vector<u64> &n_ids) {
 PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const PairOptions &opt) {
     Workspace &ws = ctx.ws;
     PairSearch ps;
-    DevBuf &list = ws.jbuf[0], &set = ws.jbuf[1];
+    DevBuf &list = ws.jbuf[0], &set = ws.jbuf[1], &mid = ws.full[0];
     // room for four pairs a node at first, slots for twice as many words (a set of
     // up to 16M slots stays in L2, where an insert costs a fifth); a level
     // that needs more is repeated on a set four times the size
@@ -266,10 +313,12 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
     // iterations, 7 pairs a node, 1.9 ms on the matrix, 0.65 on the list; a mesh of 264K nodes, 17 a
     // node in 67 levels, 20 against 3.1; random graphs past the line lose 1 to 5 % to it.
     const u64 n = hi - lo, many = std::max<u64>(16 * n, PS_SLOTS / 2);
-    if (slots * 12 > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
-    // after the counters of the list and the blocks, two arrays by level: bound and rows, each levels + 4 words
+    const u64 unit = opt.joins ? 20 : 12;  // bytes a slot: the set, half as many words, the joins' set
+    if (slots * unit > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
+    // After the counters of the list, the blocks and the joins' set, five arrays by level
+    // (PairState): bound, rows, first, middle, second, each levels + 4 words
     u64 levels = 64;
-    constexpr u64 HEAD = 8, ARRAYS = 2;
+    constexpr u64 HEAD = 8, ARRAYS = 5;
     auto words = [](u64 lv) { return HEAD + ARRAYS * (lv + 4); };
     ctx.reserve(ws.cl_levels, words(levels) * 8);
     DL_CUDA(cudaMemsetAsync(ws.cl_levels.p, 0, words(levels) * 8, ctx.stream));
@@ -279,21 +328,35 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
         st.cap = slots / 2;
         st.set = set.as<u64>();
         st.mask = slots - 1;
+        st.mid = mid.as<u64>();
         auto *b = ws.cl_levels.as<unsigned long long>();
         st.count = b;
         st.done = reinterpret_cast<u32 *>(b + 1);
+        st.mids = b + 2;
+        st.over = b + 3;
         st.bound = b + HEAD;
         st.rows = st.bound + levels + 4;
+        st.first = st.rows + levels + 4;
+        st.middle = st.first + levels + 4;
+        st.second = st.middle + levels + 4;
     };
     ctx.reserve(list, slots / 2 * 8);
     ctx.reserve(set, slots * 8);
     DL_CUDA(cudaMemsetAsync(set.p, 0xFF, slots * 8, ctx.stream));
+    if (opt.joins) ctx.reserve(mid, slots * 8);
     bind();
     ps.bound.assign(1, 0);
     auto launch = [&](u64 level, u64 pairs) {
         DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
                   pair_level_kernel<<<grid_for(pairs, PS_THREADS, ctx, 8), PS_THREADS, 0, ctx.stream>>>(
                       st, csr.off, csr.val, lo, hi, bits, (u32) level));
+        if (opt.joins && level) {
+            DL_CUDA(cudaMemsetAsync(st.mid, 0xFF, slots * 8, ctx.stream));
+            DL_CUDA(cudaMemsetAsync(st.mids, 0, 8, ctx.stream));
+            DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
+                      pair_joins_kernel<<<grid_for(pairs, PS_THREADS, ctx, 8), PS_THREADS, 0, ctx.stream>>>(
+                          st, csr.off, csr.val, bits, (u32) level));
+        }
     };
     for (u64 level = 0;;) {
         // room for the levels of this batch
@@ -316,14 +379,21 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
         const u64 batch = opt.max_levels ? std::min<u64>(PS_LEVELS, opt.max_levels - level + 1) : PS_LEVELS;
         const u64 known = level ? ps.bound[level] - ps.bound[level - 1] : n;
         for (u64 k = 0; k < batch; ++k) launch(level + k, level || k ? std::max<u64>(4 * known, 1 << 15) : known);
+        // host copies: the head's words [0, 4), then `batch` of each array (all but bound from the
+        // rows that this batch's first level counts on)
         u64 *hs = ctx.host_scalars;
         const u64 row0 = level ? level - 1 : 0;
-        DL_CUDA(cudaMemcpyAsync(hs, st.count, 8, cudaMemcpyDeviceToHost, ctx.stream));
+        DL_CUDA(cudaMemcpyAsync(hs, st.count, 32, cudaMemcpyDeviceToHost, ctx.stream));
         DL_CUDA(cudaMemcpyAsync(hs + 4, st.bound + level + 1, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
         DL_CUDA(cudaMemcpyAsync(hs + 4 + PS_LEVELS, st.rows + row0, batch * 8, cudaMemcpyDeviceToHost, ctx.stream));
+        if (opt.joins)
+            for (u64 a = 0; a < 3; ++a)
+                DL_CUDA(cudaMemcpyAsync(hs + 4 + (2 + a) * PS_LEVELS, st.first + a * (levels + 4) + row0, batch * 8,
+                                        cudaMemcpyDeviceToHost, ctx.stream));
         static_assert(4 + ARRAYS * PS_LEVELS < 2 * 31, "fits the host scalars");
         ctx.sync();
         const u64 found = hs[0], *bounds = hs + 4;
+        if (opt.joins && hs[3]) break;  // (x, b) words were not counted
         bool full = found >= st.cap, end = false;
         u64 good = batch;  // levels of the batch that are whole
         if (full) {
@@ -336,6 +406,11 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
             if (lv) {
                 const u64 at = level ? k : k - 1;
                 ps.rows.push_back(hs[4 + PS_LEVELS + at]);
+                if (opt.joins) {
+                    ps.first.push_back(hs[4 + 2 * PS_LEVELS + at]);
+                    ps.middle.push_back(hs[4 + 3 * PS_LEVELS + at]);
+                    ps.second.push_back(hs[4 + 4 * PS_LEVELS + at]);
+                }
             }
             ps.bound.push_back(bounds[k]);
             if (ps.bound[lv + 1] == ps.bound[lv]) {  // nothing new
@@ -358,13 +433,14 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
             const u64 keep = ps.bound[level];
             slots *= 4;
             DevBuf nl;
-            if (slots * 12 > opt.limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
+            if (slots * unit > opt.limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
             ctx.reserve(nl, slots / 2 * 8);
             DL_CUDA(cudaMemcpyAsync(nl.p, list.p, keep * 8, cudaMemcpyDeviceToDevice, ctx.stream));
             ctx.give_back(list);
             list = nl;
             ctx.reserve(set, slots * 8);
             DL_CUDA(cudaMemsetAsync(set.p, 0xFF, slots * 8, ctx.stream));
+            if (opt.joins) ctx.reserve(mid, slots * 8);
             bind();
             if (keep)
                 DL_LAUNCH(ctx, K_BITMAP_EXPAND, 16.0 * keep,
@@ -373,7 +449,8 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
             DL_CUDA(cudaMemcpyAsync(st.count, ps.bound.data() + level, 8, cudaMemcpyHostToDevice, ctx.stream));
             // rows counted by the levels that are repeated: the batch's last one counted rows[begun + batch - 2]
             const u64 row = level ? level - 1 : 0;
-            DL_CUDA(cudaMemsetAsync(st.rows + row, 0, (begun + batch - 1 - row) * 8, ctx.stream));
+            for (u64 a = 0; a < 4; ++a)
+                DL_CUDA(cudaMemsetAsync(st.rows + a * (levels + 4) + row, 0, (begun + batch - 1 - row) * 8, ctx.stream));
             ctx.sync();  // ps.bound is host memory
         }
     }

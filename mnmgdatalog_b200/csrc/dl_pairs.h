@@ -11,6 +11,10 @@ namespace detail {
 struct PairSearch {
     std::vector<u64> bound;  // level k holds words [bound[k], bound[k + 1])
     std::vector<u64> rows;   // rows[k]: pairs of level k whose two nodes have out-edges
+    // With the joins counted, of level k's join in two steps (x, b), then (x, y):
+    std::vector<u64> first;   // rows of the first one
+    std::vector<u64> middle;  // distinct ones
+    std::vector<u64> second;  // rows of the second one
     bool complete = false;   // the last level found nothing (or max_levels ended the search)
     u64 n_words() const { return bound.empty() ? 0 : bound.back(); }
 };
@@ -19,7 +23,7 @@ struct PairSearch {
 struct PairDegrees {
     u64 most = 0;     // the largest
     u64 edges = 0;    // all
-    u64 squares = 0;  // sum of their squares
+    u64 squares = 0;  // sum of their squares: the rows of the base rule's join
     // A pair's expansion is shared by 32 lanes at most.
     bool fits() const;
     // Mean out-edges of an edge's source (1 more than a node's mean where degrees are random).
@@ -33,10 +37,12 @@ struct PairOptions {
     u64 max_levels = 0;    // the level to stop after (0: at the fixpoint)
     bool handover = false; // stop where a matrix is the faster form (see dl_pairs.cu)
     u64 limit = ~0ull;     // bytes of the list and the set
+    bool joins = false;    // count the rows of the joins in two steps, as the sorted runs do
 };
 // The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
 // in ws.jbuf[0], unsorted. It is not complete, and its last level may lack words, where
-// it stopped for `handover` or for `limit` or half of the free memory.
+// it stopped for `handover`, for `limit` or half of the free memory, or because a level's first
+// join did not fit the table that counts it.
 PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, const PairOptions &opt);
 // counts[instance * levels + k] = words of level k of each instance (instance of
 // a word: the last one whose first rank is at most its key rank).

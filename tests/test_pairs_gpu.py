@@ -155,6 +155,40 @@ def test_sg_session_many_pairs_of_wide_sources(engine):
             assert got.deltas.tolist() == want.deltas.tolist() and np.array_equal(got.rows, want.rows)
 
 
+def _full_stats(got, want):
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    for f in ("join_rows_total", "join_rows_max", "iterations", "nodes", "output_tuples"):
+        assert getattr(got, f) == getattr(want, f), f
+    assert np.array_equal(got.rows, want.rows)
+
+
+@pytest.mark.parametrize("stop", [0, 1, 3])
+@pytest.mark.parametrize("name", ["lattice", "wide_ids", "random", "forest", "wide_tree", "loops"])
+def test_sg_past_the_matrix_reports_the_sorted_runs_joins(name, stop):
+    """Graphs whose bit matrix passes bitmap_max_gib: rows and join sizes are those of the sorted
+    runs, by the search (which counts them) or by the runs."""
+    from mnmgdatalog_b200 import Engine
+    n = 130_000
+    rng = np.random.default_rng(1)
+    e = {"lattice": lambda: graphs.lattice3d(side=52, p=0.16, seed=3),
+         "wide_ids": lambda: graphs.lattice3d(side=50, p=0.15, seed=4) * 17_001 - 2 * 10**9,
+         "random": lambda: rng.integers(0, n, (100_000, 2)),
+         "forest": lambda: np.concatenate([np.asarray(_tree(13, 3)) + 40 * k for k in range(3300)]),
+         "wide_tree": lambda: np.stack([np.arange(n) // 10, np.arange(n) + 1], 1),
+         "loops": lambda: np.concatenate([np.stack([np.arange(n), np.arange(n)], 1),
+                                          np.stack([np.arange(n - 1), np.arange(1, n)], 1)])}[name]()
+    e = np.ascontiguousarray(e).astype(np.int32)
+    if name == "wide_tree" and stop != 1:
+        pytest.skip("10^9 pairs")
+    if name == "loops" and not stop:
+        stop = 5
+    with Engine(0) as eng:
+        eng.set_tuning(bitmap_max_gib=1)
+        assert len(np.unique(e)) > 93_000
+        _full_stats(eng.sg(e, max_iterations=stop), eng.sg(e, dedup="sort", max_iterations=stop))
+
+
 def _random_above(n, m, seed):
     return np.concatenate([np.random.default_rng(seed).integers(0, n, (m, 2)), [[0, n - 1]]]).astype(np.int32)
 
