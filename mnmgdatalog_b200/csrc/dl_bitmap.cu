@@ -1120,23 +1120,24 @@ bool bitmat_choose(Context &ctx, const dl_options &opt, u64 n, bool sg) {
     if (!bitmat_row_fits(n, sg)) return false;
     // TC also keeps the per (row block, target) offsets of its result rows
     const u64 need = bitmat_bytes(n) + (sg ? 0 : bitmat_column_offset_bytes(n));
-    // a context that already holds the matrix buffer (a repeated run) needs
-    // no driver query: the memory is its own
-    if (opt.dedup == DL_DEDUP_AUTO && ctx.ws.bitmat[0].cap >= bitmat_bytes(n) &&
-        need <= ((u64) ctx.tune.bitmap_max_gib << 30))
-        return true;
+    if (opt.dedup == DL_DEDUP_AUTO) {
+        if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
+        // a context that already holds the matrix buffer (a repeated run) needs no driver
+        // query: the memory is its own
+        if (ctx.ws.bitmat[0].cap >= bitmat_bytes(n)) return true;
+        DevBuf none;
+        DevBuf &offsets = sg ? none : ctx.ws.bitmat[1];
+        return ctx.room_for({{&ctx.ws.bitmat[0], bitmat_bytes(n)},
+                             {&offsets, sg ? 0 : bitmat_column_offset_bytes(n)}},
+                            {&ctx.ws.cl_rows[0], &ctx.ws.cl_rows[1]});
+    }
     size_t free_b = 0, total_b = 0;
     DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const u64 held = ctx.ws.bitmat[0].cap + ctx.ws.bitmat[1].cap;
-    const u64 avail = (u64) free_b + held;
-    if (opt.dedup == DL_DEDUP_BITMAP) {
-        if (need > avail)
-            throw Error(DL_ERR_OUT_OF_MEMORY, "bitmap dedup needs " + std::to_string(need) + " bytes for " +
-                                                  std::to_string(n) + " nodes; " + std::to_string(avail) +
-                                                  " available");
-        return true;
-    }
-    return need <= ((u64) ctx.tune.bitmap_max_gib << 30) && need <= avail / 2;
+    const u64 avail = (u64) free_b + ctx.ws.bitmat[0].cap + ctx.ws.bitmat[1].cap;
+    if (need > avail)
+        throw Error(DL_ERR_OUT_OF_MEMORY, "bitmap dedup needs " + std::to_string(need) + " bytes for " +
+                                              std::to_string(n) + " nodes; " + std::to_string(avail) + " available");
+    return true;
 }
 
 

@@ -1622,7 +1622,8 @@ static bool tc_closure_run(Context &ctx, Run &r, const Graph &g, const u64 *edge
         const u64 need = closure_pull_bytes(n, light.n_heavy);
         if (need > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
         const u64 rows = n * pull_words(light.n_heavy) * 4;
-        if (!ctx.room_for({{&r.bm_t, rows}, {&ws.cl_rows[0], rows}, {&ws.cl_rows[1], rows}, {&ws.cl_act, 8 * n * 4}}))
+        if (!ctx.room_for({{&r.bm_t, rows}, {&ws.cl_rows[0], rows}, {&ws.cl_rows[1], rows}, {&ws.cl_act, 8 * n * 4}},
+                          {&ws.bitmat[0], &ws.bitmat[1]}))
             return false;
         // (now, before smaller requests take the cached buffers that were counted on)
         ctx.reserve(r.bm_t, rows);

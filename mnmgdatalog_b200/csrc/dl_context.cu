@@ -122,19 +122,30 @@ int Context::best_spare(const std::vector<DevBuf> &from, size_t bytes) {
     return best;
 }
 
-bool Context::room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants) {
+bool Context::room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants,
+                       std::initializer_list<DevBuf *> idle) {
     take_returned();
     std::vector<DevBuf> left = spares;
-    size_t fresh = 0;
-    for (const auto &w : wants) {
-        if (w.first->p && w.first->cap >= w.second) continue;
-        const int best = best_spare(left, w.second);
-        if (best >= 0) left.erase(left.begin() + best);
-        else fresh += w.first->p ? std::max(w.second, w.first->cap + w.first->cap / 2) : w.second;
-    }
+    auto fresh_bytes = [&] {
+        size_t fresh = 0;
+        for (const auto &w : wants) {
+            if (w.first->cap >= w.second) continue;
+            const int best = best_spare(left, w.second);
+            if (best >= 0) left.erase(left.begin() + best);
+            else fresh += w.first->p ? std::max(w.second, w.first->cap + w.first->cap / 2) : w.second;
+        }
+        return fresh;
+    };
+    size_t fresh = fresh_bytes();
     if (!fresh) return true;
     size_t free_b = 0, total_b = 0;
     DL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (fresh > free_b / 2) {  // the other forms' buffers join the cache
+        for (DevBuf *b : idle) give_back(*b);
+        left = spares;
+        if (!(fresh = fresh_bytes())) return true;
+        DL_CUDA(cudaMemGetInfo(&free_b, &total_b));  // (the cache may have been trimmed)
+    }
     size_t cached = 0;
     for (const DevBuf &b : left) cached += b.cap;
     if (fresh > (free_b + cached) / 2) return false;

@@ -245,9 +245,11 @@ struct Context {
     static int best_spare(const std::vector<DevBuf> &from, size_t bytes);
     // Whether buffers of these sizes may be reserved by a form that another one can stand
     // in for: what they would newly allocate is at most half of the free device memory (the
-    // rest is left to whoever shares the GPU). Cached buffers that none of them reuses
-    // count as free and are freed for it. No driver query when nothing would be allocated.
-    bool room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants);
+    // rest is left to whoever shares the GPU). Cached buffers that none of them reuses, and
+    // the workspace's `idle` ones, which other forms left, count as free and are freed for
+    // it. No driver query when nothing would be allocated.
+    bool room_for(std::initializer_list<std::pair<const DevBuf *, size_t>> wants,
+                  std::initializer_list<DevBuf *> idle = {});
     // A buffer that goes into a caller's hands: at most twice the size asked for.
     void reserve_tight(DevBuf &buf, size_t bytes);
     void trim_spares();

@@ -313,8 +313,9 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
     // iterations, 7 pairs a node, 1.9 ms on the matrix, 0.65 on the list; a mesh of 264K nodes, 17 a
     // node in 67 levels, 20 against 3.1; random graphs past the line lose 1 to 5 % to it.
     const u64 n = hi - lo, many = std::max<u64>(16 * n, PS_SLOTS / 2);
+    const std::initializer_list<DevBuf *> idle = {&ws.bitmat[0], &ws.bitmat[1], &ws.cl_rows[0], &ws.cl_rows[1]};
     const u64 unit = opt.joins ? 20 : 12;  // bytes a slot: the set, half as many words, the joins' set
-    if (slots * unit > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}})) return ps;
+    if (slots * unit > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}}, idle)) return ps;
     // After the counters of the list, the blocks and the joins' set, five arrays by level
     // (PairState): bound, rows, first, middle, second, each levels + 4 words
     u64 levels = 64;
@@ -433,7 +434,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
             const u64 keep = ps.bound[level];
             slots *= 4;
             DevBuf nl;
-            if (slots * unit > opt.limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}})) break;
+            if (slots * unit > opt.limit || !ctx.room_for({{&nl, slots / 2 * 8}, {&set, slots * 8}}, idle)) break;
             ctx.reserve(nl, slots / 2 * 8);
             DL_CUDA(cudaMemcpyAsync(nl.p, list.p, keep * 8, cudaMemcpyDeviceToDevice, ctx.stream));
             ctx.give_back(list);

@@ -184,7 +184,7 @@ bool self_join_rows(Context &ctx, Run &r, const Csr &in, u64 total, PhaseTimer &
     // dozen times: worth it up to 16 bytes of matrix per join word (a result
     // row per 1K bits or so).
     if (smem + 4096 > 227 * 1024 || bytes > 16 * total || bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-    if (!ctx.room_for({{&r.bm_t, bytes}})) return false;
+    if (!ctx.room_for({{&r.bm_t, bytes}}, {&ws.bitmat[0], &ws.bitmat[1], &ws.cl_rows[0], &ws.cl_rows[1]})) return false;
     pt.mark(PH_JOIN);
     try {
         ctx.reserve(r.bm_t, bytes);

@@ -367,7 +367,9 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     const u64 bytes = n * words * 4;
     if (words * 4 + 24 * 1024 > 227 * 1024) return false;  // a row in shared memory beside the queues
     if (3 * bytes > ((u64) ctx.tune.bitmap_max_gib << 30)) return false;
-    if (!ctx.room_for({{&r.bm_t, bytes}, {&ws.cl_rows[0], bytes}, {&ws.cl_rows[1], bytes}})) return false;
+    if (!ctx.room_for({{&r.bm_t, bytes}, {&ws.cl_rows[0], bytes}, {&ws.cl_rows[1], bytes}},
+                      {&ws.bitmat[0], &ws.bitmat[1]}))
+        return false;
     // (now, before smaller requests take the cached buffers that were counted on)
     ctx.reserve(r.bm_t, bytes);
     ctx.reserve(ws.cl_rows[0], bytes);

@@ -237,3 +237,23 @@ def test_the_cache_makes_room_for_bit_rows():
         del fill
         torch.cuda.empty_cache()
     assert n == of_rows and np.array_equal(got.rows, want.rows)
+
+
+def test_the_workspace_of_other_forms_makes_room_for_the_matrix():
+    """After TC on bit rows (8 GB, two thirds of it workspace) 1 GB is free: SG that goes to the bit
+    matrix (2 GB) still does, and not to the sorted runs, whose join sizes are others."""
+    import torch
+    rng = np.random.default_rng(5)
+    tc = rng.integers(0, 150_000, (430_000, 2)).astype(np.int32)
+    sg = np.concatenate([rng.integers(0, 125_000, (132_000, 2)), [[0, 124_999]]]).astype(np.int32)
+    with Engine(0) as eng:
+        want = eng.sg(sg, max_iterations=25)
+    with Engine(0) as eng:
+        eng.tc(tc, output="none")
+        torch.cuda.empty_cache()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - 2**30, dtype=torch.uint8, device="cuda")
+        got = eng.sg(sg, max_iterations=25)
+        del fill
+        torch.cuda.empty_cache()
+    assert got.join_rows.tolist() == want.join_rows.tolist() and np.array_equal(got.rows, want.rows)
+    assert got.nodes == want.nodes
