@@ -870,6 +870,123 @@ closure_pull_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, con
     }
 }
 
+// The same level for rows of P = 1 or 2 chunks (up to 2048 heavy sources), by eight lanes for a
+// target: a warp's 32 lanes, one target at a time, left most of a short row's idle,
+// and the level is a chain of dependent loads. Trees, whose heavy sources are few: 4M nodes,
+// three children each, 1.0 -> 0.26 ms a level (the whole run 24.7 -> 13.0, 12.4 on the sorted
+// runs); 1M nodes, ten children, 4.2 -> 3.0 (2.5).
+template <int P>
+__global__ void __launch_bounds__(PU_THREADS, 4)
+closure_pull_thin_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u32 *__restrict__ roff,
+                         const u32 *__restrict__ rval, const u32 *__restrict__ hub_at, u32 *__restrict__ hub_acc,
+                         u32 *__restrict__ t) {
+    const u64 n_list = st.count[st.level];
+    if (n_list == 0) return;  // the fixpoint was reached earlier
+    __shared__ unsigned long long part[2][PU_THREADS / 32];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane & 7;
+    const u64 groups = (u64) gridDim.x * (PU_THREADS / 8);
+    u64 fresh = 0, dsum = 0;
+    for (u64 i0 = ((u64) blockIdx.x * PU_THREADS + (threadIdx.x & ~31u)) / 8; i0 < n_list; i0 += groups) {
+        const u64 i = i0 + (lane >> 3);
+        const bool have = i < n_list;
+        u32 w = 0, m = 0, b = 0, n = 0;
+        if (have) {
+            w = st.list[i];
+            m = st.todo[w];
+            b = __ldg(roff + w);
+            n = __ldg(roff + w + 1) - b;
+        }
+        const u64 row = (u64) w * sh.words + l * 4;
+        uint4 old[P], acc[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            acc[p] = old[p] = make_uint4(0, 0, 0, 0);
+            if ((m >> p) & 1u) old[p] = *reinterpret_cast<const uint4 *>(t + row + 32 * p);
+        }
+        if (n > PU_SEG) {
+            u32 *hrow = hub_acc + (u64) hub_at[w] * sh.words + l * 4;
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+                if ((m >> p) & 1u) {
+                    uint4 *hp = reinterpret_cast<uint4 *>(hrow + 32 * p);
+                    acc[p] = *hp;
+                    *hp = make_uint4(0, 0, 0, 0);
+                }
+            n = 0;
+        }
+        const u32 most = __reduce_max_sync(0xffffffffu, n);
+        for (u32 k0 = 0; k0 < most; k0 += 8) {
+            u32 y = 0, a = 0;
+            if (k0 + l < n) {
+                y = __ldg(rval + b + k0 + l);
+                const uint2 tg = st.tag[y];
+                a = tg.y == st.level - 1 ? tg.x : 0u;
+            }
+            constexpr u32 FLIGHT = 4 / P;  // in-neighbours whose pieces are in flight
+            uint4 v[FLIGHT][P];
+#pragma unroll
+            for (u32 h = 0; h < 8; h += FLIGHT) {
+#pragma unroll
+                for (u32 j = 0; j < FLIGHT; ++j) {
+                    const u32 yj = __shfl_sync(0xffffffffu, y, h + j, 8), aj = __shfl_sync(0xffffffffu, a, h + j, 8);
+                    const uint4 *src = reinterpret_cast<const uint4 *>(st.cur + (u64) yj * sh.words + l * 4);
+#pragma unroll
+                    for (int p = 0; p < P; ++p) {
+                        v[j][p] = make_uint4(0, 0, 0, 0);
+                        if ((aj >> p) & 1u) v[j][p] = __ldg(src + 8 * p);
+                    }
+                }
+#pragma unroll
+                for (u32 j = 0; j < FLIGHT; ++j)
+#pragma unroll
+                    for (int p = 0; p < P; ++p) {
+                        acc[p].x |= v[j][p].x;
+                        acc[p].y |= v[j][p].y;
+                        acc[p].z |= v[j][p].z;
+                        acc[p].w |= v[j][p].w;
+                    }
+            }
+        }
+        u32 mark = 0, bits_new = 0;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const uint4 nw = make_uint4(acc[p].x & ~old[p].x, acc[p].y & ~old[p].y, acc[p].z & ~old[p].z,
+                                        acc[p].w & ~old[p].w);
+            const bool any = (nw.x | nw.y | nw.z | nw.w) != 0;
+            if (any) {
+                *reinterpret_cast<uint4 *>(t + row + 32 * p) =
+                    make_uint4(old[p].x | nw.x, old[p].y | nw.y, old[p].z | nw.z, old[p].w | nw.w);
+                bits_new += __popc(nw.x) + __popc(nw.y) + __popc(nw.z) + __popc(nw.w);
+            }
+            const u32 lines = __ballot_sync(0xffffffffu, any);
+            if ((lines >> (lane & 24)) & 0xFFu) {  // this chunk has new bits: the whole line is written
+                mark |= 1u << p;
+                *reinterpret_cast<uint4 *>(st.nxt + row + 32 * p) = nw;
+            }
+        }
+        if (have && l == 0) {
+            st.todo[w] = 0;
+            if (mark) st.tag_next[w] = make_uint2(mark, st.level);
+        }
+        if (bits_new) {
+            fresh += bits_new;
+            dsum += (u64) bits_new * (__ldg(off + w + 1) - __ldg(off + w));
+        }
+    }
+    fresh = warp_sum(fresh);
+    dsum = warp_sum(dsum);
+    if (lane == 0) {
+        part[0][warp] = fresh;
+        part[1][warp] = dsum;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long v = 0;
+        for (int i = 0; i < PU_THREADS / 32; ++i) v += part[threadIdx.x][i];
+        if (v) atomicAdd((threadIdx.x == 0 ? st.cnt : st.deg) + st.level, v);
+    }
+}
+
 // ---- results ------------------------------------------------------------
 
 // Row z's result rows by chunk: start[z * chunks + c] = (rows of z before
@@ -1475,10 +1592,13 @@ ClosureHeavy closure_pull(Context &ctx, const Csr &csr, const u64 *edges, u64 ne
                       closure_pull_hub_kernel<K><<<grid_for(n_seg * passes * 32, PU_THREADS, ctx, 8), PU_THREADS, 0,
                                                    ctx.stream>>>(sh, view(level), roff, rval, ws.cl_segs.as<uint2>(),
                                                                  n_seg, ws.cl_hub_at.as<u32>(), hub_acc));
-        const u64 wave = resident_blocks(ctx, closure_pull_kernel<K>, PU_THREADS, 0);
+        // lanes for a target: 8 for rows of one or two chunks, else a warp
+        auto kern = res.words == 32 ? closure_pull_thin_kernel<1>
+                    : res.words == 64 ? closure_pull_thin_kernel<2> : closure_pull_kernel<K>;
+        const u64 per = PU_THREADS / (res.words <= 64 ? 8 : 32);
+        const u64 wave = resident_blocks(ctx, kern, PU_THREADS, 0);
         DL_LAUNCH(ctx, K_BITMAP_EXPAND, 0,
-                  closure_pull_kernel<K><<<(unsigned) std::min<u64>(wave, (n + PU_THREADS / 32 - 1) / (PU_THREADS / 32)),
-                                           PU_THREADS, 0, ctx.stream>>>(
+                  kern<<<(unsigned) std::min<u64>(wave, (n + per - 1) / per), PU_THREADS, 0, ctx.stream>>>(
                       sh, view(level), csr.off, roff, rval, ws.cl_hub_at.as<u32>(), hub_acc, t.as<u32>()));
         push(level);
     };

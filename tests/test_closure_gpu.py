@@ -232,3 +232,26 @@ def test_tc_rows_of_many_light_sources(engine, name):
     want, got = engine.tc(e, dedup="sort"), engine.tc(e)
     assert got.deltas.tolist() == want.deltas.tolist()
     assert np.array_equal(got.rows, want.rows)
+
+
+def _kary(n, k):
+    a = np.arange(1, n)
+    return np.stack([(a - 1) // k, a], 1)
+
+
+THIN = {f"heads_{h}": _fan(4200, h) for h in (1, 1022, 1023, 1024, 2046, 2047, 2048)}
+THIN |= {"tree_3": _kary(120_000, 3), "tree_10": _kary(200_000, 10), "tree_2": _kary(60_000, 2),
+         "tree_and_back": np.concatenate([_kary(40_000, 4), [[39_000, 20_000], [38_000, 1], [30_000, 30_000]]]),
+         "in_degrees": np.concatenate([_fan(4200, 40)] + [np.stack([3 + np.arange(d) + 40 * k, np.full(d, 9000 + k)], 1)
+                                                          for k, d in enumerate((1, 7, 8, 9, 31, 32, 33, 64))])}
+
+
+@pytest.mark.parametrize("stop", [0, 4])
+@pytest.mark.parametrize("name", sorted(THIN))
+def test_tc_few_heavy_sources(engine, name, stop):
+    """Rows of one and two chunks, by eight lanes, and of three, by a warp."""
+    e = np.ascontiguousarray(THIN[name]).astype(np.int32)
+    want, got = engine.tc(e, dedup="sort", max_iterations=stop), engine.tc(e, max_iterations=stop)
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    assert np.array_equal(got.rows, want.rows)
