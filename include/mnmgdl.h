@@ -129,7 +129,8 @@ DL_API dl_status dl_context_create(int32_t device, void *stream, dl_context **ou
 DL_API dl_status dl_context_destroy(dl_context *ctx);
 DL_API dl_status dl_context_synchronize(dl_context *ctx);
 /* Waits for the context's stream, then frees the device memory the context keeps between
- * calls: its workspace and cached buffers (e.g. the bit rows or the bit matrix of the last TC run). Results of live runs and sessions are not touched; the next call allocates again.
+ * calls: its workspace and cached buffers (e.g. the bit rows or the bit matrix of the last TC
+ * run). Results of live runs and sessions are not touched; the next call allocates again.
  * No counterpart in the reference (its drivers free everything per iteration). */
 DL_API dl_status dl_context_release_memory(dl_context *ctx);
 DL_API dl_status dl_free(dl_context *ctx, void *device_ptr);
@@ -271,15 +272,16 @@ DL_API dl_status dl_run_destroy(dl_run *run);
  * No counterpart in the reference, whose drivers run one program on one
  * edge file per process (tc.cu:42-423, sg.cu:40-477, wcc.cu:58-585). A
  * session runs every admitted instance of one program (TC, SG or WCC) as one
- * union fixpoint: each iteration's joins, sorts, set difference and merge
- * process all active instances in the same launches. Instances can be
+ * union: what is admitted together is computed in the same launches, whole
+ * fixpoints at once or iteration by iteration (dl_session_step). Instances can be
  * admitted between any two steps (continuous batching) and leave the union
  * at their own fixpoint. Each instance's outputs, iteration count and delta
  * sizes are those of dl_run_program on the same edges and options.
  * A session runs on its context's device and stream and takes the context's
  * cached buffers; dl_session_destroy hands all its memory back to the
  * context, so destroy every session before its context. Calls on one session
- * must not run concurrently. */
+ * must not run concurrently, nor those that create or destroy sessions with any
+ * other call on the same context; different sessions may be read from different threads. */
 typedef struct dl_session dl_session;
 
 /* max_nodes bounds the node count of the instances alive at once
@@ -296,7 +298,11 @@ DL_API dl_status dl_session_admit(dl_session *s, const int32_t *edges, int64_t r
  * instances ranks and sorts them together. */
 DL_API dl_status dl_session_admit_many(dl_session *s, const int32_t *const *edges, const int64_t *rows,
                                        int64_t count, int32_t edges_on_device, int64_t *first_instance);
-/* One iteration of every active instance; *active = instances still running. */
+/* One iteration of every active instance; *active = instances still running. Most instances
+ * are computed to their fixpoints at once -- TC in the first step after their admission,
+ * SG (unless its degrees, its size or the memory leave it to the sorted runs) and WCC in the
+ * admission itself -- so that such a call lasts as long as the largest of them needs, and
+ * their later steps only report: an instance of k iterations finishes with its k-th step. */
 DL_API dl_status dl_session_step(dl_session *s, int64_t *active);
 /* Ids of the instances finished since the last poll, in finishing order;
  * at most `capacity` are returned and the rest stay queued. */

@@ -109,7 +109,8 @@ class Session:
         return list(range(first.value, first.value + count))
 
     def step(self) -> int:
-        """One iteration of every active instance; returns how many are still active."""
+        """One iteration of every active instance; returns how many are still active. Instances
+        computed ahead (see dl_session_step) only report theirs."""
         a = C.c_int64()
         check(lib().dl_session_step(self.handle, C.byref(a)))
         return a.value
@@ -175,9 +176,9 @@ class Session:
         from .engine import _torch
         ids = list(instances)
         res = [self.result(i, output="none") for i in ids]
-        if output not in ("host", "device", "none"):
-            raise DatalogError(1, f"output must be host, device or none, not {output!r}")
         n = len(ids)
+        if n and output not in ("host", "device", "none"):
+            raise DatalogError(1, f"output must be host, device or none, not {output!r}")
         idv = np.asarray(ids, dtype=np.int64)
         if output != "none" and n:
             sizes = np.asarray([r.output_tuples for r in res], dtype=np.int64)

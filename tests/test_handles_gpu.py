@@ -257,3 +257,10 @@ def test_the_workspace_of_other_forms_makes_room_for_the_matrix():
         torch.cuda.empty_cache()
     assert got.join_rows.tolist() == want.join_rows.tolist() and np.array_equal(got.rows, want.rows)
     assert got.nodes == want.nodes
+
+
+def test_an_empty_batch_takes_any_output():
+    with Engine(0) as eng:
+        assert eng.run_batch("tc", [], output="nowhere") == []
+        with pytest.raises(DatalogError):
+            eng.run_batch("tc", [np.array([[1, 2]], np.int32)], output="nowhere")
