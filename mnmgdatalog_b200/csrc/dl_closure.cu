@@ -29,6 +29,7 @@
 // 45.5 -> 12.0 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 3.7 ms
 // (with a warp for every source a millisecond more); DAG of 5.5K edges from and to
 // host memory 3.5 -> 0.53 ms.
+#include <cstring>
 #include <type_traits>
 
 #include "dl_closure.h"
@@ -45,6 +46,7 @@ struct SearchCounters {
     unsigned long long words;   // result words reserved
     unsigned long long left;    // sources left over
     unsigned long long levels;  // largest level of a finished source
+    unsigned long long kept;    // eight-lane searches: first word that did not fit (all ones: all did)
 };
 
 // Where a launch's words go. Finished sources leave theirs in any order;
@@ -250,22 +252,24 @@ __device__ u32 tiny_searches(const uint2 *__restrict__ rec, u32 bb, u32 bd, u64 
     if (!ok) n = levels = 0;
     const u32 incl = warp_inclusive_sum(n);
     const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+    unsigned long long p = 0;
+    if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) total);
+    p = __shfl_sync(0xffffffffu, p, 0);
+    if (p + total > to.cap) {  // no room: to the searches, which leave them over
+        if (lane == 0) atomicMin(&ctr->kept, p);
+        return 0;
+    }
     const u32 two = __popc(__ballot_sync(0xffffffffu, levels >= 2));
     const u32 three = __popc(__ballot_sync(0xffffffffu, levels >= 3));
     const u32 counts[3] = {total - two - three, two, three};
     sums.add_tiny(__popc(all), counts, cnt, deg, stride, lane);
     top = max(top, three ? 3u : two ? 2u : 1u);
-    unsigned long long p = 0;
-    if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) total);
-    p = __shfl_sync(0xffffffffu, p, 0);
     if (ok) {
         const u64 q = p + incl - n;
         to.note(xb + lane, q, n);
-        if (p + total <= to.cap) {
 #pragma unroll
-            for (u32 k = 0; k < TINY_ROW; ++k)
-                if (k < n) to.out[q + k] = ((u64) w[k] << bits) | x;
-        }
+        for (u32 k = 0; k < TINY_ROW; ++k)
+            if (k < n) to.out[q + k] = ((u64) w[k] << bits) | x;
     }
     return all;
 }
@@ -301,27 +305,30 @@ closure_group_kernel(const u32 *__restrict__ off, const uint2 *__restrict__ rec,
             CgSmem &sq = all[q >> 3];
             const bool was = __shfl_sync(0xffffffffu, act, q), ov = __shfl_sync(0xffffffffu, over, q);
             const u32 xq = __shfl_sync(0xffffffffu, x, q), tq = __shfl_sync(0xffffffffu, tail, q);
-            if (was && ov) {
-                if (lane == 0) {
-                    left[atomicAdd(&ctr->left, 1ull)] = lo + xq;
-                    to.note(xq, 0, 0);
-                }
-            } else if (was) {
+            bool fits = was && !ov;
+            unsigned long long p = 0;
+            if (fits) {
+                if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) tq);
+                p = __shfl_sync(0xffffffffu, p, 0);
+                fits = p + tq <= to.cap;
+                if (!fits && lane == 0) atomicMin(&ctr->kept, p);
+            }
+            if (fits) {
                 const u32 lq = __shfl_sync(0xffffffffu, level, q);
                 top = max(top, lq);
                 sums.add(lo + xq, lq, sq.lc, sq.ld, inst_lo, n_inst, cnt, deg, stride, lane);
-                unsigned long long p = 0;
-                if (lane == 0) p = atomicAdd(&ctr->words, (unsigned long long) tq);
-                p = __shfl_sync(0xffffffffu, p, 0);
                 if (lane == 0) to.note(xq, p, tq);
-                if (p + tq <= to.cap)
-                    for (u32 k = lane; k < tq; k += 32) to.out[p + k] = ((u64) sq.qw[k] << bits) | (lo + xq);
+                for (u32 k = lane; k < tq; k += 32) to.out[p + k] = ((u64) sq.qw[k] << bits) | (lo + xq);
+            } else if (was && lane == 0) {
+                left[atomicAdd(&ctr->left, 1ull)] = lo + xq;
+                to.note(xq, 0, 0);
             }
             while (bm == 0 && more) {
-                unsigned long long f = 0;
-                if (lane == 0) f = atomicAdd(&ctr->fetch, (unsigned long long) batch);
+                unsigned long long f = ~0ull;  // (no further sources once the room is full)
+                if (lane == 0 && *reinterpret_cast<volatile unsigned long long *>(&ctr->words) <= to.cap)
+                    f = atomicAdd(&ctr->fetch, (unsigned long long) batch);
                 xb = __shfl_sync(0xffffffffu, f, 0);
-                if (lo + xb >= hi) {
+                if (xb >= hi - lo) {
                     more = false;
                     break;
                 }
@@ -1374,11 +1381,21 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
     DL_CUDA(cudaMemsetAsync(ws.cl_seg.p, 0, ns * 8, ctx.stream));
     DevBuf &out = ws.jbuf[0];
     // room for 96 targets a source at first, up to a GiB (nothing is known of the result
-    // yet); a launch that needs more is repeated with the room it asked for
+    // yet); eight-lane searches go on with more where it was full, the others are repeated
     ctx.reserve(out, std::min<u64>(std::max<u64>(96 * ns, 1 << 16), 1ull << 27) * 8);
     SearchCounters got{};
-    // One stage: `launch(where to)` with zeroed counters; repeated when its words outgrow the room.
-    // Its level counts are added to cnt / deg when it went through.
+    // What a launch found: its words are kept, its level counts are added to cnt / deg.
+    auto account = [&] {
+        ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
+        res.n_words += got.words;
+        res.levels = (u32) std::max<u64>(res.levels, got.levels);
+        if (!got.words) return;
+        const unsigned ag = grid_for(table / 8, T256, ctx);
+        DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, table / 8));
+        if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, table / 8));
+    };
+    // One stage of warp or CTA searches: `launch(where to)` with zeroed counters; repeated when
+    // its words outgrow the room.
     auto stage = [&](auto launch) {
         for (;;) {
             DL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(got), ctx.stream));
@@ -1387,20 +1404,11 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
             launch(SearchOut{out.as<u64>() + res.n_words, room, res.n_words, ws.cl_seg.as<u64>()});
             DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctr, sizeof(got), cudaMemcpyDeviceToHost, ctx.stream));
             ctx.sync();
-            got.words = ctx.host_scalars[1];
-            got.left = ctx.host_scalars[2];
-            got.levels = ctx.host_scalars[3];
+            std::memcpy(&got, ctx.host_scalars, sizeof(got));
             if (got.words <= room) break;
             grow_keeping(ctx, out, (res.n_words + got.words) * 8, res.n_words * 8);
         }
-        ctx.prof_add_bytes(K_BITMAP_EXPAND, 8.0 * got.words);
-        res.n_words += got.words;
-        res.levels = (u32) std::max<u64>(res.levels, got.levels);
-        if (got.words) {
-            const unsigned ag = grid_for(table / 8, T256, ctx);
-            DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(cnt, c2, table / 8));
-            if (deg) DL_LAUNCH(ctx, K_PREP, 0, add_counts_kernel<<<ag, T256, 0, ctx.stream>>>(deg, d2, table / 8));
-        }
+        account();
     };
     // Few sources go to the warps at once: one launch and one wait instead of two
     // (3.6K sources of a 5.5K-edge DAG: 0.78 -> 0.67 ms for the whole run).
@@ -1423,14 +1431,33 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
         const u32 batch = (u32) std::max<u64>(4, std::min<u64>(32, ns / (warps_g * 4)));
         const unsigned grid_g = (unsigned) std::max<u64>(
             1, std::min<u64>(wave_g, (ns + batch * (CG_THREADS / 32) - 1) / (batch * (CG_THREADS / 32))));
-        stage([&](SearchOut to) {
-            DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * ns,
+        // A launch whose room is full takes no further sources; the next one goes on from there.
+        // The searches under way then (a few ten thousand) are left over, as those that
+        // outgrew their slice.
+        for (u64 begun = 0;;) {
+            SearchCounters *at = reinterpret_cast<SearchCounters *>(ctx.host_scalars + 8);
+            *at = SearchCounters{begun, 0, got.left, 0, ~0ull};
+            DL_CUDA(cudaMemcpyAsync(ctr, at, sizeof(got), cudaMemcpyHostToDevice, ctx.stream));
+            DL_CUDA(cudaMemsetAsync(c2, 0, 2 * table, ctx.stream));
+            const SearchOut to{out.as<u64>() + res.n_words, out.cap / 8 - res.n_words, res.n_words, ws.cl_seg.as<u64>()};
+            DL_LAUNCH(ctx, K_BITMAP_EXPAND, 8.0 * (ns - begun),
                       closure_group_kernel<<<grid_g, CG_THREADS, smem_g, ctx.stream>>>(
                           csr.off, ws.cl_rec.as<uint2>(), (u32) k0, lo, hi, batch, bits, inst_lo, (u32) n_inst,
                           (u32) stride, ml, c2, deg ? d2 : nullptr, to, ctr, ws.cl_left.as<u64>()));
-        });
-        if (got.left == 0) return res;
+            DL_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctr, sizeof(got), cudaMemcpyDeviceToHost, ctx.stream));
+            ctx.sync();
+            std::memcpy(&got, ctx.host_scalars, sizeof(got));
+            got.words = std::min(got.words, got.kept);
+            account();
+            if (got.fetch >= ns) break;
+            begun = got.fetch;
+            // the others find as much, or the 96 targets a source that the first room was short of
+            const u64 rest = ns - begun;
+            const u64 more = (u64) (1.25 * (double) res.n_words / (double) begun * (double) rest);
+            grow_keeping(ctx, out, (res.n_words + std::max(more, 96 * rest)) * 8, res.n_words * 8);
+        }
         nl = got.left;
+        if (nl == 0) return res;
     }
     ctx.reserve(ws.cl_heavy, nl * 8);
     grow_keeping(ctx, out, (res.n_words + std::min<u64>(nl * 512, 1ull << 27)) * 8, res.n_words * 8);

@@ -255,3 +255,21 @@ def test_tc_few_heavy_sources(engine, name, stop):
     for f in ("deltas", "join_rows", "full_rows"):
         assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
     assert np.array_equal(got.rows, want.rows)
+
+
+def test_tc_searches_go_on_with_more_room(engine):
+    """More than 2^27 words of eight-lane searches, the most that is reserved at first: sources from where
+    the room was full, and those under way then, as a run and in a batch."""
+    import torch
+    e = graphs.sized("tc", 3_200_000)
+    sets = [e, _tiny(3, 30_000), graphs.sized("tc", 200_000, seed=1)]
+    want = [engine.tc(x, dedup="sort", output="device") for x in sets]
+    assert want[0].output_tuples > 2**27
+    engine.release_memory()  # (a cached buffer may be larger than what is asked for)
+    got = engine.tc(e, output="device")
+    assert torch.equal(got.rows, want[0].rows)
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want[0], f).tolist(), f
+    del got
+    for w, b in zip(want, engine.run_batch("tc", sets, output="device")):
+        assert b.deltas.tolist() == w.deltas.tolist() and torch.equal(b.rows, w.rows)
