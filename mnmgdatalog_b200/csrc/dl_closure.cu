@@ -1411,7 +1411,8 @@ ClosureLight closure_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bi
         account();
     };
     // Few sources go to the warps at once: one launch and one wait instead of two
-    // (3.6K sources of a 5.5K-edge DAG: 0.78 -> 0.67 ms for the whole run).
+    // (3.6K sources of a 5.5K-edge DAG: 0.78 -> 0.67 ms for the whole run; the line above it, at
+    // CL_FEW, was not timed on both sides).
     const bool groups = ns > CL_FEW && k1 - k0 < CG_MAX_EDGES;
     u64 nl = ns;
     if (groups) {
