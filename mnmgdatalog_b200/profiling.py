@@ -25,16 +25,18 @@ CLASSES = [
     (r"radix_upsweep_kernel|radix_hist_kernel", "sort_histogram"),
     (r"scan_kernel<.*WordValue", "sort_spine_scan"),
     (r"radix_bucket_kernel", "sort_spine_scan"),
-    (r"scan_kernel<.*DegreeOp", "join_count_scan"),
-    (r"wcc_(first|level|close|final)_kernel", "wcc_propagate"),
+    (r"scan_kernel<.*(DegreeOp|SegmentWords)|degree_total_kernel", "join_count_scan"),
+    (r"wcc_(first|level|close)_kernel", "wcc_propagate"),
     (r"join_emit_kernel|join_emit_bucket_kernel", "join_emit"),
     (r"digit0_hist_kernel", "join_count_scan"),
     (r"bucket_starts_kernel", "join_partition"),
-    (r"bitmat_unit_step_kernel|bitmat_set_edges_kernel|closure_(group|warp|cta|pull|pull_hub|push)_kernel|self_join_kernel|pair_level_kernel|pair_refill_kernel|sg_rows_kernel", "bitmap_expand"),
-    (r"bitmat_transpose_count|bitmat_column_count|column_offsets|closure_counts|heavy_below", "bitmap_columns"),
-    (r"bitmat_extract|bitmat_column_rows|closure_rows|scan_kernel<.*(CountValue|SumValue)", "bitmap_extract"),
+    (r"bitmat_unit_step_kernel|bitmat_set_edges_kernel|sg_unit_step_kernel|closure_(group|warp|cta|pull|pull_thin|pull_hub|push)_kernel"
+     r"|self_join_kernel|pair_(level|joins|refill)_kernel|sg_rows_kernel", "bitmap_expand"),
+    (r"bitmat_transpose_count|bitmat_column_count|column_offsets|closure_counts|heavy_below|key_offsets_kernel<(u64|unsigned long)", "bitmap_columns"),
+    (r"bitmat_extract|bitmat_column_rows|bitmat_row_popc|closure_(rows|merge)_kernel|heavy_words_kernel|scan_kernel<.*(CountValue|SumValue)",
+     "bitmap_extract"),
     (r"lbs_partition_kernel", "join_partition"),
-    (r"select_kernel", "select_compact"),
+    (r"select_kernel|segments_kernel", "select_compact"),
     (r"merge_partition_kernel", "merge_partition"),
     (r"merge_kernel", "merge"),
     (r"sparse_mark_kernel|sample_kernel", "sparse_diff"),

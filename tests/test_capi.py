@@ -92,6 +92,34 @@ def test_profile_classes_match_the_ncu_summary_classes():
     assert not lib_classes - ncu_classes, sorted(lib_classes - ncu_classes)
 
 
+def test_ncu_summary_attributes_every_kernel_as_its_launch_does():
+    """A kernel that a launch counts under a class of the live profile is attributed to
+    the same class by its name in the launch-list summary."""
+    import glob
+    import re
+
+    from mnmgdatalog_b200 import profiling
+    csrc = os.path.join(ROOT, "mnmgdatalog_b200", "csrc")
+    ids = re.search(r"enum KernelId[^{]*\{(.*?)\};", open(os.path.join(csrc, "dl_internal.h")).read(), re.S).group(1)
+    ids = [k for k in re.findall(r"\bK_[A-Z_0-9]+", re.sub(r"//.*", "", ids)) if k != "K_COUNT"]
+    block = open(os.path.join(csrc, "dl_context.cu")).read()
+    block = block[block.index("static const char *names[K_COUNT]"):]
+    class_of = dict(zip(ids, re.findall(r'"([a-z_A-Z]+)"', block[:block.index("};")])))
+    # kernels picked at run time (`auto kern = ...`) are named where they are picked
+    named = {"radix_downsweep_kernel": "K_SORT_PASS", "sg_rows_kernel": "K_BITMAP_EXPAND",
+             "closure_pull_kernel": "K_BITMAP_EXPAND", "closure_pull_thin_kernel": "K_BITMAP_EXPAND",
+             "closure_rows_kernel": "K_BITMAP_EXTRACT", "segments_kernel": "K_SELECT"}
+    launches = [(n, k) for n, k in named.items()]
+    for path in glob.glob(os.path.join(csrc, "*.cu*")):
+        for k, head in re.findall(r"DL_LAUNCH\(\s*ctx,\s*(K_\w+),(.*?)<<<", open(path).read(), re.S):
+            m = re.search(r"(\w+_kernel\b(<.*>)?)\s*$", head, re.S)
+            if m:
+                launches.append((m.group(1), k))
+    assert len(launches) > 80
+    wrong = [(n, class_of[k], profiling.kernel_class(n)) for n, k in launches if profiling.kernel_class(n) != class_of[k]]
+    assert not wrong, wrong
+
+
 @pytest.mark.parametrize("lang,std", [("c", "-std=c99"), ("c++", "-std=c++17")])
 def test_public_header_compiles_as_plain_c_and_cpp(tmp_path, lang, std):
     """include/mnmgdl.h is usable from C (cgo, FFI generators) and C++ alike:
