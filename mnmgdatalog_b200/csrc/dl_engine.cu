@@ -771,6 +771,7 @@ static bool sg_pairs_fixpoint(Context &ctx, Run &r, const Graph &g, const PairDe
     // join sizes the ones to report
     po.handover = bitmat_allowed(ctx, g.n_ids, true);
     po.joins = !po.handover;
+    po.deg = deg;
     if (po.joins && pair_search_outrun(deg, {g.n_ids})) return false;
     try {
         const PairSearch ps = pair_search(ctx, g.csr, 0, g.n_ids, g.bits, po);

@@ -38,6 +38,7 @@ struct PairOptions {
     bool handover = false; // stop where a matrix is the faster form (see dl_pairs.cu)
     u64 limit = ~0ull;     // bytes of the list and the set
     bool joins = false;    // count the rows of the joins in two steps, as the sorted runs do
+    PairDegrees deg;       // of the ranks, for `handover` and `joins`
 };
 // The search from the base rule of ranks [lo, hi) of the CSR; words (x << bits) | y
 // in ws.jbuf[0], unsorted. It is not complete, and its last level may lack words, where

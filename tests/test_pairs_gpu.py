@@ -164,7 +164,7 @@ def _full_stats(got, want):
 
 
 @pytest.mark.parametrize("stop", [0, 1, 3])
-@pytest.mark.parametrize("name", ["lattice", "wide_ids", "random", "forest", "wide_tree", "loops"])
+@pytest.mark.parametrize("name", ["lattice", "wide_ids", "random", "forest", "wide_tree", "loops", "most_64"])
 def test_sg_past_the_matrix_reports_the_sorted_runs_joins(name, stop):
     """Graphs whose bit matrix passes bitmap_max_gib: rows and join sizes are those of the sorted
     runs, by the search (which counts them) or by the runs."""
@@ -175,6 +175,8 @@ def test_sg_past_the_matrix_reports_the_sorted_runs_joins(name, stop):
          "wide_ids": lambda: graphs.lattice3d(side=50, p=0.15, seed=4) * 17_001 - 2 * 10**9,
          "random": lambda: rng.integers(0, n, (100_000, 2)),
          "forest": lambda: np.concatenate([np.asarray(_tree(13, 3)) + 40 * k for k in range(3300)]),
+         # (twice 64 words a pair: more than the set has slots for the large levels, not for the last ones)
+         "most_64": lambda: np.concatenate([graphs.lattice3d(side=50, p=0.17, seed=6), np.asarray(_hubs(64)) + n]),
          "wide_tree": lambda: np.stack([np.arange(n) // 10, np.arange(n) + 1], 1),
          "loops": lambda: np.concatenate([np.stack([np.arange(n), np.arange(n)], 1),
                                           np.stack([np.arange(n - 1), np.arange(1, n)], 1)])}[name]()
