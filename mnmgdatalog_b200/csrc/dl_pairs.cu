@@ -337,6 +337,21 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
     // iterations, 7 pairs a node, 1.9 ms on the matrix, 0.65 on the list; a mesh of 264K nodes, 17 a
     // node in 67 levels, 20 against 3.1; random graphs past the line lose 1 to 5 % to it.
     const u64 n = hi - lo, many = std::max<u64>(16 * n, PS_SLOTS / 2);
+    // Whether the levels left under max_levels end with at most 128 pairs a node, if each is as many
+    // times the one before as the last whole one is (the first: as random nodes' or siblings' children):
+    // then the list is the faster form to the end. Measured, handed over or not (on the matrix
+    // alone): 220K layered nodes, two iterations, 64 a node, 16.9 / 3.5 (12.1) ms; random graph of 260K
+    // nodes and 300K edges, ten, 83 a node, 48 / 6.2 (21.7); tree of 250K nodes with five children each,
+    // two, 124 a node, 18.4 / 7.9 (7.1); mesh of 60K nodes, ten, 121 a node, 4.2 / 4.4 (3.9).
+    auto ends_soon = [&](u64 next) {
+        if (!opt.max_levels || next == 0 || opt.max_levels - next > 16) return false;
+        const double mean = (double) opt.deg.edges / (double) n;
+        double all = (double) ps.bound[next], last = all - (double) ps.bound[next - 1];
+        const double by = next < 2 ? std::max(mean * mean, opt.deg.of_sources())
+                                   : last / (double) std::max<u64>(ps.bound[next - 1] - ps.bound[next - 2], 1);
+        for (u64 k = next; k <= opt.max_levels; ++k) all += last *= by;
+        return all <= 128.0 * (double) n;
+    };
     const std::initializer_list<DevBuf *> idle = {&ws.bitmat[0], &ws.bitmat[1], &ws.cl_rows[0], &ws.cl_rows[1]};
     const u64 unit = opt.joins ? 20 : 12;  // bytes a slot: the set, half as many words, the joins' set
     if (slots * unit > opt.limit || !ctx.room_for({{&list, slots / 2 * 8}, {&set, slots * 8}}, idle)) return ps;
@@ -453,7 +468,7 @@ PairSearch pair_search(Context &ctx, const Csr &csr, u64 lo, u64 hi, int bits, c
         }
         if (opt.handover) {
             const u64 all = full ? found : ps.n_words(), last = all - (level ? ps.bound[full ? level : level - 1] : 0);
-            if (all > 512 * n + many || (all >= many && last > n)) break;
+            if (all > 512 * n + many || (all >= many && last > n && !ends_soon(level))) break;
         }
         if (full) {  // repeat level `level` with more room: the set again from the words listed before it
             const u64 keep = ps.bound[level];

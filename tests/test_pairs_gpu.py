@@ -191,6 +191,26 @@ def test_sg_past_the_matrix_reports_the_sorted_runs_joins(name, stop):
         _full_stats(eng.sg(e, max_iterations=stop), eng.sg(e, dedup="sort", max_iterations=stop))
 
 
+@pytest.mark.parametrize("children,nodes,stop,listed", [(3, 60_000, 3, True), (3, 60_000, 4, False), (2, 90_000, 5, True),
+                                                        (2, 90_000, 6, True), (2, 90_000, 7, False), (6, 50_000, 1, True),
+                                                        (11, 50_000, 1, True), (13, 50_000, 1, False)])
+def test_sg_with_few_iterations_left(children, nodes, stop, listed):
+    """Levels of more than a pair a node: the list goes on to the last iteration when that ends with
+    128 pairs a node at most, and is handed over when not; rows and sizes are the matrix's."""
+    from mnmgdatalog_b200 import Engine
+    c = np.arange(1, nodes)
+    e = np.stack([(c - 1) // children, c], 1).astype(np.int32)
+    with Engine(0) as eng:
+        want = eng.sg(e, dedup="bitmap", max_iterations=stop)
+        eng.profile(False)
+        got = eng.sg(e, max_iterations=stop)
+        by_rows = eng.profile_read()["bitmap_extract"]["launches"]
+    assert (by_rows == 0) == listed
+    for f in ("deltas", "join_rows", "full_rows"):
+        assert getattr(got, f).tolist() == getattr(want, f).tolist(), f
+    assert np.array_equal(got.rows, want.rows)
+
+
 def _random_above(n, m, seed):
     return np.concatenate([np.random.default_rng(seed).integers(0, n, (m, 2)), [[0, n - 1]]]).astype(np.int32)
 
