@@ -72,12 +72,13 @@ bool sg_rows(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, con
 // before dedup. False (nothing done) when the bit rows are not worth it or do
 // not fit; the join and the sort of its output are the better form then.
 bool self_join_rows(Context &ctx, Run &r, const Csr &in, u64 total, PhaseTimer &pt, u64 &rows);
-// The edges by source, from the np words of the edges by target: those come in the order
-// of the other field already, so half the passes do, and no duplicates are left to drop
-// (1M rows of ids that are ranked by a sort, 1.44 -> 1.28 ms for the whole run; packing
-// and sorting the rows a second time had made it slower than the two sorts of the rows
-// side by side, 1.29).
-u64 *self_join_by_source(Context &ctx, const u64 *p, u64 np, int bits);
+// Edge words by one field, ascending, as words by the other, in a or b. Those of equal second field
+// come in the order of the first already, so half the passes do, and no duplicates are left to
+// drop (single_join of 1M rows of ids that are ranked by a sort, 1.44 -> 1.28 ms for the whole run;
+// packing and sorting the rows a second time had made it slower than the two sorts of
+// the rows side by side, 1.29; TC of a tree of 4M nodes, three children each, 13.4 -> 12.3
+// with it and the row writer's shorter walk).
+u64 *edges_by_other(Context &ctx, const u64 *edges, u64 ne, int bits, DevBuf &a, DevBuf &b);
 // Sum over the edges y -> z of y's in-degree: the join rows of the self-join.
 u64 self_join_total(Context &ctx, const Csr &in);
 

@@ -1012,7 +1012,7 @@ static void run_single_join_impl(Context &ctx, Run &r, const int32_t *rows_in, u
         if (self_join_rows(ctx, r, g.csr, total, pt, nout)) {
             ctx.run_join_total = ctx.run_join_max = total;
         } else {
-            build_csr(ctx, self_join_by_source(ctx, p, np, g.bits), np, g);  // single_join.cu:165-168
+            build_csr(ctx, edges_by_other(ctx, p, np, g.bits, ws.w0, ws.w1), np, g);  // single_join.cu:165-168
             u64 nj = 0;
             u64 *j = join_and_sort(ctx, g, p, np, EmitKind::ZV, nj, nullptr, pt);  // single_join.cu:223
             nout = nj ? unique_words(ctx, j, nj, j) : 0;                           // single_join.cu:259-264

@@ -153,15 +153,14 @@ self_join_kernel(const u32 *__restrict__ off, const u32 *__restrict__ val, u64 n
 
 }  // namespace
 
-u64 *self_join_by_source(Context &ctx, const u64 *p, u64 np, int bits) {
-    Workspace &ws = ctx.ws;
-    ctx.reserve(ws.w0, np * 8);
-    ctx.reserve(ws.w1, np * 8);
-    DL_LAUNCH(ctx, K_PREP, 16.0 * np,
-              pull_swap_kernel<<<grid_for(np, T256, ctx), T256, 0, ctx.stream>>>(p, np, bits, ws.w0.as<u64>()));
+u64 *edges_by_other(Context &ctx, const u64 *edges, u64 ne, int bits, DevBuf &a, DevBuf &b) {
+    ctx.reserve(a, ne * 8);
+    ctx.reserve(b, ne * 8);
+    DL_LAUNCH(ctx, K_PREP, 16.0 * ne,
+              pull_swap_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(edges, ne, bits, a.as<u64>()));
     int w[8], nw = 0;
-    for (int b = 0; b < bits; b += 8) w[nw++] = bits + b;
-    return radix_sort_windows(ctx, ws.w0.as<u64>(), ws.w1.as<u64>(), np, w, nw);
+    for (int k = 0; k < bits; k += 8) w[nw++] = bits + k;
+    return radix_sort_windows(ctx, a.as<u64>(), b.as<u64>(), ne, w, nw);
 }
 
 u64 self_join_total(Context &ctx, const Csr &in) {

@@ -377,13 +377,7 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     pt.mark(PH_INIT);
     PullShape sh{n, (u32) words, 0};
     while ((32u << sh.shift) < words / 32) ++sh.shift;
-    // in-neighbours: the edges sorted by target
-    ctx.reserve(ws.full[0], ne * 8);
-    ctx.reserve(ws.full[1], ne * 8);
-    DL_LAUNCH(ctx, K_PREP, 16.0 * ne,
-              pull_swap_kernel<<<grid_for(ne, T256, ctx), T256, 0, ctx.stream>>>(edges, ne, g.bits,
-                                                                                ws.full[0].as<u64>()));
-    const u64 *rev = radix_sort(ctx, ws.full[0].as<u64>(), ws.full[1].as<u64>(), ne, Codec::Raw, 2 * g.bits);
+    const u64 *rev = edges_by_other(ctx, edges, ne, g.bits, ws.full[0], ws.full[1]);  // in-neighbours
     ctx.reserve(ws.cl_roff, (n + 1) * 4);
     ctx.reserve(ws.cl_rval, ne * 4);
     u32 *roff = ws.cl_roff.as<u32>(), *rval = ws.cl_rval.as<u32>();
