@@ -1197,13 +1197,19 @@ closure_rows_kernel(const u32 *__restrict__ t, u32 words, const u32 *__restrict_
             u32 slow = any & inside;
             const u32 v0 = v;
             if ((inside >> lane) & 1u) v = 0;
+            if constexpr (DENSE) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const u32 word = __shfl_sync(0xffffffffu, v, j);
-                const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
-                if constexpr (DENSE) {
+                for (int j = 0; j < 32; ++j) {
+                    const u32 word = __shfl_sync(0xffffffffu, v, j);
+                    const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
                     if ((word >> lane) & 1u) dst[p] = pack(id[j]);
-                } else {
+                }
+            } else {
+                // (of a tree's 32 words three hold bits: 1M targets 0.78 -> 0.48 ms)
+                for (u32 nz = any & ~inside; nz; nz &= nz - 1) {
+                    const u32 j = __ffs(nz) - 1;
+                    const u32 word = __shfl_sync(0xffffffffu, v, j);
+                    const u32 p = __shfl_sync(0xffffffffu, at, j) + __popc(word & lt);
                     if ((word >> lane) & 1u) dst[p] = pack(node(__ldg(cc + j * 32 + lane)));
                 }
             }
