@@ -1444,9 +1444,7 @@ u64 sg_bitmap_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_options &o
     if (nfull) {
         ctx.reserve(ws.offsets, (n + 1) * 8);
         u64 *counts = ws.offsets.as<u64>();
-        DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * n * words_used,
-                  bitmat_row_popc_kernel<<<grid_for(n * 32, T256, ctx, 8), T256, 0, ctx.stream>>>(
-                      m, n, stride, words_used, reinterpret_cast<unsigned long long *>(counts)));
+        bitmat_row_counts(ctx, m, n, stride, words_used, counts);
         ctx.reserve(ws.w0, (n + 1) * 8);
         const u64 total = exclusive_scan(ctx, counts, n, ws.w0.as<u64>());
         if (total != nfull)
@@ -1463,6 +1461,12 @@ u64 sg_bitmap_fixpoint(Context &ctx, Run &r, const Graph &g, const dl_options &o
     }
     r.from_bitmat = true;
     return nfull;
+}
+
+void bitmat_row_counts(Context &ctx, const u32 *m, u64 n, u64 stride, u64 words, u64 *counts) {
+    DL_LAUNCH(ctx, K_BITMAP_EXTRACT, 4.0 * n * words,
+              bitmat_row_popc_kernel<<<grid_for(n * 32, T256, ctx, 8), T256, 0, ctx.stream>>>(
+                  m, n, stride, words, reinterpret_cast<unsigned long long *>(counts)));
 }
 
 }  // namespace detail

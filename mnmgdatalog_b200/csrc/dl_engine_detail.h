@@ -117,6 +117,8 @@ bool bitmat_choose(Context &ctx, const dl_options &opt, u64 n, bool sg);
 bool bitmat_allowed(const Context &ctx, u64 n, bool sg);
 u64 tc_bitmap_fixpoint(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne, const dl_options &opt,
                        PhaseTimer &pt);
+// counts[x] = set bits of row x of a bit matrix.
+void bitmat_row_counts(Context &ctx, const u32 *m, u64 n, u64 stride, u64 words, u64 *counts);
 // SG with full as a bit matrix; throws DL_ERR_OVERFLOW when a step's new rows
 // outgrow the buffer the device memory allows (the caller then reruns SG on
 // the sorted runs).

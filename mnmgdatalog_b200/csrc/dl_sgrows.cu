@@ -322,6 +322,12 @@ sg_rows_kernel(PullShape sh, PullLevel st, const u32 *__restrict__ off, const u3
     }
 }
 
+// Results of fewer bits than one in this many leave by the matrix's kernels (dl_bitmap.cu), which read
+// whole rows; closure_rows_kernel takes a line at a time, whose first row it knows, and gains
+// where the lines are full. Whole runs, by lines and by rows: 220K layered nodes, three iterations, one
+// bit in 980, 18.5 / 13.0 ms; meshes of 22K nodes, one in 55 / 5.8 / 1.8, 1.37 / 1.34, 3.18 / 3.50 and
+// 13.2 / 14.2; random 40K nodes, one in 119 / 31 / 9, 2.41 / 2.16, 3.17 / 3.05 and 4.52 / 4.99.
+constexpr u64 SG_SPARSE = 32;
 constexpr u64 SG_LEVELS = 8;  // levels launched between two host waits
 
 // Targets with many in-neighbours (pull_hubs_kernel).
@@ -487,11 +493,14 @@ bool sg_rows_run(Context &ctx, Run &r, const Graph &g, const u64 *edges, u64 ne,
     pt.mark(PH_FINAL);
     if (nfull) {
         ctx.reserve(ws.offsets, (n + 1) * 8);
-        bit_rows_count(ctx, r, n, words, 0, g.bits, nullptr, ws.offsets.as<u64>());
+        const bool sparse = nfull < n * words * 32 / SG_SPARSE;
+        if (sparse) bitmat_row_counts(ctx, r.bm_t.as<u32>(), n, words, words, ws.offsets.as<u64>());
+        else bit_rows_count(ctx, r, n, words, 0, g.bits, nullptr, ws.offsets.as<u64>());
         const u64 total = bit_rows_finish(ctx, r, n, words, ws.offsets.as<u64>());
         if (total != nfull)
             throw Error(DL_ERR_INTERNAL, "bit rows hold " + std::to_string(total) + " tuples, expected " +
                                              std::to_string(nfull));
+        r.cl_rows = !sparse;
         r.bm_row_first = true;
     }
     r.from_bitmat = true;

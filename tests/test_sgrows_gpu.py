@@ -43,6 +43,15 @@ def test_sg_rows_equal_matrix(engine, name, edges, stop):
         assert np.array_equal(engine.sg(e, max_iterations=stop).rows, want.rows.cpu().numpy())
 
 
+@pytest.mark.parametrize("name,edges,stop", [
+    ("one_in_60", graphs.lattice3d(side=14, p=0.3, seed=5), 5), ("one_in_19", graphs.lattice3d(side=14, p=0.3, seed=5), 10),
+    ("one_in_119", _random(40_000, 80_000, 5), 3), ("one_in_31", _random(40_000, 80_000, 5), 4),
+    ("ids_of_a_sort", _random(3000, 4500, 4) * 700_001 - 2**31, 3), ("eight_warps_sparse", _random(135_000, 290_000, 3), 3)])
+def test_sg_rows_sparse_and_dense_results(engine, name, edges, stop):
+    """Results on both sides of the density (a bit in 32) at which their writer changes."""
+    test_sg_rows_equal_matrix(engine, name, edges, stop)
+
+
 def _into_hubs(n, m, hubs, seed):
     """A random graph, a third of whose edges go into `hubs` nodes."""
     rng = np.random.default_rng(seed)
