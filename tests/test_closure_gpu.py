@@ -83,6 +83,22 @@ def test_tc_searches_equal_sorted_runs(engine, name):
         assert np.array_equal(host.rows, want.rows.cpu().numpy())
 
 
+def _two_fans(heads, every):
+    """`heads` sources of 4,200 targets each, or 2,000 for one in `every`: past a CTA's search, and within it."""
+    x, root, small = np.arange(heads), heads, heads + 1
+    t = heads + 2 + np.arange(4200)
+    return np.concatenate([np.stack([x, np.where(x % every, root, small)], 1), np.stack([np.full(4200, root), t], 1),
+                           np.stack([np.full(2000, small), t[:2000]], 1)])
+
+
+# sources left over by most CTA searches (the later ones are then not begun), by half of them, by few
+@pytest.mark.parametrize("heads,every", [(3000, 3000), (3000, 3), (3000, 2), (511, 8), (2400, 1)])
+def test_tc_sources_that_cta_searches_leave_over(engine, heads, every, monkeypatch):
+    name = f"two_fans_{heads}_{every}"
+    monkeypatch.setitem(CASES, name, (_two_fans(heads, every), 0))
+    test_tc_searches_equal_sorted_runs(engine, name)
+
+
 def _chain(n):
     """0 -> 1 -> n leaves."""
     return np.concatenate([[[0, 1]], np.stack([np.full(n, 1), 2 + np.arange(n)], 1)])
