@@ -26,7 +26,7 @@
 // Measured on B200 against the n x n bit matrix stepped by one launch per
 // iteration (dl_bitmap.cu), edges and result rows on the device: Chung-Lu graph
 // of 317K nodes (1.88e9 pairs; 9.3K heavy sources hold 99 % of them)
-// 45.5 -> 12.0 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 3.7 ms
+// 45.5 -> 11.5 ms; DAG of 500K edges (2.5e7 pairs, 175 iterations) 89 -> 3.6 ms
 // (with a warp for every source a millisecond more); DAG of 5.5K edges from and to
 // host memory 3.5 -> 0.53 ms.
 #include <cstring>
@@ -623,7 +623,7 @@ constexpr u32 CC_EDGES = 1u << 18;
 // too, unsearched: the bit rows take them at less than a failed search costs. A prime step
 // through the sources makes the first ones a sample of all. Random graph of 20K nodes and 30K
 // edges 3.76 -> 2.50 ms, of 24K 3.53 -> 2.75.
-constexpr u64 CC_SPREAD = 2654435761ull;  // (above every number of sources)
+constexpr u64 CC_SPREAD = 2654435761ull;  // prime, and far more than the sources that come here
 constexpr u64 CC_TRIED = 512;
 
 struct CcSmem {
